@@ -232,23 +232,25 @@ struct spect_plan_s {
   size_t izN = 0;              // floats of one IZ volume (L * L * nzp)
   float* d_imgIZ = nullptr;    // forward input / OS-EM iterate (IZ)
   float* d_backIZ = nullptr;   // back-projection accumulator (IZ)
-  float* d_Hz = nullptr;       // [nset][ny][2 hs] pass weights
-  float* d_Ez = nullptr;       // [nset][ny][2 ts] forward tails, adjoint folds
-  int* d_Rz = nullptr;         // [nset][ny][8] tap-block ranges of the four passes
+  float* d_Hz = nullptr;       // [nset][ny][hs] forward pass weights
+  float* d_Ez = nullptr;       // [nset][ny][ts] forward tails
+  int* d_Rz = nullptr;         // [nset][ny][4] tap-block ranges of the forward passes
+  float* d_Zt = nullptr;       // [nset][ny][ztable_floats] adjoint pass tables
+  ZTile zat{};                 // tiling of k_zadj
   double ztaps[2] = {0, 0};    // mean kept taps per plane of the fused passes (z, x)
-  int zshape_fwd = -1, zshape_adj = -1;
+  int zshape_fwd = -1;
   // large-plane kernels (zpath == 2): task width, column / row tiles, shared
-  // memory and resident blocks per SM of k_zs_fz, k_zs_fx, k_zs_adj, and the
-  // forward's plane-tile exchange buffer
-  int zs_w = 8, zs_tx = 8, zs_tz = 4, zs_fz_nth = kZsNth / 2, zs_adj_nth = kZsNth, zs_adj_tx = 8;
-  size_t zs_smem[3] = {0, 0, 0};
-  int zs_occ[3] = {1, 1, 1};
+  // memory and resident blocks per SM of k_zs_fz, k_zs_fx, and the forward's
+  // plane-tile exchange buffer
+  int zs_w = 8, zs_tx = 8, zs_tz = 4, zs_fz_nth = kZsNth / 2;
+  size_t zs_smem[2] = {0, 0};
+  int zs_occ[2] = {1, 1};
   float* d_Q = nullptr;
   // split kernels with the gather rotation adjoint: the premultiplied adjoint
   // planes are transposed into d_Tz (z fastest) and gathered into d_backIZ
   int gadj = 0;
   float* d_Tz = nullptr;
-  size_t zfwd_smem_b = 0, zadj_smem_b = 0;
+  size_t zfwd_smem_b = 0;
   size_t bytes = 0;
   // stream on which the plan is built and its buffers are (de)allocated;
   // async_alloc: cudaMallocAsync/cudaFreeAsync on it (no device-wide sync)
@@ -278,7 +280,7 @@ void free_plan(spect_plan_s* p) {
   void* ptrs[] = {p->d_mumap, p->d_att, p->d_err, p->d_r1view, p->d_R1, p->d_gscr_r1, p->d_H,     p->d_rot,      p->d_viewset,   p->d_tw,         p->d_all,
                   p->d_idx,   p->d_P,     p->d_part,     p->d_Vs,      p->d_imgpart,    p->d_gB,
                   p->d_gacc,  p->d_gscr_adj, p->d_views_tmp, p->d_ones, p->d_asum,       p->d_flag, p->d_sub,
-                  p->d_io_img, p->d_io_views, p->d_Hsep, p->d_Tsep, p->d_imgIZ, p->d_backIZ, p->d_Hz, p->d_Ez, p->d_Tz, p->d_Rz, p->d_Q};
+                  p->d_io_img, p->d_io_views, p->d_Hsep, p->d_Tsep, p->d_imgIZ, p->d_backIZ, p->d_Hz, p->d_Ez, p->d_Tz, p->d_Rz, p->d_Zt, p->d_Q};
   for (void* q : ptrs)
     if (q) {
       if (p->async_alloc) cudaFreeAsync(q, p->home);
@@ -553,6 +555,8 @@ ZArgs zargs(const spect_plan_s* p) {
   a.H = p->d_Hz;
   a.E = p->d_Ez;
   a.R = p->d_Rz;
+  a.tab = p->d_Zt;
+  a.t = p->zat;
   a.rot = p->d_rot;
   a.viewset = p->d_viewset;
   a.err = p->d_err;
@@ -561,16 +565,6 @@ ZArgs zargs(const spect_plan_s* p) {
 
 // zpath forward of nidx views of the IZ image: k_zfwd (rotation, attenuation,
 // convolution, depth sum of chunks) then the chunk sum (+ EM ratio y/(Ax+bg))
-// depth chunks of the large-plane adjoint over nv views and `tiles` column
-// tiles: about four work items per SM (a short last wave), at most
-// nchunk_max chunks
-void zs_chunking(const spect_plan_s* p, int nv, int tiles, int* chunkY, int* nchunks) {
-  int nc = std::max(1, std::min(p->ny, cdiv(4 * p->sm_count, std::max(1, nv * tiles))));
-  nc = std::min(nc, (int)p->nchunk_max);
-  *chunkY = cdiv(p->ny, nc);
-  *nchunks = cdiv(p->ny, *chunkY);
-}
-
 int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx, int nidx, cudaStream_t st,
              const float* y, const float* bg, float* partbuf, int gmax) {
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
@@ -625,28 +619,13 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
   for (int g0 = 0; g0 < nidx; g0 += p->gmax) {
     const int nv = std::min(p->gmax, nidx - g0);
     const int* vi = vidx + g0;
-    int cy, nc;
     ZArgs a = zargs(p);
     a.views = views + (size_t)g0 * p->nxz;
     a.T = p->d_P;
     a.vidx = vi;
     a.nv = nv;
-    if (p->zpath == 2) {  // large planes: column tiles, x pass and z pass x attenuation -> T
-      const int ntx = p->nx / p->zs_adj_tx;
-      zs_chunking(p, nv, ntx, &cy, &nc);
-      a.chunkY = cy;
-      a.nchunks = nc;
-      a.tx = p->zs_adj_tx;
-      LAUNCH(p, K_CONV_ADJ, st, "k_zs_adj",
-             zs_adj_launch(p->zs_w, p->zs_adj_nth, std::min(nv * ntx * nc, p->sm_count * p->zs_occ[2]),
-                           p->zs_smem[2], st, a));
-    } else {
-      chunking(p, nv, true, &cy, &nc);
-      a.chunkY = cy;
-      a.nchunks = nc;
-      const int gs = std::min(p->sm_count, nv * nc);
-      LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(p->zshape_adj, gs, p->zadj_smem_b, st, a));
-    }
+    const int gs = (int)std::min<long long>((long long)p->sm_count * p->zat.occ, (long long)nv * p->zat.ntile * p->ny);
+    LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
     LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
            zrot_adj_launch(p->zg, grot, st, p->d_P, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
@@ -983,7 +962,7 @@ int static_scratch_address(void** out) {
 struct TuneResult {
   int fwd_cy, adj_cy, rotf_nsplit, nsplit_adj, sep, sep_adj;
   double fwd_ms, adj_ms;
-  int zshape_fwd, zshape_adj;
+  int zshape_fwd;
 };
 std::mutex g_tune_mu;
 std::vector<std::pair<std::string, TuneResult>> g_tune_cache;
@@ -1034,10 +1013,7 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
         p->nsplit_adj = kv.second.nsplit_adj;
         p->sep = kv.second.sep && p->sep_fwd_ok;
         p->sep_adj = kv.second.sep_adj && p->sep_adj_ok;
-        if (p->zpath == 1) {
-          p->zshape_fwd = kv.second.zshape_fwd;
-          p->zshape_adj = kv.second.zshape_adj;
-        }
+        if (p->zpath == 1) p->zshape_fwd = kv.second.zshape_fwd;
         *fwd_ms = kv.second.fwd_ms;
         *adj_ms = kv.second.adj_ms;
         return SPECT_OK;
@@ -1071,17 +1047,16 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
     return SPECT_OK;
   }
   if (p->zpath) {
-    // fused path: depth tile and launch shape per direction
-    std::vector<int> fsh, ash;
+    // fused path: the forward's depth tile and launch shape (the adjoint's
+    // tiling is fixed by the geometry)
+    std::vector<int> fsh;
     for (int i = 0; i < kZNShapes; ++i) {
-      if (!zshape_allowed(p->zg, i)) continue;
       const int cap = kZShapes[i].nt * kZShapes[i].nth, xtasks = p->nz * (p->nx / kZShapes[i].w);
-      if (cap >= xtasks && cap <= 2 * xtasks && zfwd_shape_ok(i)) fsh.push_back(i);
-      if (kZShapes[i].nt == 1 && kZShapes[i].nth <= 640) ash.push_back(i);
+      if (zshape_allowed(p->zg, i) && cap >= xtasks && cap <= 2 * xtasks) fsh.push_back(i);
     }
     if (fsh.empty()) fsh.push_back(p->zshape_fwd);
-    double bf = 1e300, ba = 1e300;
-    int bcy = cys[0], bacy = cys[0], bsf = p->zshape_fwd, bsa = p->zshape_adj, rc = SPECT_OK;
+    double bf = 1e300, ba = 0;
+    int bcy = cys[0], bsf = p->zshape_fwd, rc = SPECT_OK;
     for (int sh : fsh)
       for (int cy : cys) {
         p->zshape_fwd = sh;
@@ -1094,29 +1069,15 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
           bsf = sh;
         }
       }
-    for (int sh : ash)
-      for (int cy : cys) {
-        if (rc != SPECT_OK) break;
-        p->zshape_adj = sh;
-        p->tune_adj_cy = cy;
-        double t;
-        if ((rc = time_pass(p, true, nv, 2, &t)) != SPECT_OK) break;
-        if (t < ba) {
-          ba = t;
-          bacy = cy;
-          bsa = sh;
-        }
-      }
     p->zshape_fwd = bsf;
-    p->zshape_adj = bsa;
     p->tune_fwd_cy = bcy;
-    p->tune_adj_cy = bacy;
+    if (rc == SPECT_OK) rc = time_pass(p, true, nv, 2, &ba);
     p->prof.on = prof;
     if (rc != SPECT_OK) return rc;
     *fwd_ms = bf;
     *adj_ms = ba;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache.push_back({key, TuneResult{bcy, bacy, 0, 1, p->sep, p->sep_adj, bf, ba, bsf, bsa}});
+    g_tune_cache.push_back({key, TuneResult{bcy, 0, 0, 1, p->sep, p->sep_adj, bf, ba, bsf}});
     return SPECT_OK;
   }
   // convolution kernels to try: direct (separable planes) and FFT, unless
@@ -1178,7 +1139,7 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
   *fwd_ms = bf;
   *adj_ms = ba;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache.push_back({key, TuneResult{bcy, bacy, brs, bns, bsep, basep, bf, ba, -1, -1}});
+  g_tune_cache.push_back({key, TuneResult{bcy, bacy, brs, bns, bsep, basep, bf, ba, -1}});
   return SPECT_OK;
 }
 
@@ -1420,6 +1381,25 @@ void trim_taps(double* w, int n) {
   }
 }
 
+// trim_taps of every n-tap factor; the widest support 2 h + 1 left, to which
+// the factors are then cut
+int trim_factors(std::vector<double>& w, int n) {
+  const int h = (n - 1) / 2;
+  const size_t count = w.size() / n;
+  int hk = 0;
+  for (size_t q = 0; q < count; ++q) {
+    trim_taps(w.data() + q * n, n);
+    for (int d = 0; d <= h; ++d)
+      if (w[q * n + h + d] != 0 || w[q * n + h - d] != 0) hk = std::max(hk, d);
+  }
+  const int nk = 2 * hk + 1;
+  std::vector<double> cut(count * nk);
+  for (size_t q = 0; q < count; ++q)
+    std::copy(w.begin() + q * n + h - hk, w.begin() + q * n + h - hk + nk, cut.begin() + q * nk);
+  w.swap(cut);
+  return nk;
+}
+
 // taps of a pass row w[0, len) (len a multiple of 8) that a window pass runs:
 // 8-tap blocks from a 4-tap boundary, (first 4-tap block b4, block count n8)
 // covering every nonzero tap, 4 b4 + 8 n8 <= len
@@ -1438,10 +1418,15 @@ void tap_range(const float* w, int len, int* b4, int* n8) {
   *n8 = n;
 }
 
-// zpath launch shapes (no 1024-thread shape: it leaves too few registers):
-// forward -- the fewest thread slots holding every x task of a plane (ties:
-// more threads); adjoint -- the least padded x and z passes, one task per
-// thread and pass
+// the same for the pair passes: 4-tap blocks (b4, n4), 4 b4 + 4 n4 <= len
+void tap_range4(const float* w, int len, int* b4, int* n4) {
+  int lo = 0, hi = len - 1;
+  while (lo < len && w[lo] == 0.f) ++lo;
+  while (hi > lo && w[hi] == 0.f) --hi;
+  *b4 = lo >= len ? 0 : lo / 4;
+  *n4 = lo >= len ? 0 : hi / 4 + 1 - lo / 4;
+}
+
 // tiles of the large-plane kernels: task width w (16 where it divides nx,
 // SPECT_ZW=8 forces 8), column tile tx (32, 16 or 8 dividing nx), row tile
 // tz (a multiple of 4: one x task of w outputs per thread of k_zs_fx,
@@ -1452,7 +1437,7 @@ bool zs_tiles(const ZGeom& g, size_t optin, ZsTiles* t) {
   t->tx = g.nx % 32 == 0 ? 32 : (g.nx % 16 == 0 ? 16 : 8);
   t->tz = std::min(kZsNthX * t->w / g.nx / 4 * 4, zround(g.nz, 4));
   if (t->tz < 4) return false;
-  return zs_fz_smem(g, t->tx) <= optin && zs_fx_smem(g, t->tz) <= optin && zs_adj_smem(g, t->tx) <= optin;
+  return zs_fz_smem(g, t->tx) <= optin && zs_fx_smem(g, t->tz) <= optin;
 }
 
 // shapes allowed by the geometry and by SPECT_ZW=8|16 (fixes the task width)
@@ -1466,7 +1451,7 @@ bool zshape_allowed(const ZGeom& g, int i) {
 int zpick_fwd(const ZGeom& g) {
   int best = -1;
   for (int i = 0; i < kZNShapes; ++i) {
-    if (!zfwd_shape_ok(i) || !zshape_allowed(g, i)) continue;
+    if (!zshape_allowed(g, i)) continue;
     const ZShape& s = kZShapes[i];
     const int cap = s.nt * s.nth;
     if (cap < g.nz * (g.nx / s.w)) continue;
@@ -1479,25 +1464,6 @@ int zpick_fwd(const ZGeom& g) {
   }
   return best;
 }
-// adjoint: one task per thread per pass round; the least padded work in
-// 8-output units (x and z tasks, rounded up to whole rounds), wider tasks on
-// ties
-int zpick_adj(const ZGeom& g) {
-  int best = -1;
-  long long bc = 0;
-  for (int i = 0; i < kZNShapes; ++i) {
-    const ZShape& s = kZShapes[i];
-    if (s.nt != 1 || s.nth > 640 || !zshape_allowed(g, i)) continue;
-    const long long xt = (long long)g.nz * (g.nx / s.w), zt = (long long)g.nx * ((g.nz + s.w - 1) / s.w);
-    const long long c = s.nth * ((xt + s.nth - 1) / s.nth + (zt + s.nth - 1) / s.nth) * (s.w / 8);
-    if (best < 0 || c < bc || (c == bc && s.w > kZShapes[best].w)) {
-      best = i;
-      bc = c;
-    }
-  }
-  return best;
-}
-
 int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, int nview, const float* mumap,
                      const float* psfs, float dy, const float* viewangle, int interpmeth, int mode, int nthread,
                      int nthreads, const PlanOpts& opts) {
@@ -1571,7 +1537,22 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   const char* conv_env = std::getenv("SPECT_CONV");
   const bool only_fft = conv_env && std::strcmp(conv_env, "fft") == 0;
   const int pad_rot = (int)std::ceil(1.0 + nx * std::sqrt(2.0) / 2.0 - nx / 2.0);
-  const ZGeom zg = zgeom_make(nx, ny, nz, px, pz, pad_rot);
+  // the fused path's factors: outer taps below Float32 resolution zeroed
+  // (trim_taps), and the support cut to the widest kept half-widths over all
+  // planes, which sizes the passes' line padding in shared memory
+  std::vector<double> za, zb;
+  int pxk = px, pzk = pz;
+  if (sep_host) {
+    za = fa;
+    zb = fb;
+    const char* trim_env = std::getenv("SPECT_ZTRIM");
+    if (!(trim_env && trim_env[0] == '0')) {
+      pxk = trim_factors(za, px);
+      pzk = trim_factors(zb, pz);
+    }
+  }
+  const ZGeom zg = zgeom_make(nx, ny, nz, pxk, pzk, pad_rot);
+  const ZGeom zg_full = zgeom_make(nx, ny, nz, px, pz, pad_rot);
   // zkind 1: the fused pair; 2: the large-plane kernels on the same layouts
   // (planes too large for the fused kernels' shared memory; SPECT_ZSTRIP=1
   // prefers them, =0 never takes them); 0: the split kernels
@@ -1584,11 +1565,12 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
         interpmeth == SPECT_INTERP_TWO && sep_host && !only_fft && !(zenv && zenv[0] == '0') && nx % 8 == 0 &&
-        zg.zpw <= 72 && zg.xpw <= 72 &&  // pass rows of at most 9 blocks of 8 taps
+        zg_full.zpw <= 72 && zg_full.xpw <= 72 &&  // pass rows of at most 9 blocks of 8 taps
         zg.nzp <= 256 && opts.atten_cache != 0) {
-      const bool fused = zpick_fwd(zg) >= 0 && zpick_adj(zg) >= 0 && zfwd_smem(zg, 1) <= (size_t)optin &&
-                         zadj_smem(zg, 1) <= (size_t)optin;
-      const bool strip = zs_tiles(zg, (size_t)optin, &zt);
+      p->zat = zadj_tile(zg, (size_t)optin);
+      const bool adj = p->zat.w != 0;
+      const bool fused = adj && zpick_fwd(zg) >= 0 && zfwd_smem(zg, 1) <= (size_t)optin;
+      const bool strip = adj && zs_tiles(zg, (size_t)optin, &zt);
       if (fused && !(senv && senv[0] == '1')) zkind = 1;
       else if (strip && !(senv && senv[0] == '0')) zkind = 2;
       else if (fused) zkind = 1;
@@ -1633,35 +1615,21 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     // k_zs_fz: 256 threads, two blocks per SM (SPECT_ZS_FZ_THREADS=512: one of 512)
     const char* fz_env = std::getenv("SPECT_ZS_FZ_THREADS");
     p->zs_fz_nth = (fz_env && std::atoi(fz_env) == kZsNth) ? kZsNth : kZsNth / 2;
-    // k_zs_adj: 512 threads on tiles of tx columns (SPECT_ZS_ADJ_THREADS=256:
-    // 256 threads on tiles of half the width, two blocks per SM where they fit)
-    const char* adj_env = std::getenv("SPECT_ZS_ADJ_THREADS");
-    p->zs_adj_nth = kZsNth;
-    p->zs_adj_tx = zt.tx;
-    if (adj_env && std::atoi(adj_env) == kZsNth / 2 && zt.tx / 2 >= zt.w && zt.tx % 2 == 0 && (zt.tx / 2) % 4 == 0) {
-      p->zs_adj_nth = kZsNth / 2;
-      p->zs_adj_tx = zt.tx / 2;
-    }
-    p->zs_smem[2] = zs_adj_smem(zg, p->zs_adj_tx);
     cudaError_t ze = zstrip_setup((int)p->max_smem);
-    if (ze == cudaSuccess) ze = zstrip_occupancy(zt.w, p->zs_fz_nth, p->zs_adj_nth, p->zs_smem, p->zs_occ);
+    if (ze == cudaSuccess) ze = zstrip_occupancy(zt.w, p->zs_fz_nth, p->zs_smem, p->zs_occ);
+    if (ze == cudaSuccess) ze = zpath_setup((int)p->max_smem);
     if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("large-plane kernel setup: ") + cudaGetErrorString(ze)));
   }
   if (p->zpath == 1) {
     p->zg = zg;
     p->izN = (size_t)zg.L * zg.L * zg.nzp;
     p->zshape_fwd = zpick_fwd(zg);
-    p->zshape_adj = zpick_adj(zg);
-    // double-buffered adjoint x pass where it fits (SPECT_ZADJ_BUFFERS=1: one buffer)
-    const char* nwa_env = std::getenv("SPECT_ZADJ_BUFFERS");
-    p->zg.nwa = (zadj_smem(zg, 2) <= p->max_smem && !(nwa_env && nwa_env[0] == '1')) ? 2 : 1;
     // one forward staging buffer (SPECT_ZFWD_STAGES=2: two where they fit;
     // measured slower at 128x128x80: the shared-memory carve-out takes L1
     // from the gather's image reads)
     const char* nsf_env = std::getenv("SPECT_ZFWD_STAGES");
     p->zg.nsf = (zfwd_smem(zg, 2) <= p->max_smem && nsf_env && nsf_env[0] == '2') ? 2 : 1;
     p->zfwd_smem_b = zfwd_smem(p->zg, p->zg.nsf);
-    p->zadj_smem_b = zadj_smem(p->zg, p->zg.nwa);
     const cudaError_t ze = zpath_setup((int)p->max_smem);
     if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("fused kernel setup: ") + cudaGetErrorString(ze)));
   }
@@ -1902,15 +1870,14 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     const int ts = std::max(4, (2 * hxs + 2 * hzs + 3) & ~3);
     std::vector<float> H((size_t)p->nset * ny * 2 * hs, 0.f), Tl((size_t)p->nset * ny * ts, 0.f);
     const bool ok = sep_host;
-    std::vector<float> Hz, Ez;
+    std::vector<float> Hz, Ez, Zt;
     std::vector<int> Rz;
-    std::vector<double> at(px), bt(pz);
-    const char* trim_env = std::getenv("SPECT_ZTRIM");
-    const bool trim = !(trim_env && trim_env[0] == '0');
+    const int zrow = ztable_floats(zg);
     if (ok && p->zpath) {
-      Hz.assign((size_t)p->nset * ny * 2 * zg.hs, 0.f);
-      Ez.assign((size_t)p->nset * ny * 2 * zg.ts, 0.f);
-      Rz.assign((size_t)p->nset * ny * 8, 0);
+      Hz.assign((size_t)p->nset * ny * zg.hs, 0.f);
+      Ez.assign((size_t)p->nset * ny * zg.ts, 0.f);
+      Rz.assign((size_t)p->nset * ny * 4, 0);
+      Zt.assign((size_t)p->nset * ny * zrow, 0.f);
     }
     for (int u = 0; ok && u < p->nset; ++u)
       for (int y = 0; y < ny; ++y) {
@@ -1927,34 +1894,37 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
         fold_tails(a, hxs, trow, trow + hxs);
         fold_tails(b, hzs, trow + 2 * hxs, trow + 2 * hxs + hzs);
         if (!Hz.empty()) {
-          // fused path, from the trimmed factors: [fwd z | fwd x | adj z |
-          // adj x], each shifted right by its data offset minus the half
-          // width; tails [ELz ERz ELx ERx | cLx cRx cLz cRz]; the tap-block
-          // range of each pass
-          std::copy(a, a + px, at.begin());
-          std::copy(b, b + pz, bt.begin());
-          if (trim) {
-            trim_taps(at.data(), px);
-            trim_taps(bt.data(), pz);
-          }
+          // fused path, from the trimmed factors: weights of the z and x
+          // pass, each shifted right by its data offset minus the half width;
+          // tails [ELz ERz ELx ERx] and folds [cLx cRx cLz cRz]; the
+          // tap-block range of each pass
+          const size_t pl = (size_t)u * ny + y;
+          const double* at = za.data() + pl * pxk;
+          const double* bt = zb.data() + pl * pzk;
           const int sz = zg.R0 - zg.hz, sx = zg.C0 - zg.hx;
-          float* zr = Hz.data() + ((size_t)u * ny + y) * 2 * zg.hs;
-          for (int m = 0; m < pz; ++m) zr[sz + m] = (float)bt[pz - 1 - m];
-          for (int m = 0; m < px; ++m) zr[zg.zpw + sx + m] = (float)at[px - 1 - m];
-          for (int m = 0; m < pz; ++m) zr[zg.hs + sz + m] = (float)bt[m];
-          for (int m = 0; m < px; ++m) zr[zg.hs + zg.zpw + sx + m] = (float)at[m];
-          float* er = Ez.data() + ((size_t)u * ny + y) * 2 * zg.ts;
-          clamp_tails(bt.data(), pz, er, er + hzs);
-          clamp_tails(at.data(), px, er + 2 * hzs, er + 2 * hzs + hxs);
-          fold_tails(at.data(), hxs, er + zg.ts, er + zg.ts + hxs);
-          fold_tails(bt.data(), hzs, er + zg.ts + 2 * hxs, er + zg.ts + 2 * hxs + hzs);
-          for (int m = 0; m < pz; ++m) p->ztaps[0] += bt[m] != 0.0 ? 1.0 : 0.0;
-          for (int m = 0; m < px; ++m) p->ztaps[1] += at[m] != 0.0 ? 1.0 : 0.0;
-          int* rr = Rz.data() + ((size_t)u * ny + y) * 8;
+          float* zr = Hz.data() + pl * zg.hs;
+          for (int m = 0; m < pzk; ++m) zr[sz + m] = (float)bt[pzk - 1 - m];
+          for (int m = 0; m < pxk; ++m) zr[zg.zpw + sx + m] = (float)at[pxk - 1 - m];
+          float* er = Ez.data() + pl * zg.ts;
+          clamp_tails(bt, pzk, er, er + zg.hz);
+          clamp_tails(at, pxk, er + 2 * zg.hz, er + 2 * zg.hz + zg.hx);
+          int* rr = Rz.data() + pl * 4;
           tap_range(zr, zg.zpw, rr, rr + 1);
           tap_range(zr + zg.zpw, zg.xpw, rr + 2, rr + 3);
-          tap_range(zr + zg.hs, zg.zpw, rr + 4, rr + 5);
-          tap_range(zr + zg.hs + zg.zpw, zg.xpw, rr + 6, rr + 7);
+          for (int m = 0; m < pzk; ++m) p->ztaps[0] += bt[m] != 0.0 ? 1.0 : 0.0;
+          for (int m = 0; m < pxk; ++m) p->ztaps[1] += at[m] != 0.0 ? 1.0 : 0.0;
+          // adjoint table: the weights twice each, folds, ranges
+          std::vector<float> row(zg.hs, 0.f);
+          for (int m = 0; m < pzk; ++m) row[sz + m] = (float)bt[m];
+          for (int m = 0; m < pxk; ++m) row[zg.zpw + sx + m] = (float)at[m];
+          float* tr = Zt.data() + pl * zrow;
+          for (int m = 0; m < zg.hs; ++m) tr[2 * m] = tr[2 * m + 1] = row[m];
+          fold_tails(at, zg.hx, tr + 2 * zg.hs, tr + 2 * zg.hs + zg.hx);
+          fold_tails(bt, zg.hz, tr + 2 * zg.hs + 2 * zg.hx, tr + 2 * zg.hs + 2 * zg.hx + zg.hz);
+          int ra[4];
+          tap_range4(row.data(), zg.zpw, ra, ra + 1);
+          tap_range4(row.data() + zg.zpw, zg.xpw, ra + 2, ra + 3);
+          std::memcpy(tr + 2 * zg.hs + zg.ts, ra, sizeof(ra));
         }
       }
     if (!Hz.empty()) {
@@ -1962,7 +1932,8 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       p->ztaps[1] /= (double)p->nset * ny;
       if ((st = dalloc(p, &p->d_Hz, Hz.size())) || (st = up(p->d_Hz, Hz.data(), sizeof(float) * Hz.size())) ||
           (st = dalloc(p, &p->d_Ez, Ez.size())) || (st = up(p->d_Ez, Ez.data(), sizeof(float) * Ez.size())) ||
-          (st = dalloc(p, &p->d_Rz, Rz.size())) || (st = up(p->d_Rz, Rz.data(), sizeof(int) * Rz.size())))
+          (st = dalloc(p, &p->d_Rz, Rz.size())) || (st = up(p->d_Rz, Rz.data(), sizeof(int) * Rz.size())) ||
+          (st = dalloc(p, &p->d_Zt, Zt.size())) || (st = up(p->d_Zt, Zt.data(), sizeof(float) * Zt.size())))
         return bail(st);
     }
     if (ok) {

@@ -120,28 +120,83 @@ __device__ __forceinline__ void zpassw(const float* __restrict__ w, int b4, int 
   }
 }
 
-// sum_{k < n} c[k] v[step k]: four partial sums over k mod 4, added as
-// (s0 + s1) + (s2 + s3); four taps' loads per round are independent, so a
-// round waits for one load latency
-__device__ __forceinline__ float zfold(const float* c, const float* v, int step, int n) {
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    s0 = fmaf(c[k], v[step * k], s0);
-    s1 = fmaf(c[k + 1], v[step * (k + 1)], s1);
-    s2 = fmaf(c[k + 2], v[step * (k + 2)], s2);
-    s3 = fmaf(c[k + 3], v[step * (k + 3)], s3);
-  }
-  if (k < n) s0 = fmaf(c[k], v[step * k], s0);
-  if (k + 1 < n) s1 = fmaf(c[k + 1], v[step * (k + 1)], s1);
-  if (k + 2 < n) s2 = fmaf(c[k + 2], v[step * (k + 2)], s2);
-  return (s0 + s1) + (s2 + s3);
-}
-
 // q = t / n for 0 <= t < 2^20, 1 <= n <= 4096, with r = 1/n rounded to float:
 // (t + 1/2) / n is at least 1/(2n) from an integer, far above the rounding
 // error of (t + 1/2) * r, so truncation gives the exact quotient
 __device__ __forceinline__ int zdiv(int t, float r) { return (int)(((float)t + 0.5f) * r); }
+
+// ------------------------------------------------------------------------
+// Pair passes: one task runs W consecutive outputs of TWO lines whose values
+// are interleaved in shared memory (element i = (a[i], b[i])), so every FMA
+// is a packed FFMA2 (two lines a lane) and an output pair needs no register
+// moves.  The FP32 pipe takes an FFMA2 every other cycle, which leaves every
+// second issue slot to the loads and address arithmetic (measured: with one
+// integer operation per two FMAs a chain of FFMA2 keeps 63 TFLOP/s where
+// FFMA falls to 49).  Weights are stored twice ((w, w)); taps run in blocks of
+// 4, m in [4 b4, 4 b4 + 4 n4) (n4 <= 18), in ascending order for every output:
+// the same result for every W, and for either lane as for a single line.
+template <int W>
+__device__ __forceinline__ void zpass2(const float2* __restrict__ w, int b4, int n4, const float2* line,
+                                       float2 (&o)[W]) {
+  const float4* w4 = reinterpret_cast<const float4*>(w + 4 * b4);
+  const float4* l4 = reinterpret_cast<const float4*>(line + 4 * b4);
+  float2 e[W + 4 * 18];
+#pragma unroll
+  for (int i = 0; i < W / 2; ++i) {
+    const float4 q = l4[i];
+    e[2 * i] = make_float2(q.x, q.y);
+    e[2 * i + 1] = make_float2(q.z, q.w);
+  }
+#pragma unroll
+  for (int k = 0; k < 18; ++k) {
+    if (k >= n4) break;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 q = l4[2 * k + W / 2 + i];
+      e[4 * k + W + 2 * i] = make_float2(q.x, q.y);
+      e[4 * k + W + 2 * i + 1] = make_float2(q.z, q.w);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 q = w4[2 * k + h];
+#pragma unroll
+      for (int j = 0; j < W; ++j) o[j] = __ffma2_rn(make_float2(q.x, q.y), e[4 * k + 2 * h + j], o[j]);
+#pragma unroll
+      for (int j = 0; j < W; ++j) o[j] = __ffma2_rn(make_float2(q.z, q.w), e[4 * k + 2 * h + 1 + j], o[j]);
+    }
+  }
+}
+
+// sum_{k < n} c[k] v[step k] of a pair of lines: four partial sums over k mod
+// 4, added as (s0 + s1) + (s2 + s3), so a round waits for one load latency
+__device__ __forceinline__ float2 zfold2(const float* c, const float2* v, int step, int n) {
+  float2 s[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = make_float2(0.f, 0.f);
+  int k = 0;
+  for (; k + 4 <= n; k += 4)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[j] = __ffma2_rn(make_float2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    if (k + j < n) s[j] = __ffma2_rn(make_float2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
+  return __fadd2_rn(__fadd2_rn(s[0], s[1]), __fadd2_rn(s[2], s[3]));
+}
+
+// fetch the 128-byte line of p into L2
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// fetch `bytes` (a multiple of 16, p 16-byte aligned) into L2
+__device__ __forceinline__ void prefetch_l2_bulk(const void* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// 16-byte asynchronous copy global -> shared of the calling thread, and the
+// wait for all of its copies
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ------------------------------------------------------------------------
 // Layout changes between the caller's image [z][y][x] and IZ.
@@ -310,9 +365,9 @@ __global__ void __launch_bounds__(NTH, 1) k_zfwd(ZArgs a) {
     fence_proxy_async();
     mbar_expect(&bar[s], abytes + (unsigned)(hts * sizeof(float)));
     bulk_copy(&bar[s], sA, a.att + ((size_t)v * ny + y) * nx * nzp, abytes);
-    bulk_copy(&bar[s], sW, a.H + ((size_t)set * ny + y) * (2 * hs), (unsigned)(hs * sizeof(float)));
-    bulk_copy(&bar[s], sW + hs, a.E + ((size_t)set * ny + y) * (2 * ts), (unsigned)(ts * sizeof(float)));
-    bulk_copy(&bar[s], sW + hs + ts, a.R + ((size_t)set * ny + y) * 8, 4u * sizeof(int));
+    bulk_copy(&bar[s], sW, a.H + ((size_t)set * ny + y) * hs, (unsigned)(hs * sizeof(float)));
+    bulk_copy(&bar[s], sW + hs, a.E + ((size_t)set * ny + y) * ts, (unsigned)(ts * sizeof(float)));
+    bulk_copy(&bar[s], sW + hs + ts, a.R + ((size_t)set * ny + y) * 4, 4u * sizeof(int));
   };
   auto next = [&](int& item, int& y) {
     const int yend = min(ny, chunk_of(item) * a.chunkY + a.chunkY);
@@ -545,215 +600,201 @@ __global__ void __launch_bounds__(NTH, 1) k_zfwd(ZArgs a) {
 }
 
 // ------------------------------------------------------------------------
-// k_zadj<NT, NTH, W>: adjoint convolution (tasks of W outputs); work items (slot, depth chunk), the
-// block's planes walked in sequence.  Plane p's adjoint weights and folds are
-// bulk-copied three planes ahead (stage p % 3); its x pass (view rows) writes
-// the x-pass buffer WB[p % nwa] and its z pass (WB columns, times the
-// attenuation column read by 16-byte global loads at the task start) writes
-// T.  One phase between two block barriers runs the z pass of plane p and
-// the x pass of plane p + 1, so with two buffers each plane costs one barrier
-// (one more where plane p + 1 starts a new item: the view is reloaded; and,
-// with one buffer, one between the two passes).  NT only sets how the x
-// tasks are interleaved.
-template <int NT, int NTH, int W>
-__global__ void __launch_bounds__(NTH, 1) k_zadj(ZArgs a) {
+// k_zadj<W>: adjoint convolution.  A work plane is (slot, row tile of tz rows,
+// j); block b walks planes [b n / grid, (b + 1) n / grid) of the slot-major
+// list of n, so blocks differ by at most one plane.  Plane j of an item is
+// depth y = j ystep mod ny, ystep coprime to ny and near 0.618 ny: a short
+// range of j holds narrow and wide PSF planes alike.  Per plane
+//   z pass  of the view's rows (columns 2 xp, 2 xp + 1 as one pair line,
+//           loaded once per item) -> XB, the plane's rows (2 zp, 2 zp + 1 as
+//           one pair line, zero outside the image),
+//   x pass  of XB, times the attenuation -> T.
+// Each pass is the zero-padded correlation with the factor plus the folded
+// padding at the two ends (z folds where the tile holds the image's first or
+// last row).  Lanes of the x pass are consecutive row pairs, so the
+// attenuation reads and the T stores are 256 contiguous bytes a warp (the
+// former x-then-z order read and wrote 16 bytes at a column stride, one line
+// a lane: the shared-memory/L1 pipe was its bound).  The plane's table
+// (weights, folds, tap ranges) is copied one plane ahead and its attenuation
+// prefetched into L2; an x task loads its attenuation before its FMAs, which
+// hides the rest of that latency (8 outputs a task: 16 would need 32 more
+// registers).  Two barriers a plane with one XB (the host then runs several
+// blocks per SM, which fill each other's waits), one with two.
+// Bound: FFMA2 (13.1 M of 34.7 M warp instructions at 128x128x80, 37 taps, 15
+// views; the pipe is 44 % busy) and what the blocks wait for at their
+// barriers.  Measured there: 105 -> 66 us (51.9 M instructions before);
+// 64x64x64, 11 taps, 64 views 92 -> 38 us; 256x256x200, 65 taps, 8 views
+// (five row tiles, two XB) 735 -> 483 us.
+// Shared memory (float2): [VB nxp * vst][XB nxb * (tz / 2) * bst][3 tables].
+template <int W>
+__global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
   extern __shared__ float4 smem4[];
   const ZGeom& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts;
-  float* const base = reinterpret_cast<float*>(smem4);
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(base);  // three barriers
-  const int sts = hs + ts + 4;             // one stage: weights, folds, tap ranges (4 ints)
-  float* const stage = base + 8;
-  float* const VB = stage + 3 * sts;
-  float* const WB0 = VB + (size_t)nz * g.bs;
-  const size_t wbs = g.nwa > 1 ? (size_t)nx * g.ast : 0;  // offset of the second buffer
-  const int tid = threadIdx.x;
-  const int nitems = a.nv * a.nchunks;
-  const float rnc = 1.0f / a.nchunks;
-  auto slot_of = [&](int item) { return zdiv(item, rnc); };             // item / nchunks (items < 2^20)
-  auto chunk_of = [&](int item) { return item - zdiv(item, rnc) * a.nchunks; };
-  auto issue = [&](int item, int y, int s) {  // one thread
-    const int sl = slot_of(item), v = a.vidx[sl], set = a.viewset[v];
-    float* st = stage + s * sts;
-    fence_proxy_async();
-    mbar_expect(&bar[s], (unsigned)(sts * sizeof(float)));
-    bulk_copy(&bar[s], st, a.H + ((size_t)set * ny + y) * (2 * hs) + hs, (unsigned)(hs * sizeof(float)));
-    bulk_copy(&bar[s], st + hs, a.E + ((size_t)set * ny + y) * (2 * ts) + ts, (unsigned)(ts * sizeof(float)));
-    bulk_copy(&bar[s], st + hs + ts, a.R + ((size_t)set * ny + y) * 8 + 4, 4u * sizeof(int));
+  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2;
+  const int tz = a.t.tz, vst = a.t.vst, bst = a.t.bst, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
+  const int trow = ztable_floats(g), tid = threadIdx.x, nth = blockDim.x;
+  float2* const VB = reinterpret_cast<float2*>(smem4);
+  float2* const XB0 = VB + (size_t)nxp * vst;
+  const size_t xbs = a.t.nxb > 1 ? (size_t)(tz / 2) * bst : 0;  // offset of the second row buffer
+  float* const tab0 = reinterpret_cast<float*>(XB0 + (size_t)a.t.nxb * (tz / 2) * bst);
+  const int ntile = a.t.ntile, n = a.nv * ntile * ny;
+  const int p0 = (int)((long long)blockIdx.x * n / gridDim.x), p1 = (int)((long long)(blockIdx.x + 1) * n / gridDim.x);
+  if (p0 >= p1) return;
+  const int vlen = W * ((tz + W - 1) / W) + g.zpw;  // elements of a view line that the windows read
+  const float rnxp = 1.0f / nxp;
+  int st = p0 / ny, j = p0 - st * ny;  // (slot, tile) of the plane and its place in the item
+  int y = (int)((long long)j * a.t.ystep % ny);
+  int slot = st / ntile, Z0 = (st - slot * ntile) * tz, v = a.vidx[slot];
+  auto table = [&](int view, int yy, int s) {  // every thread: its 16-byte pieces of the plane's table
+    const float* src = a.tab + ((size_t)a.viewset[view] * ny + yy) * trow;
+    for (int k = 4 * tid; k < trow; k += 4 * nth) cp16(tab0 + s * trow + k, src + k);
   };
-  auto next = [&](int& item, int& y) {
-    const int yend = min(ny, chunk_of(item) * a.chunkY + a.chunkY);
-    if (y + 1 < yend) {
-      ++y;
-    } else {
-      item += gridDim.x;
-      y = chunk_of(item) * a.chunkY;
+  // view rows Z0 - R0 .. of the item as pair lines, zero outside the image;
+  // lanes on consecutive column pairs, eight elements in flight
+  auto load_view = [&]() {
+    const float* V = a.views + (size_t)slot * nz * nx;
+    const int tot = vlen * nxp;
+    for (int k0 = tid; k0 < tot; k0 += 8 * nth) {
+      float2 q[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = k0 + i * nth, e = zdiv(k, rnxp), xp = k - e * nxp, z = Z0 + e - R0;
+        const bool in = k < tot && z >= 0 && z < nz;
+        const float* s = V + (size_t)z * nx + 2 * xp;  // 4-byte aligned only: the caller's array
+        q[i].x = in ? s[0] : 0.f;
+        q[i].y = in ? s[1] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = k0 + i * nth, e = zdiv(k, rnxp), xp = k - e * nxp;
+        if (k < tot) VB[(size_t)xp * vst + e] = q[i];
+      }
     }
   };
-  // WB rows outside the data rows stay zero
-  for (int x = tid / 32; x < g.nwa * nx; x += NTH / 32)
-    for (int r = tid & 31; r < g.ast; r += 32)
-      if (r < g.R0 || r >= g.R0 + nz) WB0[(size_t)x * g.ast + r] = 0.f;
-  // planes p, p + 1, p + 2 and p + 3 (the next to issue)
-  int i0 = blockIdx.x, y0 = (blockIdx.x % a.nchunks) * a.chunkY;
-  int i1 = i0, y1 = y0;
-  next(i1, y1);
-  int i2 = i1, y2 = y1;
-  next(i2, y2);
-  int i3 = i2, y3 = y2;
-  next(i3, y3);
-  if (tid == 0) {
-    mbar_init(&bar[0]);
-    mbar_init(&bar[1]);
-    mbar_init(&bar[2]);
-    if (i0 < nitems) issue(i0, y0, 0);
-    if (i1 < nitems) issue(i1, y1, 1);
-    if (i2 < nitems) issue(i2, y2, 2);
-  }
+  table(v, y, 0);
+  for (int k = tid; k < a.t.nxb * (tz / 2) * bst; k += nth) XB0[k] = make_float2(0.f, 0.f);
+  load_view();
+  cp_wait();
   __syncthreads();
-  if (!(i0 < nitems)) return;
-  unsigned pend = (i1 < nitems ? 7u : 1u) & (i2 < nitems ? 7u : 3u);  // copies issued, not yet waited for
-  unsigned phases = 0u;                                                  // parity of each barrier's next wait
-  auto wait = [&](int s) {
-    const bool ok = mbar_wait(&bar[s], (phases >> s) & 1u);
-    if (ok) {
-      phases ^= 1u << s;
-      pend &= ~(1u << s);
+  constexpr int X = kZadjX;  // outputs of an x task
+  const int nxw = (nx + X - 1) / X;
+  int tb = 0, xb2 = 0;  // table and row buffer of the plane
+  for (int p = p0;;) {
+    const int rows = min(tz, nz - Z0), nzp2 = (rows + 1) / 2;
+    // the next plane, its table on the way
+    int st1 = st, y1 = y + a.t.ystep;
+    if (y1 >= ny) y1 -= ny;
+    if (++j == ny) {
+      j = y1 = 0;
+      ++st1;
     }
-    return ok;
-  };
-  auto give_up = [&]() {  // after a failed wait: flag it, let the copies in flight land
-    if (tid == 0) {
-      atomicExch(a.err, 1);
-      for (int s = 0; s < 3; ++s)
-        if ((pend >> s) & 1u) mbar_wait(&bar[s], (phases >> s) & 1u);
-    }
-  };
-  const int nzb = (nz + W - 1) / W, ztasks = nx * nzb, xtasks = nz * (nx / W);
-  const int ast = g.ast, bs = g.bs, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
-  const float rnx = 1.0f / nx, rnz = 1.0f / nz;
-  // the item's view into VB, zero-padded: element e = z bs + c, eight per
-  // thread and round with all eight loads issued before the stores
-  const float rbs = 1.0f / bs;
-  auto load_view = [&](int item) {
-    const float* V = a.views + (size_t)slot_of(item) * nz * nx;
-    for (int e0 = tid; e0 < nz * bs; e0 += 8 * NTH) {
-      float v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int e = e0 + j * NTH, z = zdiv(e, rbs), c = e - z * bs;
-        v[j] = (e < nz * bs && c >= C0 && c < C0 + nx) ? V[z * nx + c - C0] : 0.f;
+    const bool more = p + 1 < p1;
+    const int tb1 = tb == 2 ? 0 : tb + 1;
+    const int slot1 = st1 == st ? slot : st1 / ntile;
+    if (more) {  // the next plane's attenuation columns on their way into L2, too
+      const int v1 = slot1 == slot ? v : a.vidx[slot1], Z1 = (st1 - slot1 * ntile) * tz, ln = (min(tz, nz - Z1) + 31) / 32;
+      table(v1, y1, tb1);
+      const float* src = a.att + (((size_t)v1 * ny + y1) * nx) * nzp + Z1;
+      if (ntile == 1) {
+        if (tid == 0) prefetch_l2_bulk(src, (unsigned)(nx * nzp * sizeof(float)));
+      } else {
+        for (int x = tid; x < nx; x += nth)
+          for (int l = 0; l < ln; ++l) prefetch_l2(src + x * nzp + 32 * l);
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (e0 + j * NTH < nz * bs) VB[e0 + j * NTH] = v[j];
     }
-  };
-  // x pass of the plane whose stage is st: task (z, x block) -> WB column x, row R0 + z
-  auto xpass = [&](const float* st, float* WB, int item, int y) {
-    const int2 rg = *reinterpret_cast<const int2*>(st + hs + ts + 2);  // x-pass tap range
-    const float* ax = st + g.zpw;     // adjoint x weights (shifted)
-    const float* cLx = st + hs;       // folds
-    const float* cRx = cLx + hx;
+    const float* const Wt = tab0 + tb * trow;
+    const float2* const Wd = reinterpret_cast<const float2*>(Wt);
+    const int4 rg = *reinterpret_cast<const int4*>(Wt + 2 * hs + ts);  // tap ranges: z pass, x pass
+    float2* const XB = XB0 + xb2 * xbs;
+    {  // z pass: task (column pair, W rows) -> XB
+      const float* cLz = Wt + 2 * hs + 2 * hx;
+      const float* cRz = cLz + hz;
+      const int tasks = nxp * ((rows + W - 1) / W);
+      for (int t = tid; t < tasks; t += nth) {
+        const int zb = zdiv(t, rnxp), xp = t - zb * nxp, z0 = W * zb;
+        const float2* col = VB + (size_t)xp * vst;
+        float2 o[W];
 #pragma unroll
-    for (int i = 0; i < NT; ++i)
-      for (int t = tid + i * NTH; t < xtasks; t += NT * NTH) {
-        const int xb = zdiv(t, rnz), z = t - xb * nz, x0 = W * xb;
-        const float* row = VB + z * bs;
-        float o[W];
+        for (int k = 0; k < W; ++k) o[k] = make_float2(0.f, 0.f);
+        zpass2<W>(Wd, rg.x, rg.y, col + z0, o);
+        if (Z0 + z0 == 0) o[0] = __fadd2_rn(o[0], zfold2(cLz, col + R0, 1, hz));
+        const int kz = nz - 1 - Z0 - z0;
+        if (kz >= 0 && kz < W) {
+          const float2 s = zfold2(cRz, col + R0 + z0 + kz, -1, hz);
 #pragma unroll
-        for (int k = 0; k < W; ++k) o[k] = 0.f;
-        zpassw<W>(ax, rg.x, rg.y, row + x0, o);
-        if (x0 == 0)
-          o[0] += zfold(cLx, row + C0, 1, hx);
-        if (x0 + W == nx)
-          o[W - 1] += zfold(cRx, row + C0 + nx - 1, -1, hx);
-        float* w = WB + x0 * ast + R0 + z;
+          for (int k = 0; k < W; ++k)
+            if (k == kz) o[k] = __fadd2_rn(o[k], s);
+        }
+        float2* w = XB + (size_t)(z0 / 2) * bst + C0 + 2 * xp;
 #pragma unroll
-        for (int k = 0; k < W; ++k) w[k * ast] = o[k];
+        for (int m = 0; m < W / 2; ++m)
+          if (z0 + 2 * m < rows)
+            *reinterpret_cast<float4*>(w + (size_t)m * bst) =
+                make_float4(o[2 * m].x, o[2 * m + 1].x, o[2 * m].y, o[2 * m + 1].y);
       }
-  };
-  // z pass of plane (item, y), stage st: task (x, z block) -> T column (x, y) of the slot
-  auto zpass = [&](const float* st, const float* WB, int item, int y) {
-    const int slot = slot_of(item), v = a.vidx[slot];
-    const int2 rg = *reinterpret_cast<const int2*>(st + hs + ts);  // z-pass tap range
-    const float* az = st;             // adjoint z weights (shifted)
-    const float* cLz = st + hs + 2 * hx;
-    const float* cRz = cLz + hz;
-    const float* attv = a.att + (((size_t)v * ny + y) * nx) * nzp;
-    float* Tp = a.T + (((size_t)slot * ny + y) * nx) * nzp;
-    for (int t = tid; t < ztasks; t += NTH) {
-      // lanes on consecutive columns: conflict-free shared windows (lanes
-      // walking down a column, which coalesces the global accesses, measured
-      // slower: 2- to 3-way bank conflicts and folds in every warp)
-      const int zb = zdiv(t, rnx), x = t - zb * nx, z0 = W * zb;
-      float4 at[W / 4];
+    }
+    cp_wait();
+    __syncthreads();
+    {  // x pass: task (row pair, X columns), times the attenuation -> T
+      const float* cLx = Wt + 2 * hs;
+      const float* cRx = cLx + hx;
+      const float* attp = a.att + (((size_t)v * ny + y) * nx) * nzp + Z0;
+      float* Tp = a.T + (((size_t)slot * ny + y) * nx) * nzp + Z0;
+      const int tasks = nzp2 * nxw;
+      const float rn = 1.0f / nzp2;
+      for (int t = tid; t < tasks; t += nth) {
+        const int xb = zdiv(t, rn), zp = t - xb * nzp2, x0 = X * xb;
+        const bool whole = x0 + X <= nx;
+        const int at0 = x0 * nzp + 2 * zp;
+        // the attenuation first: its latency passes behind the window's FMAs
+        float2 at[X];
+        if (whole) {
+          const float* q = attp + at0;
 #pragma unroll
-      for (int k = 0; k < W / 4; ++k) at[k] = ld4(attv + x * nzp + z0 + 4 * k);
-      const float* col = WB + x * ast;
-      float o[W];
+          for (int k = 0; k < X; ++k, q += nzp) at[k] = *reinterpret_cast<const float2*>(q);
+        } else {
 #pragma unroll
-      for (int k = 0; k < W; ++k) o[k] = 0.f;
-      zpassw<W>(az, rg.x, rg.y, col + z0, o);
-      if (z0 == 0)
-        o[0] += zfold(cLz, col + R0, 1, hz);
-      if (z0 <= nz - 1 && nz - 1 < z0 + W) {
-        const int kz = nz - 1 - z0;
-        const float s = zfold(cRz, col + R0 + nz - 1, -1, hz);
+          for (int k = 0; k < X; ++k) at[k] = *reinterpret_cast<const float2*>(attp + at0 + min(k, nx - 1 - x0) * nzp);
+        }
+        const float2* row = XB + (size_t)zp * bst;
+        float2 o[X];
 #pragma unroll
-        for (int k = 0; k < W; ++k)
-          if (k == kz) o[k] += s;
+        for (int k = 0; k < X; ++k) o[k] = make_float2(0.f, 0.f);
+        zpass2<X>(Wd + g.zpw, rg.z, rg.w, row + x0, o);
+        if (x0 == 0) o[0] = __fadd2_rn(o[0], zfold2(cLx, row + C0, 1, hx));
+        const int kx = nx - 1 - x0;
+        if (kx < X) {
+          const float2 s = zfold2(cRx, row + C0 + nx - 1, -1, hx);
+#pragma unroll
+          for (int k = 0; k < X; ++k)
+            if (k == kx) o[k] = __fadd2_rn(o[k], s);
+        }
+        float* q = Tp + at0;
+        if (whole) {
+#pragma unroll
+          for (int k = 0; k < X; ++k, q += nzp) *reinterpret_cast<float2*>(q) = __fmul2_rn(at[k], o[k]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < X; ++k, q += nzp)
+            if (x0 + k < nx) *reinterpret_cast<float2*>(q) = __fmul2_rn(at[k], o[k]);
+        }
       }
-      float* dst = Tp + x * nzp + z0;
-#pragma unroll
-      for (int k = 0; k < W / 4; ++k)
-        st4(dst + 4 * k, make_float4(__fmul_rn(at[k].x, o[4 * k]), __fmul_rn(at[k].y, o[4 * k + 1]),
-                                     __fmul_rn(at[k].z, o[4 * k + 2]), __fmul_rn(at[k].w, o[4 * k + 3])));
     }
-  };
-  // prologue: the first view, the stages of p and p + 1, the x pass of p
-  load_view(i0);
-  {
-    bool ok = wait(0);
-    if (i1 < nitems) ok = wait(1) && ok;
-    if (__syncthreads_or(!ok)) {
-      give_up();
-      return;
+    if (!more) break;
+    ++p;
+    y = y1;
+    tb = tb1;
+    if (a.t.nxb > 1) xb2 ^= 1;
+    if (st1 != st) {  // the last reader of VB finished before the barrier above
+      st = st1;
+      slot = slot1;
+      Z0 = (st - slot * ntile) * tz;
+      v = a.vidx[slot];
+      load_view();
+      __syncthreads();
+    } else if (a.t.nxb == 1) {
+      __syncthreads();
     }
-  }
-  xpass(stage, WB0, i0, y0);
-  __syncthreads();
-  int s = 0, w = 0;  // stage and x-pass buffer of plane p
-  for (;;) {
-    const bool h1 = i1 < nitems, h2 = i2 < nitems;
-    const int s1 = s == 2 ? 0 : s + 1;
-    const bool newv = h1 && slot_of(i1) != slot_of(i0);
-    if (newv) load_view(i1);  // the last reader of VB (the x pass of p) finished before the barrier
-    zpass(stage + s * sts, WB0 + w * wbs, i0, y0);
-    if (h1) {
-      if (newv || g.nwa == 1) __syncthreads();  // uniform
-      xpass(stage + s1 * sts, WB0 + (w ^ 1) * wbs, i1, y1);
-    }
-    bool ok = true;
-    if (h2) ok = wait(s1 == 2 ? 0 : s1 + 1);
-    if (__syncthreads_or(!ok)) {
-      give_up();
-      return;
-    }
-    if (!h1) break;
-    if (i3 < nitems) {  // stage s is free again: plane p + 3
-      if (tid == 0) issue(i3, y3, s);
-      pend |= 1u << s;
-    }
-    i0 = i1;
-    y0 = y1;
-    i1 = i2;
-    y1 = y2;
-    i2 = i3;
-    y2 = y3;
-    next(i3, y3);
-    s = s1;
-    w ^= 1;
   }
 }
 

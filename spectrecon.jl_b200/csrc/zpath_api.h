@@ -17,7 +17,6 @@ struct ZGeom {
   int hs, ts;       // weight-row and tail-row lengths of one direction
   int rows, ast;    // z-pass buffer: rows per column, column stride (4 * odd)
   int bs;           // x-pass buffer row stride (4 * odd)
-  int nwa;          // k_zadj x-pass output buffers: 2 (double-buffered) or 1
   int nsf;          // k_zfwd staging buffers: 2 (two planes in flight) or 1
 };
 
@@ -50,18 +49,40 @@ inline ZGeom zgeom_make(int nx, int ny, int nz, int px, int pz, int pad) {
   g.rows = zround(nz, 16) + g.zpw;  // z tasks of 8 or 16 outputs
   g.ast = zstride4(g.rows);
   g.bs = zstride4(nx + g.xpw);
-  g.nwa = 1;
   g.nsf = 1;
   return g;
 }
 
+// smallest 2 * odd >= v: pair lines (float2 elements) whose 16-byte chunk
+// count is odd, so the eight lanes of a 128-bit shared access phase hit
+// distinct bank groups
+__host__ __device__ constexpr int zstride2(int v) {
+  return ((zround(v, 2) / 2) % 2 == 1) ? zround(v, 2) : zround(v, 2) + 2;
+}
+// floats of one plane's table of one direction: weights of the z and x pass,
+// each stored twice | tails or folds | tap ranges (first 4-tap block and
+// 4-tap blocks of the z pass, then of the x pass)
+__host__ __device__ inline int ztable_floats(const ZGeom& g) { return 2 * g.hs + g.ts + 4; }
+
+// tiling of a pair-pass kernel: task width w, row tile tz (even; ntile tiles
+// cover nz), strides (float2) of the z-pass and x-pass lines, row buffers,
+// threads, resident blocks per SM, depth step of the plane walk, shared memory
+struct ZTile {
+  int w, tz, ntile, vst, bst, nxb, nth, occ, ystep;
+  size_t smem;
+};
+constexpr int kZadjX = 8;       // outputs of an x-pass task of k_zadj
+constexpr int kZThreads = 640;  // threads per SM the pair-pass kernels' registers allow (96 each)
+
 struct ZArgs {
   ZGeom g;
+  ZTile t;
+  const float* tab;     // [set][y][ztable_floats]: adjoint tables
   const float* img;     // IZ
   const float* att;     // ATT
-  const float* H;       // [set][y][2 hs]: fwd z | fwd x | adj z | adj x
-  const float* E;       // [set][y][2 ts]: ELz ERz ELx ERx | cLx cRx cLz cRz
-  const int* R;         // [set][y][8]: (first 4-tap block, 8-tap blocks) of fwd z | fwd x | adj z | adj x
+  const float* H;       // [set][y][hs]: forward z | x weights
+  const float* E;       // [set][y][ts]: ELz ERz ELx ERx
+  const int* R;         // [set][y][4]: (first 4-tap block, 8-tap blocks) of the forward z | x pass
   const float4* rot;    // [view] (cos(2pi - theta), sin(2pi - theta), theta == 0, theta)
   const int* vidx;      // [nv] plan view of each slot
   const int* viewset;   // [nview] PSF set of each view
@@ -84,27 +105,77 @@ __host__ __device__ inline size_t zfwd_smem(const ZGeom& g, int nsf) {
   return f * sizeof(float);
 }
 
-// k_zadj shared memory (floats): [bar 8][3 stages x (weights hs | folds ts | ranges 4)]
-//   [VB nz * bs: the view, zero-padded, data columns C0..][nwb x WB nx * ast:
-//   x-pass output, column x, data rows R0..]
-__host__ __device__ inline size_t zadj_smem(const ZGeom& g, int nwb) {
-  return sizeof(float) *
-         (8 + 3 * (size_t)(g.hs + g.ts + 4) + (size_t)g.nz * g.bs + (size_t)nwb * g.nx * g.ast);
+// k_zadj shared memory (zpath.cuh)
+inline size_t zadj_smem(const ZGeom& g, const ZTile& t) {
+  return sizeof(float) * (2 * ((size_t)(g.nx / 2) * t.vst + (size_t)t.nxb * (t.tz / 2) * t.bst) +
+                          3 * (size_t)ztable_floats(g));
+}
+// depth step of a plane walk: coprime to ny, near the golden section of ny
+inline int zdepth_step(int ny) {
+  auto gcd = [](int a, int b) {
+    while (b) {
+      const int r = a % b;
+      a = b;
+      b = r;
+    }
+    return a;
+  };
+  int s = (int)(0.618 * ny);
+  if (s < 1) s = 1;
+  while (gcd(s, ny) != 1) ++s;
+  return s;
+}
+// tiling of k_zadj: the least modelled time per view and depth.  A thread's
+// task is w outputs of two lines in each pass; wider tasks read fewer shared
+// bytes per FMA, row tiles cut the shared memory of a block so that several
+// blocks (or a second row buffer) hide each other's barriers, and fewer than
+// 16 warps per SM no longer hide the latencies.
+inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
+  ZTile best{};
+  double bc = 0;
+  for (int w : {16, 8})
+    for (int nt = 1; nt <= (g.nz + 1) / 2; ++nt) {
+      ZTile t{};
+      t.w = w;
+      t.tz = zround((g.nz + nt - 1) / nt, nt > 1 ? 8 : 2);  // tiles of whole tasks
+      t.ntile = (g.nz + t.tz - 1) / t.tz;
+      if (t.ntile != nt) continue;
+      t.vst = zstride2(w * ((t.tz + w - 1) / w) + g.zpw);
+      t.bst = zstride2(kZadjX * ((g.nx + kZadjX - 1) / kZadjX) + g.xpw);
+      const int zt = (g.nx / 2) * ((t.tz + w - 1) / w), xt = (t.tz / 2) * ((g.nx + kZadjX - 1) / kZadjX);
+      const int most = w == 16 || zt > xt ? zt : xt, rounds = (most + kZThreads - 1) / kZThreads;
+      t.nth = zround((most + rounds - 1) / rounds, 32);
+      for (int nxb : {1, 2}) {
+        t.nxb = nxb;
+        t.smem = zadj_smem(g, t);
+        if (t.smem > optin) continue;
+        const int so = (int)((optin + 1024) / (t.smem + 1024)), ro = kZThreads / t.nth;
+        t.occ = so < ro ? so : ro;
+        if (t.occ > 16) t.occ = 16;
+        if (nxb > 1 && t.occ > 1) continue;  // several blocks overlap already
+        const double warps = t.occ * t.nth / 32.0;
+        const double rz = (double)((zt + t.nth - 1) / t.nth), rx = (double)((xt + t.nth - 1) / t.nth);
+        double c = t.ntile * t.nth * (rz * w * (w == 8 ? 1.15 : 1.0) + rx * kZadjX * 1.15);  // thread slots x outputs
+        c *= warps < 16 ? 16 / warps : 1.0;
+        c *= (t.occ > 1 || nxb > 1) ? 1.0 : 1.25;
+        if (!best.w || c < bc) {
+          best = t;
+          bc = c;
+        }
+      }
+    }
+  best.ystep = zdepth_step(g.ny);
+  return best;
 }
 
-// launch shapes of k_zfwd / k_zadj: NT tasks of W outputs per thread, NTH
-// threads (W = 16 needs nx % 16 == 0); fwd: the forward compiles without
-// register spills in this shape (with the accumulators, 1024 threads and the
-// largest NT leave too few registers)
+// launch shapes of k_zfwd: NT tasks of W outputs per thread, NTH threads
+// (W = 16 needs nx % 16 == 0); each compiles without register spills
 struct ZShape {
-  int nt, nth, w, fwd;
+  int nt, nth, w;
 };
-constexpr int kZNShapes = 13;
-constexpr ZShape kZShapes[kZNShapes] = {{1, 512, 8, 1},  {2, 512, 8, 1},  {3, 512, 8, 1},   {4, 512, 8, 0},
-                                        {1, 640, 8, 1},  {2, 640, 8, 1},  {3, 640, 8, 0},   {1, 1024, 8, 0},
-                                        {1, 512, 16, 1}, {2, 512, 16, 1}, {1, 640, 16, 1},  {2, 640, 16, 0},
-                                        {1, 1024, 16, 0}};
-inline bool zfwd_shape_ok(int i) { return kZShapes[i].fwd != 0; }
+constexpr int kZNShapes = 8;
+constexpr ZShape kZShapes[kZNShapes] = {{1, 512, 8}, {2, 512, 8},  {3, 512, 8},  {1, 640, 8},
+                                        {2, 640, 8}, {1, 512, 16}, {2, 512, 16}, {1, 640, 16}};
 inline bool zshape_fits(const ZGeom& g, int i) { return g.nx % kZShapes[i].w == 0; }
 
 // large-plane kernels (zstrip.cuh), shared memory in bytes
@@ -114,19 +185,16 @@ __host__ __device__ inline size_t zs_fz_smem(const ZGeom& g, int tx) {
 __host__ __device__ inline size_t zs_fx_smem(const ZGeom& g, int tz) {
   return sizeof(float) * 2 * ((size_t)tz * g.bs + g.hs + g.ts + 4);
 }
-__host__ __device__ inline size_t zs_adj_smem(const ZGeom& g, int tx) {
-  return sizeof(float) * ((size_t)g.nz * zstride4(tx + g.xpw) + (size_t)tx * g.ast + g.hs + g.ts + 4);
-}
 struct ZsTiles {
   int w, tx, tz;  // task width, column tile, row tile
 };
-constexpr int kZsNth = 512;   // k_zs_fz, k_zs_adj threads
+constexpr int kZsNth = 512;   // k_zs_fz threads
 constexpr int kZsNthX = 640;  // k_zs_fx threads (one x task each)
 
 // launchers (zpath_inst.cu)
 cudaError_t zpath_setup(int max_smem);
 cudaError_t zfwd_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
-cudaError_t zadj_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
+cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zrot_adj_launch(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot,
                             const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,
                             int mode);
@@ -135,13 +203,12 @@ cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const fl
                             const float* att, const int* vidx);
 cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, float* dst, const float* asum, int mode);
 // large-plane kernels: w = task width (8 or 16); occ = resident blocks per
-// SM of k_zs_fz, k_zs_fx, k_zs_adj at their shared-memory sizes (for the
-// persistent grids)
+// SM of k_zs_fz, k_zs_fx at their shared-memory sizes (for the persistent
+// grids)
 cudaError_t zstrip_setup(int max_smem);
-cudaError_t zstrip_occupancy(int w, int fz_nth, int adj_nth, const size_t smem[3], int occ[3]);
+cudaError_t zstrip_occupancy(int w, int fz_nth, const size_t smem[2], int occ[2]);
 cudaError_t zs_fz_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
 cudaError_t zs_fx_launch(int w, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
-cudaError_t zs_adj_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
 cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot, float dy,
                           float* att);
 

@@ -10,15 +10,11 @@ namespace spect {
 
 namespace {
 // the order of kZShapes
-#define ZSHAPES(K)                                                                                           \
-  {(const void*)K<1, 512, 8>,  (const void*)K<2, 512, 8>,   (const void*)K<3, 512, 8>,                       \
-   (const void*)K<4, 512, 8>,  (const void*)K<1, 640, 8>,   (const void*)K<2, 640, 8>,                       \
-   (const void*)K<3, 640, 8>,  (const void*)K<1, 1024, 8>,  (const void*)K<1, 512, 16>,                      \
-   (const void*)K<2, 512, 16>, (const void*)K<1, 640, 16>,  (const void*)K<2, 640, 16>,                      \
-   (const void*)K<1, 1024, 16>}
-const void* const kZfwd[kZNShapes] = ZSHAPES(k_zfwd);
-const void* const kZadj[kZNShapes] = ZSHAPES(k_zadj);
-#undef ZSHAPES
+const void* const kZfwd[kZNShapes] = {
+    (const void*)k_zfwd<1, 512, 8>, (const void*)k_zfwd<2, 512, 8>,  (const void*)k_zfwd<3, 512, 8>,
+    (const void*)k_zfwd<1, 640, 8>, (const void*)k_zfwd<2, 640, 8>,  (const void*)k_zfwd<1, 512, 16>,
+    (const void*)k_zfwd<2, 512, 16>, (const void*)k_zfwd<1, 640, 16>};
+const void* const kZadj[2] = {(const void*)k_zadj<8>, (const void*)k_zadj<16>};
 
 // k_zrot_adj's candidates per load round: the largest of 3 and 2 whose
 // rounds compile without register spills under the kernel's launch bounds
@@ -48,12 +44,12 @@ cudaError_t zrot(const ZGeom& g, int grid, cudaStream_t st, const float* T, cons
 }  // namespace
 
 cudaError_t zpath_setup(int max_smem) {
-  for (int i = 0; i < kZNShapes; ++i) {
-    cudaError_t e = cudaFuncSetAttribute(kZfwd[i], cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kZadj[i], cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (const void* k : kZfwd)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  for (const void* k : kZadj)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  return e;
 }
 
 cudaError_t zfwd_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
@@ -62,10 +58,10 @@ cudaError_t zfwd_launch(int shape, int grid, size_t smem, cudaStream_t st, const
   return cudaLaunchKernel(kZfwd[shape], dim3(grid), dim3(kZShapes[shape].nth), args, smem, st);
 }
 
-cudaError_t zadj_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
+cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {
   ZArgs c = a;
   void* args[] = {&c};
-  return cudaLaunchKernel(kZadj[shape], dim3(grid), dim3(kZShapes[shape].nth), args, smem, st);
+  return cudaLaunchKernel(kZadj[a.t.w == 16 ? 1 : 0], dim3(grid), dim3(a.t.nth), args, a.t.smem, st);
 }
 
 cudaError_t zrot_adj_launch(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot,
@@ -86,9 +82,6 @@ namespace {
 const void* const kZsFz[4] = {(const void*)k_zs_fz<kZsNth, 8>, (const void*)k_zs_fz<kZsNth, 16>,
                               (const void*)k_zs_fz<kZsNth / 2, 8>, (const void*)k_zs_fz<kZsNth / 2, 16>};
 const void* const kZsFx[2] = {(const void*)k_zs_fx<kZsNthX, 8>, (const void*)k_zs_fx<kZsNthX, 16>};
-// k_zs_adj: 512 threads (index 0, 1) or 256 (index 2, 3: narrower tiles, two blocks per SM)
-const void* const kZsAdj[4] = {(const void*)k_zs_adj<kZsNth, 8>, (const void*)k_zs_adj<kZsNth, 16>,
-                               (const void*)k_zs_adj<kZsNth / 2, 8>, (const void*)k_zs_adj<kZsNth / 2, 16>};
 cudaError_t zs_launch(const void* k, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
   ZArgs c = a;
   void* args[] = {&c};
@@ -98,18 +91,18 @@ cudaError_t zs_launch(const void* k, int nth, int grid, size_t smem, cudaStream_
 
 cudaError_t zstrip_setup(int max_smem) {
   for (int i = 0; i < 2; ++i)
-    for (const void* k : {kZsFz[i], kZsFz[i + 2], kZsFx[i], kZsAdj[i], kZsAdj[i + 2]}) {
+    for (const void* k : {kZsFz[i], kZsFz[i + 2], kZsFx[i]}) {
       const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
       if (e != cudaSuccess) return e;
     }
   return cudaSuccess;
 }
 
-cudaError_t zstrip_occupancy(int w, int fz_nth, int adj_nth, const size_t smem[3], int occ[3]) {
-  const int i = w == 16 ? 1 : 0, f = fz_nth == kZsNth ? i : i + 2, d = adj_nth == kZsNth ? i : i + 2;
-  const void* ks[3] = {kZsFz[f], kZsFx[i], kZsAdj[d]};
-  const int nth[3] = {fz_nth, kZsNthX, adj_nth};
-  for (int j = 0; j < 3; ++j) {
+cudaError_t zstrip_occupancy(int w, int fz_nth, const size_t smem[2], int occ[2]) {
+  const int i = w == 16 ? 1 : 0, f = fz_nth == kZsNth ? i : i + 2;
+  const void* ks[2] = {kZsFz[f], kZsFx[i]};
+  const int nth[2] = {fz_nth, kZsNthX};
+  for (int j = 0; j < 2; ++j) {
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[j], ks[j], nth[j], smem[j]);
     if (e != cudaSuccess) return e;
     if (occ[j] < 1) occ[j] = 1;
@@ -123,10 +116,6 @@ cudaError_t zs_fz_launch(int w, int nth, int grid, size_t smem, cudaStream_t st,
 cudaError_t zs_fx_launch(int w, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
   return zs_launch(kZsFx[w == 16 ? 1 : 0], kZsNthX, grid, smem, st, a);
 }
-cudaError_t zs_adj_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
-  return zs_launch(kZsAdj[(w == 16 ? 1 : 0) + (nth == kZsNth ? 0 : 2)], nth, grid, smem, st, a);
-}
-
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz) {
   k_to_iz<<<dim3((g.nx + 31) / 32, g.ny, (g.nzp + 31) / 32), dim3(32, 8), 0, st>>>(g, img, iz);
   return cudaGetLastError();

@@ -11,13 +11,9 @@
 //   k_zs_fx  item (slot, depth chunk, tile of tz rows): per plane the rows of
 //            Q (loaded one plane ahead into registers), x pass accumulated
 //            over the chunk -> part[slot][chunk][z][x]
-// adjoint (backproject!, src/backproject.jl:69-124), convolution half:
-//   k_zs_adj item (slot, tile of tx columns, depth chunk): the view's columns
-//            of the tile and its halo once; per plane the x pass, the z pass
-//            times the attenuation -> T[slot][y][x][nzp]
-// Every output goes through the operations of the fused kernels in the same
-// order (z then x in the forward, x then z in the adjoint), so the two paths
-// agree bit for bit.
+// The adjoint is k_zadj (zpath.cuh) on row tiles.  Every output goes through
+// the operations of the fused kernels in the same order (z then x), so the
+// two paths agree bit for bit.
 #pragma once
 #include "zpath.cuh"
 
@@ -48,14 +44,14 @@ __device__ __forceinline__ void zs_geometry(const ZGeom& g, float4 r, int x, int
   *o_out = ((j2 + g.pad) * g.L + j1 + g.pad) * g.nzp;
 }
 
-// one plane's pass table (weights hs | tails or folds ts | ranges 4 ints)
-// into shared memory: half 0 = forward, 1 = adjoint
-__device__ __forceinline__ void zs_table(const ZArgs& a, int set, int y, int half, float* Wt, int tid, int nth) {
+// one plane's forward pass table (weights hs | tails ts | ranges 4 ints) into
+// shared memory
+__device__ __forceinline__ void zs_table(const ZArgs& a, int set, int y, float* Wt, int tid, int nth) {
   const int hs = a.g.hs, ts = a.g.ts;
-  const float* Hrow = a.H + ((size_t)set * a.g.ny + y) * (2 * hs) + half * hs;
-  const float* Erow = a.E + ((size_t)set * a.g.ny + y) * (2 * ts) + half * ts;
+  const float* Hrow = a.H + ((size_t)set * a.g.ny + y) * hs;
+  const float* Erow = a.E + ((size_t)set * a.g.ny + y) * ts;
   for (int k = tid; k < hs + ts; k += nth) Wt[k] = k < hs ? Hrow[k] : Erow[k - hs];
-  if (tid < 4) reinterpret_cast<int*>(Wt + hs + ts)[tid] = a.R[((size_t)set * a.g.ny + y) * 8 + 4 * half + tid];
+  if (tid < 4) reinterpret_cast<int*>(Wt + hs + ts)[tid] = a.R[((size_t)set * a.g.ny + y) * 4 + tid];
 }
 
 // ------------------------------------------------------------------------
@@ -80,7 +76,7 @@ __global__ void __launch_bounds__(NTH) k_zs_fz(ZArgs a) {
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     const int xt = item % ntx, sy = item / ntx, slot = sy / ny, y = sy - slot * ny, X0 = xt * tx;
     const int v = a.vidx[slot], set = a.viewset[v];
-    zs_table(a, set, y, 0, Wt, tid, NTH);
+    zs_table(a, set, y, Wt, tid, NTH);
     if (tid < tx) zs_geometry(g, a.rot[v], X0 + tid, y, &geoW[tid], &geoO[tid]);
     __syncthreads();
     // rotated, attenuated columns into ZB (column x, rows R0 + z), two units a round
@@ -185,7 +181,7 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
         const int z = zdiv(e, rn4), c = e - z * n4;
         st4(base + z * bs + C0 + 4 * c, ld4(Qp + (size_t)z * nx + 4 * c));
       }
-      zs_table(a, set, y0, 0, base + tz * bs, tid, NTH);
+      zs_table(a, set, y0, base + tz * bs, tid, NTH);
     }
     __syncthreads();
     float acc[W];
@@ -239,7 +235,7 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
             st4(XN + z * bs + C0 + 4 * c, pf[j]);
           }
         }
-        zs_table(a, set, y + 1, 0, XN + tz * bs, tid, NTH);
+        zs_table(a, set, y + 1, XN + tz * bs, tid, NTH);
       }
       __syncthreads();
     }
@@ -247,100 +243,6 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
       float* o = a.part + (((size_t)slot * a.nchunks + ch) * nz + Z0 + zl) * nx + x0;
 #pragma unroll
       for (int k = 0; k < W; k += 4) st4(o + k, make_float4(acc[k], acc[k + 1], acc[k + 2], acc[k + 3]));
-    }
-  }
-}
-
-// ------------------------------------------------------------------------
-// k_zs_adj<NTH, W>: adjoint convolution of a tile of tx columns; item =
-// (slot, column tile, depth chunk).  The view's columns X0 - C0 .. X0 + tx +
-// xpw - C0 (zero outside the image) are loaded once per item as the tile's
-// zero-padded lines, the same values at the same shifted positions as
-// k_zadj's full rows; per plane the x pass (tx / W tasks a row) -> WB, the z
-// pass times the attenuation -> T.  Shared memory (floats): [VB nz * tbs]
-// [WB tx * ast: column x, data rows R0..][table hs + ts + 4], tbs =
-// zstride4(tx + xpw).
-template <int NTH, int W>
-__global__ void __launch_bounds__(NTH) k_zs_adj(ZArgs a) {
-  extern __shared__ float4 smem4[];
-  const ZGeom& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, tx = a.tx;
-  const int ast = g.ast, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx, tbs = zstride4(tx + g.xpw);
-  float* const VB = reinterpret_cast<float*>(smem4);
-  float* const WB = VB + (size_t)nz * tbs;
-  float* const Wt = WB + (size_t)tx * ast;
-  const int tid = threadIdx.x;
-  const int ntx = nx / tx, nitems = a.nv * ntx * a.nchunks, nzb = (nz + W - 1) / W;
-  const int xbs = tx / W, xtasks = nz * xbs, ztasks = tx * nzb;
-  const float rnz = 1.0f / nz, rtx = 1.0f / tx, rtbs = 1.0f / tbs;
-  for (int k = tid; k < tx * ast; k += NTH) WB[k] = 0.f;  // rows outside the data stay zero
-  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const int ch = item % a.nchunks, st = item / a.nchunks, slot = st / ntx, xt = st - slot * ntx;
-    const int X0 = xt * tx, y0 = ch * a.chunkY, y1 = min(ny, y0 + a.chunkY);
-    const int v = a.vidx[slot], set = a.viewset[v];
-    // the tile's lines: VB[z][c] = view[z][X0 + c - C0] inside the image, else
-    // zero (the previous item's last pass ended at a barrier)
-    const float* V = a.views + (size_t)slot * nz * nx;
-    for (int e = tid; e < nz * tbs; e += NTH) {
-      const int z = zdiv(e, rtbs), c = e - z * tbs, xg = X0 + c - C0;
-      VB[e] = (xg >= 0 && xg < nx) ? V[(size_t)z * nx + xg] : 0.f;
-    }
-    for (int y = y0; y < y1; ++y) {
-      zs_table(a, set, y, 1, Wt, tid, NTH);
-      __syncthreads();
-      // x pass: task (z, x block) -> WB column x, row R0 + z
-      {
-        const int2 rg = *reinterpret_cast<const int2*>(Wt + hs + ts + 2);
-        const float* cLx = Wt + hs;
-        const float* cRx = cLx + hx;
-        for (int t = tid; t < xtasks; t += NTH) {
-          const int xb = zdiv(t, rnz), z = t - xb * nz, x0 = W * xb;
-          const float* row = VB + z * tbs;
-          float o[W];
-#pragma unroll
-          for (int k = 0; k < W; ++k) o[k] = 0.f;
-          zpassw<W>(Wt + g.zpw, rg.x, rg.y, row + x0, o);
-          if (X0 + x0 == 0) o[0] += zfold(cLx, row + C0, 1, hx);
-          if (X0 + x0 + W == nx) o[W - 1] += zfold(cRx, row + C0 + x0 + W - 1, -1, hx);
-          float* w = WB + x0 * ast + R0 + z;
-#pragma unroll
-          for (int k = 0; k < W; ++k) w[k * ast] = o[k];
-        }
-      }
-      __syncthreads();
-      // z pass: task (x, z block) -> T column (X0 + x, y) of the slot
-      {
-        const int2 rg = *reinterpret_cast<const int2*>(Wt + hs + ts);
-        const float* cLz = Wt + hs + 2 * hx;
-        const float* cRz = cLz + hz;
-        const float* attv = a.att + (((size_t)v * ny + y) * nx + X0) * nzp;
-        float* Tp = a.T + (((size_t)slot * ny + y) * nx + X0) * nzp;
-        for (int t = tid; t < ztasks; t += NTH) {
-          const int zb = zdiv(t, rtx), x = t - zb * tx, z0 = W * zb;
-          float4 at[W / 4];
-#pragma unroll
-          for (int k = 0; k < W / 4; ++k) at[k] = ld4(attv + (size_t)x * nzp + z0 + 4 * k);
-          const float* col = WB + x * ast;
-          float o[W];
-#pragma unroll
-          for (int k = 0; k < W; ++k) o[k] = 0.f;
-          zpassw<W>(Wt, rg.x, rg.y, col + z0, o);
-          if (z0 == 0) o[0] += zfold(cLz, col + R0, 1, hz);
-          if (z0 <= nz - 1 && nz - 1 < z0 + W) {
-            const int kz = nz - 1 - z0;
-            const float s = zfold(cRz, col + R0 + nz - 1, -1, hz);
-#pragma unroll
-            for (int k = 0; k < W; ++k)
-              if (k == kz) o[k] += s;
-          }
-          float* dst = Tp + (size_t)x * nzp + z0;
-#pragma unroll
-          for (int k = 0; k < W / 4; ++k)
-            st4(dst + 4 * k, make_float4(__fmul_rn(at[k].x, o[4 * k]), __fmul_rn(at[k].y, o[4 * k + 1]),
-                                         __fmul_rn(at[k].z, o[4 * k + 2]), __fmul_rn(at[k].w, o[4 * k + 3])));
-        }
-      }
-      __syncthreads();
     }
   }
 }

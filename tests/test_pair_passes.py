@@ -1,0 +1,114 @@
+"""The pair-pass kernels (csrc/zpath.cuh) checked on the CPU: the index
+arithmetic of their tiles stays inside their buffers, and their walk over
+(slot, row tile, depth) planes covers every plane once.
+
+Mirrors of zadj_tile and ztable_floats (csrc/zpath_api.h); the geometry is
+zgeom of test_fused_math.
+"""
+import math
+
+import pytest
+
+from test_fused_math import zgeom, zround
+
+OPTIN = 232448
+NTH = 640
+X = 8  # outputs of an x-pass task
+
+
+def zstride2(v):
+    r = zround(v, 2)
+    return r if (r // 2) % 2 == 1 else r + 2
+
+
+def zadj_tile(g, optin=OPTIN):
+    nx, nz = g["nx"], g["nz"]
+    trow = 2 * g["hs"] + g["ts"] + 4
+    best, bc = None, 0.0
+    for w in (16, 8):
+        for nt in range(1, (nz + 1) // 2 + 1):
+            t = dict(w=w, tz=zround((nz + nt - 1) // nt, 8 if nt > 1 else 2))
+            t["ntile"] = (nz + t["tz"] - 1) // t["tz"]
+            if t["ntile"] != nt:
+                continue
+            t["vst"] = zstride2(w * ((t["tz"] + w - 1) // w) + g["zpw"])
+            t["bst"] = zstride2(X * ((nx + X - 1) // X) + g["xpw"])
+            zt = nx // 2 * ((t["tz"] + w - 1) // w)
+            xt = t["tz"] // 2 * ((nx + X - 1) // X)
+            most = zt if w == 16 else max(zt, xt)
+            rounds = (most + NTH - 1) // NTH
+            t["nth"] = zround((most + rounds - 1) // rounds, 32)
+            for nxb in (1, 2):
+                smem = 4 * (2 * (nx // 2 * t["vst"] + nxb * (t["tz"] // 2) * t["bst"]) + 3 * trow)
+                if smem > optin:
+                    continue
+                occ = min((optin + 1024) // (smem + 1024), NTH // t["nth"], 16)
+                if nxb > 1 and occ > 1:
+                    continue
+                warps = occ * t["nth"] / 32
+                rz, rx = math.ceil(zt / t["nth"]), math.ceil(xt / t["nth"])
+                c = t["ntile"] * t["nth"] * (rz * w * (1.15 if w == 8 else 1.0) + rx * X * 1.15)
+                c *= max(1.0, 16 / warps) * (1.0 if occ > 1 or nxb > 1 else 1.25)
+                if best is None or c < bc:
+                    best, bc = dict(t, nxb=nxb, smem=smem, occ=occ), c
+    return best
+
+
+SIZES = [(128, 80, 37, 37), (64, 64, 11, 11), (64, 40, 19, 19), (96, 48, 21, 21), (128, 128, 37, 37), (16, 12, 5, 3),
+         (64, 1, 11, 1), (128, 1, 11, 1), (256, 200, 65, 65), (64, 90, 21, 21), (40, 37, 9, 9), (8, 5, 5, 5),
+         (512, 96, 21, 21), (256, 17, 63, 3), (24, 230, 7, 65)]
+
+
+@pytest.mark.parametrize("nx,nz,px,pz", SIZES)
+def test_adjoint_tile_bounds(nx, nz, px, pz):
+    g = zgeom(nx, nz, px, pz)
+    t = zadj_tile(g)
+    assert t is not None and t["smem"] <= OPTIN and 32 <= t["nth"] <= NTH and t["occ"] * t["nth"] <= NTH
+    W, tz, vst, bst = t["w"], t["tz"], t["vst"], t["bst"]
+    assert tz % 2 == 0 and tz * t["ntile"] >= nz > tz * (t["ntile"] - 1)
+    assert vst % 2 == 0 and (vst // 2) % 2 == 1 and bst % 2 == 0 and (bst // 2) % 2 == 1
+    R0, C0, hz, hx, nzp = g["R0"], g["C0"], g["hz"], g["hx"], zround(nz, 16)
+    vlen = W * ((tz + W - 1) // W) + g["zpw"]
+    assert vlen <= vst and R0 >= hz and C0 >= hx
+    for tile in range(t["ntile"]):
+        Z0 = tile * tz
+        rows = min(tz, nz - Z0)
+        zb = (rows + W - 1) // W
+        # z windows and folds stay inside the loaded line
+        assert W * (zb - 1) + g["zpw"] + W <= vlen
+        if Z0 == 0 and hz:
+            assert R0 + hz - 1 < vlen
+        last = nz - 1 - Z0
+        if last < W * zb:
+            assert 0 <= R0 + last - (hz - 1) and R0 + last < vlen
+        # row pairs stored by the z pass are those the x pass reads, inside XB and the T column
+        pairs = {(z0 + 2 * m) // 2 for z0 in range(0, W * zb, W) for m in range(W // 2) if z0 + 2 * m < rows}
+        assert pairs == set(range((rows + 1) // 2)) and max(pairs) < tz // 2
+        assert Z0 + 2 * max(pairs) + 1 < nzp
+    # x windows, data columns and folds stay inside a row
+    nxw = (nx + X - 1) // X
+    assert C0 % 2 == 0 and C0 + nx <= bst and X * (nxw - 1) + g["xpw"] + X <= bst
+    assert C0 + hx - 1 < bst and C0 + nx - 1 - (hx - 1) >= 0
+    assert g["hs"] % 8 == 0 and (2 * g["hs"] + g["ts"] + 4) % 4 == 0
+
+
+@pytest.mark.parametrize("n,grid", [(1920, 296), (80 * 128, 740), (7, 7), (5, 148), (1, 1), (8 * 5 * 256, 148)])
+def test_plane_walk_covers_once(n, grid):
+    spans = [(b * n // grid, (b + 1) * n // grid) for b in range(grid)]
+    assert [q for a, b in spans for q in range(a, b)] == list(range(n))
+    assert max(b - a for a, b in spans) - min(b - a for a, b in spans) <= 1
+
+
+@pytest.mark.parametrize("ny", [2, 4, 8, 40, 64, 96, 128, 256, 512, 90, 46])
+def test_depth_step_visits_every_depth(ny):
+    s = max(1, int(0.618 * ny))
+    while math.gcd(s, ny) != 1:
+        s += 1
+    assert s < ny or ny == 2 and s == 1
+    y, seen = 0, []
+    for _ in range(ny):
+        seen.append(y)
+        y += s
+        if y >= ny:
+            y -= ny
+    assert sorted(seen) == list(range(ny))
