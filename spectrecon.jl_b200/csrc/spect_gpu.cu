@@ -2517,6 +2517,7 @@ struct spect_server_s {
   std::unordered_map<long long, ServerJob*> jobs;
   long long next_ticket = 1;
   size_t used = 0;
+  int admitting = 0;  // jobs whose plan a scheduler thread is building (their memory is taken)
   bool stop = false;
   long long n_submitted = 0, n_done = 0, n_failed = 0, max_active_seen = 0;
   // scheduler threads: each admits and retires jobs; while one prepares a
@@ -2676,6 +2677,10 @@ void server_loop(spect_server_s* S) {
       if (S->used + j->est > S->budget) break;  // wait for memory to free up
       S->pending.pop_front();
       S->used += j->est;
+      // jobs that hold device memory at once, those being prepared included (a
+      // short job may finish before the next one's plan stands)
+      ++S->admitting;
+      S->max_active_seen = std::max<long long>(S->max_active_seen, (long long)S->active.size() + S->admitting);
       lk.unlock();
       j->t_admit = Clock::now();
       const int rc = job_admit(S, j, S->budget);
@@ -2685,6 +2690,7 @@ void server_loop(spect_server_s* S) {
         job_release(S, j);
       }
       lk.lock();
+      --S->admitting;
       S->used -= j->est;
       if (rc != SPECT_OK) {
         j->state = 3;
@@ -2697,7 +2703,6 @@ void server_loop(spect_server_s* S) {
       S->used += j->bytes;
       j->state = 1;
       S->active.push_back(j);
-      S->max_active_seen = std::max<long long>(S->max_active_seen, (long long)S->active.size());
     }
     if (S->stop && S->active.empty()) break;
     if (S->active.empty() && S->pending.empty()) {
