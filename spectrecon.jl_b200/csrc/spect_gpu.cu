@@ -235,10 +235,9 @@ struct spect_plan_s {
   float* d_Hz = nullptr;       // [nset][ny][hs] forward pass weights
   float* d_Ez = nullptr;       // [nset][ny][ts] forward tails
   int* d_Rz = nullptr;         // [nset][ny][4] tap-block ranges of the forward passes
-  float* d_Zt = nullptr;       // [nset][ny][ztable_floats] adjoint pass tables
-  ZTile zat{};                 // tiling of k_zadj
+  float* d_Zt = nullptr;       // [nset][ny][2][ztable_floats] pass tables: forward, adjoint
+  ZTile zat{}, zft{};          // tilings of k_zadj, k_zfwd
   double ztaps[2] = {0, 0};    // mean kept taps per plane of the fused passes (z, x)
-  int zshape_fwd = -1;
   // large-plane kernels (zpath == 2): task width, column / row tiles, shared
   // memory and resident blocks per SM of k_zs_fz, k_zs_fx, and the forward's
   // plane-tile exchange buffer
@@ -250,7 +249,7 @@ struct spect_plan_s {
   // planes are transposed into d_Tz (z fastest) and gathered into d_backIZ
   int gadj = 0;
   float* d_Tz = nullptr;
-  size_t zfwd_smem_b = 0;
+  int part_cap = 0;            // partial views that d_part holds (fused paths)
   size_t bytes = 0;
   // stream on which the plan is built and its buffers are (de)allocated;
   // async_alloc: cudaMallocAsync/cudaFreeAsync on it (no device-wide sync)
@@ -556,51 +555,54 @@ ZArgs zargs(const spect_plan_s* p) {
   a.E = p->d_Ez;
   a.R = p->d_Rz;
   a.tab = p->d_Zt;
-  a.t = p->zat;
   a.rot = p->d_rot;
   a.viewset = p->d_viewset;
   a.err = p->d_err;
   return a;
 }
 
+// blocks of the forward walk over nv views with room for cap partial views
+// (block + slot).  The fused and the large-plane kernels share the walk, so
+// their partial sums agree bit for bit.
+int zwalk_blocks(const spect_plan_s* p, int nv, int cap) {
+  const long long n = (long long)nv * p->ny;
+  long long G = (long long)p->sm_count * std::max(1, p->zft.occ);
+  G = std::min(G, std::max(1LL, (n + 1) / 2));  // two planes a block at least
+  return (int)std::max(1LL, std::min<long long>(G, cap - nv));
+}
+
 // zpath forward of nidx views of the IZ image: k_zfwd (rotation, attenuation,
-// convolution, depth sum of chunks) then the chunk sum (+ EM ratio y/(Ax+bg))
+// convolution, depth sum of a block's planes) then the sum of the partial
+// views (+ EM ratio y/(Ax+bg)); partbuf holds cap partial views
 int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx, int nidx, cudaStream_t st,
-             const float* y, const float* bg, float* partbuf, int gmax) {
+             const float* y, const float* bg, float* partbuf, int cap, int gmax) {
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
     const int nv = std::min(gmax, nidx - g0);
     const int* vi = vidx + g0;
-    int cy, nc;
     ZArgs a = zargs(p);
+    a.t = p->zft;
     a.img = imgIZ;
     a.vidx = vi;
     a.nv = nv;
     a.part = partbuf;
+    a.G = zwalk_blocks(p, nv, cap);
     if (p->zpath == 2) {  // large planes: gather + z pass -> Q, x pass + depth sum -> part
-      // the fused kernel's depth chunks: the same partial sums, bit for bit
       const int ntz = cdiv(p->nz, p->zs_tz);
-      chunking(p, nv, false, &cy, &nc);
-      a.chunkY = cy;
-      a.nchunks = nc;
       a.Q = p->d_Q;
       a.tx = p->zs_tx;
       a.tz = p->zs_tz;
-      const int n1 = nv * p->ny * (p->nx / p->zs_tx), n2 = nv * nc * ntz;
+      const int n1 = nv * p->ny * (p->nx / p->zs_tx), n2 = (a.G + nv) * ntz;
       LAUNCH(p, K_CONV_FWD, st, "k_zs_fz",
              zs_fz_launch(p->zs_w, p->zs_fz_nth, std::min(n1, p->sm_count * p->zs_occ[0]), p->zs_smem[0], st, a));
       LAUNCH(p, K_CONV_FWD, st, "k_zs_fx",
              zs_fx_launch(p->zs_w, std::min(n2, p->sm_count * p->zs_occ[1]), p->zs_smem[1], st, a));
     } else {
-      chunking(p, nv, false, &cy, &nc);
-      a.chunkY = cy;
-      a.nchunks = nc;
-      const int gs = std::min(p->sm_count, nv * nc);
-      LAUNCH(p, K_CONV_FWD, st, "k_zfwd", zfwd_launch(p->zshape_fwd, gs, p->zfwd_smem_b, st, a));
+      LAUNCH(p, K_CONV_FWD, st, "k_zfwd", zfwd_launch(a.G, st, a));
     }
-    const size_t n = (size_t)nv * p->nxz;
+    const size_t n = (size_t)nv * p->nxz / (p->nxz % 4 == 0 ? 4 : 1);
     const int rb = (int)std::min<size_t>((n + 255) / 256, (size_t)p->sm_count * 16);
-    LAUNCH(p, K_REDUCE_VIEWS, st, "k_reduce_views",
-           k_reduce_views<<<rb, 256, 0, st>>>(partbuf, nv, nc, (int)p->nxz, views + (size_t)g0 * p->nxz, y, bg, vi));
+    LAUNCH(p, K_REDUCE_VIEWS, st, "k_reduce_parts",
+           zreduce_launch(rb, st, partbuf, nv, p->ny, a.G, (int)p->nxz, views + (size_t)g0 * p->nxz, y, bg, vi));
   }
   return SPECT_OK;
 }
@@ -624,6 +626,7 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
     a.T = p->d_P;
     a.vidx = vi;
     a.nv = nv;
+    a.t = p->zat;
     const int gs = (int)std::min<long long>((long long)p->sm_count * p->zat.occ, (long long)nv * p->zat.ntile * p->ny);
     LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
@@ -637,10 +640,10 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
 // forward projection of nidx views (device index list vidx) into views;
 // with y/bg non-null the output is the EM ratio y/(A x + bg).
 int forward_scratch(spect_plan_s* p, float* views, const float* image, const int* vidx, int nidx, cudaStream_t st,
-                    const float* y, const float* bg, float* Pbuf, float* partbuf, int gmax) {
+                    const float* y, const float* bg, float* Pbuf, float* partbuf, int cap, int gmax) {
   if (p->zpath) {
     LAUNCH(p, K_OTHER, st, "k_to_iz", zto_iz_launch(p->zg, st, image, p->d_imgIZ));
-    return zforward(p, views, p->d_imgIZ, vidx, nidx, st, y, bg, partbuf, gmax);
+    return zforward(p, views, p->d_imgIZ, vidx, nidx, st, y, bg, partbuf, cap, gmax);
   }
   const Geom& g = p->g;
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
@@ -710,7 +713,7 @@ int forward_scratch(spect_plan_s* p, float* views, const float* image, const int
 
 int forward(spect_plan_s* p, float* views, const float* image, const int* vidx, int nidx, cudaStream_t st,
             const float* y, const float* bg) {
-  return forward_scratch(p, views, image, vidx, nidx, st, y, bg, p->d_P, p->d_part, p->gmax);
+  return forward_scratch(p, views, image, vidx, nidx, st, y, bg, p->d_P, p->d_part, p->part_cap, p->gmax);
 }
 
 // back-projection of nidx views.  mode 0: image = A' views; mode 1: image =
@@ -895,7 +898,7 @@ int enqueue_osem(spect_plan_s* p, float* out, const float* x0, const float* y, c
     for (int it = 0; it < niter; ++it)
       for (int b = 0; b < nblocks; ++b) {
         const int* vi = p->d_sub + (size_t)b * nsub;
-        STATUS_TRY(zforward(p, p->d_views_tmp, p->d_imgIZ, vi, nsub, st, y, bg, p->d_part, p->gmax));
+        STATUS_TRY(zforward(p, p->d_views_tmp, p->d_imgIZ, vi, nsub, st, y, bg, p->d_part, p->part_cap, p->gmax));
         STATUS_TRY(zbackward(p, p->d_imgIZ, p->d_views_tmp, vi, nsub, st, 2, p->d_imgIZ,
                              p->d_asum + (size_t)b * p->izN));
       }
@@ -962,7 +965,6 @@ int static_scratch_address(void** out) {
 struct TuneResult {
   int fwd_cy, adj_cy, rotf_nsplit, nsplit_adj, sep, sep_adj;
   double fwd_ms, adj_ms;
-  int zshape_fwd;
 };
 std::mutex g_tune_mu;
 std::vector<std::pair<std::string, TuneResult>> g_tune_cache;
@@ -974,8 +976,6 @@ std::string tune_key(const spect_plan_s* p, int nv) {
          "/s" + std::to_string(p->sep_fwd_ok) + std::to_string(p->sep_adj_ok) + std::to_string(p->sep_forced) +
          "/z" + std::to_string(p->zpath) + "/y" + std::to_string(p->ny);
 }
-
-bool zshape_allowed(const ZGeom& g, int i);
 
 int time_pass(spect_plan_s* p, bool adj, int nv, int reps, double* ms) {
   cudaStream_t st = p->home;
@@ -1013,7 +1013,6 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
         p->nsplit_adj = kv.second.nsplit_adj;
         p->sep = kv.second.sep && p->sep_fwd_ok;
         p->sep_adj = kv.second.sep_adj && p->sep_adj_ok;
-        if (p->zpath == 1) p->zshape_fwd = kv.second.zshape_fwd;
         *fwd_ms = kv.second.fwd_ms;
         *adj_ms = kv.second.adj_ms;
         return SPECT_OK;
@@ -1034,9 +1033,9 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
     int c = best_chunk(p, nv, c0);
     if (std::find(cys.begin(), cys.end(), c) == cys.end()) cys.push_back(c);
   }
-  if (p->zpath == 2) {
-    // large-plane kernels: their tiles and chunks are fixed by the geometry;
-    // the timings are recorded for the caller
+  if (p->zpath) {
+    // fused paths: their tilings are fixed by the geometry; the timings are
+    // recorded for the caller
     double tf = 0, ta = 0;
     int rc = time_pass(p, false, nv, 2, &tf);
     if (rc == SPECT_OK) rc = time_pass(p, true, nv, 2, &ta);
@@ -1044,40 +1043,8 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
     if (rc != SPECT_OK) return rc;
     *fwd_ms = tf;
     *adj_ms = ta;
-    return SPECT_OK;
-  }
-  if (p->zpath) {
-    // fused path: the forward's depth tile and launch shape (the adjoint's
-    // tiling is fixed by the geometry)
-    std::vector<int> fsh;
-    for (int i = 0; i < kZNShapes; ++i) {
-      const int cap = kZShapes[i].nt * kZShapes[i].nth, xtasks = p->nz * (p->nx / kZShapes[i].w);
-      if (zshape_allowed(p->zg, i) && cap >= xtasks && cap <= 2 * xtasks) fsh.push_back(i);
-    }
-    if (fsh.empty()) fsh.push_back(p->zshape_fwd);
-    double bf = 1e300, ba = 0;
-    int bcy = cys[0], bsf = p->zshape_fwd, rc = SPECT_OK;
-    for (int sh : fsh)
-      for (int cy : cys) {
-        p->zshape_fwd = sh;
-        p->tune_fwd_cy = cy;
-        double t;
-        if ((rc = time_pass(p, false, nv, 2, &t)) != SPECT_OK) break;
-        if (t < bf) {
-          bf = t;
-          bcy = cy;
-          bsf = sh;
-        }
-      }
-    p->zshape_fwd = bsf;
-    p->tune_fwd_cy = bcy;
-    if (rc == SPECT_OK) rc = time_pass(p, true, nv, 2, &ba);
-    p->prof.on = prof;
-    if (rc != SPECT_OK) return rc;
-    *fwd_ms = bf;
-    *adj_ms = ba;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache.push_back({key, TuneResult{bcy, 0, 0, 1, p->sep, p->sep_adj, bf, ba, bsf}});
+    g_tune_cache.push_back({key, TuneResult{0, 0, 0, 1, p->sep, p->sep_adj, tf, ta}});
     return SPECT_OK;
   }
   // convolution kernels to try: direct (separable planes) and FFT, unless
@@ -1139,7 +1106,7 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
   *fwd_ms = bf;
   *adj_ms = ba;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache.push_back({key, TuneResult{bcy, bacy, brs, bns, bsep, basep, bf, ba, -1}});
+  g_tune_cache.push_back({key, TuneResult{bcy, bacy, brs, bns, bsep, basep, bf, ba}});
   return SPECT_OK;
 }
 
@@ -1440,30 +1407,6 @@ bool zs_tiles(const ZGeom& g, size_t optin, ZsTiles* t) {
   return zs_fz_smem(g, t->tx) <= optin && zs_fx_smem(g, t->tz) <= optin;
 }
 
-// shapes allowed by the geometry and by SPECT_ZW=8|16 (fixes the task width)
-bool zshape_allowed(const ZGeom& g, int i) {
-  const char* e = std::getenv("SPECT_ZW");
-  const int force = e ? std::atoi(e) : 0;
-  return zshape_fits(g, i) && (force == 0 || kZShapes[i].w == force);
-}
-// forward: the widest tasks, then the least thread capacity holding all x
-// tasks (their outputs stay in registers), then more threads
-int zpick_fwd(const ZGeom& g) {
-  int best = -1;
-  for (int i = 0; i < kZNShapes; ++i) {
-    if (!zshape_allowed(g, i)) continue;
-    const ZShape& s = kZShapes[i];
-    const int cap = s.nt * s.nth;
-    if (cap < g.nz * (g.nx / s.w)) continue;
-    if (best < 0) {
-      best = i;
-      continue;
-    }
-    const ZShape& b = kZShapes[best];
-    if (s.w > b.w || (s.w == b.w && (cap < b.nt * b.nth || (cap == b.nt * b.nth && s.nth > b.nth)))) best = i;
-  }
-  return best;
-}
 int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, int nview, const float* mumap,
                      const float* psfs, float dy, const float* viewangle, int interpmeth, int mode, int nthread,
                      int nthreads, const PlanOpts& opts) {
@@ -1569,7 +1512,9 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
         zg.nzp <= 256 && opts.atten_cache != 0) {
       p->zat = zadj_tile(zg, (size_t)optin);
       const bool adj = p->zat.w != 0;
-      const bool fused = adj && zpick_fwd(zg) >= 0 && zfwd_smem(zg, 1) <= (size_t)optin;
+      p->zft = zfwd_tile(zg, (size_t)optin);
+      const bool fused = adj && p->zft.w != 0;
+      if (!fused) p->zft.ystep = zdepth_step(ny);  // the walk of the large-plane kernels
       const bool strip = adj && zs_tiles(zg, (size_t)optin, &zt);
       if (fused && !(senv && senv[0] == '1')) zkind = 1;
       else if (strip && !(senv && senv[0] == '0')) zkind = 2;
@@ -1623,13 +1568,6 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   if (p->zpath == 1) {
     p->zg = zg;
     p->izN = (size_t)zg.L * zg.L * zg.nzp;
-    p->zshape_fwd = zpick_fwd(zg);
-    // one forward staging buffer (SPECT_ZFWD_STAGES=2: two where they fit;
-    // measured slower at 128x128x80: the shared-memory carve-out takes L1
-    // from the gather's image reads)
-    const char* nsf_env = std::getenv("SPECT_ZFWD_STAGES");
-    p->zg.nsf = (zfwd_smem(zg, 2) <= p->max_smem && nsf_env && nsf_env[0] == '2') ? 2 : 1;
-    p->zfwd_smem_b = zfwd_smem(p->zg, p->zg.nsf);
     const cudaError_t ze = zpath_setup((int)p->max_smem);
     if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("fused kernel setup: ") + cudaGetErrorString(ze)));
   }
@@ -1663,7 +1601,9 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       (st = dalloc(p, &p->d_H, (size_t)p->nset * ny * (p->cg.Q + 1) * Npx)) ||
       (st = dalloc(p, &p->d_P, (size_t)p->gmax * slot)) ||
       (st = ((p->nchunk_max = ((size_t)p->gmax * 32 * p->nxz * 4 <= ((size_t)256 << 20)) ? 32 : 16),
-             dalloc(p, &p->d_part, (size_t)p->gmax * p->nchunk_max * p->nxz))) ||
+             p->part_cap = p->zpath ? std::max(p->gmax * p->nchunk_max, p->sm_count * std::max(1, p->zft.occ) + p->gmax)
+                                    : p->gmax * p->nchunk_max,
+             dalloc(p, &p->d_part, (size_t)p->part_cap * p->nxz))) ||
       (st = dalloc(p, &p->d_Vs, (size_t)p->gmax * p->cg.Q * Npx)) ||
       (st = dalloc(p, &p->d_imgpart, (size_t)p->nsplit_adj_max * p->N)))
     return bail(st);
@@ -1877,7 +1817,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       Hz.assign((size_t)p->nset * ny * zg.hs, 0.f);
       Ez.assign((size_t)p->nset * ny * zg.ts, 0.f);
       Rz.assign((size_t)p->nset * ny * 4, 0);
-      Zt.assign((size_t)p->nset * ny * zrow, 0.f);
+      Zt.assign((size_t)p->nset * ny * 2 * zrow, 0.f);
     }
     for (int u = 0; ok && u < p->nset; ++u)
       for (int y = 0; y < ny; ++y) {
@@ -1913,18 +1853,26 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
           tap_range(zr + zg.zpw, zg.xpw, rr + 2, rr + 3);
           for (int m = 0; m < pzk; ++m) p->ztaps[0] += bt[m] != 0.0 ? 1.0 : 0.0;
           for (int m = 0; m < pxk; ++m) p->ztaps[1] += at[m] != 0.0 ? 1.0 : 0.0;
-          // adjoint table: the weights twice each, folds, ranges
-          std::vector<float> row(zg.hs, 0.f);
-          for (int m = 0; m < pzk; ++m) row[sz + m] = (float)bt[m];
-          for (int m = 0; m < pxk; ++m) row[zg.zpw + sx + m] = (float)at[m];
-          float* tr = Zt.data() + pl * zrow;
-          for (int m = 0; m < zg.hs; ++m) tr[2 * m] = tr[2 * m + 1] = row[m];
-          fold_tails(at, zg.hx, tr + 2 * zg.hs, tr + 2 * zg.hs + zg.hx);
-          fold_tails(bt, zg.hz, tr + 2 * zg.hs + 2 * zg.hx, tr + 2 * zg.hs + 2 * zg.hx + zg.hz);
-          int ra[4];
-          tap_range4(row.data(), zg.zpw, ra, ra + 1);
-          tap_range4(row.data() + zg.zpw, zg.xpw, ra + 2, ra + 3);
-          std::memcpy(tr + 2 * zg.hs + zg.ts, ra, sizeof(ra));
+          // pass tables: the weights twice each, tails or folds, ranges
+          for (int d = 0; d < 2; ++d) {
+            std::vector<float> row(zg.hs, 0.f);
+            for (int m = 0; m < pzk; ++m) row[sz + m] = (float)bt[d ? m : pzk - 1 - m];
+            for (int m = 0; m < pxk; ++m) row[zg.zpw + sx + m] = (float)at[d ? m : pxk - 1 - m];
+            float* tr = Zt.data() + (pl * 2 + d) * zrow;
+            for (int m = 0; m < zg.hs; ++m) tr[2 * m] = tr[2 * m + 1] = row[m];
+            float* ft = tr + 2 * zg.hs;
+            if (d) {
+              fold_tails(at, zg.hx, ft, ft + zg.hx);
+              fold_tails(bt, zg.hz, ft + 2 * zg.hx, ft + 2 * zg.hx + zg.hz);
+            } else {
+              clamp_tails(bt, pzk, ft, ft + zg.hz);
+              clamp_tails(at, pxk, ft + 2 * zg.hz, ft + 2 * zg.hz + zg.hx);
+            }
+            int ra[4];
+            tap_range4(row.data(), zg.zpw, ra, ra + 1);
+            tap_range4(row.data() + zg.zpw, zg.xpw, ra + 2, ra + 3);
+            std::memcpy(ft + zg.ts, ra, sizeof(ra));
+          }
         }
       }
     if (!Hz.empty()) {
@@ -2056,7 +2004,8 @@ int spect_project_static_scratch(spect_plan_t p, float* views, const float* imag
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   const bool prof = p->prof.on;
   p->prof.on = false;  // no event creation on this path
-  int rc = forward_scratch(p, views, image, vi, nindex, st, nullptr, nullptr, Pbuf, partbuf, gmax);
+  int rc = forward_scratch(p, views, image, vi, nindex, st, nullptr, nullptr, Pbuf, partbuf, gmax * p->nchunk_max,
+                           gmax);
   p->prof.on = prof;
   return rc;
 }

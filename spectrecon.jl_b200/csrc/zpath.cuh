@@ -59,14 +59,12 @@
 #include "bulk_copy.cuh"
 #include "zpath_api.h"
 
-#ifndef ZFWD_GU
-#define ZFWD_GU 2
-#endif
-
 namespace spect {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+// four floats as two packed pairs
+__device__ __forceinline__ ulonglong2 ldp(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 // 8-byte read-only global load issued only where pred holds; (0, 0) elsewhere
 // (no memory access for those lanes).  p must be 8-byte aligned.
 __device__ __forceinline__ float2 ldg2_if(const float* p, bool pred) {
@@ -135,52 +133,84 @@ __device__ __forceinline__ int zdiv(int t, float r) { return (int)(((float)t + 0
 // FFMA falls to 49).  Weights are stored twice ((w, w)); taps run in blocks of
 // 4, m in [4 b4, 4 b4 + 4 n4) (n4 <= 18), in ascending order for every output:
 // the same result for every W, and for either lane as for a single line.
+using f2 = unsigned long long;  // two packed floats in one 64-bit register (pair)
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(f2 d) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(d));
+  return v;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 template <int W>
-__device__ __forceinline__ void zpass2(const float2* __restrict__ w, int b4, int n4, const float2* line,
-                                       float2 (&o)[W]) {
-  const float4* w4 = reinterpret_cast<const float4*>(w + 4 * b4);
-  const float4* l4 = reinterpret_cast<const float4*>(line + 4 * b4);
-  float2 e[W + 4 * 18];
+__device__ __forceinline__ void zpass2(const f2* __restrict__ w, int b4, int n4, const f2* line, f2 (&o)[W]) {
+  const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(w + 4 * b4);
+  const ulonglong2* l4 = reinterpret_cast<const ulonglong2*>(line + 4 * b4);
+  f2 e[W + 4 * 18];
 #pragma unroll
   for (int i = 0; i < W / 2; ++i) {
-    const float4 q = l4[i];
-    e[2 * i] = make_float2(q.x, q.y);
-    e[2 * i + 1] = make_float2(q.z, q.w);
+    const ulonglong2 q = l4[i];
+    e[2 * i] = q.x;
+    e[2 * i + 1] = q.y;
   }
 #pragma unroll
   for (int k = 0; k < 18; ++k) {
     if (k >= n4) break;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const float4 q = l4[2 * k + W / 2 + i];
-      e[4 * k + W + 2 * i] = make_float2(q.x, q.y);
-      e[4 * k + W + 2 * i + 1] = make_float2(q.z, q.w);
+      const ulonglong2 q = l4[2 * k + W / 2 + i];
+      e[4 * k + W + 2 * i] = q.x;
+      e[4 * k + W + 2 * i + 1] = q.y;
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float4 q = w4[2 * k + h];
+      const ulonglong2 q = w4[2 * k + h];
 #pragma unroll
-      for (int j = 0; j < W; ++j) o[j] = __ffma2_rn(make_float2(q.x, q.y), e[4 * k + 2 * h + j], o[j]);
+      for (int j = 0; j < W; ++j) o[j] = fma2(q.x, e[4 * k + 2 * h + j], o[j]);
 #pragma unroll
-      for (int j = 0; j < W; ++j) o[j] = __ffma2_rn(make_float2(q.z, q.w), e[4 * k + 2 * h + 1 + j], o[j]);
+      for (int j = 0; j < W; ++j) o[j] = fma2(q.y, e[4 * k + 2 * h + 1 + j], o[j]);
     }
   }
 }
 
 // sum_{k < n} c[k] v[step k] of a pair of lines: four partial sums over k mod
 // 4, added as (s0 + s1) + (s2 + s3), so a round waits for one load latency
-__device__ __forceinline__ float2 zfold2(const float* c, const float2* v, int step, int n) {
-  float2 s[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) s[j] = make_float2(0.f, 0.f);
+__device__ __forceinline__ f2 zfold2(const float* c, const f2* v, int step, int n) {
+  f2 s[4] = {0, 0, 0, 0};
   int k = 0;
   for (; k + 4 <= n; k += 4)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s[j] = __ffma2_rn(make_float2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
+    for (int j = 0; j < 4; ++j) s[j] = fma2(pack2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
 #pragma unroll
   for (int j = 0; j < 3; ++j)
-    if (k + j < n) s[j] = __ffma2_rn(make_float2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
-  return __fadd2_rn(__fadd2_rn(s[0], s[1]), __fadd2_rn(s[2], s[3]));
+    if (k + j < n) s[j] = fma2(pack2(c[k + j], c[k + j]), v[step * (k + j)], s[j]);
+  return add2(add2(s[0], s[1]), add2(s[2], s[3]));
+}
+
+// the outputs (2 m, 2 m + 1) of a task over the pair (a, b) of lines, as two
+// elements (line pairs of the other direction): (o[2m].a, o[2m+1].a),
+// (o[2m].b, o[2m+1].b)
+__device__ __forceinline__ float4 zturn(f2 p, f2 q) {
+  const float2 u = unpack2(p), v = unpack2(q);
+  return make_float4(u.x, v.x, u.y, v.y);
 }
 
 // fetch the 128-byte line of p into L2
@@ -327,275 +357,281 @@ __global__ void __launch_bounds__(256) k_zatten(ZGeom g, const float* __restrict
 }
 
 // ------------------------------------------------------------------------
-// k_zfwd<NT, NTH, W>: persistent forward, one block per SM, NTH threads; NT
-// x-pass tasks of W outputs per thread, all of a plane's x tasks resident
-// (NT * NTH >= nz * nx / W) since their outputs accumulate over the chunk.
-// The block walks its planes in sequence; the attenuation plane and weights
-// of the next nsf planes are bulk-copied while plane p is worked on (stage
-// q % nsf holds plane q).  Two block barriers per plane: phase A runs the z
-// pass of plane p (ZB -> XB) and the sample geometry of plane p + 1; phase B
-// the x pass of plane p (XB -> registers) and the gather of plane p + 1
-// (rotated, attenuated image -> ZB).
-template <int NT, int NTH, int W>
-__global__ void __launch_bounds__(NTH, 1) k_zfwd(ZArgs a) {
-  constexpr int GU = ZFWD_GU;  // gather units per thread and round (4 measured ~1 % faster, with spills in some shapes)
+// Walk over the depth planes of a group: plane q = (slot, j) of the slot-major
+// list of n = nv ny is depth y = j ystep mod ny of the slot's view (ystep
+// coprime to ny and near 0.618 ny: a short range of j holds narrow and wide
+// PSF planes alike), and block b of a grid of G owns planes [b n / G,
+// (b + 1) n / G).  The forward sums a block's planes of one slot into one
+// partial view, number b + slot (different for every pair that occurs).
+// k_reduce_parts adds a slot's partials in block order (+ the EM ratio
+// y / (A x + bg), src/ml-os-em.jl:38,119).
+__device__ __forceinline__ int zblock_of(long long q, int n, int G) { return (int)(((q + 1) * G - 1) / n); }
+
+// four view elements a thread where nxz % 4 == 0 (V = 4), else one
+template <int V>
+__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nv, int ny, int G, int nxz,
+                                                      float* __restrict__ out, const float* __restrict__ y,
+                                                      const float* __restrict__ bg, const int* __restrict__ vidx) {
+  const int per = nxz / V, n = nv * ny;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv * per; k += gridDim.x * blockDim.x) {
+    const int slot = k / per, e = V * (k - slot * per);
+    const int b0 = zblock_of((long long)slot * ny, n, G), b1 = zblock_of((long long)(slot + 1) * ny - 1, n, G);
+    const float* p = part + (size_t)(b0 + slot) * nxz + e;
+    float s[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) s[i] = 0.f;
+#pragma unroll 4
+    for (int b = b0; b <= b1; ++b, p += nxz) {
+      if constexpr (V == 4) {
+        const float4 q = ld4(p);
+        s[0] += q.x;
+        s[1] += q.y;
+        s[2] += q.z;
+        s[3] += q.w;
+      } else {
+        s[0] += p[0];
+      }
+    }
+    const size_t src = y ? (size_t)vidx[slot] * nxz + e : 0, dst = (size_t)slot * nxz + e;
+#pragma unroll
+    for (int i = 0; i < V; ++i) out[dst + i] = y ? y[src + i] / (s[i] + bg[src + i]) : s[i];
+  }
+}
+
+// ------------------------------------------------------------------------
+// k_zfwd<NT>: forward.  Per plane: the rotated, attenuated image columns 2 xp,
+// 2 xp + 1 as pair lines ZB (gather), the z pass -> rows 2 zp, 2 zp + 1 as
+// pair lines XB, the x pass accumulated in registers over the block's planes
+// of the view (NT tasks of X outputs a thread).  Two barriers a plane:
+// phase A runs the z pass of plane p and the sample geometry of plane p + 1,
+// phase B the x pass of plane p and the gather of plane p + 1; its table is
+// copied and its attenuation prefetched into L2 during phase A.  Small planes
+// take a few warps a block and several blocks an SM, so that one's barriers
+// and gather latency pass behind another's FMAs; tasks of 8 outputs keep a
+// thread at 96 registers, x outputs included (16 spilled them).
+// Bound: the shared-memory/L1 pipe (63 % busy at 128x128x80, 37 taps) and the
+// gather's L2 latency between the barriers; FFMA2 is 37 % of the
+// instructions.  Measured there: 15 views 107.7 -> 78.3 us, 120 views 695 ->
+// 573 us; 64x64x40, 19 taps, 60 views 107 -> 38 us; 128x128x1, 80 views 229 ->
+// 50 us (the former kernel staged the attenuation plane in shared memory, ran
+// one line a lane and one block per SM, and dealt chunks of 15 planes).
+// Shared memory: [2 tables][geoW nx x (w00 w00 w10 w10 | w01 w01 w11 w11)]
+// [geoO nx int][ZB nxp * vst][XB (nz + 1) / 2 * bst] (lines: float2).
+template <int NT>
+__global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
   extern __shared__ float4 smem4[];
+  constexpr int X = kZfwdX, W = kZfwdZ;
   const ZGeom& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nsf = g.nsf;
-  float* const base = reinterpret_cast<float*>(smem4);
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(base);  // nsf barriers
-  const int hts = hs + ts + 4;         // weights, tails, tap ranges of one plane (4 ints)
-  const int sts = nx * nzp + hts;      // stage: attenuation plane [x][nzp], then those
-  float* const stage = base + 4;
-  float* const Hw0 = stage + nsf * sts;           // working weights, tails, ranges: two planes
-  float4* const geoW = reinterpret_cast<float4*>(Hw0 + 2 * hts);
-  int* const geoO = reinterpret_cast<int*>(geoW + nx);
-  float* const ZB = reinterpret_cast<float*>(geoO + zround(nx, 4));  // [x][ast], data rows R0..R0+nz-1
-  float* const XB = ZB + (size_t)nx * g.ast;                          // [z][bs], data columns C0..C0+nx-1
-  const int tid = threadIdx.x;
-  const int nitems = a.nv * a.nchunks;
-  const float rnc = 1.0f / a.nchunks;
-  auto slot_of = [&](int item) { return zdiv(item, rnc); };             // item / nchunks (items < 2^20)
-  auto chunk_of = [&](int item) { return item - zdiv(item, rnc) * a.nchunks; };
-  const unsigned abytes = (unsigned)((size_t)nx * nzp * sizeof(float));
-  auto issue = [&](int item, int y, int s) {  // one thread: attenuation plane, weights, tails of plane y
-    const int sl = slot_of(item), v = a.vidx[sl], set = a.viewset[v];
-    float* sA = stage + s * sts;
-    float* sW = sA + nx * nzp;
-    fence_proxy_async();
-    mbar_expect(&bar[s], abytes + (unsigned)(hts * sizeof(float)));
-    bulk_copy(&bar[s], sA, a.att + ((size_t)v * ny + y) * nx * nzp, abytes);
-    bulk_copy(&bar[s], sW, a.H + ((size_t)set * ny + y) * hs, (unsigned)(hs * sizeof(float)));
-    bulk_copy(&bar[s], sW + hs, a.E + ((size_t)set * ny + y) * ts, (unsigned)(ts * sizeof(float)));
-    bulk_copy(&bar[s], sW + hs + ts, a.R + ((size_t)set * ny + y) * 4, 4u * sizeof(int));
-  };
-  auto next = [&](int& item, int& y) {
-    const int yend = min(ny, chunk_of(item) * a.chunkY + a.chunkY);
-    if (y + 1 < yend) {
-      ++y;
-    } else {
-      item += gridDim.x;
-      y = chunk_of(item) * a.chunkY;
-    }
-  };
-  // the padded buffers start zero; only their data rows / columns are written later
-  for (size_t k = tid; k < (size_t)nx * g.ast + (size_t)nz * g.bs; k += NTH) ZB[k] = 0.f;
-  int i0 = blockIdx.x, y0 = (blockIdx.x % a.nchunks) * a.chunkY;  // plane p
-  int i1 = i0, y1 = y0;
-  next(i1, y1);  // p + 1
-  int iq = i1, yq = y1;  // the next plane to issue
-  unsigned pend = 0u;    // stages with a copy issued and not yet waited for (same in every thread)
-  if (tid == 0) {
-    for (int s = 0; s < nsf; ++s) mbar_init(&bar[s]);
-    if (i0 < nitems) issue(i0, y0, 0);
-  }
-  pend = 1u;
-  if (nsf > 1) {
-    if (tid == 0 && iq < nitems) issue(iq, yq, 1);
-    if (iq < nitems) pend |= 2u;
-    next(iq, yq);
-  }
-  __syncthreads();
-  if (!(i0 < nitems)) return;
-  const int nzb = (nz + W - 1) / W, ztasks = nx * nzb, nz4 = (nz + 3) / 4, units = nx * nz4;
-  const int xtasks = nz * (nx / W);
+  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2, nzp2 = (nz + 1) / 2;
+  const int vst = a.t.vst, bst = a.t.bst, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
+  const int trow = ztable_floats(g), tid = threadIdx.x, nth = blockDim.x;
+  float* const tab0 = reinterpret_cast<float*>(smem4);
+  float4* const geoW = reinterpret_cast<float4*>(tab0 + 2 * trow);
+  int* const geoO = reinterpret_cast<int*>(geoW + 2 * nx);
+  f2* const ZB = reinterpret_cast<f2*>(geoO + zround(nx, 4));
+  f2* const XB = ZB + (size_t)nxp * vst;
+  const int n = a.nv * ny;
+  const int p0 = (int)((long long)blockIdx.x * n / gridDim.x), p1 = (int)((long long)(blockIdx.x + 1) * n / gridDim.x);
+  if (p0 >= p1) return;
   const size_t Lz = (size_t)g.L * nzp;
-  const int ast = g.ast, bs = g.bs, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
-  const int zpw = g.zpw;
-  const float rnx = 1.0f / nx, rnz = 1.0f / nz, rnz4 = 1.0f / nz4;
-  unsigned phases = 0u;  // parity of each barrier's next wait
-  // wait for stage s; false (every thread) when a wait gave up, after the
-  // copies in flight have landed
-  auto staged = [&](int s) {
-    const bool ok = mbar_wait(&bar[s], (phases >> s) & 1u);
-    if (ok) {
-      phases ^= 1u << s;
-      pend &= ~(1u << s);
-    }
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) {
-        atomicExch(a.err, 1);
-        for (int k = 0; k < nsf; ++k)
-          if ((pend >> k) & 1u) mbar_wait(&bar[k], (phases >> k) & 1u);
-      }
-      return false;
-    }
-    return true;
+  int slot = p0 / ny, j = p0 - slot * ny;
+  int y = (int)((long long)j * a.t.ystep % ny), v = a.vidx[slot];
+  auto table = [&](int view, int yy, int s) {  // every thread: its 16-byte pieces of the plane's table
+    if (4 * tid >= trow) return;
+    const float* src = a.tab + (((size_t)a.viewset[view] * ny + yy) * 2) * trow;
+    for (int k = 4 * tid; k < trow; k += 4 * nth) cp16(tab0 + s * trow + k, src + k);
   };
-  // sample geometry of plane (item, y), one rotated-grid column per thread:
-  // the position arithmetic of RotPos::pos with the view's (cos, sin)
-  auto geometry = [&](int item, int y) {
-    if (tid < nx) {
-      const float4 r = a.rot[a.vidx[slot_of(item)]];
-      int j1 = tid, j2 = y;
-      float4 w = make_float4(1.f, 0.f, 0.f, 0.f);
-      if (r.z == 0.f) {
-        const float cs = r.x, sn = r.y;
-        const float d1 = __fsub_rn((float)tid, g.c0), d2 = __fsub_rn((float)y, g.c0);
-        const float s1 = __fadd_rn(g.c0, __fsub_rn(__fmul_rn(cs, d1), __fmul_rn(sn, d2)));
-        const float s2 = __fadd_rn(g.c0, __fadd_rn(__fmul_rn(sn, d1), __fmul_rn(cs, d2)));
-        const float f1 = floorf(s1), f2 = floorf(s2);
-        const float t1 = __fsub_rn(s1, f1), t2 = __fsub_rn(s2, f2);
-        const float u1 = __fsub_rn(1.0f, t1), u2 = __fsub_rn(1.0f, t2);
-        j1 = (int)f1;
-        j2 = (int)f2;
-        w = make_float4(__fmul_rn(u1, u2), __fmul_rn(t1, u2), __fmul_rn(u1, t2), __fmul_rn(t1, t2));
-        if (j1 < -g.pad || j1 > nx + g.pad - 2 || j2 < -g.pad || j2 > nx + g.pad - 2) {
-          j1 = j2 = 0;
-          w = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-      geoW[tid] = w;
-      geoO[tid] = ((j2 + g.pad) * g.L + j1 + g.pad) * nzp;
+  auto geometry = [&](int view, int yy) {
+    if (tid >= nx) return;
+    const float4 r = a.rot[view];
+    for (int x = tid; x < nx; x += nth) {
+      float4 w;
+      int off;
+      zgeo(g, r.x, r.y, r.z != 0.f, x, yy, w, off);
+      geoW[2 * x] = make_float4(w.x, w.x, w.y, w.y);
+      geoW[2 * x + 1] = make_float4(w.z, w.z, w.w, w.w);
+      geoO[x] = off;
     }
   };
-  // staged weights of stage s into working buffer hb; rotated, attenuated
-  // plane into ZB (column x, rows R0 + z), four z at a time
-  auto gather = [&](int s, int hb) {
-    const float* const sA = stage + s * sts;
-    const float* const sW = sA + nx * nzp;
-    float* const Hw = Hw0 + hb * hts;
-    for (int k = tid; k < hs + ts; k += NTH) Hw[k] = sW[k];
-    if (tid < 4) reinterpret_cast<int*>(Hw + hs + ts)[tid] = reinterpret_cast<const int*>(sW + hs + ts)[tid];
-    // GU units per round, all their image loads issued before any is used
-    for (int u0 = tid; u0 < units; u0 += GU * NTH) {
-      float4 t[GU][4];
-      int xs[GU], zs[GU];
-#pragma unroll
-      for (int j = 0; j < GU; ++j) {
-        const int u = min(u0 + j * NTH, units - 1);  // a repeated last unit stores the same values
-        xs[j] = zdiv(u, rnz4);
-        zs[j] = u - xs[j] * nz4;
-        const float* p = a.img + geoO[xs[j]] + 4 * zs[j];
-        t[j][0] = ld4(p);
-        t[j][1] = ld4(p + nzp);
-        t[j][2] = ld4(p + Lz);
-        t[j][3] = ld4(p + Lz + nzp);
-      }
-#pragma unroll
-      for (int j = 0; j < GU; ++j) {
-        const float4 w = geoW[xs[j]];
-        const float4 at = ld4(sA + xs[j] * nzp + 4 * zs[j]);
-        const float4 t0 = t[j][0], t1 = t[j][1], t2 = t[j][2], t3 = t[j][3];
-        float4 o;
-        o.x = __fmul_rn(fmaf(w.w, t3.x, fmaf(w.z, t2.x, fmaf(w.y, t1.x, __fmul_rn(w.x, t0.x)))), at.x);
-        o.y = __fmul_rn(fmaf(w.w, t3.y, fmaf(w.z, t2.y, fmaf(w.y, t1.y, __fmul_rn(w.x, t0.y)))), at.y);
-        o.z = __fmul_rn(fmaf(w.w, t3.z, fmaf(w.z, t2.z, fmaf(w.y, t1.z, __fmul_rn(w.x, t0.z)))), at.z);
-        o.w = __fmul_rn(fmaf(w.w, t3.w, fmaf(w.z, t2.w, fmaf(w.y, t1.w, __fmul_rn(w.x, t0.w)))), at.w);
-        st4(ZB + xs[j] * ast + R0 + 4 * zs[j], o);
+  // rotated, attenuated column x at z group z4: four z as two packed pairs
+  const int nz4 = (nz + 3) / 4, dq = nth / nz4, dr = nth - dq * nz4, q0 = tid / nz4, r0 = tid - q0 * nz4;
+  auto sample = [&](const float* att, int x, int z4, f2& lo, f2& hi) {
+    const float* p = a.img + geoO[x] + 4 * z4;
+    const ulonglong2 t0 = ldp(p), t1 = ldp(p + nzp), t2 = ldp(p + Lz), t3 = ldp(p + Lz + nzp);
+    const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
+    const ulonglong2 wa = reinterpret_cast<const ulonglong2*>(geoW)[2 * x];  // (w00, w00), (w10, w10)
+    const ulonglong2 wb = reinterpret_cast<const ulonglong2*>(geoW)[2 * x + 1];
+    lo = mul2(fma2(wb.y, t3.x, fma2(wb.x, t2.x, fma2(wa.y, t1.x, mul2(wa.x, t0.x)))), at.x);
+    hi = mul2(fma2(wb.y, t3.y, fma2(wb.x, t2.y, fma2(wa.y, t1.y, mul2(wa.x, t0.y)))), at.y);
+  };
+  const int hi4 = (tid >> 2) & 1;
+  auto gather = [&](int view, int yy) {  // unit (column pair, z group)
+    const float* att = a.att + (((size_t)view * ny + yy) * nx) * nzp;
+    for (int xp = q0, z4 = r0; xp < nxp;) {
+      f2 al, ah, bl, bh;
+      sample(att, 2 * xp, z4, al, ah);
+      sample(att, 2 * xp + 1, z4, bl, bh);
+      // a lane's 32 bytes as two stores, the halves in turn by lane group of
+      // four: the eight lanes of an access phase hit distinct bank groups
+      float4* o = reinterpret_cast<float4*>(ZB + xp * vst + R0 + 4 * z4);
+      o[hi4] = zturn(hi4 ? ah : al, hi4 ? bh : bl);
+      o[hi4 ^ 1] = zturn(hi4 ? al : ah, hi4 ? bl : bh);
+      xp += dq;
+      z4 += dr;
+      if (z4 >= nz4) {
+        z4 -= nz4;
+        ++xp;
       }
     }
   };
-  float acc[NT][W];
+  table(v, y, 0);
+  geometry(v, y);
+  // the lines start zero; only their data elements are written later
+  for (int k = tid; k < nxp * vst + nzp2 * bst; k += nth) ZB[k] = 0;
+  cp_wait();
+  __syncthreads();
+  gather(v, y);
+  // this thread's x tasks: rows 2 zp, 2 zp + 1, columns x0 .. x0 + X - 1
+  f2 acc[NT][X];
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc[i][k] = 0.f;
-  // the stage that plane p's copy used is free again: the plane nsf ahead
-  auto refill = [&](int s) {
-    if (iq < nitems) {
-      if (tid == 0) issue(iq, yq, s);
-      pend |= 1u << s;
-    }
-    next(iq, yq);
-  };
-  // prologue: plane p's geometry and staged data, its gather
-  geometry(i0, y0);
-  if (!staged(0)) return;
-  gather(0, 0);
+    for (int k = 0; k < X; ++k) acc[i][k] = 0;
   __syncthreads();
-  refill(0);
-  int hb = 0, s1 = nsf > 1 ? 1 : 0;  // working-weight buffer of plane p, stage of plane p + 1
-  for (;;) {
-    const bool h1 = i1 < nitems;
-    const float* Hw = Hw0 + hb * hts;
-    const int4 rg = *reinterpret_cast<const int4*>(Hw + hs + ts);  // tap ranges: z pass, x pass
-    // phase A: z pass of p, task (x, z block) -> XB rows z, column C0 + x
-    const float* ELz = Hw + hs;
-    const float* ERz = ELz + hz;
-    for (int t = tid; t < ztasks; t += NTH) {
-      const int zb = zdiv(t, rnx), x = t - zb * nx, z0 = W * zb;
-      float o[W];
+  const int nzb = (nz + W - 1) / W;
+  // this thread's first z task and the step to its next; its x tasks
+  const int zb0 = tid / nxp, xp0 = tid - zb0 * nxp, dzb = nth / nxp, dxz = nth - dzb * nxp;
+  int xs0[NT], rowo[NT];
 #pragma unroll
-      for (int k = 0; k < W; ++k) o[k] = 0.f;
-      const float* col = ZB + x * ast;
-      zpassw<W>(Hw, rg.x, rg.y, col + z0, o);
+  for (int i = 0; i < NT; ++i) {
+    const int xb = (tid + i * nth) / nzp2;
+    xs0[i] = X * xb;
+    rowo[i] = (tid + i * nth - xb * nzp2) * bst;
+  }
+  int tb = 0;
+  for (int p = p0;; ++p) {
+    int slot1 = slot, y1 = y + a.t.ystep;
+    if (y1 >= ny) y1 -= ny;
+    if (++j == ny) {
+      j = y1 = 0;
+      ++slot1;
+    }
+    const bool more = p + 1 < p1;
+    const int v1 = more && slot1 != slot ? a.vidx[slot1] : v;
+    const float* const Wt = tab0 + tb * trow;
+    const f2* const Wd = reinterpret_cast<const f2*>(Wt);
+    const int4 rg = *reinterpret_cast<const int4*>(Wt + 2 * hs + ts);  // tap ranges: z pass, x pass
+    if (more) {
+      table(v1, y1, tb ^ 1);
+      if (tid == 0)
+        prefetch_l2_bulk(a.att + (((size_t)v1 * ny + y1) * nx) * nzp, (unsigned)(nx * nzp * sizeof(float)));
+    }
+    // phase A: z pass of p, task (column pair, W rows) -> XB
+    const float* ELz = Wt + 2 * hs;
+    const float* ERz = ELz + hz;
+    for (int zb = zb0, xp = xp0; zb < nzb;) {
+      const int z0 = W * zb;
+      const f2* col = ZB + xp * vst;
+      f2 o[W];
+#pragma unroll
+      for (int k = 0; k < W; ++k) o[k] = 0;
+      zpass2<W>(Wd, rg.x, rg.y, col + z0, o);
       if (z0 < hz) {  // clamped rows above the plane
-        const float e0 = col[R0];
+        const f2 e0 = col[R0];
 #pragma unroll
         for (int k = 0; k < W; ++k)
-          if (z0 + k < hz) o[k] = fmaf(ELz[z0 + k], e0, o[k]);
+          if (z0 + k < hz) o[k] = fma2(pack2(ELz[z0 + k], ELz[z0 + k]), e0, o[k]);
       }
       if (z0 + W > nz - hz) {  // clamped rows below
-        const float e1 = col[R0 + nz - 1];
+        const f2 e1 = col[R0 + nz - 1];
 #pragma unroll
         for (int k = 0; k < W; ++k) {
           const int kk = nz - 1 - z0 - k;
-          if (kk >= 0 && kk < hz) o[k] = fmaf(ERz[kk], e1, o[k]);
+          if (kk >= 0 && kk < hz) o[k] = fma2(pack2(ERz[kk], ERz[kk]), e1, o[k]);
         }
       }
-      float* xo = XB + z0 * bs + C0 + x;
+      f2* w = XB + (z0 / 2) * bst + C0 + 2 * xp;
 #pragma unroll
-      for (int k = 0; k < W; ++k)
-        if (z0 + k < nz) xo[k * bs] = o[k];
+      for (int m = 0; m < W / 2; ++m)
+        if (z0 + 2 * m < nz)
+          *reinterpret_cast<float4*>(w + m * bst) = zturn(o[2 * m], o[2 * m + 1]);
+      xp += dxz;
+      zb += dzb;
+      if (xp >= nxp) {
+        xp -= nxp;
+        ++zb;
+      }
     }
-    if (h1) {
-      geometry(i1, y1);
-      if (!staged(s1)) return;
-    } else {
-      __syncthreads();
-    }
-    // phase B: x pass of p, accumulated over the chunk; gather of p + 1
+    if (more) geometry(v1, y1);
+    cp_wait();
+    __syncthreads();
+    // phase B: x pass of p, accumulated; gather of p + 1
     const float* ELx = ERz + hz;
     const float* ERx = ELx + hx;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const int t = tid + i * NTH;
-      if (t < xtasks) {
-        const int xb = zdiv(t, rnz), z = t - xb * nz, x0 = W * xb;
-        const float* row = XB + z * bs;
-        zpassw<W>(Hw + zpw, rg.z, rg.w, row + x0, acc[i]);
+      const int x0 = xs0[i];
+      if (x0 < nx) {
+        const f2* const row = XB + rowo[i];
+        // the plane's own sum first, then onto the depth sum: short chains
+        f2 o[X];
+#pragma unroll
+        for (int k = 0; k < X; ++k) o[k] = 0;
+        zpass2<X>(Wd + g.zpw, rg.z, rg.w, row + x0, o);
         if (x0 < hx) {
-          const float e0 = row[C0];
+          const f2 e0 = row[C0];
 #pragma unroll
-          for (int k = 0; k < W; ++k)
-            if (x0 + k < hx) acc[i][k] = fmaf(ELx[x0 + k], e0, acc[i][k]);
+          for (int k = 0; k < X; ++k)
+            if (x0 + k < hx) o[k] = fma2(pack2(ELx[x0 + k], ELx[x0 + k]), e0, o[k]);
         }
-        if (x0 + W > nx - hx) {
-          const float e1 = row[C0 + nx - 1];
+        if (x0 + X > nx - hx) {
+          const f2 e1 = row[C0 + nx - 1];
 #pragma unroll
-          for (int k = 0; k < W; ++k) {
+          for (int k = 0; k < X; ++k) {
             const int kk = nx - 1 - x0 - k;
-            if (kk < hx) acc[i][k] = fmaf(ERx[kk], e1, acc[i][k]);
+            if (kk >= 0 && kk < hx) o[k] = fma2(pack2(ERx[kk], ERx[kk]), e1, o[k]);
           }
         }
+#pragma unroll
+        for (int k = 0; k < X; ++k) acc[i][k] = add2(acc[i][k], o[k]);
       }
     }
-    if (h1) gather(s1, hb ^ 1);
-    if (!h1 || i1 != i0) {  // p ends its item: partial view of the chunk, part[slot][ch][z][x]
-      const int slot = slot_of(i0), ch = i0 - slot * a.nchunks;
-      float* out = a.part + ((size_t)slot * a.nchunks + ch) * nz * nx;
+    if (more) gather(v1, y1);
+    if (!more || slot1 != slot) {  // p ends the block's planes of this view: its partial view
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        const int t = tid + i * NTH;
-        if (t < xtasks) {
-          const int xb = zdiv(t, rnz), z = t - xb * nz;
-          float* o = out + (size_t)z * nx + W * xb;
+        const int x0 = xs0[i], zp = (tid + i * nth) % nzp2;
+        if (x0 < nx) {
+          float* q = a.part + (size_t)(blockIdx.x + slot) * nz * nx + (size_t)(2 * zp) * nx + x0;
+          const bool two = 2 * zp + 1 < nz;
+          if (nx % 4 == 0) {
 #pragma unroll
-          for (int k = 0; k < W; k += 4) st4(o + k, make_float4(acc[i][k], acc[i][k + 1], acc[i][k + 2], acc[i][k + 3]));
+            for (int k = 0; k < X; k += 4)
+              if (x0 + k < nx) {
+                const float4 u = zturn(acc[i][k], acc[i][k + 1]), w = zturn(acc[i][k + 2], acc[i][k + 3]);
+                st4(q + k, make_float4(u.x, u.y, w.x, w.y));
+                if (two) st4(q + nx + k, make_float4(u.z, u.w, w.z, w.w));
+              }
+          } else {
+#pragma unroll
+            for (int k = 0; k < X; ++k)
+              if (x0 + k < nx) {
+                const float2 u = unpack2(acc[i][k]);
+                q[k] = u.x;
+                if (two) q[nx + k] = u.y;
+              }
+          }
         }
 #pragma unroll
-        for (int k = 0; k < W; ++k) acc[i][k] = 0.f;
+        for (int k = 0; k < X; ++k) acc[i][k] = 0;
       }
     }
-    if (!h1) break;
+    if (!more) break;
     __syncthreads();
-    refill(s1);
-    i0 = i1;
-    y0 = y1;
-    next(i1, y1);
-    hb ^= 1;
-    s1 = nsf > 1 ? s1 ^ 1 : 0;
+    slot = slot1;
+    y = y1;
+    v = v1;
+    tb ^= 1;
   }
 }
 
@@ -633,8 +669,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
   const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2;
   const int tz = a.t.tz, vst = a.t.vst, bst = a.t.bst, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
   const int trow = ztable_floats(g), tid = threadIdx.x, nth = blockDim.x;
-  float2* const VB = reinterpret_cast<float2*>(smem4);
-  float2* const XB0 = VB + (size_t)nxp * vst;
+  f2* const VB = reinterpret_cast<f2*>(smem4);
+  f2* const XB0 = VB + (size_t)nxp * vst;
   const size_t xbs = a.t.nxb > 1 ? (size_t)(tz / 2) * bst : 0;  // offset of the second row buffer
   float* const tab0 = reinterpret_cast<float*>(XB0 + (size_t)a.t.nxb * (tz / 2) * bst);
   const int ntile = a.t.ntile, n = a.nv * ntile * ny;
@@ -646,7 +682,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
   int y = (int)((long long)j * a.t.ystep % ny);
   int slot = st / ntile, Z0 = (st - slot * ntile) * tz, v = a.vidx[slot];
   auto table = [&](int view, int yy, int s) {  // every thread: its 16-byte pieces of the plane's table
-    const float* src = a.tab + ((size_t)a.viewset[view] * ny + yy) * trow;
+    const float* src = a.tab + (((size_t)a.viewset[view] * ny + yy) * 2 + 1) * trow;
     for (int k = 4 * tid; k < trow; k += 4 * nth) cp16(tab0 + s * trow + k, src + k);
   };
   // view rows Z0 - R0 .. of the item as pair lines, zero outside the image;
@@ -667,12 +703,12 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int k = k0 + i * nth, e = zdiv(k, rnxp), xp = k - e * nxp;
-        if (k < tot) VB[(size_t)xp * vst + e] = q[i];
+        if (k < tot) VB[(size_t)xp * vst + e] = pack2(q[i].x, q[i].y);
       }
     }
   };
   table(v, y, 0);
-  for (int k = tid; k < a.t.nxb * (tz / 2) * bst; k += nth) XB0[k] = make_float2(0.f, 0.f);
+  for (int k = tid; k < a.t.nxb * (tz / 2) * bst; k += nth) XB0[k] = 0;
   load_view();
   cp_wait();
   __syncthreads();
@@ -703,34 +739,34 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
       }
     }
     const float* const Wt = tab0 + tb * trow;
-    const float2* const Wd = reinterpret_cast<const float2*>(Wt);
+    const f2* const Wd = reinterpret_cast<const f2*>(Wt);
     const int4 rg = *reinterpret_cast<const int4*>(Wt + 2 * hs + ts);  // tap ranges: z pass, x pass
-    float2* const XB = XB0 + xb2 * xbs;
+    f2* const XB = XB0 + xb2 * xbs;
     {  // z pass: task (column pair, W rows) -> XB
       const float* cLz = Wt + 2 * hs + 2 * hx;
       const float* cRz = cLz + hz;
       const int tasks = nxp * ((rows + W - 1) / W);
       for (int t = tid; t < tasks; t += nth) {
         const int zb = zdiv(t, rnxp), xp = t - zb * nxp, z0 = W * zb;
-        const float2* col = VB + (size_t)xp * vst;
-        float2 o[W];
+        const f2* col = VB + (size_t)xp * vst;
+        f2 o[W];
 #pragma unroll
-        for (int k = 0; k < W; ++k) o[k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < W; ++k) o[k] = 0;
         zpass2<W>(Wd, rg.x, rg.y, col + z0, o);
-        if (Z0 + z0 == 0) o[0] = __fadd2_rn(o[0], zfold2(cLz, col + R0, 1, hz));
+        if (Z0 + z0 == 0) o[0] = add2(o[0], zfold2(cLz, col + R0, 1, hz));
         const int kz = nz - 1 - Z0 - z0;
         if (kz >= 0 && kz < W) {
-          const float2 s = zfold2(cRz, col + R0 + z0 + kz, -1, hz);
+          const f2 s = zfold2(cRz, col + R0 + z0 + kz, -1, hz);
 #pragma unroll
           for (int k = 0; k < W; ++k)
-            if (k == kz) o[k] = __fadd2_rn(o[k], s);
+            if (k == kz) o[k] = add2(o[k], s);
         }
-        float2* w = XB + (size_t)(z0 / 2) * bst + C0 + 2 * xp;
+        f2* w = XB + (size_t)(z0 / 2) * bst + C0 + 2 * xp;
 #pragma unroll
         for (int m = 0; m < W / 2; ++m)
           if (z0 + 2 * m < rows)
             *reinterpret_cast<float4*>(w + (size_t)m * bst) =
-                make_float4(o[2 * m].x, o[2 * m + 1].x, o[2 * m].y, o[2 * m + 1].y);
+                zturn(o[2 * m], o[2 * m + 1]);
       }
     }
     cp_wait();
@@ -747,36 +783,36 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
         const bool whole = x0 + X <= nx;
         const int at0 = x0 * nzp + 2 * zp;
         // the attenuation first: its latency passes behind the window's FMAs
-        float2 at[X];
+        f2 at[X];
         if (whole) {
           const float* q = attp + at0;
 #pragma unroll
-          for (int k = 0; k < X; ++k, q += nzp) at[k] = *reinterpret_cast<const float2*>(q);
+          for (int k = 0; k < X; ++k, q += nzp) at[k] = *reinterpret_cast<const f2*>(q);
         } else {
 #pragma unroll
-          for (int k = 0; k < X; ++k) at[k] = *reinterpret_cast<const float2*>(attp + at0 + min(k, nx - 1 - x0) * nzp);
+          for (int k = 0; k < X; ++k) at[k] = *reinterpret_cast<const f2*>(attp + at0 + min(k, nx - 1 - x0) * nzp);
         }
-        const float2* row = XB + (size_t)zp * bst;
-        float2 o[X];
+        const f2* row = XB + (size_t)zp * bst;
+        f2 o[X];
 #pragma unroll
-        for (int k = 0; k < X; ++k) o[k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < X; ++k) o[k] = 0;
         zpass2<X>(Wd + g.zpw, rg.z, rg.w, row + x0, o);
-        if (x0 == 0) o[0] = __fadd2_rn(o[0], zfold2(cLx, row + C0, 1, hx));
+        if (x0 == 0) o[0] = add2(o[0], zfold2(cLx, row + C0, 1, hx));
         const int kx = nx - 1 - x0;
         if (kx < X) {
-          const float2 s = zfold2(cRx, row + C0 + nx - 1, -1, hx);
+          const f2 s = zfold2(cRx, row + C0 + nx - 1, -1, hx);
 #pragma unroll
           for (int k = 0; k < X; ++k)
-            if (k == kx) o[k] = __fadd2_rn(o[k], s);
+            if (k == kx) o[k] = add2(o[k], s);
         }
         float* q = Tp + at0;
         if (whole) {
 #pragma unroll
-          for (int k = 0; k < X; ++k, q += nzp) *reinterpret_cast<float2*>(q) = __fmul2_rn(at[k], o[k]);
+          for (int k = 0; k < X; ++k, q += nzp) *reinterpret_cast<f2*>(q) = mul2(at[k], o[k]);
         } else {
 #pragma unroll
           for (int k = 0; k < X; ++k, q += nzp)
-            if (x0 + k < nx) *reinterpret_cast<float2*>(q) = __fmul2_rn(at[k], o[k]);
+            if (x0 + k < nx) *reinterpret_cast<f2*>(q) = mul2(at[k], o[k]);
         }
       }
     }

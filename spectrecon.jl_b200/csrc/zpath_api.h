@@ -17,7 +17,6 @@ struct ZGeom {
   int hs, ts;       // weight-row and tail-row lengths of one direction
   int rows, ast;    // z-pass buffer: rows per column, column stride (4 * odd)
   int bs;           // x-pass buffer row stride (4 * odd)
-  int nsf;          // k_zfwd staging buffers: 2 (two planes in flight) or 1
 };
 
 __host__ __device__ constexpr int zround(int v, int m) { return (v + m - 1) / m * m; }
@@ -49,7 +48,6 @@ inline ZGeom zgeom_make(int nx, int ny, int nz, int px, int pz, int pad) {
   g.rows = zround(nz, 16) + g.zpw;  // z tasks of 8 or 16 outputs
   g.ast = zstride4(g.rows);
   g.bs = zstride4(nx + g.xpw);
-  g.nsf = 1;
   return g;
 }
 
@@ -66,18 +64,22 @@ __host__ __device__ inline int ztable_floats(const ZGeom& g) { return 2 * g.hs +
 
 // tiling of a pair-pass kernel: task width w, row tile tz (even; ntile tiles
 // cover nz), strides (float2) of the z-pass and x-pass lines, row buffers,
-// threads, resident blocks per SM, depth step of the plane walk, shared memory
+// threads, resident blocks per SM, depth step of the plane walk, x tasks a
+// thread (k_zfwd), shared memory
 struct ZTile {
-  int w, tz, ntile, vst, bst, nxb, nth, occ, ystep;
+  int w, tz, ntile, vst, bst, nxb, nth, occ, ystep, nxt;
   size_t smem;
 };
+constexpr int kZfwdX = 8;       // outputs of an x-pass and of a z-pass task of k_zfwd
+constexpr int kZfwdZ = 8;
+constexpr int kZfwdNT = 2;      // x tasks a thread at most (their outputs stay in registers)
 constexpr int kZadjX = 8;       // outputs of an x-pass task of k_zadj
 constexpr int kZThreads = 640;  // threads per SM the pair-pass kernels' registers allow (96 each)
 
 struct ZArgs {
   ZGeom g;
   ZTile t;
-  const float* tab;     // [set][y][ztable_floats]: adjoint tables
+  const float* tab;     // [set][y][2][ztable_floats]: forward, adjoint tables
   const float* img;     // IZ
   const float* att;     // ATT
   const float* H;       // [set][y][hs]: forward z | x weights
@@ -86,8 +88,9 @@ struct ZArgs {
   const float4* rot;    // [view] (cos(2pi - theta), sin(2pi - theta), theta == 0, theta)
   const int* vidx;      // [nv] plan view of each slot
   const int* viewset;   // [nview] PSF set of each view
-  int nv, chunkY, nchunks;
-  float* part;          // k_zfwd output [nv][nchunks][nz][nx]
+  int nv;
+  int G;                // blocks of the forward walk (partial views: block + slot)
+  float* part;          // partial views [G + nv][nz][nx]
   const float* views;   // k_zadj input [nv][nz][nx]
   float* T;             // k_zadj output [nv][ny][nx][nzp]
   int* err;
@@ -95,16 +98,11 @@ struct ZArgs {
   int tx, tz;           // their column and row tile sizes
 };
 
-// k_zfwd shared memory (floats; every region 16-byte aligned):
-//   [bar 4][nsf stages: att plane nx*nzp | weights hs | tails ts | ranges 4]
-//   [Hw 2 x (hs + ts + 4)][geoW nx (float4)][geoO nx (int), rounded to 4]
-//   [ZB nx * ast][XB nz * bs]
-__host__ __device__ inline size_t zfwd_smem(const ZGeom& g, int nsf) {
-  const size_t f = 4 + nsf * ((size_t)g.nx * g.nzp + g.hs + g.ts + 4) + 2 * (size_t)(g.hs + g.ts + 4) +
-                   4 * (size_t)g.nx + zround(g.nx, 4) + (size_t)g.nx * g.ast + (size_t)g.nz * g.bs;
-  return f * sizeof(float);
+// k_zfwd shared memory (zpath.cuh)
+inline size_t zfwd_smem(const ZGeom& g, const ZTile& t) {
+  return sizeof(float) * (2 * (size_t)ztable_floats(g) + 8 * (size_t)g.nx + zround(g.nx, 4) +
+                          2 * ((size_t)(g.nx / 2) * t.vst + (size_t)((g.nz + 1) / 2) * t.bst));
 }
-
 // k_zadj shared memory (zpath.cuh)
 inline size_t zadj_smem(const ZGeom& g, const ZTile& t) {
   return sizeof(float) * (2 * ((size_t)(g.nx / 2) * t.vst + (size_t)t.nxb * (t.tz / 2) * t.bst) +
@@ -168,15 +166,30 @@ inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
   return best;
 }
 
-// launch shapes of k_zfwd: NT tasks of W outputs per thread, NTH threads
-// (W = 16 needs nx % 16 == 0); each compiles without register spills
-struct ZShape {
-  int nt, nth, w;
-};
-constexpr int kZNShapes = 8;
-constexpr ZShape kZShapes[kZNShapes] = {{1, 512, 8}, {2, 512, 8},  {3, 512, 8},  {1, 640, 8},
-                                        {2, 640, 8}, {1, 512, 16}, {2, 512, 16}, {1, 640, 16}};
-inline bool zshape_fits(const ZGeom& g, int i) { return g.nx % kZShapes[i].w == 0; }
+// tiling of k_zfwd (w == 0: the plane does not fit): kZfwdNT x tasks a thread
+// (their outputs stay in registers over the planes); threads for them, for
+// half the z tasks and for a quarter of the gather units
+inline ZTile zfwd_tile(const ZGeom& g, size_t optin) {
+  ZTile t{};
+  const int nxw = (g.nx + kZfwdX - 1) / kZfwdX, nzb = (g.nz + kZfwdZ - 1) / kZfwdZ, xt = (g.nz + 1) / 2 * nxw;
+  if (xt > kZfwdNT * kZThreads) return t;
+  t.tz = zround(g.nz, 2);
+  t.ntile = t.nxb = 1;
+  t.vst = zstride2(kZfwdZ * nzb + g.zpw);
+  t.bst = zstride2(kZfwdX * nxw + g.xpw);
+  t.smem = zfwd_smem(g, t);
+  if (t.smem > optin) return t;
+  const int zh = ((g.nx / 2) * nzb + 1) / 2, gq = ((g.nx / 2) * ((g.nz + 3) / 4) + 3) / 4;
+  t.nxt = xt <= kZThreads ? 1 : kZfwdNT;
+  const int xh = (xt + t.nxt - 1) / t.nxt, most = xh > zh ? xh : zh;
+  t.nth = zround(most > gq ? most : gq, 32);
+  if (t.nth > kZThreads) t.nth = kZThreads;
+  const int so = (int)((optin + 1024) / (t.smem + 1024)), ro = kZThreads / t.nth;
+  t.occ = so < ro ? so : ro;
+  t.ystep = zdepth_step(g.ny);
+  t.w = kZfwdX;
+  return t;
+}
 
 // large-plane kernels (zstrip.cuh), shared memory in bytes
 __host__ __device__ inline size_t zs_fz_smem(const ZGeom& g, int tx) {
@@ -193,7 +206,10 @@ constexpr int kZsNthX = 640;  // k_zs_fx threads (one x task each)
 
 // launchers (zpath_inst.cu)
 cudaError_t zpath_setup(int max_smem);
-cudaError_t zfwd_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
+cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
+// views (EM ratio with y, bg) of nv slots from the partial views of a walk by G blocks
+cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
+                           const float* y, const float* bg, const int* vidx);
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zrot_adj_launch(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot,
                             const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,

@@ -9,11 +9,6 @@
 namespace spect {
 
 namespace {
-// the order of kZShapes
-const void* const kZfwd[kZNShapes] = {
-    (const void*)k_zfwd<1, 512, 8>, (const void*)k_zfwd<2, 512, 8>,  (const void*)k_zfwd<3, 512, 8>,
-    (const void*)k_zfwd<1, 640, 8>, (const void*)k_zfwd<2, 640, 8>,  (const void*)k_zfwd<1, 512, 16>,
-    (const void*)k_zfwd<2, 512, 16>, (const void*)k_zfwd<1, 640, 16>};
 const void* const kZadj[2] = {(const void*)k_zadj<8>, (const void*)k_zadj<16>};
 
 // k_zrot_adj's candidates per load round: the largest of 3 and 2 whose
@@ -45,17 +40,24 @@ cudaError_t zrot(const ZGeom& g, int grid, cudaStream_t st, const float* T, cons
 
 cudaError_t zpath_setup(int max_smem) {
   cudaError_t e = cudaSuccess;
-  for (const void* k : kZfwd)
+  for (const void* k : {(const void*)k_zfwd<1>, (const void*)k_zfwd<2>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   for (const void* k : kZadj)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   return e;
 }
 
-cudaError_t zfwd_launch(int shape, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
-  ZArgs c = a;
-  void* args[] = {&c};
-  return cudaLaunchKernel(kZfwd[shape], dim3(grid), dim3(kZShapes[shape].nth), args, smem, st);
+cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a) {
+  if (a.t.nxt == 1) k_zfwd<1><<<grid, a.t.nth, a.t.smem, st>>>(a);
+  else k_zfwd<2><<<grid, a.t.nth, a.t.smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
+                           const float* y, const float* bg, const int* vidx) {
+  if (nxz % 4 == 0) k_reduce_parts<4><<<grid, 256, 0, st>>>(part, nv, ny, G, nxz, out, y, bg, vidx);
+  else k_reduce_parts<1><<<grid, 256, 0, st>>>(part, nv, ny, G, nxz, out, y, bg, vidx);
+  return cudaGetLastError();
 }
 
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {

@@ -8,9 +8,9 @@
 // forward (project!, src/project.jl:77-135):
 //   k_zs_fz  item (slot, y, tile of tx columns): gather the rotated,
 //            attenuated columns (as k_zfwd), z pass, rows -> Q[slot][y][z][x]
-//   k_zs_fx  item (slot, depth chunk, tile of tz rows): per plane the rows of
-//            Q (loaded one plane ahead into registers), x pass accumulated
-//            over the chunk -> part[slot][chunk][z][x]
+//   k_zs_fx  item (partial view of the forward walk, tile of tz rows): per
+//            plane the rows of Q (loaded one plane ahead into registers), x
+//            pass accumulated over the partial's planes -> part
 // The adjoint is k_zadj (zpath.cuh) on row tiles.  Every output goes through
 // the operations of the fused kernels in the same order (z then x), so the
 // two paths agree bit for bit.
@@ -148,6 +148,24 @@ __global__ void __launch_bounds__(NTH) k_zs_fz(ZArgs a) {
   }
 }
 
+// planes [j0, j1) of partial view id (walk block + slot) of the forward walk;
+// false where no block and slot of that sum meet
+__device__ __forceinline__ bool zs_segment(const ZArgs& a, int id, int& slot, int& j0, int& j1) {
+  const int ny = a.g.ny, n = a.nv * ny, G = a.G;
+  // the walk's blocks and slots grow together: find the slot whose ids hold id
+  for (slot = 0; slot < a.nv; ++slot) {
+    const int b1 = zblock_of((long long)(slot + 1) * ny - 1, n, G);
+    if (id <= b1 + slot) break;
+  }
+  if (slot == a.nv) return false;
+  const int b = id - slot;
+  if (b < zblock_of((long long)slot * ny, n, G)) return false;
+  const int q0 = (int)((long long)b * n / G), q1 = (int)((long long)(b + 1) * n / G);
+  j0 = max(q0 - slot * ny, 0);
+  j1 = min(q1 - slot * ny, ny);
+  return j0 < j1;
+}
+
 // ------------------------------------------------------------------------
 // k_zs_fx<NTH, W>: forward x pass and depth sum, one task of W outputs per
 // thread and plane (tz * nx / W <= NTH; the host picks tz).  Shared memory
@@ -160,42 +178,46 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
   const int bufsz = tz * bs + hs + ts + 4;
   float* const base = reinterpret_cast<float*>(smem4);
   const int tid = threadIdx.x;
-  const int ntz = (nz + tz - 1) / tz, nitems = a.nv * a.nchunks * ntz, n4 = nx / 4, xbs = nx / W;
+  const int ntz = (nz + tz - 1) / tz, nitems = (a.G + a.nv) * ntz, n4 = nx / 4, xbs = nx / W;
   const float rn4 = 1.0f / n4, rtz = 1.0f / tz;
   for (int k = tid; k < 2 * bufsz; k += NTH) base[k] = 0.f;  // padding columns stay zero
   __syncthreads();
   // this thread's task: row zl, x block xb
   const int xb = zdiv(tid, rtz), zl = tid - xb * tz, x0 = W * xb;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const int zt = item % ntz, sc = item / ntz, slot = sc / a.nchunks, ch = sc - slot * a.nchunks;
+    // partial view id = walk block + slot, planes j0 .. j1 - 1 of the slot
+    const int zt = item % ntz, id = item / ntz;
+    int slot, j0, j1;
+    if (!zs_segment(a, id, slot, j0, j1)) continue;
     const int Z0 = zt * tz, rows = min(tz, nz - Z0);
-    const int y0 = ch * a.chunkY, y1 = min(ny, y0 + a.chunkY);
     const int v = a.vidx[slot], set = a.viewset[v];
+    int y = (int)((long long)j0 * a.t.ystep % ny);
     const bool mine = tid < tz * xbs && zl < rows;
     const int tot4 = rows * n4;
     auto src = [&](int y) { return a.Q + (((size_t)slot * ny + y) * nz + Z0) * nx; };
-    // plane y0 straight into buffer 0
+    // the first plane straight into buffer 0
     {
-      const float* Qp = src(y0);
+      const float* Qp = src(y);
       for (int e = tid; e < tot4; e += NTH) {
         const int z = zdiv(e, rn4), c = e - z * n4;
         st4(base + z * bs + C0 + 4 * c, ld4(Qp + (size_t)z * nx + 4 * c));
       }
-      zs_table(a, set, y0, base + tz * bs, tid, NTH);
+      zs_table(a, set, y, base + tz * bs, tid, NTH);
     }
     __syncthreads();
     float acc[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) acc[k] = 0.f;
-    for (int y = y0; y < y1; ++y) {
-      float* const XB = base + ((y - y0) & 1) * bufsz;
-      float* const XN = base + (((y - y0) & 1) ^ 1) * bufsz;
+    for (int jj = j0; jj < j1; ++jj) {
+      float* const XB = base + ((jj - j0) & 1) * bufsz;
+      float* const XN = base + (((jj - j0) & 1) ^ 1) * bufsz;
+      const int yn = y + a.t.ystep < ny ? y + a.t.ystep : y + a.t.ystep - ny;
       const float* Wt = XB + tz * bs;
       // the next plane's rows into registers first (four float4 a thread at most)
       float4 pf[4];
-      const bool more = y + 1 < y1;
+      const bool more = jj + 1 < j1;
       if (more) {
-        const float* Qp = src(y + 1);
+        const float* Qp = src(yn);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int e = tid + j * NTH;
@@ -210,21 +232,26 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
         const float* ELx = Wt + hs + 2 * g.hz;
         const float* ERx = ELx + hx;
         const float* row = XB + zl * bs;
-        zpassw<W>(Wt + g.zpw, rg.x, rg.y, row + x0, acc);
+        float o[W];  // the plane's own sum, then onto the depth sum, as k_zfwd
+#pragma unroll
+        for (int k = 0; k < W; ++k) o[k] = 0.f;
+        zpassw<W>(Wt + g.zpw, rg.x, rg.y, row + x0, o);
         if (x0 < hx) {
           const float e0 = row[C0];
 #pragma unroll
           for (int k = 0; k < W; ++k)
-            if (x0 + k < hx) acc[k] = fmaf(ELx[x0 + k], e0, acc[k]);
+            if (x0 + k < hx) o[k] = fmaf(ELx[x0 + k], e0, o[k]);
         }
         if (x0 + W > nx - hx) {
           const float e1 = row[C0 + nx - 1];
 #pragma unroll
           for (int k = 0; k < W; ++k) {
             const int kk = nx - 1 - x0 - k;
-            if (kk < hx) acc[k] = fmaf(ERx[kk], e1, acc[k]);
+            if (kk < hx) o[k] = fmaf(ERx[kk], e1, o[k]);
           }
         }
+#pragma unroll
+        for (int k = 0; k < W; ++k) acc[k] += o[k];
       }
       if (more) {
 #pragma unroll
@@ -235,12 +262,13 @@ __global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
             st4(XN + z * bs + C0 + 4 * c, pf[j]);
           }
         }
-        zs_table(a, set, y + 1, XN + tz * bs, tid, NTH);
+        zs_table(a, set, yn, XN + tz * bs, tid, NTH);
       }
+      y = yn;
       __syncthreads();
     }
-    if (mine) {  // partial view of this chunk: part[slot][ch][z][x]
-      float* o = a.part + (((size_t)slot * a.nchunks + ch) * nz + Z0 + zl) * nx + x0;
+    if (mine) {
+      float* o = a.part + ((size_t)id * nz + Z0 + zl) * nx + x0;
 #pragma unroll
       for (int k = 0; k < W; k += 4) st4(o + k, make_float4(acc[k], acc[k + 1], acc[k + 2], acc[k + 3]));
     }

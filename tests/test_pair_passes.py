@@ -112,3 +112,80 @@ def test_depth_step_visits_every_depth(ny):
         if y >= ny:
             y -= ny
     assert sorted(seen) == list(range(ny))
+
+
+def zfwd_tile(g, optin=OPTIN):
+    """Mirror of zfwd_tile (csrc/zpath_api.h): None where the plane does not fit."""
+    nx, nz = g["nx"], g["nz"]
+    nxw, nzb = (nx + 7) // 8, (nz + 7) // 8
+    xt = (nz + 1) // 2 * nxw
+    if xt > 2 * NTH:
+        return None
+    t = dict(vst=zstride2(8 * nzb + g["zpw"]), bst=zstride2(8 * nxw + g["xpw"]))
+    trow = 2 * g["hs"] + g["ts"] + 4
+    t["smem"] = 4 * (2 * trow + 8 * nx + zround(nx, 4) + 2 * (nx // 2 * t["vst"] + (nz + 1) // 2 * t["bst"]))
+    if t["smem"] > optin:
+        return None
+    t["nxt"] = 1 if xt <= NTH else 2
+    zh, gq = (nx // 2 * nzb + 1) // 2, (nx // 2 * ((nz + 3) // 4) + 3) // 4
+    t["nth"] = min(NTH, zround(max((xt + t["nxt"] - 1) // t["nxt"], zh, gq), 32))
+    return t
+
+
+@pytest.mark.parametrize("nx,nz,px,pz", SIZES)
+def test_forward_tile_bounds(nx, nz, px, pz):
+    g = zgeom(nx, nz, px, pz)
+    t = zfwd_tile(g)
+    if t is None:  # the large-plane kernels
+        assert nx * nz > 8000
+        return
+    R0, C0, hz, hx, vst, bst, nth = g["R0"], g["C0"], g["hz"], g["hx"], t["vst"], t["bst"], t["nth"]
+    nzb, nz4, nxp, nzp2, nxw = (nz + 7) // 8, (nz + 3) // 4, nx // 2, (nz + 1) // 2, (nx + 7) // 8
+    assert (vst // 2) % 2 == 1 and (bst // 2) % 2 == 1 and R0 % 2 == 0 and C0 % 2 == 0
+    # every x task has a thread slot; the z tasks and gather units are walked by constant steps
+    assert t["nxt"] * nth >= nzp2 * nxw
+    for tid in (0, 1, nth // 2, nth - 1):
+        dq, dr = divmod(nth, nz4)
+        xp, z4 = divmod(tid, nz4)
+        got = []
+        while xp < nxp:
+            got.append(xp * nz4 + z4)
+            xp, z4 = xp + dq, z4 + dr
+            if z4 >= nz4:
+                xp, z4 = xp + 1, z4 - nz4
+        assert got == list(range(tid, nxp * nz4, nth))
+        dq, dr = divmod(nth, nxp)
+        zb, xp = divmod(tid, nxp)
+        got = []
+        while zb < nzb:
+            got.append(zb * nxp + xp)
+            zb, xp = zb + dq, xp + dr
+            if xp >= nxp:
+                zb, xp = zb + 1, xp - nxp
+        assert got == list(range(tid, nxp * nzb, nth))
+    # lines: gather stores, windows, clamped edges; rows stored by the z pass
+    assert R0 + 4 * nz4 <= vst and 8 * (nzb - 1) + g["zpw"] + 8 <= vst
+    assert C0 + nx <= bst and 8 * (nxw - 1) + g["xpw"] + 8 <= bst
+    assert max(z0 // 2 + m for z0 in range(0, 8 * nzb, 8) for m in range(4) if z0 + 2 * m < nz) == nzp2 - 1
+
+
+@pytest.mark.parametrize("nv,ny,grid", [(15, 128, 148), (8, 256, 296), (3, 40, 60), (1, 64, 31), (120, 128, 148),
+                                        (2, 8, 8), (1, 2, 1)])
+def test_partial_views_of_the_forward_walk(nv, ny, grid):
+    """Partial view block + slot is unique, a slot's partials are consecutive
+    (zblock_of), and they cover its planes once, in order."""
+    n = nv * ny
+
+    def block_of(q):
+        return ((q + 1) * grid - 1) // n
+
+    seen = {}
+    for b in range(grid):
+        for q in range(b * n // grid, (b + 1) * n // grid):
+            assert block_of(q) == b
+            seen.setdefault((b, q // ny), []).append(q % ny)
+    ids = [b + s for b, s in seen]
+    assert len(set(ids)) == len(ids) and max(ids) < grid + nv
+    for s in range(nv):
+        b0, b1 = block_of(s * ny), block_of((s + 1) * ny - 1)
+        assert sum((seen[(b, s)] for b in range(b0, b1 + 1)), []) == list(range(ny))
