@@ -249,6 +249,7 @@ struct spect_plan_s {
   // planes are transposed into d_Tz (z fastest) and gathered into d_backIZ
   int gadj = 0;
   float* d_Tz = nullptr;
+  size_t tzero = 0;            // offset of the zero column behind the z-fastest adjoint planes (d_P or d_Tz)
   int part_cap = 0;            // partial views that d_part holds (fused paths)
   size_t bytes = 0;
   // stream on which the plan is built and its buffers are (de)allocated;
@@ -617,7 +618,6 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
     CUDA_TRY(cudaMemsetAsync(outIZ, 0, sizeof(float) * p->izN, st));
     return SPECT_OK;
   }
-  const int grot = std::max(1, cdiv((long long)p->nx * p->nx * 16, 256));  // 16 lanes per image column
   for (int g0 = 0; g0 < nidx; g0 += p->gmax) {
     const int nv = std::min(p->gmax, nidx - g0);
     const int* vi = vidx + g0;
@@ -631,7 +631,7 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
     LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
     LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-           zrot_adj_launch(p->zg, grot, st, p->d_P, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
+           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
                            last ? outIZ : p->d_backIZ, xIZ, asumIZ, last ? mode : 0));
   }
   return SPECT_OK;
@@ -769,9 +769,8 @@ int backward(spect_plan_s* p, float* image, const float* views, const int* vidx,
     if (p->gadj) {  // premultiplied planes -> z fastest -> gather into the IZ accumulator
       LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
              zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
-      const int grot = std::max(1, cdiv((long long)p->nx * p->nx * 16, 256));
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-             zrot_adj_launch(p->zg, grot, st, p->d_Tz, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
+             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
                              nullptr, nullptr, 0));
     } else if (p->interp == SPECT_INTERP_ONE) {
       const size_t n = (size_t)nv * p->N;
@@ -1599,7 +1598,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       (st = (cudaMemsetAsync(p->d_err, 0, sizeof(int), p->home) == cudaSuccess) ? SPECT_OK
                                                                                  : fail(SPECT_ERR_CUDA, "memset")) ||
       (st = dalloc(p, &p->d_H, (size_t)p->nset * ny * (p->cg.Q + 1) * Npx)) ||
-      (st = dalloc(p, &p->d_P, (size_t)p->gmax * slot)) ||
+      (st = dalloc(p, &p->d_P, (size_t)p->gmax * slot + (p->zpath ? zg.nzp : 0))) ||
       (st = ((p->nchunk_max = ((size_t)p->gmax * 32 * p->nxz * 4 <= ((size_t)256 << 20)) ? 32 : 16),
              p->part_cap = p->zpath ? std::max(p->gmax * p->nchunk_max, p->sm_count * std::max(1, p->zft.occ) + p->gmax)
                                     : p->gmax * p->nchunk_max,
@@ -1616,9 +1615,11 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       p->zg = zg;
       p->izN = (size_t)zg.L * zg.L * zg.nzp;
       if ((st = dalloc(p, &p->d_backIZ, p->izN)) ||
-          (st = dalloc(p, &p->d_Tz, (size_t)p->gmax * ny * nx * zg.nzp)))
+          (st = dalloc(p, &p->d_Tz, (size_t)p->gmax * ny * nx * zg.nzp + zg.nzp)))
         return bail(st);
-      if (cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess)
+      p->tzero = (size_t)p->gmax * ny * nx * zg.nzp;
+      if (cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
+          cudaMemsetAsync(p->d_Tz + p->tzero, 0, sizeof(float) * zg.nzp, p->home) != cudaSuccess)
         return bail(fail(SPECT_ERR_CUDA, "memset"));
     }
   }
@@ -1629,7 +1630,8 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       return bail(st);
     cudaError_t e = cudaMemsetAsync(p->d_imgIZ, 0, sizeof(float) * p->izN, p->home);
     if (e == cudaSuccess) e = cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_P, 0, sizeof(float) * (size_t)p->gmax * slot, p->home);
+    p->tzero = (size_t)p->gmax * slot;
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_P, 0, sizeof(float) * (p->tzero + zg.nzp), p->home);
     if (e != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e)));
   }
 

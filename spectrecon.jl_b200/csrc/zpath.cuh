@@ -29,9 +29,8 @@
 // The kernels for planes too large for these kernels' shared memory are in
 // zstrip.cuh (same layouts and passes, over plane tiles).
 // k_zrot_adj  imrotate_adj! :two (src/rotatez.jl:390-416) and the view sum
-//          (src/backproject.jl:146-153): output-stationary gather.  Groups of
-//          8 lanes own one image column (x, y) over all z (8 lanes x ZPL) and
-//          sum, over their views in order, the bilinear weights of the
+//          (src/backproject.jl:146-153): output-stationary gather.  Every image
+//          column sums, over the views in order, the bilinear weights of the
 //          rotated-grid points whose footprint covers it: the exact transpose
 //          of the forward sampling, without atomics.  The EM update
 //          (src/ml-os-em.jl:111-126) is its epilogue.
@@ -65,17 +64,6 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 // four floats as two packed pairs
 __device__ __forceinline__ ulonglong2 ldp(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
-// 8-byte read-only global load issued only where pred holds; (0, 0) elsewhere
-// (no memory access for those lanes).  p must be 8-byte aligned.
-__device__ __forceinline__ float2 ldg2_if(const float* p, bool pred) {
-  unsigned a, b;
-  asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t"
-      "@q ld.global.nc.v2.b32 {%0, %1}, [%2];\n\t}"
-      : "=r"(a), "=r"(b)
-      : "l"(p), "r"((int)pred));
-  return make_float2(__uint_as_float(a), __uint_as_float(b));
-}
-
 // one W-output task (W = 8 or 16) over a zero-padded line, the taps
 // m in [4 b4, 4 b4 + 8 nblk) in blocks of 8 (nblk <= 9): o[k] += sum_m w[m]
 // line[k + m] (line and w 16-byte aligned; reads line[4 b4, 4 b4 + 8 nblk +
@@ -835,146 +823,186 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
 }
 
 // ------------------------------------------------------------------------
-// k_zrot_adj<ZPL, RB>: two 8-lane groups of a warp own image column p = (j1, j2)
-// (grid-stride), lane l of a group the z pairs 2 l + 16 q, q < ZPL / 2 (nzp =
-// 8 ZPL): 64 contiguous bytes per group and 8-byte load.  The first group
-// sums the even slots, the second the odd ones; a shuffle adds the two
-// partial sums (a fixed order).  Per slot, lane l of a group evaluates
-// candidate l (and every lane candidate 8) and the group shares the nine by
-// shuffles, summing them in the order 0..8.  For
-// every slot, the rotated-grid points (x, y) whose bilinear footprint contains
+// k_zrot_adj: a block owns a tile of C = tx ty image columns over all z.  Its
+// units (column, four z) are dealt to the threads of a group, kZrotU a thread,
+// lanes on consecutive z of a column (16-byte loads, whole sectors); S groups
+// take every S-th slot and their sums are added in group order.  The
+// rotated-grid points (x, y) whose bilinear footprint contains image column
 // (j1, j2) -- those with floor(s1) in {j1-1, j1} and floor(s2) in {j2-1, j2}
 // -- lie within |cos| + |sin| of the inverse-rotated pixel centre, so the
-// candidates are at most 3 x 3 points; each is tested with the forward's own
-// position arithmetic and weighted with the forward's weight product.
-// RB = 0: a hit candidate's loads are issued under a branch on its offset,
-// so the candidates' load latencies follow one another.  RB > 0: the
-// candidates go in rounds of RB whose loads are all issued (predicated off
-// for misses, which then read zero) before the round's FMAs, so up to
-// RB x ZPL / 2 loads per lane are in flight; a miss adds fmaf(0, 0, acc) ==
-// acc, so both forms give the same bits.
+// candidates are at most 3 x 3 points (four hit as a rule, three to five but
+// for a few; a weight of zero is no hit).  One thread tests the nine of a
+// (slot, column) pair with the forward's own position arithmetic and lists the
+// hits (T column, weight) in shared memory, vb slots of the tile at a time,
+// one batch ahead of the sums; lists of fewer than four end in the zero column
+// zcol, so that a unit runs four unconditional loads a slot, the others under
+// a branch.  A group's sum runs over its slots and hits in order.
+// Bound: L1 (its tag stage is 55 % busy where an SM works: a column's 320
+// bytes straddle lines) and the latency of the misses.  Measured (the former
+// kernel tested the candidates in every 8-lane group): 128x128x80, 15 views 49
+// -> 46 us; 64x64x64, 64 views 57 -> 31 us; 64x64x40, 60 views 45 -> 24 us;
+// 256x256x200, 8 views 252 -> 216 us.
 // Epilogue (IZ layout): v = acc (+ prev); mode 1: zeros -> +Inf; mode 2:
 // v = x * (v / asum); out = v (z < nz only; out may be prev or x).
-template <int ZPL, int RB>
-__global__ void __launch_bounds__(256, (ZPL <= 14 ? 4 : 2)) k_zrot_adj(ZGeom g, const float* __restrict__ T,
-                                                 const float4* __restrict__ rot, const int* __restrict__ vidx, int nv,
-                                                 const float* prev, float* out, const float* x,
-                                                 const float* __restrict__ asum, int mode) {
-  const int lane = threadIdx.x & 7, half = (threadIdx.x >> 3) & 1;
-  const int npix = (gridDim.x * blockDim.x) >> 4;
-  const int nx = g.nx, ny = g.ny, nzp = g.nzp;
+__global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* __restrict__ T,
+                                                             int zcol, const float4* __restrict__ rot,
+                                                             const int* __restrict__ vidx, int nv, const float* prev,
+                                                             float* out, const float* x,
+                                                             const float* __restrict__ asum, int mode) {
+  constexpr int U = kZrotU, E = kZrotList;
+  extern __shared__ float4 smem4[];
+  const int nth = blockDim.x, tid = threadIdx.x, nx = g.nx, ny = g.ny, n4 = g.nzp / 4, C = r.tx * r.ty;
   const float c0 = g.c0;
-  // every warp runs the same number of iterations (the shuffle needs all lanes)
-  for (int p0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 4; p0 < nx * nx; p0 += npix) {
-    const int p = min(p0 + ((threadIdx.x >> 4) & 1), nx * nx - 1);
-    const bool own = p0 + ((threadIdx.x >> 4) & 1) < nx * nx;
-    const int j2 = p / nx, j1 = p - j2 * nx;
-    const float fj1 = (float)j1, fj2 = (float)j2;
-    float2 acc[ZPL / 2];
-#pragma unroll
-    for (int q = 0; q < ZPL / 2; ++q) acc[q] = make_float2(0.f, 0.f);
-    // every lane runs the same number of rounds (the shuffles need them all)
-    for (int s0 = 0; s0 < nv; s0 += 2) {
-      const bool live = s0 + half < nv;
-      const int s = live ? s0 + half : s0;
-      const float4 r = rot[vidx[s]];
-      const float cs = r.x, sn = r.y;
-      const float d1 = fj1 - c0, d2 = fj2 - c0;
+  // [2][nth][E]: the hits (T column, weight); the first entry's top five bits
+  // hold their count
+  int2* const list = reinterpret_cast<int2*>(smem4);
+  const int ntx = (nx + r.tx - 1) / r.tx;
+  const int X0 = (blockIdx.x % ntx) * r.tx, Y0 = (blockIdx.x / ntx) * r.ty;
+  // hits of the batch of slots from s0 on: thread q's pair is slot s0 + q / C, column q % C
+  const int ps = tid / C, pc = tid - ps * C, pj1 = X0 + pc % r.tx, pj2 = Y0 + pc / r.tx;
+  const float fj1 = (float)pj1, fj2 = (float)pj2, d1 = fj1 - c0, d2 = fj2 - c0;
+  auto hits = [&](int s0, int buf) {
+    const int s = s0 + ps;
+    int2* const L0 = list + (buf * nth + tid) * E;
+    int2* L = L0;
+    if (ps < r.vb && s < nv && pj1 < nx && pj2 < nx) {
+      const float4 rt = rot[vidx[s]];
+      const float cs = rt.x, sn = rt.y;
       const float xc = c0 + cs * d1 + sn * d2, yc = c0 - sn * d1 + cs * d2;
       const float rr = fabsf(cs) + fabsf(sn) + 0.01f;
-      const int xlo = max(0, (int)ceilf(xc - rr)), xhi = min(nx - 1, (int)floorf(xc + rr));
-      const int ylo = max(0, (int)ceilf(yc - rr)), yhi = min(ny - 1, (int)floorf(yc + rr));
-      const float* Ts = T + (size_t)s * ny * nx * nzp + 2 * lane;
-      // candidate c = 3 i + k (x offset i, y offset k): weight and column
-      // offset (-1: no footprint), with the forward's own operations
-      auto cand = [&](int c, float& w, int& o) {
-        const int i = (c * 11) >> 5, k = c - 3 * i;  // c / 3 for c <= 8
-        const int xx = min(xlo + i, nx - 1), yy = min(ylo + k, ny - 1);
-        const float di = __fsub_rn((float)xx, c0), dj = __fsub_rn((float)yy, c0);
-        const float s1 = __fadd_rn(c0, __fsub_rn(__fmul_rn(cs, di), __fmul_rn(sn, dj)));
-        const float s2 = __fadd_rn(c0, __fadd_rn(__fmul_rn(sn, di), __fmul_rn(cs, dj)));
-        const bool ok = live && xlo + i <= xhi && ylo + k <= yhi && s1 >= fj1 - 1.f && s1 < fj1 + 1.f &&
-                        s2 >= fj2 - 1.f && s2 < fj2 + 1.f;
-        const float f1 = floorf(s1), f2 = floorf(s2);
-        const float t1 = __fsub_rn(s1, f1), t2 = __fsub_rn(s2, f2);
-        const float a1 = f1 == fj1 ? __fsub_rn(1.0f, t1) : t1;
-        const float a2 = f2 == fj2 ? __fsub_rn(1.0f, t2) : t2;
-        w = ok ? __fmul_rn(a1, a2) : 0.f;
-        o = ok ? (yy * nx + xx) * nzp : -1;
-      };
-      // lane l of the group evaluates candidate l, every lane candidate 8;
-      // the group shares them by shuffles and sums them in the order c = 0..8
-      float wl, w8;
-      int ol, o8;
-      cand(lane, wl, ol);
-      cand(8, w8, o8);
-      if constexpr (RB == 0) {
+      const int xlo = max(0, (int)ceilf(xc - rr)), nxc = min(nx - 1, (int)floorf(xc + rr)) - xlo;
+      const int ylo = max(0, (int)ceilf(yc - rr)), nyc = min(ny - 1, (int)floorf(yc + rr)) - ylo;
+      const int base = (s * ny + ylo) * nx + xlo;
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-          const float w = c < 8 ? __shfl_sync(0xffffffffu, wl, c, 8) : w8;
-          const int o = c < 8 ? __shfl_sync(0xffffffffu, ol, c, 8) : o8;
-          if (o >= 0) {
-            const float* tp = Ts + o;
+      for (int i = 0; i < 3; ++i) {
+        const float di = __fsub_rn((float)(xlo + i), c0), ci = __fmul_rn(cs, di), si = __fmul_rn(sn, di);
 #pragma unroll
-            for (int q = 0; q < ZPL / 2; ++q) {
-              const float2 t = *reinterpret_cast<const float2*>(tp + 16 * q);
-              acc[q].x = fmaf(w, t.x, acc[q].x);
-              acc[q].y = fmaf(w, t.y, acc[q].y);
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c0 = 0; c0 < 9; c0 += RB) {
-          float wk[RB];
-          float2 tk[RB][ZPL / 2];
-#pragma unroll
-          for (int k = 0; k < RB; ++k) {
-            const int c = c0 + k;
-            wk[k] = 0.f;
-            if (c < 9) {  // resolved at compile time
-              wk[k] = c < 8 ? __shfl_sync(0xffffffffu, wl, c, 8) : w8;
-              const int o = c < 8 ? __shfl_sync(0xffffffffu, ol, c, 8) : o8;
-              const float* tp = Ts + max(o, 0);
-#pragma unroll
-              for (int q = 0; q < ZPL / 2; ++q) tk[k][q] = ldg2_if(tp + 16 * q, o >= 0);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < RB; ++k) {
-            if (c0 + k < 9) {
-#pragma unroll
-              for (int q = 0; q < ZPL / 2; ++q) {
-                acc[q].x = fmaf(wk[k], tk[k][q].x, acc[q].x);
-                acc[q].y = fmaf(wk[k], tk[k][q].y, acc[q].y);
-              }
-            }
+        for (int k = 0; k < 3; ++k) {
+          const float dj = __fsub_rn((float)(ylo + k), c0);
+          const float s1 = __fadd_rn(c0, __fsub_rn(ci, __fmul_rn(sn, dj)));
+          const float s2 = __fadd_rn(c0, __fadd_rn(si, __fmul_rn(cs, dj)));
+          // floor(s) == j: 1 - (s - j); floor(s) == j - 1: s - (j - 1); not positive elsewhere
+          const float a1 = s1 >= fj1 ? __fsub_rn(1.0f, __fsub_rn(s1, fj1)) : __fsub_rn(s1, fj1 - 1.f);
+          const float a2 = s2 >= fj2 ? __fsub_rn(1.0f, __fsub_rn(s2, fj2)) : __fsub_rn(s2, fj2 - 1.f);
+          if (i <= nxc && k <= nyc && fminf(a1, a2) > 0.f) {
+            *L++ = make_int2(base + k * nx + i, __float_as_int(__fmul_rn(a1, a2)));
           }
         }
       }
     }
+    const int m = (int)(L - L0);
+    for (; L < L0 + 4; ++L) *L = make_int2(zcol, 0);
+    L0->x |= m << 27;
+  };
+  // this thread's units: group, column of the tile, z group (a unit past the
+  // last repeats it and is not stored)
+  const int gth = nth / r.S, grp = tid / gth, gt = tid - grp * gth, units = C * n4;
+  const unsigned cb = (unsigned)g.nzp * (unsigned)sizeof(float);  // bytes of a T column
+  int col[U];
+  const char* Tz[U];
+  float4 acc[U];
 #pragma unroll
-    for (int q = 0; q < ZPL / 2; ++q) {  // even + odd slots
-      acc[q].x += __shfl_xor_sync(0xffffffffu, acc[q].x, 8);
-      acc[q].y += __shfl_xor_sync(0xffffffffu, acc[q].y, 8);
-    }
-    if (half || !own) continue;
-    const size_t o = ((size_t)(j2 + g.pad) * g.L + j1 + g.pad) * nzp + 2 * lane;
+  for (int i = 0; i < U; ++i) {
+    const int u = min(gt + i * gth, units - 1);
+    col[i] = u / n4;
+    Tz[i] = reinterpret_cast<const char*>(T) + 16 * (u - col[i] * n4);
+    acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  auto load = [&](int i, int c) {
+    return __ldg(reinterpret_cast<const float4*>(Tz[i] + (unsigned long long)(unsigned)c * cb));
+  };
+  auto add = [&](float4& v, int wi, const float4& t) {
+    const float w = __int_as_float(wi);
+    v.x = fmaf(w, t.x, v.x);
+    v.y = fmaf(w, t.y, v.y);
+    v.z = fmaf(w, t.z, v.z);
+    v.w = fmaf(w, t.w, v.w);
+  };
+  hits(0, 0);
+  __syncthreads();
+  for (int s0 = 0, buf = 0; s0 < nv; s0 += r.vb, buf ^= 1) {
+    if (s0 + r.vb < nv) hits(s0 + r.vb, buf ^ 1);
+    const int nb = min(r.vb, nv - s0);
+    for (int b = grp; b < nb; b += r.S) {
+      const int2* const L = list + (buf * nth + b * C) * E;
 #pragma unroll
-    for (int q = 0; q < ZPL / 2; ++q) {
-      const float vq[2] = {acc[q].x, acc[q].y};
+      for (int i0 = 0; i0 < U; i0 += 2) {  // two units: eight loads before the sums
+        float4 t[2][4];
+        int w[2][4], m[2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const size_t oe = o + 16 * q + e;
-        if (2 * lane + 16 * q + e < g.nz) {
-          float v = vq[e];
-          if (prev) v += prev[oe];
-          if (mode == 1 && v == 0.f) v = __int_as_float(0x7f800000);
-          if (mode == 2) v = x[oe] * (v / asum[oe]);
-          out[oe] = v;
+        for (int i = 0; i < 2; ++i) {
+          const int2* const q = L + col[i0 + i] * E;
+          const int2 e0 = q[0], e1 = q[1], e2 = q[2], e3 = q[3];
+          m[i] = (int)((unsigned)e0.x >> 27);
+          t[i][0] = load(i0 + i, e0.x & 0x07ffffff);
+          t[i][1] = load(i0 + i, e1.x);
+          t[i][2] = load(i0 + i, e2.x);
+          t[i][3] = load(i0 + i, e3.x);
+          w[i][0] = e0.y;
+          w[i][1] = e1.y;
+          w[i][2] = e2.y;
+          w[i][3] = e3.y;
+        }
+        // the slot's own sum first, then onto the view sum: short chains
+        float4 v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int h = 0; h < 4; ++h) add(v[i], w[i][h], t[i][h]);
+        }
+        for (int h = 4; h < max(m[0], m[1]); ++h)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (h < m[i]) {
+              const int2 e = L[col[i0 + i] * E + h];
+              add(v[i], e.y, load(i0 + i, e.x));
+            }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          acc[i0 + i].x += v[i].x;
+          acc[i0 + i].y += v[i].y;
+          acc[i0 + i].z += v[i].z;
+          acc[i0 + i].w += v[i].w;
         }
       }
     }
+    __syncthreads();
+  }
+  if (r.S > 1) {  // sums of groups 1 .. S - 1 to group 0, in order
+    float4* const part = smem4;
+    if (grp > 0)
+#pragma unroll
+      for (int i = 0; i < U; ++i) part[((grp - 1) * U + i) * gth + gt] = acc[i];
+    __syncthreads();
+    if (grp > 0) return;
+    for (int q = 0; q < r.S - 1; ++q)
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const float4 v = part[(q * U + i) * gth + gt];
+        acc[i].x += v.x;
+        acc[i].y += v.y;
+        acc[i].z += v.z;
+        acc[i].w += v.w;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    if (gt + i * gth >= units) continue;
+    const int z = 4 * (gt + i * gth - col[i] * n4);
+    const int j1 = X0 + col[i] % r.tx, j2 = Y0 + col[i] / r.tx;
+    if (j1 >= nx || j2 >= nx) continue;
+    const size_t o = ((size_t)(j2 + g.pad) * g.L + j1 + g.pad) * g.nzp + z;
+    const float vq[4] = {acc[i].x, acc[i].y, acc[i].z, acc[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (z + e < g.nz) {
+        float v = vq[e];
+        if (prev) v += prev[o + e];
+        if (mode == 1 && v == 0.f) v = __int_as_float(0x7f800000);
+        if (mode == 2) v = x[o + e] * (v / asum[o + e]);
+        out[o + e] = v;
+      }
   }
 }
 

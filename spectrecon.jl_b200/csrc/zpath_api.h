@@ -204,6 +204,37 @@ struct ZsTiles {
 constexpr int kZsNth = 512;   // k_zs_fz threads
 constexpr int kZsNthX = 640;  // k_zs_fx threads (one x task each)
 
+// tiling of k_zrot_adj: tiles of tx x ty image columns, S groups of threads
+// over the slots, vb slots whose hits are listed at a time (one thread tests
+// one column of one slot).  16 columns a tile (8 of over 160 z): the blocks
+// are short enough to fill the last wave (128x128x80, 15 views: 46 us; 32
+// columns 48 us, 8 columns 46 us; 256x256x200, 8 views: 226 us, 8 columns 216
+// us), and images that leave the SMs short of threads split the slots
+// (64x64x64, 64 views: 32 columns 47 us, 16 columns in four groups 31 us).
+constexpr int kZrotU = 2;          // units (column, four z) a thread
+constexpr int kZrotList = 9;       // list entries of a pair: its candidates at most
+constexpr int kZrotThreads = 512;  // nzp <= 256: 8 columns x 64 units / 2 = 256 a group at most
+struct ZRotTile {
+  int tx, ty, S, vb, nth, grid;
+  size_t smem;
+};
+inline ZRotTile zrot_tile(const ZGeom& g, int nv, int sms) {
+  ZRotTile r{};
+  const int n4 = g.nzp / 4, C = n4 <= 40 ? 16 : 8;
+  r.tx = 4;
+  r.ty = C / 4;
+  r.grid = ((g.nx + r.tx - 1) / r.tx) * ((g.nx + r.ty - 1) / r.ty);
+  const int gth = zround((C * n4 + kZrotU - 1) / kZrotU, 32);
+  r.S = (int)((long long)sms * 2 * kZrotThreads / ((long long)r.grid * gth));
+  if (r.S > nv) r.S = nv;
+  if (r.S > kZrotThreads / gth) r.S = kZrotThreads / gth;
+  if (r.S < 1) r.S = 1;
+  r.nth = r.S * gth;
+  r.vb = r.nth / C;
+  r.smem = (size_t)r.nth * 2 * kZrotList * 8;
+  return r;
+}
+
 // launchers (zpath_inst.cu)
 cudaError_t zpath_setup(int max_smem);
 cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
@@ -211,9 +242,9 @@ cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
                            const float* y, const float* bg, const int* vidx);
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
-cudaError_t zrot_adj_launch(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot,
+cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
                             const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,
-                            int mode);
+                            int mode);  // T[zero ..]: a column of zeros
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz);
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx);

@@ -1,8 +1,6 @@
 // zpath_inst.cu -- instantiations and launchers of the fused projector pair
 // (zpath.cuh) and of the large-plane kernels (zstrip.cuh), compiled as a unit
 // of its own.
-#include <cstdlib>
-
 #include "zpath.cuh"
 #include "zstrip.cuh"
 
@@ -11,31 +9,6 @@ namespace spect {
 namespace {
 const void* const kZadj[2] = {(const void*)k_zadj<8>, (const void*)k_zadj<16>};
 
-// k_zrot_adj's candidates per load round: the largest of 3 and 2 whose
-// rounds compile without register spills under the kernel's launch bounds
-// (64 registers per thread for ZPL <= 14, 128 above; from ptxas -v for
-// every ZPL); 0 (one branch per candidate) where both spill.
-// SPECT_ZROT_RB=0 selects the branch form everywhere; read once per process.
-constexpr int zrot_rounds(int zpl) {
-  return (zpl <= 10 || (zpl >= 16 && zpl <= 24)) ? 3 : (zpl == 26 || zpl >= 30) ? 2 : 0;
-}
-bool zrot_branch_form() {
-  static const bool b = [] {
-    const char* e = getenv("SPECT_ZROT_RB");
-    return e != nullptr && e[0] == '0' && e[1] == 0;
-  }();
-  return b;
-}
-
-template <int ZPL>
-cudaError_t zrot(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot, const int* vidx,
-                 int nv, const float* prev, float* out, const float* x, const float* asum, int mode) {
-  if (zrot_branch_form())
-    k_zrot_adj<ZPL, 0><<<grid, 256, 0, st>>>(g, T, rot, vidx, nv, prev, out, x, asum, mode);
-  else
-    k_zrot_adj<ZPL, zrot_rounds(ZPL)><<<grid, 256, 0, st>>>(g, T, rot, vidx, nv, prev, out, x, asum, mode);
-  return cudaGetLastError();
-}
 }  // namespace
 
 cudaError_t zpath_setup(int max_smem) {
@@ -66,17 +39,17 @@ cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {
   return cudaLaunchKernel(kZadj[a.t.w == 16 ? 1 : 0], dim3(grid), dim3(a.t.nth), args, a.t.smem, st);
 }
 
-cudaError_t zrot_adj_launch(const ZGeom& g, int grid, cudaStream_t st, const float* T, const float4* rot,
+cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
                             const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,
                             int mode) {
-  switch (g.nzp / 8) {  // nzp is a multiple of 16
-#define ZCASE(n) \
-  case n: return zrot<n>(g, grid, st, T, rot, vidx, nv, prev, out, x, asum, mode);
-    ZCASE(2) ZCASE(4) ZCASE(6) ZCASE(8) ZCASE(10) ZCASE(12) ZCASE(14) ZCASE(16)
-    ZCASE(18) ZCASE(20) ZCASE(22) ZCASE(24) ZCASE(26) ZCASE(28) ZCASE(30) ZCASE(32)
-#undef ZCASE
+  const ZRotTile r = zrot_tile(g, nv, sms);
+  if (r.smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute((const void*)k_zrot_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kZrotThreads * 2 * kZrotList * 8);
+    if (e != cudaSuccess) return e;
   }
-  return cudaErrorInvalidValue;
+  k_zrot_adj<<<r.grid, r.nth, r.smem, st>>>(g, r, T, (int)(zero / g.nzp), rot, vidx, nv, prev, out, x, asum, mode);
+  return cudaGetLastError();
 }
 
 namespace {

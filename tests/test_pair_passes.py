@@ -189,3 +189,34 @@ def test_partial_views_of_the_forward_walk(nv, ny, grid):
     for s in range(nv):
         b0, b1 = block_of(s * ny), block_of((s + 1) * ny - 1)
         assert sum((seen[(b, s)] for b in range(b0, b1 + 1)), []) == list(range(ny))
+
+
+def zrot_tile(g, nv, sms=148):
+    """Mirror of zrot_tile (csrc/zpath_api.h)."""
+    n4 = zround(g["nz"], 16) // 4
+    C = 16 if n4 <= 40 else 8
+    tx, ty = 4, C // 4
+    grid = -(-g["nx"] // tx) * -(-g["nx"] // ty)
+    gth = zround((C * n4 + 1) // 2, 32)
+    S = max(1, min(sms * 1024 // (grid * gth), nv, 512 // gth))
+    return dict(C=C, tx=tx, ty=ty, grid=grid, gth=gth, S=S, nth=S * gth, vb=S * gth // C, n4=n4)
+
+
+@pytest.mark.parametrize("nx,nz,px,pz", SIZES + [(90, 53, 5, 5), (32, 160, 5, 5), (512, 250, 5, 5)])
+@pytest.mark.parametrize("nv", [1, 2, 15, 128])
+def test_gather_adjoint_tile(nx, nz, px, pz, nv):
+    g = zgeom(nx, nz, px, pz)
+    t = zrot_tile(g, nv)
+    assert t["nth"] <= 512 and t["vb"] >= 1 and t["vb"] * t["C"] <= t["nth"]
+    # every unit of a tile has a thread, the group sums fit in the lists' memory
+    assert 2 * t["gth"] >= t["C"] * t["n4"]
+    assert (t["S"] - 1) * 2 * t["gth"] * 16 <= t["nth"] * 2 * 9 * 8
+    # the groups take every slot of a batch once
+    slots = []
+    for s0 in range(0, nv, t["vb"]):
+        nb = min(t["vb"], nv - s0)
+        for grp in range(t["S"]):
+            slots += [s0 + b for b in range(grp, nb, t["S"])]
+    assert sorted(slots) == list(range(nv))
+    # tiles cover the image
+    assert -(-nx // t["tx"]) * t["tx"] >= nx and -(-nx // t["ty"]) * t["ty"] >= nx
