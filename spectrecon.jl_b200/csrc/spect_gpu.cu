@@ -1506,7 +1506,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     const char* senv = std::getenv("SPECT_ZSTRIP");
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
-        interpmeth == SPECT_INTERP_TWO && sep_host && !only_fft && !(zenv && zenv[0] == '0') && nx % 8 == 0 &&
+        interpmeth == SPECT_INTERP_TWO && sep_host && !only_fft && !(zenv && zenv[0] == '0') &&
         zg_full.zpw <= 72 && zg_full.xpw <= 72 &&  // pass rows of at most 9 blocks of 8 taps
         zg.nzp <= 256 && opts.atten_cache != 0) {
       p->zat = zadj_tile(zg, (size_t)optin);
@@ -1514,7 +1514,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       p->zft = zfwd_tile(zg, (size_t)optin);
       const bool fused = adj && p->zft.w != 0;
       if (!fused) p->zft.ystep = zdepth_step(ny);  // the walk of the large-plane kernels
-      const bool strip = adj && zs_tiles(zg, (size_t)optin, &zt);
+      const bool strip = adj && nx % 8 == 0 && zs_tiles(zg, (size_t)optin, &zt);
       if (fused && !(senv && senv[0] == '1')) zkind = 1;
       else if (strip && !(senv && senv[0] == '0')) zkind = 2;
       else if (fused) zkind = 1;

@@ -1,0 +1,69 @@
+"""The fused projector pair on matrices that no task width divides (any even
+nx, any nz, px != pz), against the split kernels (SPECT_ZPATH=0) of the same
+plan and against the Float32 and Float64 oracles.
+
+Tolerances: 1e-4 against the oracles, the bound of the other parity tests
+(max|gpu - oracle| / max|oracle|); 1e-5 between the two GPU paths, which carry
+~1e-6 each (Float32 FFT and direct sums of up to 65 taps).
+"""
+import numpy as np
+import pytest
+
+from conftest import relerr
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-4
+
+
+def _plan_inputs(S, nx, nz, px, pz, nview, seed):
+    rng = np.random.default_rng(seed)
+    mumap = np.asfortranarray(0.01 * rng.random((nx, nx, nz)), np.float32)
+    psf = S.psf_gauss(ny=nx, px=px, pz=pz, fwhm_start=1, fwhm_end=max(1.5, px / 5))
+    psfs = np.asfortranarray(np.repeat(psf[:, :, :, None], nview, axis=3), np.float32)
+    x = np.asfortranarray(rng.random((nx, nx, nz)), np.float32)
+    y = np.asfortranarray(rng.random((nx, nz, nview)), np.float32)
+    return mumap, psfs, x, y
+
+
+@pytest.mark.parametrize("nx,nz,px,pz,nview,idx", [
+    (90, 53, 21, 17, 12, [11, 0, 4]),  # a partial x task of two columns, an odd last row
+    (46, 80, 7, 7, 10, None),          # six columns in the last x task
+    (34, 9, 5, 3, 9, [8, 2]),          # one z task and a row
+    (10, 3, 3, 3, 7, None),            # one x task and two columns
+    (2, 1, 1, 1, 4, None),             # the smallest image, no blur
+    (66, 1, 9, 1, 16, [3, 15]),        # one slice
+    (122, 66, 25, 25, 5, [4, 1]),      # several warps of partial tasks
+])
+def test_ragged_fused_pair(S, O, monkeypatch, nx, nz, px, pz, nview, idx):
+    mumap, psfs, x, y = _plan_inputs(S, nx, nz, px, pz, nview, 7 * nx + nz)
+    ii = None if idx is None else np.array(idx, np.int32)
+    ys = y if ii is None else np.asfortranarray(y[:, :, ii])
+    out = {}
+    for path in ("fused", "split"):
+        monkeypatch.setenv("SPECT_ZPATH", "1" if path == "fused" else "0")
+        plan = S.SPECTplan(mumap, psfs, 4.8)
+        assert plan.path == path
+        out[path] = (S.project(x, plan, index=ii), S.backproject(ys, plan, index=ii))
+        plan.close()
+    for a, b in zip(out["fused"], out["split"]):
+        assert relerr(a, b) <= 1e-5
+    for dtype in (np.float32, np.float64):
+        G = O.Geometry(mumap, psfs, 4.8, dtype=dtype)
+        assert relerr(out["fused"][0], G.project(x, index=ii)) <= TOL
+        assert relerr(out["fused"][1], G.backproject(ys, index=ii)) <= TOL
+
+
+def test_ragged_osem_and_view_dependent_psfs(S, O):
+    """OS-EM with a PSF stack of its own for every view (a body-contouring
+    orbit) on a matrix of 38 columns and 21 rows."""
+    nx, nz, p, nview = 38, 21, 9, 8
+    mumap, _, x, _ = _plan_inputs(S, nx, nz, p, p, nview, 3)
+    psfs = np.stack([S.psf_gauss(ny=nx, px=p, fwhm_start=1, fwhm_end=1.5 + 0.1 * v) for v in range(nview)], axis=3)
+    psfs = np.asfortranarray(psfs, np.float32)
+    plan = S.SPECTplan(mumap, psfs, 4.8)
+    assert plan.path == "fused" and plan.info()["nset"] == nview
+    G = O.Geometry(mumap, psfs, 4.8)
+    yn = np.asfortranarray(G.project(x) + 0.1, np.float32)
+    bg = np.full(yn.shape, 0.05, np.float32, order="F")
+    x0 = np.ones(x.shape, np.float32, order="F")
+    assert relerr(S.osem(x0, yn, bg, S.Ablock(plan, 4), niter=2), G.osem(x0, yn, bg, 4, 2)) <= TOL

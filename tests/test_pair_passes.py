@@ -56,7 +56,8 @@ def zadj_tile(g, optin=OPTIN):
 
 SIZES = [(128, 80, 37, 37), (64, 64, 11, 11), (64, 40, 19, 19), (96, 48, 21, 21), (128, 128, 37, 37), (16, 12, 5, 3),
          (64, 1, 11, 1), (128, 1, 11, 1), (256, 200, 65, 65), (64, 90, 21, 21), (40, 37, 9, 9), (8, 5, 5, 5),
-         (512, 96, 21, 21), (256, 17, 63, 3), (24, 230, 7, 65)]
+         (512, 96, 21, 21), (256, 17, 63, 3), (24, 230, 7, 65), (90, 53, 21, 17), (46, 80, 7, 7), (82, 73, 17, 17),
+         (34, 9, 5, 3), (2, 1, 1, 1), (6, 3, 3, 3), (170, 1, 7, 1), (122, 100, 25, 25)]
 
 
 @pytest.mark.parametrize("nx,nz,px,pz", SIZES)
