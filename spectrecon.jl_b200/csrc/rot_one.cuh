@@ -14,6 +14,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "zpath_api.h"  // Rot1View
+
 namespace spect {
 
 constexpr int kRot1Threads = 512;
@@ -21,14 +23,6 @@ constexpr int kRot1Warps = kRot1Threads / 32;
 
 struct Rot1Geom {
   int nx, ny, nz, L, pad, LS;
-};
-
-// per view: mode 0 copy (theta == 0 mod 2pi), 1 rot_f90 only (theta close
-// to m*pi/2), 2 rot_f90 + shears; tn = tan(phi/2), sn = -sin(phi),
-// phi = theta - m*pi/2 (src/rotatez.jl:249-272)
-struct Rot1View {
-  double tn, sn;
-  int m, mode;
 };
 
 // linearinterp!(A, s, e, len) for the line with 1-based index i; the output
@@ -87,7 +81,9 @@ __device__ __forceinline__ void line_adj(const Line1& P, const float* __restrict
       if (qh >= 0 && qh < L) acc = __fadd_rn(acc, __fmul_rn(P.chi, x[qh]));
       if (ql >= 0 && ql < L) acc = __fadd_rn(acc, __fmul_rn(P.clo, x[ql]));
     } else {
-      for (int q = 0; q < L; ++q) {
+      // only the clamped range of q reaches the edge (the others' J differ)
+      const int q0 = P.caseA ? 0 : max(0, L - P.F - 1), q1 = P.caseA ? min(L - 1, 1 + L - P.K) : L - 1;
+      for (int q = q0; q <= q1; ++q) {
         if (P.jlo(q, L) == j) acc = __fadd_rn(acc, __fmul_rn(P.clo, x[q]));
         if (P.jhi(q, L) == j) acc = __fadd_rn(acc, __fmul_rn(P.chi, x[q]));
       }

@@ -558,6 +558,7 @@ ZArgs zargs(const spect_plan_s* p) {
   a.tab = p->d_Zt;
   a.rot = p->d_rot;
   a.viewset = p->d_viewset;
+  a.r1 = p->interp == SPECT_INTERP_ONE ? p->d_r1view : nullptr;
   a.err = p->d_err;
   return a;
 }
@@ -631,7 +632,7 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
     LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
     LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
+           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, a.r1, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
                            last ? outIZ : p->d_backIZ, xIZ, asumIZ, last ? mode : 0));
   }
   return SPECT_OK;
@@ -770,7 +771,7 @@ int backward(spect_plan_s* p, float* image, const float* views, const int* vidx,
       LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
              zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, vi, nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
+             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, vi, nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
                              nullptr, nullptr, 0));
     } else if (p->interp == SPECT_INTERP_ONE) {
       const size_t n = (size_t)nv * p->N;
@@ -1506,15 +1507,16 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     const char* senv = std::getenv("SPECT_ZSTRIP");
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
-        interpmeth == SPECT_INTERP_TWO && sep_host && !only_fft && !(zenv && zenv[0] == '0') &&
+        sep_host && !only_fft && !(zenv && zenv[0] == '0') &&
         zg_full.zpw <= 72 && zg_full.xpw <= 72 &&  // pass rows of at most 9 blocks of 8 taps
         zg.nzp <= 256 && opts.atten_cache != 0) {
       p->zat = zadj_tile(zg, (size_t)optin);
       const bool adj = p->zat.w != 0;
-      p->zft = zfwd_tile(zg, (size_t)optin);
+      const bool one = interpmeth == SPECT_INTERP_ONE;
+      p->zft = zfwd_tile(zg, (size_t)optin, one);
       const bool fused = adj && p->zft.w != 0;
       if (!fused) p->zft.ystep = zdepth_step(ny);  // the walk of the large-plane kernels
-      const bool strip = adj && nx % 8 == 0 && zs_tiles(zg, (size_t)optin, &zt);
+      const bool strip = adj && !one && nx % 8 == 0 && zs_tiles(zg, (size_t)optin, &zt);
       if (fused && !(senv && senv[0] == '1')) zkind = 1;
       else if (strip && !(senv && senv[0] == '0')) zkind = 2;
       else if (fused) zkind = 1;
@@ -1536,15 +1538,16 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     }
     bool want = !(env && env[0] == '0') && need <= std::min(fr / 4, (size_t)32 << 30);
     if (opts.atten_cache >= 0) want = opts.atten_cache == 1;
-    if (interpmeth == SPECT_INTERP_ONE) {
-      // the :one path reads its attenuation from the cache
-      int st1 = dalloc(p, &p->d_att, p->N * (size_t)nview);
-      if (st1 != SPECT_OK) return bail(st1);
-    } else if (want && dalloc(p, &p->d_att, cnt) != SPECT_OK) {
+    if ((interpmeth == SPECT_INTERP_TWO || zcand) && want && dalloc(p, &p->d_att, cnt) != SPECT_OK) {
       p->d_att = nullptr;
       g_err.clear();
     }
     p->zpath = (zcand && p->d_att) ? zkind : 0;
+    if (interpmeth == SPECT_INTERP_ONE && !p->d_att) {
+      // the split :one path reads its attenuation from the cache
+      int st1 = dalloc(p, &p->d_att, p->N * (size_t)nview);
+      if (st1 != SPECT_OK) return bail(st1);
+    }
   }
   int st = configure(p);
   if (st != SPECT_OK) return bail(st);
@@ -1618,6 +1621,8 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
           (st = dalloc(p, &p->d_Tz, (size_t)p->gmax * ny * nx * zg.nzp + zg.nzp)))
         return bail(st);
       p->tzero = (size_t)p->gmax * ny * nx * zg.nzp;
+      const cudaError_t ze = zrot_adj_setup();
+      if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("gather adjoint setup: ") + cudaGetErrorString(ze)));
       if (cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
           cudaMemsetAsync(p->d_Tz + p->tzero, 0, sizeof(float) * zg.nzp, p->home) != cudaSuccess)
         return bail(fail(SPECT_ERR_CUDA, "memset"));
@@ -1667,10 +1672,11 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       return bail(fail(SPECT_ERR_CUDA, "k_rot1_adj shared memory"));
     p->r1_grid_y = std::max(1, cdiv(4 * p->sm_count, nz));
     size_t gs = 0;
+    if (p->zpath) p->r1f_smem_ok = p->r1a_smem_ok = 1;  // the fused pair runs neither kernel
     if (!p->r1f_smem_ok) gs = std::max(gs, (size_t)nz * p->r1_grid_y * (p->r1f_smem / sizeof(float)));
     if (!p->r1a_smem_ok) gs = std::max(gs, (size_t)nz * p->nsplit_adj_max * (p->r1a_smem / sizeof(float)));
     if (gs && (st = dalloc(p, &p->d_gscr_r1, gs))) return bail(st);
-    if ((st = dalloc(p, &p->d_R1, (size_t)p->gmax * p->N)) || (st = dalloc(p, &p->d_r1view, nview)))
+    if ((!p->zpath && (st = dalloc(p, &p->d_R1, (size_t)p->gmax * p->N))) || (st = dalloc(p, &p->d_r1view, nview)))
       return bail(st);
     std::vector<Rot1View> rv(nview);
     const double kHalfPi = 1.5707963267948966;
@@ -1697,7 +1703,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     if ((st = up(p->d_r1view, rv.data(), sizeof(Rot1View) * nview))) return bail(st);
   }
 
-  if (p->d_att && interpmeth == SPECT_INTERP_ONE) {
+  if (p->d_att && interpmeth == SPECT_INTERP_ONE && !p->zpath) {
     // :one-rotated mu-map per group of views, then the depth scan
     cudaError_t e = cudaSuccess;
     for (int v0 = 0; v0 < nview && e == cudaSuccess; v0 += p->gmax) {
@@ -1722,7 +1728,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
                                    : cudaMalloc((void**)&muz, sizeof(float) * p->izN);
     if (e == cudaSuccess) e = cudaMemsetAsync(muz, 0, sizeof(float) * p->izN, hs);
     if (e == cudaSuccess) e = zto_iz_launch(p->zg, hs, p->d_mumap, muz);
-    if (e == cudaSuccess) e = zatten_launch(p->zg, nview, hs, muz, p->d_rot, dy, p->d_att);
+    if (e == cudaSuccess) e = zatten_launch(p->zg, nview, hs, muz, p->d_rot, p->d_r1view, dy, p->d_att);
     if (e == cudaSuccess) e = cudaStreamSynchronize(hs);
     if (muz) dfree(p, muz);
     if (e != cudaSuccess) {
@@ -2442,7 +2448,7 @@ size_t est_job_bytes(const ServerJob& j, bool att) {
              + 8 * N + 2 * (size_t)j.nview * nxz + (size_t)j.nblocks * N  // imgpart, EM buffers
              + 2 * N + 2 * (size_t)j.nview * nxz;     // job buffers
   if (j.interp == SPECT_INTERP_ONE) f += nsub * N;
-  else f += 2 * nsub * (size_t)j.nx * j.nx * ((j.nz + 15) / 16 * 16) + 2 * N;  // z-fastest planes and tiles, IZ volumes
+  f += 2 * nsub * (size_t)j.nx * j.nx * ((j.nz + 15) / 16 * 16) + 2 * N;  // z-fastest planes and tiles, IZ volumes
   size_t b = 4 * f + (size_t)j.nview * 32;
   // per-CTA global slabs of large planes (B, spectra accumulators)
   if ((size_t)j.nx * (Q + 1) * 8 + 8192 > 227 * 1024) b += (size_t)148 * j.nx * (Q + 1) * 8;

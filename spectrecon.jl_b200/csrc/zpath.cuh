@@ -316,28 +316,142 @@ __device__ __forceinline__ void zgeo(const ZGeom& g, float cs, float sn, bool id
   off = ((j2 + g.pad) * g.L + j1 + g.pad) * g.nzp;
 }
 
+// The three shears of imrotate! :one (src/rotatez.jl:240-322) as one gather.
+// A line's shear is out(q) = lo in(q + off) + (1 - lo) in(q + off + 1)
+// (linearinterp!, src/rotatez.jl:21-51: positions in Float64), so an output
+// point of the cropped grid is the sum of 2 x 2 x 2 taps of the padded image.
+// The index clamps of linearinterp! never reach such a point with a nonzero
+// value: its own x shear stays inside the padded grid, and a clamped y or
+// first x shear reads the grid's zero ring.  Weights are products in Float64,
+// rounded once.
+// Measured, 96x96x48, 15 of 90 views, 21 taps, forward and adjoint: 1437 us of
+// kernels with the line-by-line passes (k_rot1_fwd, k_rot1_adj, the convolution
+// and attenuation kernels around them), 100 us here.
+struct OneLine {
+  double lo;
+  int off;
+};
+__device__ __forceinline__ OneLine one_line(int i, double t, int L) {  // 0-based line i
+  const double s = (i + 1 - (L + 1) / 2.0) * t + 1;
+  const double c = ceil(s);
+  return OneLine{c - s, s <= 1 ? (int)c - 2 : (int)floor(s) - 1};
+}
+// taps of rotated-grid point (x, y): off[k], off[k] + delta with the weights
+// w[2 k], w[2 k + 1]; delta = one_delta(view): the next element along the
+// first shear's lines, in IZ, after rot_f90! by m
+__device__ __forceinline__ int one_delta(const ZGeom& g, int m) {
+  return m == 0 ? g.nzp : m == 1 ? -g.L * g.nzp : m == 2 ? -g.nzp : g.L * g.nzp;
+}
+__device__ __forceinline__ void one_geo(const ZGeom& g, const Rot1View& V, int x, int y, float (&w)[8], int (&off)[4]) {
+  const int L = g.L, a = g.pad + x, b = g.pad + y, m = V.mode == 0 ? 0 : V.m;
+  auto pos = [&](int p, int q) {  // IZ column of element (p, q) after rot_f90! by m
+    const int u = m == 0 ? p : m == 1 ? q : m == 2 ? L - 1 - p : L - 1 - q;
+    const int v = m == 0 ? q : m == 1 ? L - 1 - p : m == 2 ? L - 1 - q : p;
+    return (v * L + u) * g.nzp;
+  };
+  const int ring = (L + 1) * g.nzp;  // column (1, 1): zero, and its neighbours too (pad >= 2)
+#pragma unroll
+  for (int k = 0; k < 8; ++k) w[k] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) off[k] = ring;
+  if (V.mode != 2) {
+    off[0] = pos(a, b);
+    w[0] = 1.f;
+    return;
+  }
+  const OneLine l3 = one_line(b, V.tn, L);
+#pragma unroll
+  for (int e3 = 0; e3 < 2; ++e3) {
+    const int a1 = a + l3.off + e3;
+    if (a1 < 0 || a1 >= L) continue;
+    const OneLine l2 = one_line(a1, V.sn, L);
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int b1 = b + l2.off + e2;
+      if (b1 < 0 || b1 >= L) continue;
+      const OneLine l1 = one_line(b1, V.tn, L);
+      const int a0 = a1 + l1.off;
+      if (a0 < 0 || a0 > L - 2) continue;
+      const double w32 = (e3 ? 1.0 - l3.lo : l3.lo) * (e2 ? 1.0 - l2.lo : l2.lo);
+      off[2 * e3 + e2] = pos(a0, b1);
+      w[4 * e3 + 2 * e2] = (float)(w32 * l1.lo);
+      w[4 * e3 + 2 * e2 + 1] = (float)(w32 * (1.0 - l1.lo));
+    }
+  }
+}
+
+// the transpose of one_geo: hit(x, y, w) for the rotated-grid points that read
+// image column (j1, j2) with a weight that is not zero
+template <class F>
+__device__ __forceinline__ void one_hits(const ZGeom& g, const Rot1View& V, int j1, int j2, F hit) {
+  const int L = g.L, p = g.pad + j1, q = g.pad + j2, m = V.mode == 0 ? 0 : V.m, nx = g.nx, pad = g.pad;
+  const int A = m == 0 ? p : m == 1 ? L - 1 - q : m == 2 ? L - 1 - p : q;  // rot_f90! by m
+  const int B = m == 0 ? q : m == 1 ? p : m == 2 ? L - 1 - q : L - 1 - p;
+  if (V.mode != 2) {
+    if (A >= pad && A < pad + nx && B >= pad && B < pad + nx) hit(A - pad, B - pad, 1.f);
+    return;
+  }
+  const OneLine l1 = one_line(B, V.tn, L);
+#pragma unroll
+  for (int e1 = 0; e1 < 2; ++e1) {
+    const int a1 = A - l1.off - e1;
+    if (a1 < 0 || a1 >= L) continue;
+    const OneLine l2 = one_line(a1, V.sn, L);
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int b = B - l2.off - e2;
+      if (b < pad || b >= pad + nx) continue;
+      const OneLine l3 = one_line(b, V.tn, L);
+#pragma unroll
+      for (int e3 = 0; e3 < 2; ++e3) {
+        const int a = a1 - l3.off - e3;
+        if (a < pad || a >= pad + nx) continue;
+        const float w = (float)((e1 ? 1.0 - l1.lo : l1.lo) * (e2 ? 1.0 - l2.lo : l2.lo) * (e3 ? 1.0 - l3.lo : l3.lo));
+        if (w != 0.f) hit(a - pad, b - pad, w);
+      }
+    }
+  }
+}
+
 // Attenuation cache in the ATT layout: block (column x, view v), one thread
 // per z (nzp threads); each walks y and scans the rotated mu-map (bilinear
 // sample of the IZ-laid-out mu-map with bilinear()'s fmul/fadd order), as
 // k_atten_build does.
+template <bool ONE>
 __global__ void __launch_bounds__(256) k_zatten(ZGeom g, const float* __restrict__ muz,
-                                               const float4* __restrict__ rot, float dy, float* __restrict__ att) {
+                                               const float4* __restrict__ rot, const Rot1View* __restrict__ r1, float dy,
+                                               float* __restrict__ att) {
   const int x = blockIdx.x, v = blockIdx.y, z = threadIdx.x;
   if (z >= g.nzp) return;
-  const float4 r = rot[v];
-  const bool ident = r.z != 0.f;
   const float mdy = -dy;
   float prefix = 0.f;
   const size_t Lz = (size_t)g.L * g.nzp;
   for (int y = 0; y < g.ny; ++y) {
-    float4 w;
-    int off;
-    zgeo(g, r.x, r.y, ident, x, y, w, off);
-    const float* p = muz + off + z;
-    float m = __fmul_rn(w.x, p[0]);
-    m = __fadd_rn(m, __fmul_rn(w.y, p[g.nzp]));
-    m = __fadd_rn(m, __fmul_rn(w.z, p[Lz]));
-    m = __fadd_rn(m, __fmul_rn(w.w, p[Lz + g.nzp]));
+    float m;
+    if constexpr (ONE) {
+      float w[8];
+      int off[4];
+      const Rot1View V = r1[v];
+      const int d = one_delta(g, V.mode == 0 ? 0 : V.m);
+      one_geo(g, V, x, y, w, off);
+      m = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float* p = muz + off[k] + z;
+        m = fmaf(w[2 * k], p[0], m);
+        m = fmaf(w[2 * k + 1], p[d], m);
+      }
+    } else {
+      const float4 r = rot[v];
+      float4 w;
+      int off;
+      zgeo(g, r.x, r.y, r.z != 0.f, x, y, w, off);
+      const float* p = muz + off + z;
+      m = __fmul_rn(w.x, p[0]);
+      m = __fadd_rn(m, __fmul_rn(w.y, p[g.nzp]));
+      m = __fadd_rn(m, __fmul_rn(w.z, p[Lz]));
+      m = __fadd_rn(m, __fmul_rn(w.w, p[Lz + g.nzp]));
+    }
     const float e = __fadd_rn(prefix, __fmul_rn(0.5f, m));
     att[(((size_t)v * g.ny + y) * g.nx + x) * g.nzp + z] = z < g.nz ? expf(__fmul_rn(e, mdy)) : 0.f;
     prefix = __fadd_rn(prefix, m);
@@ -403,9 +517,10 @@ __global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ 
 // 573 us; 64x64x40, 19 taps, 60 views 107 -> 38 us; 128x128x1, 80 views 229 ->
 // 50 us (the former kernel staged the attenuation plane in shared memory, ran
 // one line a lane and one block per SM, and dealt chunks of 15 planes).
+// ONE: the :one rotation (eight taps a column, one_geo).
 // Shared memory: [2 tables][geoW nx x (w00 w00 w10 w10 | w01 w01 w11 w11)]
 // [geoO nx int][ZB nxp * vst][XB (nz + 1) / 2 * bst] (lines: float2).
-template <int NT>
+template <int NT, bool ONE>
 __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int X = kZfwdX, W = kZfwdZ;
@@ -415,8 +530,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
   const int trow = ztable_floats(g), tid = threadIdx.x, nth = blockDim.x;
   float* const tab0 = reinterpret_cast<float*>(smem4);
   float4* const geoW = reinterpret_cast<float4*>(tab0 + 2 * trow);
-  int* const geoO = reinterpret_cast<int*>(geoW + 2 * nx);
-  f2* const ZB = reinterpret_cast<f2*>(geoO + zround(nx, 4));
+  int* const geoO = reinterpret_cast<int*>(geoW + (ONE ? 4 : 2) * nx);
+  f2* const ZB = reinterpret_cast<f2*>(geoO + (ONE ? 4 * nx : zround(nx, 4)));
   f2* const XB = ZB + (size_t)nxp * vst;
   const int n = a.nv * ny;
   const int p0 = (int)((long long)blockIdx.x * n / gridDim.x), p1 = (int)((long long)(blockIdx.x + 1) * n / gridDim.x);
@@ -431,34 +546,65 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
   };
   auto geometry = [&](int view, int yy) {
     if (tid >= nx) return;
-    const float4 r = a.rot[view];
-    for (int x = tid; x < nx; x += nth) {
-      float4 w;
-      int off;
-      zgeo(g, r.x, r.y, r.z != 0.f, x, yy, w, off);
-      geoW[2 * x] = make_float4(w.x, w.x, w.y, w.y);
-      geoW[2 * x + 1] = make_float4(w.z, w.z, w.w, w.w);
-      geoO[x] = off;
+    if constexpr (ONE) {
+      const Rot1View V = a.r1[view];
+      for (int x = tid; x < nx; x += nth) {
+        float w[8];
+        int off[4];
+        one_geo(g, V, x, yy, w, off);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) geoW[4 * x + k] = make_float4(w[2 * k], w[2 * k], w[2 * k + 1], w[2 * k + 1]);
+        reinterpret_cast<int4*>(geoO)[x] = make_int4(off[0], off[1], off[2], off[3]);
+      }
+    } else {
+      const float4 r = a.rot[view];
+      for (int x = tid; x < nx; x += nth) {
+        float4 w;
+        int off;
+        zgeo(g, r.x, r.y, r.z != 0.f, x, yy, w, off);
+        geoW[2 * x] = make_float4(w.x, w.x, w.y, w.y);
+        geoW[2 * x + 1] = make_float4(w.z, w.z, w.w, w.w);
+        geoO[x] = off;
+      }
     }
   };
   // rotated, attenuated column x at z group z4: four z as two packed pairs
   const int nz4 = (nz + 3) / 4, dq = nth / nz4, dr = nth - dq * nz4, q0 = tid / nz4, r0 = tid - q0 * nz4;
-  auto sample = [&](const float* att, int x, int z4, f2& lo, f2& hi) {
-    const float* p = a.img + geoO[x] + 4 * z4;
-    const ulonglong2 t0 = ldp(p), t1 = ldp(p + nzp), t2 = ldp(p + Lz), t3 = ldp(p + Lz + nzp);
-    const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
-    const ulonglong2 wa = reinterpret_cast<const ulonglong2*>(geoW)[2 * x];  // (w00, w00), (w10, w10)
-    const ulonglong2 wb = reinterpret_cast<const ulonglong2*>(geoW)[2 * x + 1];
-    lo = mul2(fma2(wb.y, t3.x, fma2(wb.x, t2.x, fma2(wa.y, t1.x, mul2(wa.x, t0.x)))), at.x);
-    hi = mul2(fma2(wb.y, t3.y, fma2(wb.x, t2.y, fma2(wa.y, t1.y, mul2(wa.x, t0.y)))), at.y);
+  auto sample = [&](const float* att, int d, int x, int z4, f2& lo, f2& hi) {
+    if constexpr (ONE) {
+      const int4 o4 = reinterpret_cast<const int4*>(geoO)[x];
+      const int os[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float* p = a.img + os[k] + 4 * z4;
+        const ulonglong2 t0 = ldp(p), t1 = ldp(p + d);
+        const ulonglong2 w = reinterpret_cast<const ulonglong2*>(geoW)[4 * x + k];
+        lo = fma2(w.y, t1.x, k ? fma2(w.x, t0.x, lo) : mul2(w.x, t0.x));
+        hi = fma2(w.y, t1.y, k ? fma2(w.x, t0.y, hi) : mul2(w.x, t0.y));
+      }
+      const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
+      lo = mul2(lo, at.x);
+      hi = mul2(hi, at.y);
+      return;
+    } else {
+      const float* p = a.img + geoO[x] + 4 * z4;
+      const ulonglong2 t0 = ldp(p), t1 = ldp(p + nzp), t2 = ldp(p + Lz), t3 = ldp(p + Lz + nzp);
+      const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
+      const ulonglong2 wa = reinterpret_cast<const ulonglong2*>(geoW)[2 * x];  // (w00, w00), (w10, w10)
+      const ulonglong2 wb = reinterpret_cast<const ulonglong2*>(geoW)[2 * x + 1];
+      lo = mul2(fma2(wb.y, t3.x, fma2(wb.x, t2.x, fma2(wa.y, t1.x, mul2(wa.x, t0.x)))), at.x);
+      hi = mul2(fma2(wb.y, t3.y, fma2(wb.x, t2.y, fma2(wa.y, t1.y, mul2(wa.x, t0.y)))), at.y);
+    }
   };
   const int hi4 = (tid >> 2) & 1;
   auto gather = [&](int view, int yy) {  // unit (column pair, z group)
     const float* att = a.att + (((size_t)view * ny + yy) * nx) * nzp;
+    int d = 0;
+    if constexpr (ONE) d = one_delta(g, a.r1[view].mode == 0 ? 0 : a.r1[view].m);
     for (int xp = q0, z4 = r0; xp < nxp;) {
       f2 al, ah, bl, bh;
-      sample(att, 2 * xp, z4, al, ah);
-      sample(att, 2 * xp + 1, z4, bl, bh);
+      sample(att, d, 2 * xp, z4, al, ah);
+      sample(att, d, 2 * xp + 1, z4, bl, bh);
       // a lane's 32 bytes as two stores, the halves in turn by lane group of
       // four: the eight lanes of an access phase hit distinct bank groups
       float4* o = reinterpret_cast<float4*>(ZB + xp * vst + R0 + 4 * z4);
@@ -844,8 +990,10 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
 // 256x256x200, 8 views 252 -> 216 us.
 // Epilogue (IZ layout): v = acc (+ prev); mode 1: zeros -> +Inf; mode 2:
 // v = x * (v / asum); out = v (z < nz only; out may be prev or x).
+template <bool ONE>
 __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* __restrict__ T,
                                                              int zcol, const float4* __restrict__ rot,
+                                                             const Rot1View* __restrict__ r1,
                                                              const int* __restrict__ vidx, int nv, const float* prev,
                                                              float* out, const float* x,
                                                              const float* __restrict__ asum, int mode) {
@@ -866,26 +1014,32 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
     int2* const L0 = list + (buf * nth + tid) * E;
     int2* L = L0;
     if (ps < r.vb && s < nv && pj1 < nx && pj2 < nx) {
-      const float4 rt = rot[vidx[s]];
-      const float cs = rt.x, sn = rt.y;
-      const float xc = c0 + cs * d1 + sn * d2, yc = c0 - sn * d1 + cs * d2;
-      const float rr = fabsf(cs) + fabsf(sn) + 0.01f;
-      const int xlo = max(0, (int)ceilf(xc - rr)), nxc = min(nx - 1, (int)floorf(xc + rr)) - xlo;
-      const int ylo = max(0, (int)ceilf(yc - rr)), nyc = min(ny - 1, (int)floorf(yc + rr)) - ylo;
-      const int base = (s * ny + ylo) * nx + xlo;
+      if constexpr (ONE) {
+        one_hits(g, r1[vidx[s]], pj1, pj2, [&](int xx, int yy, float w) {
+          *L++ = make_int2((s * ny + yy) * nx + xx, __float_as_int(w));
+        });
+      } else {
+        const float4 rt = rot[vidx[s]];
+        const float cs = rt.x, sn = rt.y;
+        const float xc = c0 + cs * d1 + sn * d2, yc = c0 - sn * d1 + cs * d2;
+        const float rr = fabsf(cs) + fabsf(sn) + 0.01f;
+        const int xlo = max(0, (int)ceilf(xc - rr)), nxc = min(nx - 1, (int)floorf(xc + rr)) - xlo;
+        const int ylo = max(0, (int)ceilf(yc - rr)), nyc = min(ny - 1, (int)floorf(yc + rr)) - ylo;
+        const int base = (s * ny + ylo) * nx + xlo;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const float di = __fsub_rn((float)(xlo + i), c0), ci = __fmul_rn(cs, di), si = __fmul_rn(sn, di);
+        for (int i = 0; i < 3; ++i) {
+          const float di = __fsub_rn((float)(xlo + i), c0), ci = __fmul_rn(cs, di), si = __fmul_rn(sn, di);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float dj = __fsub_rn((float)(ylo + k), c0);
-          const float s1 = __fadd_rn(c0, __fsub_rn(ci, __fmul_rn(sn, dj)));
-          const float s2 = __fadd_rn(c0, __fadd_rn(si, __fmul_rn(cs, dj)));
-          // floor(s) == j: 1 - (s - j); floor(s) == j - 1: s - (j - 1); not positive elsewhere
-          const float a1 = s1 >= fj1 ? __fsub_rn(1.0f, __fsub_rn(s1, fj1)) : __fsub_rn(s1, fj1 - 1.f);
-          const float a2 = s2 >= fj2 ? __fsub_rn(1.0f, __fsub_rn(s2, fj2)) : __fsub_rn(s2, fj2 - 1.f);
-          if (i <= nxc && k <= nyc && fminf(a1, a2) > 0.f) {
-            *L++ = make_int2(base + k * nx + i, __float_as_int(__fmul_rn(a1, a2)));
+          for (int k = 0; k < 3; ++k) {
+            const float dj = __fsub_rn((float)(ylo + k), c0);
+            const float s1 = __fadd_rn(c0, __fsub_rn(ci, __fmul_rn(sn, dj)));
+            const float s2 = __fadd_rn(c0, __fadd_rn(si, __fmul_rn(cs, dj)));
+            // floor(s) == j: 1 - (s - j); floor(s) == j - 1: s - (j - 1); not positive elsewhere
+            const float a1 = s1 >= fj1 ? __fsub_rn(1.0f, __fsub_rn(s1, fj1)) : __fsub_rn(s1, fj1 - 1.f);
+            const float a2 = s2 >= fj2 ? __fsub_rn(1.0f, __fsub_rn(s2, fj2)) : __fsub_rn(s2, fj2 - 1.f);
+            if (i <= nxc && k <= nyc && fminf(a1, a2) > 0.f) {
+              *L++ = make_int2(base + k * nx + i, __float_as_int(__fmul_rn(a1, a2)));
+            }
           }
         }
       }

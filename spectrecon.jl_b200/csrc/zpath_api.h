@@ -76,9 +76,18 @@ constexpr int kZfwdNT = 2;      // x tasks a thread at most (their outputs stay 
 constexpr int kZadjX = 8;       // outputs of an x-pass task of k_zadj
 constexpr int kZThreads = 640;  // threads per SM the pair-pass kernels' registers allow (96 each)
 
+// :one rotation of a view (src/rotatez.jl:240-322): mode 0 copy (theta == 0
+// mod 2pi), 1 rot_f90 only (theta close to m*pi/2), 2 rot_f90 + shears; tn =
+// tan(phi/2), sn = -sin(phi), phi = theta - m*pi/2 (src/rotatez.jl:249-272)
+struct Rot1View {
+  double tn, sn;
+  int m, mode;
+};
+
 struct ZArgs {
   ZGeom g;
   ZTile t;
+  const Rot1View* r1;   // [nview] :one rotation; null for :two
   const float* tab;     // [set][y][2][ztable_floats]: forward, adjoint tables
   const float* img;     // IZ
   const float* att;     // ATT
@@ -99,8 +108,9 @@ struct ZArgs {
 };
 
 // k_zfwd shared memory (zpath.cuh)
-inline size_t zfwd_smem(const ZGeom& g, const ZTile& t) {
-  return sizeof(float) * (2 * (size_t)ztable_floats(g) + 8 * (size_t)g.nx + zround(g.nx, 4) +
+// (one: the eight taps a column of the :one rotation in place of four)
+inline size_t zfwd_smem(const ZGeom& g, const ZTile& t, bool one) {
+  return sizeof(float) * (2 * (size_t)ztable_floats(g) + (one ? 20 : 8) * (size_t)g.nx + (one ? 0 : zround(g.nx, 4)) +
                           2 * ((size_t)(g.nx / 2) * t.vst + (size_t)((g.nz + 1) / 2) * t.bst));
 }
 // k_zadj shared memory (zpath.cuh)
@@ -169,7 +179,7 @@ inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
 // tiling of k_zfwd (w == 0: the plane does not fit): kZfwdNT x tasks a thread
 // (their outputs stay in registers over the planes); threads for them, for
 // half the z tasks and for a quarter of the gather units
-inline ZTile zfwd_tile(const ZGeom& g, size_t optin) {
+inline ZTile zfwd_tile(const ZGeom& g, size_t optin, bool one) {
   ZTile t{};
   const int nxw = (g.nx + kZfwdX - 1) / kZfwdX, nzb = (g.nz + kZfwdZ - 1) / kZfwdZ, xt = (g.nz + 1) / 2 * nxw;
   if (xt > kZfwdNT * kZThreads) return t;
@@ -177,7 +187,7 @@ inline ZTile zfwd_tile(const ZGeom& g, size_t optin) {
   t.ntile = t.nxb = 1;
   t.vst = zstride2(kZfwdZ * nzb + g.zpw);
   t.bst = zstride2(kZfwdX * nxw + g.xpw);
-  t.smem = zfwd_smem(g, t);
+  t.smem = zfwd_smem(g, t, one);
   if (t.smem > optin) return t;
   const int zh = ((g.nx / 2) * nzb + 1) / 2, gq = ((g.nx / 2) * ((g.nz + 3) / 4) + 3) / 4;
   t.nxt = xt <= kZThreads ? 1 : kZfwdNT;
@@ -236,15 +246,16 @@ inline ZRotTile zrot_tile(const ZGeom& g, int nv, int sms) {
 }
 
 // launchers (zpath_inst.cu)
-cudaError_t zpath_setup(int max_smem);
+cudaError_t zpath_setup(int max_smem);  // shared-memory limits of the fused kernels (zrot_adj_setup's too)
+cudaError_t zrot_adj_setup();
 cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
 // views (EM ratio with y, bg) of nv slots from the partial views of a walk by G blocks
 cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
                            const float* y, const float* bg, const int* vidx);
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
-                            const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,
-                            int mode);  // T[zero ..]: a column of zeros
+                            const Rot1View* r1, const int* vidx, int nv, const float* prev, float* out, const float* x,
+                            const float* asum, int mode);  // T[zero ..]: a column of zeros; r1: null for :two
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz);
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx);
@@ -256,7 +267,7 @@ cudaError_t zstrip_setup(int max_smem);
 cudaError_t zstrip_occupancy(int w, int fz_nth, const size_t smem[2], int occ[2]);
 cudaError_t zs_fz_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
 cudaError_t zs_fx_launch(int w, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
-cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot, float dy,
-                          float* att);
+cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot,
+                          const Rot1View* r1, float dy, float* att);
 
 }  // namespace spect

@@ -7,13 +7,24 @@
 namespace spect {
 
 namespace {
+// [x tasks a thread - 1][rotation :two, :one]
+const void* const kZfwd[2][2] = {{(const void*)k_zfwd<1, false>, (const void*)k_zfwd<1, true>},
+                                 {(const void*)k_zfwd<2, false>, (const void*)k_zfwd<2, true>}};
 const void* const kZadj[2] = {(const void*)k_zadj<8>, (const void*)k_zadj<16>};
 
 }  // namespace
 
-cudaError_t zpath_setup(int max_smem) {
+cudaError_t zrot_adj_setup() {
   cudaError_t e = cudaSuccess;
-  for (const void* k : {(const void*)k_zfwd<1>, (const void*)k_zfwd<2>})
+  for (const void* k : {(const void*)k_zrot_adj<false>, (const void*)k_zrot_adj<true>})
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kZrotThreads * 2 * kZrotList * 8);
+  return e;
+}
+
+cudaError_t zpath_setup(int max_smem) {
+  cudaError_t e = zrot_adj_setup();
+  for (const void* k : {kZfwd[0][0], kZfwd[0][1], kZfwd[1][0], kZfwd[1][1]})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   for (const void* k : kZadj)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
@@ -21,9 +32,9 @@ cudaError_t zpath_setup(int max_smem) {
 }
 
 cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a) {
-  if (a.t.nxt == 1) k_zfwd<1><<<grid, a.t.nth, a.t.smem, st>>>(a);
-  else k_zfwd<2><<<grid, a.t.nth, a.t.smem, st>>>(a);
-  return cudaGetLastError();
+  ZArgs c = a;
+  void* args[] = {&c};
+  return cudaLaunchKernel(kZfwd[a.t.nxt - 1][a.r1 ? 1 : 0], dim3(grid), dim3(a.t.nth), args, a.t.smem, st);
 }
 
 cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
@@ -40,15 +51,11 @@ cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {
 }
 
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
-                            const int* vidx, int nv, const float* prev, float* out, const float* x, const float* asum,
-                            int mode) {
+                            const Rot1View* r1, const int* vidx, int nv, const float* prev, float* out, const float* x,
+                            const float* asum, int mode) {
   const ZRotTile r = zrot_tile(g, nv, sms);
-  if (r.smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute((const void*)k_zrot_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kZrotThreads * 2 * kZrotList * 8);
-    if (e != cudaSuccess) return e;
-  }
-  k_zrot_adj<<<r.grid, r.nth, r.smem, st>>>(g, r, T, (int)(zero / g.nzp), rot, vidx, nv, prev, out, x, asum, mode);
+  const auto kernel = r1 ? k_zrot_adj<true> : k_zrot_adj<false>;
+  kernel<<<r.grid, r.nth, r.smem, st>>>(g, r, T, (int)(zero / g.nzp), rot, r1, vidx, nv, prev, out, x, asum, mode);
   return cudaGetLastError();
 }
 
@@ -107,9 +114,10 @@ cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, fl
   return cudaGetLastError();
 }
 
-cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot, float dy,
-                          float* att) {
-  k_zatten<<<dim3(g.nx, nview), g.nzp, 0, st>>>(g, muz, rot, dy, att);
+cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot,
+                          const Rot1View* r1, float dy, float* att) {
+  if (r1) k_zatten<true><<<dim3(g.nx, nview), g.nzp, 0, st>>>(g, muz, rot, r1, dy, att);
+  else k_zatten<false><<<dim3(g.nx, nview), g.nzp, 0, st>>>(g, muz, rot, r1, dy, att);
   return cudaGetLastError();
 }
 

@@ -67,3 +67,31 @@ def test_ragged_osem_and_view_dependent_psfs(S, O):
     bg = np.full(yn.shape, 0.05, np.float32, order="F")
     x0 = np.ones(x.shape, np.float32, order="F")
     assert relerr(S.osem(x0, yn, bg, S.Ablock(plan, 4), niter=2), G.osem(x0, yn, bg, 4, 2)) <= TOL
+
+
+@pytest.mark.parametrize("nx,nz,px,pz,nview,idx", [
+    (32, 20, 5, 3, 8, None),           # views at multiples of 45 and 90 degrees
+    (46, 17, 7, 7, 11, [10, 0, 3]),    # a partial x task, an odd last row
+    (2, 1, 1, 1, 5, None),
+    (128, 80, 37, 37, 120, [0, 30, 44, 97]),
+])
+def test_shear_rotation_on_the_fused_pair(S, O, monkeypatch, nx, nz, px, pz, nview, idx):
+    """:one (three shears) as one gather of eight taps and its transpose,
+    against the line-by-line kernels of the split path and the oracles; image
+    and views are dense up to the corners, where the shears reach the edge of
+    the padded grid."""
+    mumap, psfs, x, y = _plan_inputs(S, nx, nz, px, pz, nview, 5 * nx + nz)
+    ii = None if idx is None else np.array(idx, np.int32)
+    ys = y if ii is None else np.asfortranarray(y[:, :, ii])
+    out = {}
+    for path in ("fused", "split"):
+        monkeypatch.setenv("SPECT_ZPATH", "1" if path == "fused" else "0")
+        plan = S.SPECTplan(mumap, psfs, 4.8, interpmeth="one")
+        assert plan.path == path
+        out[path] = (S.project(x, plan, index=ii), S.backproject(ys, plan, index=ii))
+        plan.close()
+    for a, b in zip(out["fused"], out["split"]):
+        assert relerr(a, b) <= 1e-5
+    G = O.Geometry(mumap, psfs, 4.8, interp="one")
+    assert relerr(out["fused"][0], G.project(x, index=ii)) <= TOL
+    assert relerr(out["fused"][1], G.backproject(ys, index=ii)) <= TOL
