@@ -232,18 +232,10 @@ struct spect_plan_s {
   size_t izN = 0;              // floats of one IZ volume (L * L * nzp)
   float* d_imgIZ = nullptr;    // forward input / OS-EM iterate (IZ)
   float* d_backIZ = nullptr;   // back-projection accumulator (IZ)
-  float* d_Hz = nullptr;       // [nset][ny][hs] forward pass weights
-  float* d_Ez = nullptr;       // [nset][ny][ts] forward tails
-  int* d_Rz = nullptr;         // [nset][ny][4] tap-block ranges of the forward passes
   float* d_Zt = nullptr;       // [nset][ny][2][ztable_floats] pass tables: forward, adjoint
   ZTile zat{}, zft{};          // tilings of k_zadj, k_zfwd
   double ztaps[2] = {0, 0};    // mean kept taps per plane of the fused passes (z, x)
-  // large-plane kernels (zpath == 2): task width, column / row tiles, shared
-  // memory and resident blocks per SM of k_zs_fz, k_zs_fx, and the forward's
-  // plane-tile exchange buffer
-  int zs_w = 8, zs_tx = 8, zs_tz = 4, zs_fz_nth = kZsNth / 2;
-  size_t zs_smem[2] = {0, 0};
-  int zs_occ[2] = {1, 1};
+  ZsTiles zst{};               // tiling of the large-plane kernels (zpath == 2), their plane exchange buffer
   float* d_Q = nullptr;
   // split kernels with the gather rotation adjoint: the premultiplied adjoint
   // planes are transposed into d_Tz (z fastest) and gathered into d_backIZ
@@ -280,7 +272,7 @@ void free_plan(spect_plan_s* p) {
   void* ptrs[] = {p->d_mumap, p->d_att, p->d_err, p->d_r1view, p->d_R1, p->d_gscr_r1, p->d_H,     p->d_rot,      p->d_viewset,   p->d_tw,         p->d_all,
                   p->d_idx,   p->d_P,     p->d_part,     p->d_Vs,      p->d_imgpart,    p->d_gB,
                   p->d_gacc,  p->d_gscr_adj, p->d_views_tmp, p->d_ones, p->d_asum,       p->d_flag, p->d_sub,
-                  p->d_io_img, p->d_io_views, p->d_Hsep, p->d_Tsep, p->d_imgIZ, p->d_backIZ, p->d_Hz, p->d_Ez, p->d_Tz, p->d_Rz, p->d_Zt, p->d_Q};
+                  p->d_io_img, p->d_io_views, p->d_Hsep, p->d_Tsep, p->d_imgIZ, p->d_backIZ, p->d_Tz, p->d_Zt, p->d_Q};
   for (void* q : ptrs)
     if (q) {
       if (p->async_alloc) cudaFreeAsync(q, p->home);
@@ -552,9 +544,6 @@ ZArgs zargs(const spect_plan_s* p) {
   a.g = p->zg;
   a.img = p->d_imgIZ;
   a.att = p->d_att;
-  a.H = p->d_Hz;
-  a.E = p->d_Ez;
-  a.R = p->d_Rz;
   a.tab = p->d_Zt;
   a.rot = p->d_rot;
   a.viewset = p->d_viewset;
@@ -589,15 +578,15 @@ int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx,
     a.part = partbuf;
     a.G = zwalk_blocks(p, nv, cap);
     if (p->zpath == 2) {  // large planes: gather + z pass -> Q, x pass + depth sum -> part
-      const int ntz = cdiv(p->nz, p->zs_tz);
+      const ZsTiles& t = p->zst;
       a.Q = p->d_Q;
-      a.tx = p->zs_tx;
-      a.tz = p->zs_tz;
-      const int n1 = nv * p->ny * (p->nx / p->zs_tx), n2 = (a.G + nv) * ntz;
-      LAUNCH(p, K_CONV_FWD, st, "k_zs_fz",
-             zs_fz_launch(p->zs_w, p->zs_fz_nth, std::min(n1, p->sm_count * p->zs_occ[0]), p->zs_smem[0], st, a));
-      LAUNCH(p, K_CONV_FWD, st, "k_zs_fx",
-             zs_fx_launch(p->zs_w, std::min(n2, p->sm_count * p->zs_occ[1]), p->zs_smem[1], st, a));
+      a.tx = t.tx;
+      a.tz = t.tz;
+      a.zvst = t.zvst;
+      a.xbst = t.xbst;
+      const int n1 = nv * p->ny * cdiv(p->nx, t.tx), n2 = (a.G + nv) * cdiv((p->nz + 1) / 2, t.tz / 2);
+      LAUNCH(p, K_CONV_FWD, st, "k_zs_fz", zs_fz_launch(t, std::min(n1, p->sm_count * t.fz_occ), st, a));
+      LAUNCH(p, K_CONV_FWD, st, "k_zs_fx", zs_fx_launch(t, std::min(n2, p->sm_count * t.fx_occ), st, a));
     } else {
       LAUNCH(p, K_CONV_FWD, st, "k_zfwd", zfwd_launch(a.G, st, a));
     }
@@ -1367,44 +1356,14 @@ int trim_factors(std::vector<double>& w, int n) {
   return nk;
 }
 
-// taps of a pass row w[0, len) (len a multiple of 8) that a window pass runs:
-// 8-tap blocks from a 4-tap boundary, (first 4-tap block b4, block count n8)
-// covering every nonzero tap, 4 b4 + 8 n8 <= len
-void tap_range(const float* w, int len, int* b4, int* n8) {
-  int lo = 0, hi = len - 1;
-  while (lo < len && w[lo] == 0.f) ++lo;
-  while (hi > lo && w[hi] == 0.f) --hi;
-  if (lo >= len) {  // no tap (cannot happen for a plane factor)
-    *b4 = 0;
-    *n8 = 0;
-    return;
-  }
-  int b = lo / 4, n = (hi + 1 - 4 * b + 7) / 8;
-  if (4 * b + 8 * n > len) --b;  // 4 past the end: start 4 taps earlier (zeros)
-  *b4 = b;
-  *n8 = n;
-}
-
-// the same for the pair passes: 4-tap blocks (b4, n4), 4 b4 + 4 n4 <= len
+// taps of a pass row w[0, len) (len a multiple of 4) that a pass runs: n4
+// 4-tap blocks from block b4 on, covering every nonzero tap
 void tap_range4(const float* w, int len, int* b4, int* n4) {
   int lo = 0, hi = len - 1;
   while (lo < len && w[lo] == 0.f) ++lo;
   while (hi > lo && w[hi] == 0.f) --hi;
   *b4 = lo >= len ? 0 : lo / 4;
   *n4 = lo >= len ? 0 : hi / 4 + 1 - lo / 4;
-}
-
-// tiles of the large-plane kernels: task width w (16 where it divides nx,
-// SPECT_ZW=8 forces 8), column tile tx (32, 16 or 8 dividing nx), row tile
-// tz (a multiple of 4: one x task of w outputs per thread of k_zs_fx,
-// tz * nx / w <= kZsNthX); false when a kernel's shared memory does not fit
-bool zs_tiles(const ZGeom& g, size_t optin, ZsTiles* t) {
-  const char* e = std::getenv("SPECT_ZW");
-  t->w = (g.nx % 16 == 0 && !(e && std::atoi(e) == 8)) ? 16 : 8;
-  t->tx = g.nx % 32 == 0 ? 32 : (g.nx % 16 == 0 ? 16 : 8);
-  t->tz = std::min(kZsNthX * t->w / g.nx / 4 * 4, zround(g.nz, 4));
-  if (t->tz < 4) return false;
-  return zs_fz_smem(g, t->tx) <= optin && zs_fx_smem(g, t->tz) <= optin;
 }
 
 int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, int nview, const float* mumap,
@@ -1500,7 +1459,6 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   // (planes too large for the fused kernels' shared memory; SPECT_ZSTRIP=1
   // prefers them, =0 never takes them); 0: the split kernels
   int zkind = 0;
-  ZsTiles zt{};
   {
     int dev = 0, optin = 0;
     const char* zenv = std::getenv("SPECT_ZPATH");
@@ -1516,7 +1474,8 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       p->zft = zfwd_tile(zg, (size_t)optin, one);
       const bool fused = adj && p->zft.w != 0;
       if (!fused) p->zft.ystep = zdepth_step(ny);  // the walk of the large-plane kernels
-      const bool strip = adj && !one && nx % 8 == 0 && zs_tiles(zg, (size_t)optin, &zt);
+      p->zst = zs_tiles(zg, (size_t)optin);
+      const bool strip = adj && !one && p->zst.fz_nth != 0;
       if (fused && !(senv && senv[0] == '1')) zkind = 1;
       else if (strip && !(senv && senv[0] == '0')) zkind = 2;
       else if (fused) zkind = 1;
@@ -1554,17 +1513,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   if (p->zpath == 2) {
     p->zg = zg;
     p->izN = (size_t)zg.L * zg.L * zg.nzp;
-    p->zs_w = zt.w;
-    p->zs_tx = zt.tx;
-    p->zs_tz = zt.tz;
-    p->zs_smem[0] = zs_fz_smem(zg, zt.tx);
-    p->zs_smem[1] = zs_fx_smem(zg, zt.tz);
-    // k_zs_fz: 256 threads, two blocks per SM (SPECT_ZS_FZ_THREADS=512: one of 512)
-    const char* fz_env = std::getenv("SPECT_ZS_FZ_THREADS");
-    p->zs_fz_nth = (fz_env && std::atoi(fz_env) == kZsNth) ? kZsNth : kZsNth / 2;
-    cudaError_t ze = zstrip_setup((int)p->max_smem);
-    if (ze == cudaSuccess) ze = zstrip_occupancy(zt.w, p->zs_fz_nth, p->zs_smem, p->zs_occ);
-    if (ze == cudaSuccess) ze = zpath_setup((int)p->max_smem);
+    const cudaError_t ze = zpath_setup((int)p->max_smem);
     if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("large-plane kernel setup: ") + cudaGetErrorString(ze)));
   }
   if (p->zpath == 1) {
@@ -1818,13 +1767,9 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     const int ts = std::max(4, (2 * hxs + 2 * hzs + 3) & ~3);
     std::vector<float> H((size_t)p->nset * ny * 2 * hs, 0.f), Tl((size_t)p->nset * ny * ts, 0.f);
     const bool ok = sep_host;
-    std::vector<float> Hz, Ez, Zt;
-    std::vector<int> Rz;
+    std::vector<float> Zt;
     const int zrow = ztable_floats(zg);
     if (ok && p->zpath) {
-      Hz.assign((size_t)p->nset * ny * zg.hs, 0.f);
-      Ez.assign((size_t)p->nset * ny * zg.ts, 0.f);
-      Rz.assign((size_t)p->nset * ny * 4, 0);
       Zt.assign((size_t)p->nset * ny * 2 * zrow, 0.f);
     }
     for (int u = 0; ok && u < p->nset; ++u)
@@ -1841,7 +1786,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
         float* trow = Tl.data() + ((size_t)u * ny + y) * ts;
         fold_tails(a, hxs, trow, trow + hxs);
         fold_tails(b, hzs, trow + 2 * hxs, trow + 2 * hxs + hzs);
-        if (!Hz.empty()) {
+        if (!Zt.empty()) {
           // fused path, from the trimmed factors: weights of the z and x
           // pass, each shifted right by its data offset minus the half width;
           // tails [ELz ERz ELx ERx] and folds [cLx cRx cLz cRz]; the
@@ -1850,15 +1795,6 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
           const double* at = za.data() + pl * pxk;
           const double* bt = zb.data() + pl * pzk;
           const int sz = zg.R0 - zg.hz, sx = zg.C0 - zg.hx;
-          float* zr = Hz.data() + pl * zg.hs;
-          for (int m = 0; m < pzk; ++m) zr[sz + m] = (float)bt[pzk - 1 - m];
-          for (int m = 0; m < pxk; ++m) zr[zg.zpw + sx + m] = (float)at[pxk - 1 - m];
-          float* er = Ez.data() + pl * zg.ts;
-          clamp_tails(bt, pzk, er, er + zg.hz);
-          clamp_tails(at, pxk, er + 2 * zg.hz, er + 2 * zg.hz + zg.hx);
-          int* rr = Rz.data() + pl * 4;
-          tap_range(zr, zg.zpw, rr, rr + 1);
-          tap_range(zr + zg.zpw, zg.xpw, rr + 2, rr + 3);
           for (int m = 0; m < pzk; ++m) p->ztaps[0] += bt[m] != 0.0 ? 1.0 : 0.0;
           for (int m = 0; m < pxk; ++m) p->ztaps[1] += at[m] != 0.0 ? 1.0 : 0.0;
           // pass tables: the weights twice each, tails or folds, ranges
@@ -1883,13 +1819,10 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
           }
         }
       }
-    if (!Hz.empty()) {
+    if (!Zt.empty()) {
       p->ztaps[0] /= (double)p->nset * ny;
       p->ztaps[1] /= (double)p->nset * ny;
-      if ((st = dalloc(p, &p->d_Hz, Hz.size())) || (st = up(p->d_Hz, Hz.data(), sizeof(float) * Hz.size())) ||
-          (st = dalloc(p, &p->d_Ez, Ez.size())) || (st = up(p->d_Ez, Ez.data(), sizeof(float) * Ez.size())) ||
-          (st = dalloc(p, &p->d_Rz, Rz.size())) || (st = up(p->d_Rz, Rz.data(), sizeof(int) * Rz.size())) ||
-          (st = dalloc(p, &p->d_Zt, Zt.size())) || (st = up(p->d_Zt, Zt.data(), sizeof(float) * Zt.size())))
+      if ((st = dalloc(p, &p->d_Zt, Zt.size())) || (st = up(p->d_Zt, Zt.data(), sizeof(float) * Zt.size())))
         return bail(st);
     }
     if (ok) {

@@ -62,50 +62,10 @@ namespace spect {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-// four floats as two packed pairs
+// four floats as two packed pairs; ldp_cs: read once (the image that the
+// gather reads again and again stays in L2 instead)
 __device__ __forceinline__ ulonglong2 ldp(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
-// one W-output task (W = 8 or 16) over a zero-padded line, the taps
-// m in [4 b4, 4 b4 + 8 nblk) in blocks of 8 (nblk <= 9): o[k] += sum_m w[m]
-// line[k + m] (line and w 16-byte aligned; reads line[4 b4, 4 b4 + 8 nblk +
-// W)).  Fully unrolled with a uniform early exit; the window elements are
-// named by constant indices (registers, no moves): per block two new quads
-// of the line and two weight quads feed 8 W FMAs.  Every output sums its
-// taps in ascending m, so W does not change the result.
-template <int W>
-__device__ __forceinline__ void zpassw(const float* __restrict__ w, int b4, int nblk, const float* line,
-                                       float (&o)[W]) {
-  w += 4 * b4;
-  line += 4 * b4;
-  float e[W + 8 * 9];
-#pragma unroll
-  for (int i = 0; i < W / 4; ++i) {
-    const float4 q = ld4(line + 4 * i);
-    e[4 * i] = q.x;
-    e[4 * i + 1] = q.y;
-    e[4 * i + 2] = q.z;
-    e[4 * i + 3] = q.w;
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    if (k >= nblk) break;
-    const float4 q0 = ld4(line + 8 * k + W), q1 = ld4(line + 8 * k + W + 4);
-    e[8 * k + W] = q0.x;
-    e[8 * k + W + 1] = q0.y;
-    e[8 * k + W + 2] = q0.z;
-    e[8 * k + W + 3] = q0.w;
-    e[8 * k + W + 4] = q1.x;
-    e[8 * k + W + 5] = q1.y;
-    e[8 * k + W + 6] = q1.z;
-    e[8 * k + W + 7] = q1.w;
-    const float4 w0 = ld4(w + 8 * k), w1 = ld4(w + 8 * k + 4);
-    const float ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-    for (int s2 = 0; s2 < 8; ++s2)
-#pragma unroll
-      for (int j = 0; j < W; ++j) o[j] = fmaf(ws[s2], e[8 * k + s2 + j], o[j]);
-  }
-}
-
+__device__ __forceinline__ ulonglong2 ldp_cs(const float* p) { return __ldcs(reinterpret_cast<const ulonglong2*>(p)); }
 // q = t / n for 0 <= t < 2^20, 1 <= n <= 4096, with r = 1/n rounded to float:
 // (t + 1/2) / n is at least 1/(2n) from an integer, far above the rounding
 // error of (t + 1/2) * r, so truncation gives the exact quotient
@@ -199,6 +159,60 @@ __device__ __forceinline__ f2 zfold2(const float* c, const f2* v, int step, int 
 __device__ __forceinline__ float4 zturn(f2 p, f2 q) {
   const float2 u = unpack2(p), v = unpack2(q);
   return make_float4(u.x, v.x, u.y, v.y);
+}
+
+// four z of a rotated, attenuated column as two packed pairs: the four taps at
+// p, p + nzp, p + Lz, p + Lz + nzp with the doubled weights w4[0] = (w00 w00
+// w10 w10), w4[1] = (w01 w01 w11 w11), times the attenuation at att
+__device__ __forceinline__ void zsample4(const float* p, int nzp, size_t Lz, const float4* w4, const float* att, f2& lo,
+                                         f2& hi) {
+  const ulonglong2 t0 = ldp(p), t1 = ldp(p + nzp), t2 = ldp(p + Lz), t3 = ldp(p + Lz + nzp);
+  const ulonglong2 at = ldp_cs(att);
+  const ulonglong2 wa = reinterpret_cast<const ulonglong2*>(w4)[0], wb = reinterpret_cast<const ulonglong2*>(w4)[1];
+  lo = mul2(fma2(wb.y, t3.x, fma2(wb.x, t2.x, fma2(wa.y, t1.x, mul2(wa.x, t0.x)))), at.x);
+  hi = mul2(fma2(wb.y, t3.y, fma2(wb.x, t2.y, fma2(wa.y, t1.y, mul2(wa.x, t0.y)))), at.y);
+}
+
+// the clamped boundary of a forward task's outputs i0 .. i0 + W - 1 of a line
+// of n elements with edge values e0, e1: + EL[i] e0 (i < h), + ER[n-1-i] e1
+template <int W>
+__device__ __forceinline__ void zclamp(f2 (&o)[W], const float* EL, const float* ER, int h, int i0, int n, f2 e0, f2 e1) {
+  if (i0 < h) {
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (i0 + k < h) o[k] = fma2(pack2(EL[i0 + k], EL[i0 + k]), e0, o[k]);
+  }
+  if (i0 + W > n - h) {
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const int kk = n - 1 - i0 - k;
+      if (kk >= 0 && kk < h) o[k] = fma2(pack2(ER[kk], ER[kk]), e1, o[k]);
+    }
+  }
+}
+
+// a task's outputs (rows z, z + 1, columns x0 ..) into a partial view [nz][nx]
+template <int X>
+__device__ __forceinline__ void zstore_part(float* part, const f2 (&acc)[X], int nx, int nz, int z, int x0) {
+  float* q = part + (size_t)z * nx + x0;
+  const bool two = z + 1 < nz;
+  if (nx % 4 == 0) {
+#pragma unroll
+    for (int k = 0; k < X; k += 4)
+      if (x0 + k < nx) {
+        const float4 u = zturn(acc[k], acc[k + 1]), w = zturn(acc[k + 2], acc[k + 3]);
+        st4(q + k, make_float4(u.x, u.y, w.x, w.y));
+        if (two) st4(q + nx + k, make_float4(u.z, u.w, w.z, w.w));
+      }
+  } else {
+#pragma unroll
+    for (int k = 0; k < X; ++k)
+      if (x0 + k < nx) {
+        const float2 u = unpack2(acc[k]);
+        q[k] = u.x;
+        if (two) q[nx + k] = u.y;
+      }
+  }
 }
 
 // fetch the 128-byte line of p into L2
@@ -582,18 +596,12 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
         lo = fma2(w.y, t1.x, k ? fma2(w.x, t0.x, lo) : mul2(w.x, t0.x));
         hi = fma2(w.y, t1.y, k ? fma2(w.x, t0.y, hi) : mul2(w.x, t0.y));
       }
-      const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
+      const ulonglong2 at = ldp_cs(att + x * nzp + 4 * z4);
       lo = mul2(lo, at.x);
       hi = mul2(hi, at.y);
       return;
     } else {
-      const float* p = a.img + geoO[x] + 4 * z4;
-      const ulonglong2 t0 = ldp(p), t1 = ldp(p + nzp), t2 = ldp(p + Lz), t3 = ldp(p + Lz + nzp);
-      const ulonglong2 at = ldp(att + x * nzp + 4 * z4);
-      const ulonglong2 wa = reinterpret_cast<const ulonglong2*>(geoW)[2 * x];  // (w00, w00), (w10, w10)
-      const ulonglong2 wb = reinterpret_cast<const ulonglong2*>(geoW)[2 * x + 1];
-      lo = mul2(fma2(wb.y, t3.x, fma2(wb.x, t2.x, fma2(wa.y, t1.x, mul2(wa.x, t0.x)))), at.x);
-      hi = mul2(fma2(wb.y, t3.y, fma2(wb.x, t2.y, fma2(wa.y, t1.y, mul2(wa.x, t0.y)))), at.y);
+      zsample4(a.img + geoO[x] + 4 * z4, nzp, Lz, geoW + 2 * x, att + x * nzp + 4 * z4, lo, hi);
     }
   };
   const int hi4 = (tid >> 2) & 1;
@@ -670,20 +678,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
 #pragma unroll
       for (int k = 0; k < W; ++k) o[k] = 0;
       zpass2<W>(Wd, rg.x, rg.y, col + z0, o);
-      if (z0 < hz) {  // clamped rows above the plane
-        const f2 e0 = col[R0];
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-          if (z0 + k < hz) o[k] = fma2(pack2(ELz[z0 + k], ELz[z0 + k]), e0, o[k]);
-      }
-      if (z0 + W > nz - hz) {  // clamped rows below
-        const f2 e1 = col[R0 + nz - 1];
-#pragma unroll
-        for (int k = 0; k < W; ++k) {
-          const int kk = nz - 1 - z0 - k;
-          if (kk >= 0 && kk < hz) o[k] = fma2(pack2(ERz[kk], ERz[kk]), e1, o[k]);
-        }
-      }
+      zclamp<W>(o, ELz, ERz, hz, z0, nz, col[R0], col[R0 + nz - 1]);
       f2* w = XB + (z0 / 2) * bst + C0 + 2 * xp;
 #pragma unroll
       for (int m = 0; m < W / 2; ++m)
@@ -712,20 +707,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
 #pragma unroll
         for (int k = 0; k < X; ++k) o[k] = 0;
         zpass2<X>(Wd + g.zpw, rg.z, rg.w, row + x0, o);
-        if (x0 < hx) {
-          const f2 e0 = row[C0];
-#pragma unroll
-          for (int k = 0; k < X; ++k)
-            if (x0 + k < hx) o[k] = fma2(pack2(ELx[x0 + k], ELx[x0 + k]), e0, o[k]);
-        }
-        if (x0 + X > nx - hx) {
-          const f2 e1 = row[C0 + nx - 1];
-#pragma unroll
-          for (int k = 0; k < X; ++k) {
-            const int kk = nx - 1 - x0 - k;
-            if (kk >= 0 && kk < hx) o[k] = fma2(pack2(ERx[kk], ERx[kk]), e1, o[k]);
-          }
-        }
+        zclamp<X>(o, ELx, ERx, hx, x0, nx, row[C0], row[C0 + nx - 1]);
 #pragma unroll
         for (int k = 0; k < X; ++k) acc[i][k] = add2(acc[i][k], o[k]);
       }
@@ -735,27 +717,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
         const int x0 = xs0[i], zp = (tid + i * nth) % nzp2;
-        if (x0 < nx) {
-          float* q = a.part + (size_t)(blockIdx.x + slot) * nz * nx + (size_t)(2 * zp) * nx + x0;
-          const bool two = 2 * zp + 1 < nz;
-          if (nx % 4 == 0) {
-#pragma unroll
-            for (int k = 0; k < X; k += 4)
-              if (x0 + k < nx) {
-                const float4 u = zturn(acc[i][k], acc[i][k + 1]), w = zturn(acc[i][k + 2], acc[i][k + 3]);
-                st4(q + k, make_float4(u.x, u.y, w.x, w.y));
-                if (two) st4(q + nx + k, make_float4(u.z, u.w, w.z, w.w));
-              }
-          } else {
-#pragma unroll
-            for (int k = 0; k < X; ++k)
-              if (x0 + k < nx) {
-                const float2 u = unpack2(acc[i][k]);
-                q[k] = u.x;
-                if (two) q[nx + k] = u.y;
-              }
-          }
-        }
+        if (x0 < nx) zstore_part<X>(a.part + (size_t)(blockIdx.x + slot) * nz * nx, acc[i], nx, nz, 2 * zp, x0);
 #pragma unroll
         for (int k = 0; k < X; ++k) acc[i][k] = 0;
       }

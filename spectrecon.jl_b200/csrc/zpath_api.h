@@ -91,9 +91,6 @@ struct ZArgs {
   const float* tab;     // [set][y][2][ztable_floats]: forward, adjoint tables
   const float* img;     // IZ
   const float* att;     // ATT
-  const float* H;       // [set][y][hs]: forward z | x weights
-  const float* E;       // [set][y][ts]: ELz ERz ELx ERx
-  const int* R;         // [set][y][4]: (first 4-tap block, 8-tap blocks) of the forward z | x pass
   const float4* rot;    // [view] (cos(2pi - theta), sin(2pi - theta), theta == 0, theta)
   const int* vidx;      // [nv] plan view of each slot
   const int* viewset;   // [nview] PSF set of each view
@@ -103,8 +100,9 @@ struct ZArgs {
   const float* views;   // k_zadj input [nv][nz][nx]
   float* T;             // k_zadj output [nv][ny][nx][nzp]
   int* err;
-  float* Q;             // plane-tile exchange of the large-plane kernels (zstrip.cuh)
+  float* Q;             // plane exchange of the large-plane kernels (zstrip.cuh), [nv][ny][row pair][nx][2]
   int tx, tz;           // their column and row tile sizes
+  int zvst, xbst;       // their line strides (f2)
 };
 
 // k_zfwd shared memory (zpath.cuh)
@@ -201,18 +199,45 @@ inline ZTile zfwd_tile(const ZGeom& g, size_t optin, bool one) {
   return t;
 }
 
-// large-plane kernels (zstrip.cuh), shared memory in bytes
-__host__ __device__ inline size_t zs_fz_smem(const ZGeom& g, int tx) {
-  return sizeof(float) * ((size_t)g.hs + g.ts + 4 + 5 * (size_t)tx + (size_t)tx * g.ast + (size_t)g.nz * tx);
-}
-__host__ __device__ inline size_t zs_fx_smem(const ZGeom& g, int tz) {
-  return sizeof(float) * 2 * ((size_t)tz * g.bs + g.hs + g.ts + 4);
-}
+// tiling of the large-plane kernels (zstrip.cuh): k_zs_fz on equal tiles of tx
+// columns in two planes with a thread for two of its 8-output tasks, k_zs_fx on tiles of
+// tz rows (about 320 tasks of kZfwdX outputs of a row pair, one a thread, so
+// that two blocks share an SM); nth = 0: a tile does not fit
+constexpr int kZsThreads = 320;  // k_zs_fz threads, three blocks an SM
 struct ZsTiles {
-  int w, tx, tz;  // task width, column tile, row tile
+  int tx, zvst, fz_nth, fz_occ, tz, xbst, fx_nth, fx_occ;
+  size_t fz_smem, fx_smem;
 };
-constexpr int kZsNth = 512;   // k_zs_fz threads
-constexpr int kZsNthX = 640;  // k_zs_fx threads (one x task each)
+inline ZsTiles zs_tiles(const ZGeom& g, size_t optin) {
+  ZsTiles t{};
+  auto occupancy = [&](size_t smem, int nth, int threads) {
+    const int so = (int)((optin + 1024) / (smem + 1024)), ro = threads / nth;
+    return so < ro ? so : ro;
+  };
+  const int nzb = (g.nz + 7) / 8;
+  int tmax = 2 * (320 / nzb);
+  if (tmax > 32) tmax = 32;
+  t.tx = zround((g.nx + (g.nx + tmax - 1) / tmax - 1) / ((g.nx + tmax - 1) / tmax), 4);
+  if (t.tx > g.nx) t.tx = g.nx;
+  t.zvst = zstride2(8 * nzb + g.zpw);
+  t.fz_smem = sizeof(float) * (4 * ((size_t)ztable_floats(g) + 8 * t.tx + zround(t.tx, 4)) + 2 * (size_t)t.tx * t.zvst);
+  int nth = 2 * zround((t.tx / 2 * nzb + 1) / 2, 32);  // two tasks a thread
+  if (nth > kZsThreads) nth = kZsThreads;
+  const int nxw = (g.nx + kZfwdX - 1) / kZfwdX, nrp = (g.nz + 1) / 2;
+  int tzp = 320 / nxw;
+  if (tzp < 1) tzp = 1;
+  if (tzp > nrp) tzp = nrp;
+  t.tz = 2 * tzp;
+  t.xbst = zstride2(kZfwdX * nxw + g.xpw);
+  t.fx_smem = sizeof(float) * 2 * (2 * (size_t)tzp * t.xbst + ztable_floats(g));
+  const int fxn = zround(tzp * nxw, 32);
+  if (t.fz_smem > optin || t.fx_smem > optin || fxn > kZThreads) return t;
+  t.fz_nth = nth;
+  t.fx_nth = fxn;
+  t.fz_occ = occupancy(t.fz_smem, nth, 3 * kZsThreads);
+  t.fx_occ = occupancy(t.fx_smem, fxn, kZThreads);
+  return t;
+}
 
 // tiling of k_zrot_adj: tiles of tx x ty image columns, S groups of threads
 // over the slots, vb slots whose hits are listed at a time (one thread tests
@@ -260,13 +285,9 @@ cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, flo
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx);
 cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, float* dst, const float* asum, int mode);
-// large-plane kernels: w = task width (8 or 16); occ = resident blocks per
-// SM of k_zs_fz, k_zs_fx at their shared-memory sizes (for the persistent
-// grids)
-cudaError_t zstrip_setup(int max_smem);
-cudaError_t zstrip_occupancy(int w, int fz_nth, const size_t smem[2], int occ[2]);
-cudaError_t zs_fz_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
-cudaError_t zs_fx_launch(int w, int grid, size_t smem, cudaStream_t st, const ZArgs& a);
+// large-plane kernels
+cudaError_t zs_fz_launch(const ZsTiles& t, int grid, cudaStream_t st, const ZArgs& a);
+cudaError_t zs_fx_launch(const ZsTiles& t, int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot,
                           const Rot1View* r1, float dy, float* att);
 

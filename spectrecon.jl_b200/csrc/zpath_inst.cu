@@ -26,6 +26,8 @@ cudaError_t zpath_setup(int max_smem) {
   cudaError_t e = zrot_adj_setup();
   for (const void* k : {kZfwd[0][0], kZfwd[0][1], kZfwd[1][0], kZfwd[1][1]})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  for (const void* k : {(const void*)k_zs_fz, (const void*)k_zs_fx})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   for (const void* k : kZadj)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   return e;
@@ -59,45 +61,15 @@ cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const floa
   return cudaGetLastError();
 }
 
-namespace {
-// k_zs_fz: 512 threads (index 0, 1) or 256 (index 2, 3: two blocks per SM at these registers)
-const void* const kZsFz[4] = {(const void*)k_zs_fz<kZsNth, 8>, (const void*)k_zs_fz<kZsNth, 16>,
-                              (const void*)k_zs_fz<kZsNth / 2, 8>, (const void*)k_zs_fz<kZsNth / 2, 16>};
-const void* const kZsFx[2] = {(const void*)k_zs_fx<kZsNthX, 8>, (const void*)k_zs_fx<kZsNthX, 16>};
-cudaError_t zs_launch(const void* k, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
-  ZArgs c = a;
-  void* args[] = {&c};
-  return cudaLaunchKernel(k, dim3(grid), dim3(nth), args, smem, st);
+cudaError_t zs_fz_launch(const ZsTiles& t, int grid, cudaStream_t st, const ZArgs& a) {
+  k_zs_fz<<<grid, t.fz_nth, t.fz_smem, st>>>(a);
+  return cudaGetLastError();
 }
-}  // namespace
-
-cudaError_t zstrip_setup(int max_smem) {
-  for (int i = 0; i < 2; ++i)
-    for (const void* k : {kZsFz[i], kZsFz[i + 2], kZsFx[i]}) {
-      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-      if (e != cudaSuccess) return e;
-    }
-  return cudaSuccess;
+cudaError_t zs_fx_launch(const ZsTiles& t, int grid, cudaStream_t st, const ZArgs& a) {
+  k_zs_fx<<<grid, t.fx_nth, t.fx_smem, st>>>(a);
+  return cudaGetLastError();
 }
 
-cudaError_t zstrip_occupancy(int w, int fz_nth, const size_t smem[2], int occ[2]) {
-  const int i = w == 16 ? 1 : 0, f = fz_nth == kZsNth ? i : i + 2;
-  const void* ks[2] = {kZsFz[f], kZsFx[i]};
-  const int nth[2] = {fz_nth, kZsNthX};
-  for (int j = 0; j < 2; ++j) {
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[j], ks[j], nth[j], smem[j]);
-    if (e != cudaSuccess) return e;
-    if (occ[j] < 1) occ[j] = 1;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t zs_fz_launch(int w, int nth, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
-  return zs_launch(kZsFz[(w == 16 ? 1 : 0) + (nth == kZsNth ? 0 : 2)], nth, grid, smem, st, a);
-}
-cudaError_t zs_fx_launch(int w, int grid, size_t smem, cudaStream_t st, const ZArgs& a) {
-  return zs_launch(kZsFx[w == 16 ? 1 : 0], kZsNthX, grid, smem, st, a);
-}
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz) {
   k_to_iz<<<dim3((g.nx + 31) / 32, g.ny, (g.nzp + 31) / 32), dim3(32, 8), 0, st>>>(g, img, iz);
   return cudaGetLastError();

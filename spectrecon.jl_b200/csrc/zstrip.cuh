@@ -1,16 +1,16 @@
-// zstrip.cuh -- the projector pair for planes too large for the fused
-// kernels' shared memory (e.g. 256x256x200 with a 65-tap PSF), on the same
-// z-fastest layouts (IZ image, ATT cache, T adjoint planes) and with the same
-// trimmed separable passes (zpassw, tail and fold tables, tap ranges) as
-// zpath.cuh, over plane tiles; the forward's two passes are kernels of their
-// own that exchange planes through the device buffer Q.
+// zstrip.cuh -- the forward projector for planes too large for k_zfwd's
+// shared memory (e.g. 256x256x200 with a 65-tap PSF), on the same z-fastest
+// layouts and with the same sampling, pair passes and plane walk as zpath.cuh,
+// over plane tiles; the two passes are kernels of their own that exchange
+// planes through the device buffer Q, whose rows are already the x pass's
+// pair lines.
 //
 // forward (project!, src/project.jl:77-135):
-//   k_zs_fz  item (slot, y, tile of tx columns): gather the rotated,
-//            attenuated columns (as k_zfwd), z pass, rows -> Q[slot][y][z][x]
-//   k_zs_fx  item (partial view of the forward walk, tile of tz rows): per
-//            plane the rows of Q (loaded one plane ahead into registers), x
-//            pass accumulated over the partial's planes -> part
+//   k_zs_fz  item (slot, two planes y, tile of tx columns): gather the rotated,
+//            attenuated columns, z pass -> Q[slot][y][row pair][x][2]
+//   k_zs_fx  item (partial view of the forward walk, tile of row pairs): per
+//            plane the rows of Q (copied one plane ahead), x pass accumulated
+//            over the partial's planes -> part
 // The adjoint is k_zadj (zpath.cuh) on row tiles.  Every output goes through
 // the operations of the fused kernels in the same order (z then x), so the
 // two paths agree bit for bit.
@@ -19,132 +19,128 @@
 
 namespace spect {
 
-// the sample geometry of column x of plane y for the view's (cos, sin):
-// k_zfwd's geometry, one column
-__device__ __forceinline__ void zs_geometry(const ZGeom& g, float4 r, int x, int y, float4* w_out, int* o_out) {
-  int j1 = x, j2 = y;
-  float4 w = make_float4(1.f, 0.f, 0.f, 0.f);
-  if (r.z == 0.f) {
-    const float cs = r.x, sn = r.y;
-    const float d1 = __fsub_rn((float)x, g.c0), d2 = __fsub_rn((float)y, g.c0);
-    const float s1 = __fadd_rn(g.c0, __fsub_rn(__fmul_rn(cs, d1), __fmul_rn(sn, d2)));
-    const float s2 = __fadd_rn(g.c0, __fadd_rn(__fmul_rn(sn, d1), __fmul_rn(cs, d2)));
-    const float f1 = floorf(s1), f2 = floorf(s2);
-    const float t1 = __fsub_rn(s1, f1), t2 = __fsub_rn(s2, f2);
-    const float u1 = __fsub_rn(1.0f, t1), u2 = __fsub_rn(1.0f, t2);
-    j1 = (int)f1;
-    j2 = (int)f2;
-    w = make_float4(__fmul_rn(u1, u2), __fmul_rn(t1, u2), __fmul_rn(u1, t2), __fmul_rn(t1, t2));
-    if (j1 < -g.pad || j1 > g.nx + g.pad - 2 || j2 < -g.pad || j2 > g.nx + g.pad - 2) {
-      j1 = j2 = 0;
-      w = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  *w_out = w;
-  *o_out = ((j2 + g.pad) * g.L + j1 + g.pad) * g.nzp;
-}
-
-// one plane's forward pass table (weights hs | tails ts | ranges 4 ints) into
-// shared memory
-__device__ __forceinline__ void zs_table(const ZArgs& a, int set, int y, float* Wt, int tid, int nth) {
-  const int hs = a.g.hs, ts = a.g.ts;
-  const float* Hrow = a.H + ((size_t)set * a.g.ny + y) * hs;
-  const float* Erow = a.E + ((size_t)set * a.g.ny + y) * ts;
-  for (int k = tid; k < hs + ts; k += nth) Wt[k] = k < hs ? Hrow[k] : Erow[k - hs];
-  if (tid < 4) reinterpret_cast<int*>(Wt + hs + ts)[tid] = a.R[((size_t)set * a.g.ny + y) * 4 + tid];
-}
-
 // ------------------------------------------------------------------------
-// k_zs_fz<NTH, W>: forward gather and z pass.  Shared memory (floats):
-// [table hs + ts + 4][geoW tx float4][geoO tx int][ZB tx * ast][OB nz * tx]
-template <int NTH, int W>
-__global__ void __launch_bounds__(NTH) k_zs_fz(ZArgs a) {
+// k_zs_fz: forward gather and z pass of a tile of tx columns in two adjacent
+// planes (their samples share taps: about 3.3 image columns are read for the
+// eight taps of an x, where one plane reads 2.4 for four), tasks of 8 outputs
+// of a column pair; the first half of the warps runs the first plane's, so a
+// warp's weights stay uniform.  Two barriers an item: the z pass runs while
+// the next item's taps and attenuation are prefetched into L2.  64 registers
+// and tiles for 320 threads, three blocks an SM: the bound is HBM (attenuation
+// and image read, Q written: 1.1 GB for 8 views of 256x256x200, 65 taps) and
+// the latency of the gather's loads, not the FMAs.  Measured there: 392 us
+// (16-output tasks on two blocks 411 us, one plane an item 425 us, double ZB
+// with one barrier 511 us -- it takes the L1; the former single-line kernel,
+// which needed nx % 8 == 0, 394 us).
+// Shared memory: [2 x 2 x (table | geoW tx x 2 float4 | geoO tx int)]
+// [ZB 2 x tx / 2 * vst f2].
+__global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(ZArgs a) {
   extern __shared__ float4 smem4[];
+  constexpr int W = 8;
   const ZGeom& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, tx = a.tx;
-  float* const Wt = reinterpret_cast<float*>(smem4);
-  float4* const geoW = reinterpret_cast<float4*>(Wt + hs + ts + 4);
-  int* const geoO = reinterpret_cast<int*>(geoW + tx);
-  float* const ZB = reinterpret_cast<float*>(geoO + tx);
-  float* const OB = ZB + (size_t)tx * g.ast;
-  const int tid = threadIdx.x, ast = g.ast, R0 = g.R0, hz = g.hz;
-  const int ntx = nx / tx, nitems = a.nv * ny * ntx;
-  const int nz4 = (nz + 3) / 4, units = tx * nz4, nzb = (nz + W - 1) / W, ztasks = tx * nzb, q4 = tx / 4;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, tx = a.tx, vst = a.zvst;
+  const int trow = ztable_floats(g), tid = threadIdx.x, nth = blockDim.x, R0 = g.R0, hz = g.hz;
+  const int bufsz = trow + 8 * tx + zround(tx, 4), zbs = (tx / 2) * vst;
+  float* const base = reinterpret_cast<float*>(smem4);
+  f2* const ZB0 = reinterpret_cast<f2*>(base + 4 * bufsz);
+  const int ntx = (nx + tx - 1) / tx, nyp = ny / 2, nitems = a.nv * nyp * ntx, nz4 = (nz + 3) / 4, nzb = (nz + W - 1) / W;
+  const int nrp = (nz + 1) / 2;
   const size_t Lz = (size_t)g.L * nzp;
-  const float rnz4 = 1.0f / nz4, rtx = 1.0f / tx, rq4 = 1.0f / q4;
-  for (int k = tid; k < tx * ast; k += NTH) ZB[k] = 0.f;  // rows outside the data stay zero
-  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const int xt = item % ntx, sy = item / ntx, slot = sy / ny, y = sy - slot * ny, X0 = xt * tx;
-    const int v = a.vidx[slot], set = a.viewset[v];
-    zs_table(a, set, y, Wt, tid, NTH);
-    if (tid < tx) zs_geometry(g, a.rot[v], X0 + tid, y, &geoW[tid], &geoO[tid]);
-    __syncthreads();
-    // rotated, attenuated columns into ZB (column x, rows R0 + z), two units a round
-    const float* attp = a.att + (((size_t)v * ny + y) * nx + X0) * nzp;
-    for (int u0 = tid; u0 < units; u0 += 2 * NTH) {
-      float4 t[2][4], at[2];
-      int xs[2], zs[2];
+  const float rnz4 = 1.0f / nz4;
+  auto place = [&](int item, int& slot, int& y, int& X0) {  // the item's slot, first plane and column
+    const int xt = item % ntx, sy = item / ntx;
+    slot = sy / nyp;
+    y = 2 * (sy - slot * nyp);
+    X0 = xt * tx;
+  };
+  auto prepare = [&](int item, float* buf) {  // tables and sample geometry of an item
+    int slot, y, X0;
+    place(item, slot, y, X0);
+    const int v = a.vidx[slot];
+    const float* src = a.tab + (((size_t)a.viewset[v] * ny + y) * 2) * trow;
+    for (int k = 4 * tid; k < trow; k += 4 * nth) {
+      cp16(buf + k, src + k);
+      cp16(buf + bufsz + k, src + 2 * trow + k);
+    }
+    const float4 r = a.rot[v];
+    const int cols = min(tx, nx - X0);
+    for (int c = tid; c < 2 * cols; c += nth) {
+      const int p = c >= cols, x = c - p * cols;
+      float4* const geoW = reinterpret_cast<float4*>(buf + p * bufsz + trow);
+      float4 w;
+      int off;
+      zgeo(g, r.x, r.y, r.z != 0.f, X0 + x, y + p, w, off);
+      geoW[2 * x] = make_float4(w.x, w.x, w.y, w.y);
+      geoW[2 * x + 1] = make_float4(w.z, w.z, w.w, w.w);
+      reinterpret_cast<int*>(geoW + 2 * tx)[x] = off;
+    }
+  };
+  for (int k = tid; k < 2 * zbs; k += nth) ZB0[k] = 0;  // rows outside the data stay zero
+  int item = blockIdx.x, hb = 0;
+  if (item < nitems) prepare(item, base);
+  cp_wait();
+  __syncthreads();
+  const int hi4 = (tid >> 2) & 1, hth = nth / 2, pz = tid >= hth, tz = tid - pz * hth;
+  for (; item < nitems; item += gridDim.x, hb ^= 1) {
+    int slot, y, X0;
+    place(item, slot, y, X0);
+    const int txp = min(tx, nx - X0) / 2;
+    const float* const buf = base + 2 * hb * bufsz;
+    float* const next = base + 2 * (hb ^ 1) * bufsz;
+    const bool more = item + gridDim.x < nitems;
+    if (more) prepare(item + gridDim.x, next);
+    for (int p = 0; p < 2; ++p) {
+      const float4* const geoW = reinterpret_cast<const float4*>(buf + p * bufsz + trow);
+      const int* const geoO = reinterpret_cast<const int*>(geoW + 2 * tx);
+      const float* att = a.att + (((size_t)a.vidx[slot] * ny + y + p) * nx + X0) * nzp;
+      for (int u = tid; u < txp * nz4; u += nth) {  // unit (column pair, z group)
+        const int xp = zdiv(u, rnz4), z4 = u - xp * nz4;
+        f2 lo[2], hi[2];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int u = min(u0 + j * NTH, units - 1);  // a repeated last unit stores the same values
-        xs[j] = zdiv(u, rnz4);
-        zs[j] = u - xs[j] * nz4;
-        const float* p = a.img + geoO[xs[j]] + 4 * zs[j];
-        t[j][0] = ld4(p);
-        t[j][1] = ld4(p + nzp);
-        t[j][2] = ld4(p + Lz);
-        t[j][3] = ld4(p + Lz + nzp);
-        at[j] = ld4(attp + (size_t)xs[j] * nzp + 4 * zs[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float4 w = geoW[xs[j]];
-        const float4 t0 = t[j][0], t1 = t[j][1], t2 = t[j][2], t3 = t[j][3];
-        float4 o;
-        o.x = __fmul_rn(fmaf(w.w, t3.x, fmaf(w.z, t2.x, fmaf(w.y, t1.x, __fmul_rn(w.x, t0.x)))), at[j].x);
-        o.y = __fmul_rn(fmaf(w.w, t3.y, fmaf(w.z, t2.y, fmaf(w.y, t1.y, __fmul_rn(w.x, t0.y)))), at[j].y);
-        o.z = __fmul_rn(fmaf(w.w, t3.z, fmaf(w.z, t2.z, fmaf(w.y, t1.z, __fmul_rn(w.x, t0.z)))), at[j].z);
-        o.w = __fmul_rn(fmaf(w.w, t3.w, fmaf(w.z, t2.w, fmaf(w.y, t1.w, __fmul_rn(w.x, t0.w)))), at[j].w);
-        st4(ZB + xs[j] * ast + R0 + 4 * zs[j], o);
+        for (int c = 0; c < 2; ++c)
+          zsample4(a.img + geoO[2 * xp + c] + 4 * z4, nzp, Lz, geoW + 2 * (2 * xp + c),
+                   att + (2 * xp + c) * nzp + 4 * z4, lo[c], hi[c]);
+        float4* o = reinterpret_cast<float4*>(ZB0 + p * zbs + xp * vst + R0 + 4 * z4);
+        o[hi4] = zturn(hi4 ? hi[0] : lo[0], hi4 ? hi[1] : lo[1]);
+        o[hi4 ^ 1] = zturn(hi4 ? lo[0] : hi[0], hi4 ? lo[1] : hi[1]);
       }
     }
+    cp_wait();
     __syncthreads();
-    // z pass: task (x, z block) -> OB rows z, column x
-    const int2 rg = *reinterpret_cast<const int2*>(Wt + hs + ts);
-    const float* ELz = Wt + hs;
-    const float* ERz = ELz + hz;
-    for (int t = tid; t < ztasks; t += NTH) {
-      const int zb = zdiv(t, rtx), x = t - zb * tx, z0 = W * zb;
-      float o[W];
-#pragma unroll
-      for (int k = 0; k < W; ++k) o[k] = 0.f;
-      const float* col = ZB + x * ast;
-      zpassw<W>(Wt, rg.x, rg.y, col + z0, o);
-      if (z0 < hz) {
-        const float e0 = col[R0];
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-          if (z0 + k < hz) o[k] = fmaf(ELz[z0 + k], e0, o[k]);
+    if (more) {  // the next item's taps (two runs of two columns) and attenuation on their way into L2
+      int slot1, y1, X1;
+      place(item + gridDim.x, slot1, y1, X1);
+      const int cols = min(tx, nx - X1);
+      for (int c = tid; c < 2 * cols; c += nth) {
+        const int p = c >= cols, x = c - p * cols;
+        const int off = reinterpret_cast<const int*>(next + p * bufsz + trow + 8 * tx)[x];
+        prefetch_l2_bulk(a.img + off, 2 * nzp * (unsigned)sizeof(float));
+        prefetch_l2_bulk(a.img + off + Lz, 2 * nzp * (unsigned)sizeof(float));
+        if (x == 0)
+          prefetch_l2_bulk(a.att + (((size_t)a.vidx[slot1] * ny + y1 + p) * nx + X1) * nzp,
+                           cols * nzp * (unsigned)sizeof(float));
       }
-      if (z0 + W > nz - hz) {
-        const float e1 = col[R0 + nz - 1];
+    }
+    // z pass: task (column pair, 16 rows) of plane y + pz -> Q
+    const float* const Wt = buf + pz * bufsz;
+    const f2* const Wd = reinterpret_cast<const f2*>(Wt);
+    const int2 rg = *reinterpret_cast<const int2*>(Wt + 2 * hs + ts);
+    f2* const Qp = reinterpret_cast<f2*>(a.Q) + ((size_t)slot * ny + y + pz) * nrp * nx + X0;
+    const float rtxp = 1.0f / txp;
+    for (int t = tz; t < txp * nzb; t += hth) {
+      const int zb = zdiv(t, rtxp), xp = t - zb * txp, z0 = W * zb;
+      f2 o[W];
 #pragma unroll
-        for (int k = 0; k < W; ++k) {
-          const int kk = nz - 1 - z0 - k;
-          if (kk >= 0 && kk < hz) o[k] = fmaf(ERz[kk], e1, o[k]);
-        }
-      }
+      for (int k = 0; k < W; ++k) o[k] = 0;
+      const f2* col = ZB0 + pz * zbs + xp * vst;
+      zpass2<W>(Wd, rg.x, rg.y, col + z0, o);
+      zclamp<W>(o, Wt + 2 * hs, Wt + 2 * hs + hz, hz, z0, nz, col[R0], col[R0 + nz - 1]);
+      f2* q = Qp + (size_t)(z0 / 2) * nx + 2 * xp;
 #pragma unroll
-      for (int k = 0; k < W; ++k)
-        if (z0 + k < nz) OB[(z0 + k) * tx + x] = o[k];
+      for (int m = 0; m < W / 2; ++m)
+        if (z0 + 2 * m < nz) __stcs(reinterpret_cast<float4*>(q + (size_t)m * nx), zturn(o[2 * m], o[2 * m + 1]));
     }
     __syncthreads();
-    // the tile's rows -> Q[slot][y][z][X0 ..]
-    float* Qp = a.Q + ((size_t)slot * ny + y) * nz * nx + X0;
-    for (int e = tid; e < nz * q4; e += NTH) {
-      const int z = zdiv(e, rq4), c = e - z * q4;
-      st4(Qp + (size_t)z * nx + 4 * c, ld4(OB + z * tx + 4 * c));
-    }
   }
 }
 
@@ -167,111 +163,71 @@ __device__ __forceinline__ bool zs_segment(const ZArgs& a, int id, int& slot, in
 }
 
 // ------------------------------------------------------------------------
-// k_zs_fx<NTH, W>: forward x pass and depth sum, one task of W outputs per
-// thread and plane (tz * nx / W <= NTH; the host picks tz).  Shared memory
-// (floats): 2 x [XB tz * bs (data columns C0..)][table hs + ts + 4].
-template <int NTH, int W>
-__global__ void __launch_bounds__(NTH, 1) k_zs_fx(ZArgs a) {
+// k_zs_fx: forward x pass and depth sum, one task of kZfwdX outputs a thread
+// and plane; the rows of Q and the table of the next plane are copied
+// (cp.async) while a plane is worked on, one barrier a plane, two blocks an
+// SM.  Bound: FFMA2 and the shared-memory pipe; 256x256x200, 8 views 295 ->
+// 255 us.  Shared memory: 2 x [XB tzp * bst f2 | table].
+__global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(ZArgs a) {
   extern __shared__ float4 smem4[];
+  constexpr int X = kZfwdX;
   const ZGeom& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, hs = g.hs, ts = g.ts, tz = a.tz, bs = g.bs, C0 = g.C0, hx = g.hx;
-  const int bufsz = tz * bs + hs + ts + 4;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, hs = g.hs, ts = g.ts, tzp = a.tz / 2, bst = a.xbst, C0 = g.C0, hx = g.hx;
+  const int trow = ztable_floats(g), bufsz = 2 * tzp * bst + trow, tid = threadIdx.x, nth = blockDim.x;
   float* const base = reinterpret_cast<float*>(smem4);
-  const int tid = threadIdx.x;
-  const int ntz = (nz + tz - 1) / tz, nitems = (a.G + a.nv) * ntz, n4 = nx / 4, xbs = nx / W;
-  const float rn4 = 1.0f / n4, rtz = 1.0f / tz;
-  for (int k = tid; k < 2 * bufsz; k += NTH) base[k] = 0.f;  // padding columns stay zero
+  const int nrp = (nz + 1) / 2, ntz = (nrp + tzp - 1) / tzp, nitems = (a.G + a.nv) * ntz, n2 = nx / 2;
+  for (int k = tid; k < 2 * bufsz; k += nth) base[k] = 0.f;  // columns outside the data stay zero
   __syncthreads();
-  // this thread's task: row zl, x block xb
-  const int xb = zdiv(tid, rtz), zl = tid - xb * tz, x0 = W * xb;
+  const int xb = tid / tzp, zl = tid - xb * tzp, x0 = X * xb;  // this thread's task: row pair zl, columns x0 ..
+  const int dr = nth / n2, dc = nth - dr * n2, r0 = tid / n2, c0 = tid - r0 * n2;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    // partial view id = walk block + slot, planes j0 .. j1 - 1 of the slot
-    const int zt = item % ntz, id = item / ntz;
+    const int zt = item % ntz, id = item / ntz;  // partial view, planes j0 .. j1 - 1 of its slot
     int slot, j0, j1;
     if (!zs_segment(a, id, slot, j0, j1)) continue;
-    const int Z0 = zt * tz, rows = min(tz, nz - Z0);
-    const int v = a.vidx[slot], set = a.viewset[v];
+    const int Z0 = zt * tzp, rows = min(tzp, nrp - Z0), set = a.viewset[a.vidx[slot]];
     int y = (int)((long long)j0 * a.t.ystep % ny);
-    const bool mine = tid < tz * xbs && zl < rows;
-    const int tot4 = rows * n4;
-    auto src = [&](int y) { return a.Q + (((size_t)slot * ny + y) * nz + Z0) * nx; };
-    // the first plane straight into buffer 0
-    {
-      const float* Qp = src(y);
-      for (int e = tid; e < tot4; e += NTH) {
-        const int z = zdiv(e, rn4), c = e - z * n4;
-        st4(base + z * bs + C0 + 4 * c, ld4(Qp + (size_t)z * nx + 4 * c));
+    const bool mine = x0 < nx && zl < rows;
+    auto fetch = [&](int yy, float* buf) {  // rows (16 bytes: columns 2 c, 2 c + 1 of a row pair) and table
+      const float* Qp = a.Q + (((size_t)slot * ny + yy) * nrp + Z0) * 2 * nx;
+      for (int r = r0, c = c0; r < rows;) {
+        cp16(buf + 2 * (r * bst + C0 + 2 * c), Qp + (size_t)r * 2 * nx + 4 * c);
+        r += dr;
+        c += dc;
+        if (c >= n2) {
+          c -= n2;
+          ++r;
+        }
       }
-      zs_table(a, set, y, base + tz * bs, tid, NTH);
-    }
+      const float* src = a.tab + (((size_t)set * ny + yy) * 2) * trow;
+      for (int k = 4 * tid; k < trow; k += 4 * nth) cp16(buf + 2 * tzp * bst + k, src + k);
+    };
+    fetch(y, base);
+    cp_wait();
     __syncthreads();
-    float acc[W];
+    f2 acc[X];
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc[k] = 0.f;
+    for (int k = 0; k < X; ++k) acc[k] = 0;
     for (int jj = j0; jj < j1; ++jj) {
-      float* const XB = base + ((jj - j0) & 1) * bufsz;
-      float* const XN = base + (((jj - j0) & 1) ^ 1) * bufsz;
-      const int yn = y + a.t.ystep < ny ? y + a.t.ystep : y + a.t.ystep - ny;
-      const float* Wt = XB + tz * bs;
-      // the next plane's rows into registers first (four float4 a thread at most)
-      float4 pf[4];
-      const bool more = jj + 1 < j1;
-      if (more) {
-        const float* Qp = src(yn);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int e = tid + j * NTH;
-          if (e < tot4) {
-            const int z = zdiv(e, rn4), c = e - z * n4;
-            pf[j] = ld4(Qp + (size_t)z * nx + 4 * c);
-          }
-        }
-      }
+      float* const buf = base + ((jj - j0) & 1) * bufsz;
+      y = y + a.t.ystep < ny ? y + a.t.ystep : y + a.t.ystep - ny;
+      if (jj + 1 < j1) fetch(y, base + (((jj - j0) & 1) ^ 1) * bufsz);
       if (mine) {
-        const int2 rg = *reinterpret_cast<const int2*>(Wt + hs + ts + 2);
-        const float* ELx = Wt + hs + 2 * g.hz;
-        const float* ERx = ELx + hx;
-        const float* row = XB + zl * bs;
-        float o[W];  // the plane's own sum, then onto the depth sum, as k_zfwd
+        const float* Wt = buf + 2 * tzp * bst;
+        const int2 rg = *reinterpret_cast<const int2*>(Wt + 2 * hs + ts + 2);
+        const f2* row = reinterpret_cast<const f2*>(buf) + zl * bst;
+        f2 o[X];  // the plane's own sum, then onto the depth sum, as k_zfwd
 #pragma unroll
-        for (int k = 0; k < W; ++k) o[k] = 0.f;
-        zpassw<W>(Wt + g.zpw, rg.x, rg.y, row + x0, o);
-        if (x0 < hx) {
-          const float e0 = row[C0];
+        for (int k = 0; k < X; ++k) o[k] = 0;
+        zpass2<X>(reinterpret_cast<const f2*>(Wt) + g.zpw, rg.x, rg.y, row + x0, o);
+        const float* EL = Wt + 2 * hs + 2 * g.hz;
+        zclamp<X>(o, EL, EL + hx, hx, x0, nx, row[C0], row[C0 + nx - 1]);
 #pragma unroll
-          for (int k = 0; k < W; ++k)
-            if (x0 + k < hx) o[k] = fmaf(ELx[x0 + k], e0, o[k]);
-        }
-        if (x0 + W > nx - hx) {
-          const float e1 = row[C0 + nx - 1];
-#pragma unroll
-          for (int k = 0; k < W; ++k) {
-            const int kk = nx - 1 - x0 - k;
-            if (kk < hx) o[k] = fmaf(ERx[kk], e1, o[k]);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < W; ++k) acc[k] += o[k];
+        for (int k = 0; k < X; ++k) acc[k] = add2(acc[k], o[k]);
       }
-      if (more) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int e = tid + j * NTH;
-          if (e < tot4) {
-            const int z = zdiv(e, rn4), c = e - z * n4;
-            st4(XN + z * bs + C0 + 4 * c, pf[j]);
-          }
-        }
-        zs_table(a, set, yn, XN + tz * bs, tid, NTH);
-      }
-      y = yn;
+      cp_wait();
       __syncthreads();
     }
-    if (mine) {
-      float* o = a.part + ((size_t)id * nz + Z0 + zl) * nx + x0;
-#pragma unroll
-      for (int k = 0; k < W; k += 4) st4(o + k, make_float4(acc[k], acc[k + 1], acc[k + 2], acc[k + 3]));
-    }
+    if (mine) zstore_part<X>(a.part + (size_t)id * nz * nx, acc, nx, nz, 2 * (Z0 + zl), x0);
   }
 }
 

@@ -95,3 +95,25 @@ def test_shear_rotation_on_the_fused_pair(S, O, monkeypatch, nx, nz, px, pz, nvi
     G = O.Geometry(mumap, psfs, 4.8, interp="one")
     assert relerr(out["fused"][0], G.project(x, index=ii)) <= TOL
     assert relerr(out["fused"][1], G.backproject(ys, index=ii)) <= TOL
+
+
+@pytest.mark.parametrize("nx,nz,px,pz,nview,idx", [
+    (90, 53, 21, 17, 12, [11, 0, 4]),  # three column tiles, the last of 26 columns; an odd last row
+    (34, 9, 5, 3, 9, None),            # two tiles of 20 and 14 columns
+    (10, 3, 3, 3, 7, None),
+    (2, 1, 1, 1, 4, None),
+])
+def test_ragged_large_plane_kernels(S, O, monkeypatch, nx, nz, px, pz, nview, idx):
+    """The large-plane forward kernels (forced) on ragged matrices equal the
+    fused kernel bit for bit."""
+    mumap, psfs, x, y = _plan_inputs(S, nx, nz, px, pz, nview, 11 * nx + nz)
+    ii = None if idx is None else np.array(idx, np.int32)
+    out = {}
+    for strip in ("0", "1"):
+        monkeypatch.setenv("SPECT_ZSTRIP", strip)
+        plan = S.SPECTplan(mumap, psfs, 4.8)
+        assert plan.path == ("strip" if strip == "1" else "fused")
+        out[strip] = S.project(x, plan, index=ii)
+        plan.close()
+    assert np.array_equal(out["0"], out["1"])
+    assert relerr(out["1"], O.Geometry(mumap, psfs, 4.8).project(x, index=ii)) <= TOL

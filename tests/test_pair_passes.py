@@ -221,3 +221,40 @@ def test_gather_adjoint_tile(nx, nz, px, pz, nv):
     assert sorted(slots) == list(range(nv))
     # tiles cover the image
     assert -(-nx // t["tx"]) * t["tx"] >= nx and -(-nx // t["ty"]) * t["ty"] >= nx
+
+
+@pytest.mark.parametrize("nx,nz,px,pz", SIZES + [(222, 150, 41, 41), (254, 199, 65, 65), (512, 230, 65, 65)])
+def test_large_plane_forward_tiles(nx, nz, px, pz):
+    """Mirror of zs_tiles (csrc/zpath_api.h): the indexes of k_zs_fz and
+    k_zs_fx stay inside their buffers, and every task has a thread."""
+    g = zgeom(nx, nz, px, pz)
+    trow = 2 * g["hs"] + g["ts"] + 4
+    nzb, nrp, nxw = (nz + 7) // 8, (nz + 1) // 2, (nx + 7) // 8
+    tmax = min(32, 2 * (320 // nzb))
+    ntile = -(-nx // tmax)
+    tx = min(nx, zround(-(-nx // ntile), 4))
+    zvst, xbst = zstride2(8 * nzb + g["zpw"]), zstride2(8 * nxw + g["xpw"])
+    tzp = min(max(1, 320 // nxw), nrp)
+    fz, fx = 4 * (4 * (trow + 8 * tx + zround(tx, 4)) + 2 * tx * zvst), 4 * 2 * (2 * tzp * xbst + trow)
+    assert fz <= OPTIN and fx <= OPTIN and zround(tzp * nxw, 32) <= NTH
+    assert min(320, 2 * zround((tx // 2 * nzb + 1) // 2, 32)) % 64 == 0  # whole warps a plane
+    # k_zs_fz: gather stores, windows; the last tile has an even number of columns
+    assert tx % 2 == 0 and (nx - (nx - 1) // tx * tx) % 2 == 0
+    assert g["R0"] + 4 * ((nz + 3) // 4) <= zvst and 8 * (nzb - 1) + g["zpw"] + 8 <= zvst
+    # rows it stores are the row pairs k_zs_fx reads
+    assert {(z0 + 2 * m) // 2 for z0 in range(0, 8 * nzb, 8) for m in range(4) if z0 + 2 * m < nz} == set(range(nrp))
+    # k_zs_fx: data columns and windows
+    assert g["C0"] + nx <= xbst and 8 * (nxw - 1) + g["xpw"] + 8 <= xbst
+    # planes of the exchange buffer fit its allocation (nzp values a column)
+    assert 2 * nrp * nx <= zround(nz, 16) * nx
+    n2, nth = nx // 2, zround(tzp * nxw, 32)
+    for tid in (0, 1, nth - 1):
+        dr, dc = divmod(nth, n2)
+        r, c = divmod(tid, n2)
+        got = []
+        while r < tzp:
+            got.append(r * n2 + c)
+            r, c = r + dr, c + dc
+            if c >= n2:
+                r, c = r + 1, c - n2
+        assert got == list(range(tid, tzp * n2, nth))
