@@ -590,10 +590,12 @@ int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx,
     } else {
       LAUNCH(p, K_CONV_FWD, st, "k_zfwd", zfwd_launch(a.G, st, a));
     }
-    const size_t n = (size_t)nv * p->nxz / (p->nxz % 4 == 0 ? 4 : 1);
+    // four elements a thread where that leaves a warp for every scheduler
+    const int vec = p->nxz % 4 == 0 && (size_t)nv * p->nxz >= (size_t)512 * p->sm_count ? 4 : 1;
+    const size_t n = (size_t)nv * p->nxz / vec;
     const int rb = (int)std::min<size_t>((n + 255) / 256, (size_t)p->sm_count * 16);
     LAUNCH(p, K_REDUCE_VIEWS, st, "k_reduce_parts",
-           zreduce_launch(rb, st, partbuf, nv, p->ny, a.G, (int)p->nxz, views + (size_t)g0 * p->nxz, y, bg, vi));
+           zreduce_launch(rb, st, partbuf, nv, p->ny, a.G, (int)p->nxz, vec, views + (size_t)g0 * p->nxz, y, bg, vi));
   }
   return SPECT_OK;
 }

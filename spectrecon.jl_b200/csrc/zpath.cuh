@@ -215,6 +215,18 @@ __device__ __forceinline__ void zstore_part(float* part, const f2 (&acc)[X], int
   }
 }
 
+// programmatic dependent launch: wait until the kernels before this one in the
+// stream have completed, then let the next one's blocks start where room is
+// (they wait here in turn).  What a kernel does before it touches nothing
+// that an earlier kernel writes or reads: its own shared memory, the plan's
+// constant tables, the view list.  Data that such kernels exchange is read by
+// plain loads: a pointer marked __restrict__ or a read-only load could be
+// moved above the wait.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // fetch the 128-byte line of p into L2
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -234,10 +246,11 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::
 // Layout changes between the caller's image [z][y][x] and IZ.
 // k_to_iz: IZ interior (and its z padding) from img; grid (ceil(nx/32),
 // ny, ceil(nzp/32)), block (32, 8).
-__global__ void __launch_bounds__(256) k_to_iz(ZGeom g, const float* __restrict__ img, float* __restrict__ iz) {
+__global__ void __launch_bounds__(256) k_to_iz(ZGeom g, const float* img, float* iz) {
   __shared__ float tile[32][33];
   const int x0 = blockIdx.x * 32, y = blockIdx.y, z0 = blockIdx.z * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
+  grid_wait();
   for (int k = ty; k < 32; k += 8) {  // tile[z][x], coalesced over x
     const int z = z0 + k, x = x0 + tx;
     tile[k][tx] = (z < g.nz && x < g.nx) ? img[((size_t)z * g.ny + y) * g.nx + x] : 0.f;
@@ -252,11 +265,12 @@ __global__ void __launch_bounds__(256) k_to_iz(ZGeom g, const float* __restrict_
 // k_from_iz: dst (caller layout) from the IZ interior.  mode 0: dst = v;
 // 1: dst = v, zeros -> +Inf (EM sensitivity, src/ml-os-em.jl:111-114);
 // 2: dst = dst * (v / asum) (EM update, asum in the caller layout).
-__global__ void __launch_bounds__(256) k_from_iz(ZGeom g, const float* __restrict__ iz, float* dst,
-                                                 const float* __restrict__ asum, int mode) {
+__global__ void __launch_bounds__(256) k_from_iz(ZGeom g, const float* iz, float* dst, const float* asum,
+                                                 int mode) {
   __shared__ float tile[32][33];
   const int x0 = blockIdx.x * 32, y = blockIdx.y, z0 = blockIdx.z * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
+  grid_wait();
   for (int k = ty; k < 32; k += 8) {  // tile[x][z], coalesced over z
     const int x = x0 + k, z = z0 + tx;
     tile[k][tx] = (x < g.nx && z < g.nz) ? iz[((size_t)(y + g.pad) * g.L + x + g.pad) * g.nzp + z] : 0.f;
@@ -485,10 +499,10 @@ __device__ __forceinline__ int zblock_of(long long q, int n, int G) { return (in
 
 // four view elements a thread where nxz % 4 == 0 (V = 4), else one
 template <int V>
-__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nv, int ny, int G, int nxz,
-                                                      float* __restrict__ out, const float* __restrict__ y,
-                                                      const float* __restrict__ bg, const int* __restrict__ vidx) {
+__global__ void __launch_bounds__(256) k_reduce_parts(const float* part, int nv, int ny, int G, int nxz, float* out,
+                                                      const float* y, const float* bg, const int* vidx) {
   const int per = nxz / V, n = nv * ny;
+  grid_wait();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv * per; k += gridDim.x * blockDim.x) {
     const int slot = k / per, e = V * (k - slot * per);
     const int b0 = zblock_of((long long)slot * ny, n, G), b1 = zblock_of((long long)(slot + 1) * ny - 1, n, G);
@@ -496,7 +510,7 @@ __global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ 
     float s[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) s[i] = 0.f;
-#pragma unroll 4
+#pragma unroll 8
     for (int b = b0; b <= b1; ++b, p += nxz) {
       if constexpr (V == 4) {
         const float4 q = ld4(p);
@@ -632,6 +646,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
   for (int k = tid; k < nxp * vst + nzp2 * bst; k += nth) ZB[k] = 0;
   cp_wait();
   __syncthreads();
+  grid_wait();
   gather(v, y);
   // this thread's x tasks: rows 2 zp, 2 zp + 1, columns x0 .. x0 + X - 1
   f2 acc[NT][X];
@@ -805,6 +820,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
   };
   table(v, y, 0);
   for (int k = tid; k < a.t.nxb * (tz / 2) * bst; k += nth) XB0[k] = 0;
+  grid_wait();
   load_view();
   cp_wait();
   __syncthreads();
@@ -953,12 +969,12 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
 // Epilogue (IZ layout): v = acc (+ prev); mode 1: zeros -> +Inf; mode 2:
 // v = x * (v / asum); out = v (z < nz only; out may be prev or x).
 template <bool ONE>
-__global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* __restrict__ T,
+__global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* T,
                                                              int zcol, const float4* __restrict__ rot,
                                                              const Rot1View* __restrict__ r1,
                                                              const int* __restrict__ vidx, int nv, const float* prev,
-                                                             float* out, const float* x,
-                                                             const float* __restrict__ asum, int mode) {
+                                                             float* out, const float* x, const float* asum,
+                                                             int mode) {
   constexpr int U = kZrotU, E = kZrotList;
   extern __shared__ float4 smem4[];
   const int nth = blockDim.x, tid = threadIdx.x, nx = g.nx, ny = g.ny, n4 = g.nzp / 4, C = r.tx * r.ty;
@@ -1025,7 +1041,7 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
     acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   auto load = [&](int i, int c) {
-    return __ldg(reinterpret_cast<const float4*>(Tz[i] + (unsigned long long)(unsigned)c * cb));
+    return *reinterpret_cast<const float4*>(Tz[i] + (unsigned long long)(unsigned)c * cb);
   };
   auto add = [&](float4& v, int wi, const float4& t) {
     const float w = __int_as_float(wi);
@@ -1036,6 +1052,7 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
   };
   hits(0, 0);
   __syncthreads();
+  grid_wait();
   for (int s0 = 0, buf = 0; s0 < nv; s0 += r.vb, buf ^= 1) {
     if (s0 + r.vb < nv) hits(s0 + r.vb, buf ^ 1);
     const int nb = min(r.vb, nv - s0);

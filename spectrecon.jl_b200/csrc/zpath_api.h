@@ -270,13 +270,17 @@ inline ZRotTile zrot_tile(const ZGeom& g, int nv, int sms) {
   return r;
 }
 
+// short work (about 100 us a kernel at most): nv planes stacks of nx x nx x nz
+inline bool zearly(const ZGeom& g, int nv) { return (long long)nv * g.nx * g.ny * g.nz <= (1LL << 25); }
+
 // launchers (zpath_inst.cu)
 cudaError_t zpath_setup(int max_smem);  // shared-memory limits of the fused kernels (zrot_adj_setup's too)
 cudaError_t zrot_adj_setup();
 cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
-// views (EM ratio with y, bg) of nv slots from the partial views of a walk by G blocks
-cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, float* out,
-                           const float* y, const float* bg, const int* vidx);
+// views (EM ratio with y, bg) of nv slots from the partial views of a walk by
+// G blocks, vec (4 or 1) elements a thread
+cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, int vec,
+                           float* out, const float* y, const float* bg, const int* vidx);
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
                             const Rot1View* r1, const int* vidx, int nv, const float* prev, float* out, const float* x,

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(ZArgs a) {
   if (item < nitems) prepare(item, base);
   cp_wait();
   __syncthreads();
+  grid_wait();
   const int hi4 = (tid >> 2) & 1, hth = nth / 2, pz = tid >= hth, tz = tid - pz * hth;
   for (; item < nitems; item += gridDim.x, hb ^= 1) {
     int slot, y, X0;
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(ZArgs a) {
   const int nrp = (nz + 1) / 2, ntz = (nrp + tzp - 1) / tzp, nitems = (a.G + a.nv) * ntz, n2 = nx / 2;
   for (int k = tid; k < 2 * bufsz; k += nth) base[k] = 0.f;  // columns outside the data stay zero
   __syncthreads();
+  grid_wait();
   const int xb = tid / tzp, zl = tid - xb * tzp, x0 = X * xb;  // this thread's task: row pair zl, columns x0 ..
   const int dr = nth / n2, dc = nth - dr * n2, r0 = tid / n2, c0 = tid - r0 * n2;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {

@@ -117,3 +117,41 @@ def test_ragged_large_plane_kernels(S, O, monkeypatch, nx, nz, px, pz, nview, id
         plan.close()
     assert np.array_equal(out["0"], out["1"])
     assert relerr(out["1"], O.Geometry(mumap, psfs, 4.8).project(x, index=ii)) <= TOL
+
+
+def test_unsynchronised_chain_equals_synchronised(S):
+    """Kernels of consecutive calls overlap at their ends (programmatic
+    dependent launch): a chain of projections and back-projections in which
+    every call reads what the call before it wrote gives the same bits as with
+    a synchronisation after each, on the default and on another stream."""
+    import torch
+
+    nx, nz, nview = 48, 21, 12
+    mumap, psfs, x, y = _plan_inputs(S, nx, nz, 7, 5, nview, 9)
+    plan = S.SPECTplan(mumap, psfs, 4.8)
+    idx = [np.array([3, 0, 7], np.int32), None, np.array([11, 2], np.int32)]
+    x0 = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    ref = None
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        for sync in (True, False):
+            with torch.cuda.stream(stream):
+                stream.wait_stream(torch.cuda.default_stream())
+                im = x0.clone()
+                got = []
+                for step in range(9):
+                    ii = idx[step % 3]
+                    n = nview if ii is None else len(ii)
+                    v = torch.empty((n, nz, nx), device="cuda")
+                    S.project_(v.permute(2, 1, 0), im.permute(2, 1, 0), plan, index=ii, stream=stream)
+                    if sync:
+                        torch.cuda.synchronize()
+                    out = torch.empty_like(im)
+                    S.backproject_(out.permute(2, 1, 0), v.permute(2, 1, 0), plan, index=ii, stream=stream)
+                    if sync:
+                        torch.cuda.synchronize()
+                    im = out / out.abs().max()
+                    got += [v, im]
+                torch.cuda.synchronize()
+            if ref is None:
+                ref = got
+            assert all(torch.equal(a, b) for a, b in zip(got, ref))
