@@ -552,6 +552,20 @@ ZArgs zargs(const spect_plan_s* p) {
   return a;
 }
 
+// views of a call: a device table, or the caller's host list (fused paths:
+// handed over in the kernels' parameters, kViewsInline at a time)
+struct ViewSel {
+  const int* dev;
+  const int32_t* host;
+};
+ViewList view_list(const ViewSel& s, int g0, int nv) {
+  ViewList l;
+  l.p = s.host ? nullptr : s.dev + g0;
+  for (int i = 0; s.host && i < nv; ++i) l.v[i] = (unsigned short)s.host[g0 + i];
+  return l;
+}
+int view_group(const ViewSel& s, int gmax) { return s.host ? std::min(gmax, kViewsInline) : gmax; }
+
 // blocks of the forward walk over nv views with room for cap partial views
 // (block + slot).  The fused and the large-plane kernels share the walk, so
 // their partial sums agree bit for bit.
@@ -565,15 +579,15 @@ int zwalk_blocks(const spect_plan_s* p, int nv, int cap) {
 // zpath forward of nidx views of the IZ image: k_zfwd (rotation, attenuation,
 // convolution, depth sum of a block's planes) then the sum of the partial
 // views (+ EM ratio y/(Ax+bg)); partbuf holds cap partial views
-int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx, int nidx, cudaStream_t st,
+int zforward(spect_plan_s* p, float* views, const float* imgIZ, const ViewSel& vsel, int nidx, cudaStream_t st,
              const float* y, const float* bg, float* partbuf, int cap, int gmax) {
+  gmax = view_group(vsel, gmax);
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
     const int nv = std::min(gmax, nidx - g0);
-    const int* vi = vidx + g0;
     ZArgs a = zargs(p);
     a.t = p->zft;
     a.img = imgIZ;
-    a.vidx = vi;
+    a.vidx = view_list(vsel, g0, nv);
     a.nv = nv;
     a.part = partbuf;
     a.G = zwalk_blocks(p, nv, cap);
@@ -595,7 +609,7 @@ int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx,
     const size_t n = (size_t)nv * p->nxz / vec;
     const int rb = (int)std::min<size_t>((n + 255) / 256, (size_t)p->sm_count * 16);
     LAUNCH(p, K_REDUCE_VIEWS, st, "k_reduce_parts",
-           zreduce_launch(rb, st, partbuf, nv, p->ny, a.G, (int)p->nxz, vec, views + (size_t)g0 * p->nxz, y, bg, vi));
+           zreduce_launch(rb, st, partbuf, nv, p->ny, a.G, (int)p->nxz, vec, views + (size_t)g0 * p->nxz, y, bg, a.vidx));
   }
   return SPECT_OK;
 }
@@ -604,26 +618,26 @@ int zforward(spect_plan_s* p, float* views, const float* imgIZ, const int* vidx,
 // planes) then k_zrot_adj (gather over the group's views; groups after the
 // first add to the accumulator).  mode 0: out = A' views; 1: zeros -> Inf;
 // 2: out = x .* (A' views) ./ asum (x, asum in IZ; out may be x).
-int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx, int nidx, cudaStream_t st, int mode,
+int zbackward(spect_plan_s* p, float* outIZ, const float* views, const ViewSel& vsel, int nidx, cudaStream_t st, int mode,
               const float* xIZ, const float* asumIZ) {
   if (nidx == 0) {
     CUDA_TRY(cudaMemsetAsync(outIZ, 0, sizeof(float) * p->izN, st));
     return SPECT_OK;
   }
-  for (int g0 = 0; g0 < nidx; g0 += p->gmax) {
-    const int nv = std::min(p->gmax, nidx - g0);
-    const int* vi = vidx + g0;
+  const int gmax = view_group(vsel, p->gmax);
+  for (int g0 = 0; g0 < nidx; g0 += gmax) {
+    const int nv = std::min(gmax, nidx - g0);
     ZArgs a = zargs(p);
     a.views = views + (size_t)g0 * p->nxz;
     a.T = p->d_P;
-    a.vidx = vi;
+    a.vidx = view_list(vsel, g0, nv);
     a.nv = nv;
     a.t = p->zat;
     const int gs = (int)std::min<long long>((long long)p->sm_count * p->zat.occ, (long long)nv * p->zat.ntile * p->ny);
     LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
     LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, a.r1, vi, nv, g0 > 0 ? p->d_backIZ : nullptr,
+           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, a.r1, a.vidx, nv, g0 > 0 ? p->d_backIZ : nullptr,
                            last ? outIZ : p->d_backIZ, xIZ, asumIZ, last ? mode : 0));
   }
   return SPECT_OK;
@@ -631,12 +645,13 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const int* vidx
 
 // forward projection of nidx views (device index list vidx) into views;
 // with y/bg non-null the output is the EM ratio y/(A x + bg).
-int forward_scratch(spect_plan_s* p, float* views, const float* image, const int* vidx, int nidx, cudaStream_t st,
+int forward_scratch(spect_plan_s* p, float* views, const float* image, const ViewSel& vsel, int nidx, cudaStream_t st,
                     const float* y, const float* bg, float* Pbuf, float* partbuf, int cap, int gmax) {
   if (p->zpath) {
     LAUNCH(p, K_OTHER, st, "k_to_iz", zto_iz_launch(p->zg, st, image, p->d_imgIZ));
-    return zforward(p, views, p->d_imgIZ, vidx, nidx, st, y, bg, partbuf, cap, gmax);
+    return zforward(p, views, p->d_imgIZ, vsel, nidx, st, y, bg, partbuf, cap, gmax);
   }
+  const int* const vidx = vsel.dev;
   const Geom& g = p->g;
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
     const int nv = std::min(gmax, nidx - g0);
@@ -703,20 +718,21 @@ int forward_scratch(spect_plan_s* p, float* views, const float* image, const int
   return SPECT_OK;
 }
 
-int forward(spect_plan_s* p, float* views, const float* image, const int* vidx, int nidx, cudaStream_t st,
+int forward(spect_plan_s* p, float* views, const float* image, const ViewSel& vsel, int nidx, cudaStream_t st,
             const float* y, const float* bg) {
-  return forward_scratch(p, views, image, vidx, nidx, st, y, bg, p->d_P, p->d_part, p->part_cap, p->gmax);
+  return forward_scratch(p, views, image, vsel, nidx, st, y, bg, p->d_P, p->d_part, p->part_cap, p->gmax);
 }
 
 // back-projection of nidx views.  mode 0: image = A' views; mode 1: image =
 // A' views with zeros -> Inf (EM sensitivity); mode 2: image .*= (A' views) ./ asum
-int backward(spect_plan_s* p, float* image, const float* views, const int* vidx, int nidx, cudaStream_t st,
+int backward(spect_plan_s* p, float* image, const float* views, const ViewSel& vsel, int nidx, cudaStream_t st,
              int mode, const float* asum) {
   if (p->zpath) {
-    STATUS_TRY(zbackward(p, p->d_backIZ, views, vidx, nidx, st, 0, nullptr, nullptr));
+    STATUS_TRY(zbackward(p, p->d_backIZ, views, vsel, nidx, st, 0, nullptr, nullptr));
     LAUNCH(p, K_REDUCE_IMAGE, st, "k_from_iz", zfrom_iz_launch(p->zg, st, p->d_backIZ, image, asum, mode));
     return SPECT_OK;
   }
+  const int* const vidx = vsel.dev;
   const Geom& g = p->g;
   const int nsplit = p->nsplit_adj;
   if (nidx == 0) {
@@ -762,7 +778,7 @@ int backward(spect_plan_s* p, float* image, const float* views, const int* vidx,
       LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
              zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, vi, nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
+             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, view_list(ViewSel{vi, nullptr}, 0, nv), nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
                              nullptr, nullptr, 0));
     } else if (p->interp == SPECT_INTERP_ONE) {
       const size_t n = (size_t)nv * p->N;
@@ -799,10 +815,10 @@ int backward(spect_plan_s* p, float* image, const float* views, const int* vidx,
   return SPECT_OK;
 }
 
-int stage_index(spect_plan_s* p, const int32_t* index, int nindex, cudaStream_t st, const int** dev) {
+int stage_index(spect_plan_s* p, const int32_t* index, int nindex, cudaStream_t st, ViewSel* sel) {
   if (!index) {
     if (nindex != p->nview) return fail(SPECT_ERR_DIM, "DimensionMismatch: index=NULL needs nindex == nview");
-    *dev = p->d_all;
+    *sel = ViewSel{p->d_all, nullptr};
     return SPECT_OK;
   }
   if (nindex < 0 || nindex > p->nview)
@@ -811,8 +827,12 @@ int stage_index(spect_plan_s* p, const int32_t* index, int nindex, cudaStream_t 
     if (index[i] < 0 || index[i] >= p->nview)
       return fail(SPECT_ERR_INDEX, "BoundsError: view index " + std::to_string(index[i]) + " not in 0.." +
                                        std::to_string(p->nview - 1));
+  if (p->zpath && p->nview <= 65536) {
+    *sel = ViewSel{nullptr, index};
+    return SPECT_OK;
+  }
   CUDA_TRY(cudaMemcpyAsync(p->d_idx, index, sizeof(int) * nindex, cudaMemcpyHostToDevice, st));
-  *dev = p->d_idx;
+  *sel = ViewSel{p->d_idx, nullptr};
   return SPECT_OK;
 }
 
@@ -884,11 +904,11 @@ int enqueue_osem(spect_plan_s* p, float* out, const float* x0, const float* y, c
   if (p->zpath) {  // the iterate and the sensitivities stay in the IZ layout
     LAUNCH(p, K_OTHER, st, "k_to_iz", zto_iz_launch(p->zg, st, x0, p->d_imgIZ));
     for (int b = 0; b < nblocks; ++b)
-      STATUS_TRY(zbackward(p, p->d_asum + (size_t)b * p->izN, p->d_ones, p->d_sub + (size_t)b * nsub, nsub, st, 1,
+      STATUS_TRY(zbackward(p, p->d_asum + (size_t)b * p->izN, p->d_ones, ViewSel{p->d_sub + (size_t)b * nsub, nullptr}, nsub, st, 1,
                            nullptr, nullptr));
     for (int it = 0; it < niter; ++it)
       for (int b = 0; b < nblocks; ++b) {
-        const int* vi = p->d_sub + (size_t)b * nsub;
+        const ViewSel vi{p->d_sub + (size_t)b * nsub, nullptr};
         STATUS_TRY(zforward(p, p->d_views_tmp, p->d_imgIZ, vi, nsub, st, y, bg, p->d_part, p->part_cap, p->gmax));
         STATUS_TRY(zbackward(p, p->d_imgIZ, p->d_views_tmp, vi, nsub, st, 2, p->d_imgIZ,
                              p->d_asum + (size_t)b * p->izN));
@@ -897,12 +917,12 @@ int enqueue_osem(spect_plan_s* p, float* out, const float* x0, const float* y, c
     return SPECT_OK;
   }
   for (int b = 0; b < nblocks; ++b)
-    STATUS_TRY(backward(p, p->d_asum + (size_t)b * p->N, p->d_ones, p->d_sub + (size_t)b * nsub, nsub, st, 1,
+    STATUS_TRY(backward(p, p->d_asum + (size_t)b * p->N, p->d_ones, ViewSel{p->d_sub + (size_t)b * nsub, nullptr}, nsub, st, 1,
                         nullptr));
   if (out != x0) CUDA_TRY(cudaMemcpyAsync(out, x0, sizeof(float) * p->N, cudaMemcpyDeviceToDevice, st));
   for (int it = 0; it < niter; ++it)
     for (int b = 0; b < nblocks; ++b) {
-      const int* vi = p->d_sub + (size_t)b * nsub;
+      const ViewSel vi{p->d_sub + (size_t)b * nsub, nullptr};
       STATUS_TRY(forward(p, p->d_views_tmp, out, vi, nsub, st, y, bg));
       STATUS_TRY(backward(p, out, p->d_views_tmp, vi, nsub, st, 2, p->d_asum + (size_t)b * p->N));
     }
@@ -977,8 +997,8 @@ int time_pass(spect_plan_s* p, bool adj, int nv, int reps, double* ms) {
   int rc = SPECT_OK;
   for (int r = 0; r <= reps && rc == SPECT_OK; ++r) {  // r = 0: warm-up
     cudaEventRecord(a, st);
-    rc = adj ? backward(p, p->d_io_img, p->d_io_views, p->d_all, nv, st, 0, nullptr)
-             : forward(p, p->d_io_views, p->d_io_img, p->d_all, nv, st, nullptr, nullptr);
+    rc = adj ? backward(p, p->d_io_img, p->d_io_views, ViewSel{p->d_all, nullptr}, nv, st, 0, nullptr)
+             : forward(p, p->d_io_views, p->d_io_img, ViewSel{p->d_all, nullptr}, nv, st, nullptr, nullptr);
     cudaEventRecord(b, st);
     if (cudaEventSynchronize(b) != cudaSuccess) rc = fail(SPECT_ERR_CUDA, "autotune timing");
     float t = 0;
@@ -1913,7 +1933,7 @@ int spect_project(spect_plan_t p, float* views, const float* image, const int32_
   if (!p || !views || !image) return fail(SPECT_ERR_ARG, "null pointer argument");
   std::lock_guard<std::mutex> lk(p->mu);
   cudaStream_t st = (cudaStream_t)stream;
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   return forward(p, views, image, vi, nindex, st, nullptr, nullptr);
 }
@@ -1943,7 +1963,7 @@ int spect_project_static_scratch(spect_plan_t p, float* views, const float* imag
   size_t off = (sizeof(float) * (size_t)gmax * p->N + 255) & ~(size_t)255;
   float* partbuf = reinterpret_cast<float*>(static_cast<unsigned char*>(base) + off);
   cudaStream_t st = (cudaStream_t)stream;
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   const bool prof = p->prof.on;
   p->prof.on = false;  // no event creation on this path
@@ -1971,7 +1991,7 @@ int spect_project_host(spect_plan_t p, float* views, const float* image, const i
   std::lock_guard<std::mutex> lk(p->mu);
   STATUS_TRY(ensure_io(p));
   cudaStream_t st = 0;
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   CUDA_TRY(cudaMemcpyAsync(p->d_io_img, image, sizeof(float) * p->N, cudaMemcpyHostToDevice, st));
   STATUS_TRY(forward(p, p->d_io_views, p->d_io_img, vi, nindex, st, nullptr, nullptr));
@@ -1984,7 +2004,7 @@ int spect_backproject(spect_plan_t p, float* image, const float* views, const in
   if (!p || !views || !image) return fail(SPECT_ERR_ARG, "null pointer argument");
   std::lock_guard<std::mutex> lk(p->mu);
   cudaStream_t st = (cudaStream_t)stream;
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   return backward(p, image, views, vi, nindex, st, 0, nullptr);
 }
@@ -1994,7 +2014,7 @@ int spect_backproject_host(spect_plan_t p, float* image, const float* views, con
   std::lock_guard<std::mutex> lk(p->mu);
   STATUS_TRY(ensure_io(p));
   cudaStream_t st = 0;
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   CUDA_TRY(cudaMemcpyAsync(p->d_io_views, views, sizeof(float) * nindex * p->nxz, cudaMemcpyHostToDevice, st));
   STATUS_TRY(backward(p, p->d_io_img, p->d_io_views, vi, nindex, st, 0, nullptr));
@@ -2045,7 +2065,7 @@ int spect_em_subset_update(spect_plan_t p, float* x, const float* ynoisy, const 
   std::lock_guard<std::mutex> lk(p->mu);
   cudaStream_t st = (cudaStream_t)stream;
   STATUS_TRY(ensure_em(p, 1));
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   STATUS_TRY(forward(p, p->d_views_tmp, x, vi, nindex, st, ynoisy, background));
   return backward(p, x, p->d_views_tmp, vi, nindex, st, 2, asum);
@@ -2056,7 +2076,7 @@ int spect_subset_sensitivity(spect_plan_t p, float* asum, const int32_t* index, 
   std::lock_guard<std::mutex> lk(p->mu);
   cudaStream_t st = (cudaStream_t)stream;
   STATUS_TRY(ensure_em(p, 1));
-  const int* vi;
+  ViewSel vi;
   STATUS_TRY(stage_index(p, index, nindex, st, &vi));
   return backward(p, asum, p->d_ones, vi, nindex, st, 1, nullptr);
 }

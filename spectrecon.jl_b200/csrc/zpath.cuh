@@ -500,7 +500,8 @@ __device__ __forceinline__ int zblock_of(long long q, int n, int G) { return (in
 // four view elements a thread where nxz % 4 == 0 (V = 4), else one
 template <int V>
 __global__ void __launch_bounds__(256) k_reduce_parts(const float* part, int nv, int ny, int G, int nxz, float* out,
-                                                      const float* y, const float* bg, const int* vidx) {
+                                                      const float* y, const float* bg,
+                                                      const __grid_constant__ ViewList vidx) {
   const int per = nxz / V, n = nv * ny;
   grid_wait();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv * per; k += gridDim.x * blockDim.x) {
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(256) k_reduce_parts(const float* part, int nv,
 // Shared memory: [2 tables][geoW nx x (w00 w00 w10 w10 | w01 w01 w11 w11)]
 // [geoO nx int][ZB nxp * vst][XB (nz + 1) / 2 * bst] (lines: float2).
 template <int NT, bool ONE>
-__global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
+__global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int X = kZfwdX, W = kZfwdZ;
   const ZGeom& g = a.g;
@@ -774,7 +775,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(ZArgs a) {
 // (five row tiles, two XB) 735 -> 483 us.
 // Shared memory (float2): [VB nxp * vst][XB nxb * (tz / 2) * bst][3 tables].
 template <int W>
-__global__ void __launch_bounds__(kZThreads, 1) k_zadj(ZArgs a) {
+__global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
   const ZGeom& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2;
@@ -972,7 +973,7 @@ template <bool ONE>
 __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* T,
                                                              int zcol, const float4* __restrict__ rot,
                                                              const Rot1View* __restrict__ r1,
-                                                             const int* __restrict__ vidx, int nv, const float* prev,
+                                                             const __grid_constant__ ViewList vidx, int nv, const float* prev,
                                                              float* out, const float* x, const float* asum,
                                                              int mode) {
   constexpr int U = kZrotU, E = kZrotList;

@@ -84,6 +84,16 @@ struct Rot1View {
   int m, mode;
 };
 
+// plan views of a call's slots: a device table, or up to kViewsInline of them
+// in the kernel's own parameters (a caller's index list then needs no copy to
+// the device, about 6 us a call and a break in the kernels' overlap)
+constexpr int kViewsInline = 256;
+struct ViewList {
+  const int* p;
+  unsigned short v[kViewsInline];
+  __host__ __device__ int operator[](int i) const { return p ? p[i] : v[i]; }
+};
+
 struct ZArgs {
   ZGeom g;
   ZTile t;
@@ -92,7 +102,7 @@ struct ZArgs {
   const float* img;     // IZ
   const float* att;     // ATT
   const float4* rot;    // [view] (cos(2pi - theta), sin(2pi - theta), theta == 0, theta)
-  const int* vidx;      // [nv] plan view of each slot
+  ViewList vidx;        // plan view of each slot
   const int* viewset;   // [nview] PSF set of each view
   int nv;
   int G;                // blocks of the forward walk (partial views: block + slot)
@@ -280,10 +290,10 @@ cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a);
 // views (EM ratio with y, bg) of nv slots from the partial views of a walk by
 // G blocks, vec (4 or 1) elements a thread
 cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, int vec,
-                           float* out, const float* y, const float* bg, const int* vidx);
+                           float* out, const float* y, const float* bg, const ViewList& vidx);
 cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a);
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
-                            const Rot1View* r1, const int* vidx, int nv, const float* prev, float* out, const float* x,
+                            const Rot1View* r1, const ViewList& vidx, int nv, const float* prev, float* out, const float* x,
                             const float* asum, int mode);  // T[zero ..]: a column of zeros; r1: null for :two
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz);
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,

@@ -8,7 +8,7 @@ namespace spect {
 
 namespace {
 // [x tasks a thread - 1][rotation :two, :one]
-void (*const kZfwd[2][2])(ZArgs) = {{k_zfwd<1, false>, k_zfwd<1, true>}, {k_zfwd<2, false>, k_zfwd<2, true>}};
+void (*const kZfwd[2][2])(const ZArgs) = {{k_zfwd<1, false>, k_zfwd<1, true>}, {k_zfwd<2, false>, k_zfwd<2, true>}};
 // launch with programmatic stream serialisation (grid_wait, zpath.cuh) where
 // `early`: the blocks of a kernel start as the one before it in the stream
 // runs out, which hides its launch latency and its prologue; a kernel after
@@ -32,7 +32,7 @@ cudaError_t launch_next(bool early, void (*kernel)(P...), dim3 grid, dim3 block,
   c.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
-void (*const kZadj[2])(ZArgs) = {k_zadj<8>, k_zadj<16>};
+void (*const kZadj[2])(const ZArgs) = {k_zadj<8>, k_zadj<16>};
 
 }  // namespace
 
@@ -56,7 +56,7 @@ cudaError_t zfwd_launch(int grid, cudaStream_t st, const ZArgs& a) {
 }
 
 cudaError_t zreduce_launch(int grid, cudaStream_t st, const float* part, int nv, int ny, int G, int nxz, int vec,
-                           float* out, const float* y, const float* bg, const int* vidx) {
+                           float* out, const float* y, const float* bg, const ViewList& vidx) {
   return launch_next(true, vec == 4 ? k_reduce_parts<4> : k_reduce_parts<1>, grid, 256, 0, st, part, nv, ny, G, nxz, out, y,
                      bg, vidx);
 }
@@ -66,7 +66,7 @@ cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {
 }
 
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
-                            const Rot1View* r1, const int* vidx, int nv, const float* prev, float* out, const float* x,
+                            const Rot1View* r1, const ViewList& vidx, int nv, const float* prev, float* out, const float* x,
                             const float* asum, int mode) {
   const ZRotTile r = zrot_tile(g, nv, sms);
   const auto kernel = r1 ? k_zrot_adj<true> : k_zrot_adj<false>;

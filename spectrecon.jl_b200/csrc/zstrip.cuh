@@ -34,7 +34,7 @@ namespace spect {
 // which needed nx % 8 == 0, 394 us).
 // Shared memory: [2 x 2 x (table | geoW tx x 2 float4 | geoO tx int)]
 // [ZB 2 x tx / 2 * vst f2].
-__global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(ZArgs a) {
+__global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int W = 8;
   const ZGeom& g = a.g;
@@ -169,7 +169,7 @@ __device__ __forceinline__ bool zs_segment(const ZArgs& a, int id, int& slot, in
 // (cp.async) while a plane is worked on, one barrier a plane, two blocks an
 // SM.  Bound: FFMA2 and the shared-memory pipe; 256x256x200, 8 views 295 ->
 // 255 us.  Shared memory: 2 x [XB tzp * bst f2 | table].
-__global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(ZArgs a) {
+__global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int X = kZfwdX;
   const ZGeom& g = a.g;
