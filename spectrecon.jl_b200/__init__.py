@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 import numpy as np
 
@@ -46,11 +47,28 @@ def nthreads() -> int:
     return int(os.environ.get("SPECT_NTHREADS", os.cpu_count() or 1))
 
 
+def _cuda_tensor(a) -> bool:
+    """A plain float32 CUDA tensor, whose shape, strides and pointer are read
+    directly: building __cuda_array_interface__ takes about 5 us an argument.
+    Every other array goes by the interface (and meets its errors there)."""
+    torch = sys.modules.get("torch")
+    return (torch is not None and type(a) is torch.Tensor and a.is_cuda and a.dtype is torch.float32
+            and not a.requires_grad and a.layout is torch.strided and a.numel() > 0)
+
+
 def _is_device(a) -> bool:
-    return hasattr(a, "__cuda_array_interface__")
+    return _cuda_tensor(a) or hasattr(a, "__cuda_array_interface__")
 
 
 def _dev_ptr(a, shape, name):
+    if _cuda_tensor(a) and a.shape == tuple(shape):
+        want = 1
+        for n, st in zip(shape, a.stride()):
+            if n > 1 and st != want:
+                break
+            want *= n
+        else:
+            return a.data_ptr()
     cai = a.__cuda_array_interface__
     if tuple(cai["shape"]) != tuple(shape):
         raise SpectError(8, f"DimensionMismatch: {name} has shape {tuple(cai['shape'])}, expected {tuple(shape)}")
@@ -81,7 +99,7 @@ def _index(index):
     if index is None:
         return None, None
     idx = np.ascontiguousarray(np.asarray(index, dtype=np.int32).ravel())
-    return idx, _ptr(idx)
+    return idx, idx.ctypes.data
 
 
 def _stream_ptr(stream):

@@ -40,10 +40,11 @@ def to_julia_layout(t):
     """``t`` (Julia shape) as float32, column-major, on its device (copies
     only when its layout differs)."""
     torch = _torch()
-    t = t.detach().to(torch.float32)
-    nd = t.dim()
-    perm = tuple(reversed(range(nd)))
-    return t.permute(*perm).contiguous().permute(*perm)
+    t = t.detach()
+    perm = tuple(reversed(range(t.dim())))
+    if t.dtype is torch.float32 and t.permute(perm).is_contiguous():
+        return t
+    return t.to(torch.float32).permute(perm).contiguous().permute(perm)
 
 
 class SPECTOperator:
@@ -70,8 +71,13 @@ class SPECTOperator:
 
     H = T
 
-    def _stream(self):
-        return _torch().cuda.current_stream()
+    @staticmethod
+    def _stream():
+        """torch's current stream (its handle where torch gives that without
+        building a Stream object, about 5 us)."""
+        torch = _torch()
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return torch.cuda.current_stream() if raw is None else raw(torch.cuda.current_device())
 
     def forward(self, x):
         """views = P x (project!); ``x`` is a CUDA tensor of the image shape."""

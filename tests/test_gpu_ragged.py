@@ -155,3 +155,34 @@ def test_unsynchronised_chain_equals_synchronised(S):
             if ref is None:
                 ref = got
             assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+def test_device_array_checks(S):
+    """Device arrays meet the same checks however they are read: shape, type,
+    strides, gradients; arrays that only offer the interface still work, and
+    an index list longer than a kernel's own list gives the same views."""
+    import torch
+
+    nx, nz, nview = 16, 5, 300
+    mumap, psfs, x, _ = _plan_inputs(S, nx, nz, 3, 3, nview, 1)
+    plan = S.SPECTplan(mumap, psfs, 4.8)
+    im = torch.from_numpy(np.ascontiguousarray(x.T)).cuda().permute(2, 1, 0)
+    out = torch.empty((nview, nz, nx), device="cuda").permute(2, 1, 0)
+    S.project_(out, im, plan)
+    with pytest.raises(S.SpectError):
+        S.project_(out[:, :, :2], im, plan)
+    with pytest.raises(TypeError):
+        S.project_(out, im.double(), plan)
+    with pytest.raises(ValueError):
+        S.project_(out, im.permute(1, 0, 2), plan)
+    with pytest.raises(RuntimeError):
+        S.project_(out, im.clone().requires_grad_(True), plan)
+
+    class Interface:
+        def __init__(self, t):
+            self.__cuda_array_interface__ = t.__cuda_array_interface__
+
+    again = torch.empty_like(out)
+    S.project_(Interface(again), Interface(im), plan, index=np.arange(nview, dtype=np.int32))
+    torch.cuda.synchronize()
+    assert relerr(again.cpu().numpy(), out.cpu().numpy()) <= 1e-6  # other groups, other partial sums
