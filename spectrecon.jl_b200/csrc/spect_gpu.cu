@@ -552,8 +552,8 @@ ZArgs zargs(const spect_plan_s* p) {
   return a;
 }
 
-// views of a call: a device table, or the caller's host list (fused paths:
-// handed over in the kernels' parameters, kViewsInline at a time)
+// views of a call: a device table, or the caller's host list (fused paths, at
+// most kViewsInline: handed over in the kernels' parameters)
 struct ViewSel {
   const int* dev;
   const int32_t* host;
@@ -561,10 +561,9 @@ struct ViewSel {
 ViewList view_list(const ViewSel& s, int g0, int nv) {
   ViewList l;
   l.p = s.host ? nullptr : s.dev + g0;
-  for (int i = 0; s.host && i < nv; ++i) l.v[i] = (unsigned short)s.host[g0 + i];
+  for (int i = 0; s.host && i < nv; ++i) l.v[i] = s.host[g0 + i];
   return l;
 }
-int view_group(const ViewSel& s, int gmax) { return s.host ? std::min(gmax, kViewsInline) : gmax; }
 
 // blocks of the forward walk over nv views with room for cap partial views
 // (block + slot).  The fused and the large-plane kernels share the walk, so
@@ -581,7 +580,6 @@ int zwalk_blocks(const spect_plan_s* p, int nv, int cap) {
 // views (+ EM ratio y/(Ax+bg)); partbuf holds cap partial views
 int zforward(spect_plan_s* p, float* views, const float* imgIZ, const ViewSel& vsel, int nidx, cudaStream_t st,
              const float* y, const float* bg, float* partbuf, int cap, int gmax) {
-  gmax = view_group(vsel, gmax);
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
     const int nv = std::min(gmax, nidx - g0);
     ZArgs a = zargs(p);
@@ -624,9 +622,8 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const ViewSel& 
     CUDA_TRY(cudaMemsetAsync(outIZ, 0, sizeof(float) * p->izN, st));
     return SPECT_OK;
   }
-  const int gmax = view_group(vsel, p->gmax);
-  for (int g0 = 0; g0 < nidx; g0 += gmax) {
-    const int nv = std::min(gmax, nidx - g0);
+  for (int g0 = 0; g0 < nidx; g0 += p->gmax) {
+    const int nv = std::min(p->gmax, nidx - g0);
     ZArgs a = zargs(p);
     a.views = views + (size_t)g0 * p->nxz;
     a.T = p->d_P;
@@ -827,7 +824,7 @@ int stage_index(spect_plan_s* p, const int32_t* index, int nindex, cudaStream_t 
     if (index[i] < 0 || index[i] >= p->nview)
       return fail(SPECT_ERR_INDEX, "BoundsError: view index " + std::to_string(index[i]) + " not in 0.." +
                                        std::to_string(p->nview - 1));
-  if (p->zpath && p->nview <= 65536) {
+  if (p->zpath && nindex <= kViewsInline) {
     *sel = ViewSel{nullptr, index};
     return SPECT_OK;
   }

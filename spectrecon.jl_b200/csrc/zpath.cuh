@@ -501,7 +501,8 @@ __device__ __forceinline__ int zblock_of(long long q, int n, int G) { return (in
 template <int V>
 __global__ void __launch_bounds__(256) k_reduce_parts(const float* part, int nv, int ny, int G, int nxz, float* out,
                                                       const float* y, const float* bg,
-                                                      const __grid_constant__ ViewList vidx) {
+                                                      const __grid_constant__ ViewList list) {
+  const int* const vidx = list.ptr();
   const int per = nxz / V, n = nv * ny;
   grid_wait();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv * per; k += gridDim.x * blockDim.x) {
@@ -553,6 +554,7 @@ template <int NT, bool ONE>
 __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
   constexpr int X = kZfwdX, W = kZfwdZ;
+  const int* const vidx = a.vidx.ptr();
   const ZGeom& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2, nzp2 = (nz + 1) / 2;
   const int vst = a.t.vst, bst = a.t.bst, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
@@ -567,7 +569,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ Z
   if (p0 >= p1) return;
   const size_t Lz = (size_t)g.L * nzp;
   int slot = p0 / ny, j = p0 - slot * ny;
-  int y = (int)((long long)j * a.t.ystep % ny), v = a.vidx[slot];
+  int y = (int)((long long)j * a.t.ystep % ny), v = vidx[slot];
   auto table = [&](int view, int yy, int s) {  // every thread: its 16-byte pieces of the plane's table
     if (4 * tid >= trow) return;
     const float* src = a.tab + (((size_t)a.viewset[view] * ny + yy) * 2) * trow;
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ Z
       ++slot1;
     }
     const bool more = p + 1 < p1;
-    const int v1 = more && slot1 != slot ? a.vidx[slot1] : v;
+    const int v1 = more && slot1 != slot ? vidx[slot1] : v;
     const float* const Wt = tab0 + tb * trow;
     const f2* const Wd = reinterpret_cast<const f2*>(Wt);
     const int4 rg = *reinterpret_cast<const int4*>(Wt + 2 * hs + ts);  // tap ranges: z pass, x pass
@@ -777,6 +779,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ Z
 template <int W>
 __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ ZArgs a) {
   extern __shared__ float4 smem4[];
+  const int* const vidx = a.vidx.ptr();
   const ZGeom& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nzp = g.nzp, hs = g.hs, ts = g.ts, nxp = nx / 2;
   const int tz = a.t.tz, vst = a.t.vst, bst = a.t.bst, R0 = g.R0, C0 = g.C0, hz = g.hz, hx = g.hx;
@@ -792,7 +795,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ Z
   const float rnxp = 1.0f / nxp;
   int st = p0 / ny, j = p0 - st * ny;  // (slot, tile) of the plane and its place in the item
   int y = (int)((long long)j * a.t.ystep % ny);
-  int slot = st / ntile, Z0 = (st - slot * ntile) * tz, v = a.vidx[slot];
+  int slot = st / ntile, Z0 = (st - slot * ntile) * tz, v = vidx[slot];
   auto table = [&](int view, int yy, int s) {  // every thread: its 16-byte pieces of the plane's table
     const float* src = a.tab + (((size_t)a.viewset[view] * ny + yy) * 2 + 1) * trow;
     for (int k = 4 * tid; k < trow; k += 4 * nth) cp16(tab0 + s * trow + k, src + k);
@@ -841,7 +844,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ Z
     const int tb1 = tb == 2 ? 0 : tb + 1;
     const int slot1 = st1 == st ? slot : st1 / ntile;
     if (more) {  // the next plane's attenuation columns on their way into L2, too
-      const int v1 = slot1 == slot ? v : a.vidx[slot1], Z1 = (st1 - slot1 * ntile) * tz, ln = (min(tz, nz - Z1) + 31) / 32;
+      const int v1 = slot1 == slot ? v : vidx[slot1], Z1 = (st1 - slot1 * ntile) * tz, ln = (min(tz, nz - Z1) + 31) / 32;
       table(v1, y1, tb1);
       const float* src = a.att + (((size_t)v1 * ny + y1) * nx) * nzp + Z1;
       if (ntile == 1) {
@@ -938,7 +941,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ Z
       st = st1;
       slot = slot1;
       Z0 = (st - slot * ntile) * tz;
-      v = a.vidx[slot];
+      v = vidx[slot];
       load_view();
       __syncthreads();
     } else if (a.t.nxb == 1) {
@@ -973,10 +976,11 @@ template <bool ONE>
 __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile r, const float* T,
                                                              int zcol, const float4* __restrict__ rot,
                                                              const Rot1View* __restrict__ r1,
-                                                             const __grid_constant__ ViewList vidx, int nv, const float* prev,
+                                                             const __grid_constant__ ViewList views, int nv, const float* prev,
                                                              float* out, const float* x, const float* asum,
                                                              int mode) {
   constexpr int U = kZrotU, E = kZrotList;
+  const int* const vidx = views.ptr();
   extern __shared__ float4 smem4[];
   const int nth = blockDim.x, tid = threadIdx.x, nx = g.nx, ny = g.ny, n4 = g.nzp / 4, C = r.tx * r.ty;
   const float c0 = g.c0;

@@ -85,13 +85,15 @@ struct Rot1View {
 };
 
 // plan views of a call's slots: a device table, or up to kViewsInline of them
-// in the kernel's own parameters (a caller's index list then needs no copy to
-// the device, about 6 us a call and a break in the kernels' overlap)
-constexpr int kViewsInline = 256;
+// in the kernel's own parameters (a short index list of a caller then needs no
+// copy to the device, about 6 us a call and a break in the kernels' overlap)
+constexpr int kViewsInline = 32;
 struct ViewList {
   const int* p;
-  unsigned short v[kViewsInline];
-  __host__ __device__ int operator[](int i) const { return p ? p[i] : v[i]; }
+  int v[kViewsInline];
+  // one pointer for either, taken once a kernel (parameter memory is
+  // addressable there): a choice at every read cost k_zfwd up to 8 %
+  __device__ const int* ptr() const { return p ? p : v; }
 };
 
 struct ZArgs {

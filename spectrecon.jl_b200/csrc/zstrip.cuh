@@ -35,6 +35,7 @@ namespace spect {
 // Shared memory: [2 x 2 x (table | geoW tx x 2 float4 | geoO tx int)]
 // [ZB 2 x tx / 2 * vst f2].
 __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__ ZArgs a) {
+  const int* const vidx = a.vidx.ptr();
   extern __shared__ float4 smem4[];
   constexpr int W = 8;
   const ZGeom& g = a.g;
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__
   auto prepare = [&](int item, float* buf) {  // tables and sample geometry of an item
     int slot, y, X0;
     place(item, slot, y, X0);
-    const int v = a.vidx[slot];
+    const int v = vidx[slot];
     const float* src = a.tab + (((size_t)a.viewset[v] * ny + y) * 2) * trow;
     for (int k = 4 * tid; k < trow; k += 4 * nth) {
       cp16(buf + k, src + k);
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__
     for (int p = 0; p < 2; ++p) {
       const float4* const geoW = reinterpret_cast<const float4*>(buf + p * bufsz + trow);
       const int* const geoO = reinterpret_cast<const int*>(geoW + 2 * tx);
-      const float* att = a.att + (((size_t)a.vidx[slot] * ny + y + p) * nx + X0) * nzp;
+      const float* att = a.att + (((size_t)vidx[slot] * ny + y + p) * nx + X0) * nzp;
       for (int u = tid; u < txp * nz4; u += nth) {  // unit (column pair, z group)
         const int xp = zdiv(u, rnz4), z4 = u - xp * nz4;
         f2 lo[2], hi[2];
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__
         prefetch_l2_bulk(a.img + off, 2 * nzp * (unsigned)sizeof(float));
         prefetch_l2_bulk(a.img + off + Lz, 2 * nzp * (unsigned)sizeof(float));
         if (x == 0)
-          prefetch_l2_bulk(a.att + (((size_t)a.vidx[slot1] * ny + y1 + p) * nx + X1) * nzp,
+          prefetch_l2_bulk(a.att + (((size_t)vidx[slot1] * ny + y1 + p) * nx + X1) * nzp,
                            cols * nzp * (unsigned)sizeof(float));
       }
     }
@@ -170,6 +171,7 @@ __device__ __forceinline__ bool zs_segment(const ZArgs& a, int id, int& slot, in
 // SM.  Bound: FFMA2 and the shared-memory pipe; 256x256x200, 8 views 295 ->
 // 255 us.  Shared memory: 2 x [XB tzp * bst f2 | table].
 __global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(const __grid_constant__ ZArgs a) {
+  const int* const vidx = a.vidx.ptr();
   extern __shared__ float4 smem4[];
   constexpr int X = kZfwdX;
   const ZGeom& g = a.g;
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zs_fx(const __grid_constant__ 
     const int zt = item % ntz, id = item / ntz;  // partial view, planes j0 .. j1 - 1 of its slot
     int slot, j0, j1;
     if (!zs_segment(a, id, slot, j0, j1)) continue;
-    const int Z0 = zt * tzp, rows = min(tzp, nrp - Z0), set = a.viewset[a.vidx[slot]];
+    const int Z0 = zt * tzp, rows = min(tzp, nrp - Z0), set = a.viewset[vidx[slot]];
     int y = (int)((long long)j0 * a.t.ystep % ny);
     const bool mine = x0 < nx && zl < rows;
     auto fetch = [&](int yy, float* buf) {  // rows (16 bytes: columns 2 c, 2 c + 1 of a row pair) and table

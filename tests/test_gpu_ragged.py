@@ -185,4 +185,4 @@ def test_device_array_checks(S):
     again = torch.empty_like(out)
     S.project_(Interface(again), Interface(im), plan, index=np.arange(nview, dtype=np.int32))
     torch.cuda.synchronize()
-    assert relerr(again.cpu().numpy(), out.cpu().numpy()) <= 1e-6  # other groups, other partial sums
+    assert relerr(again.cpu().numpy(), out.cpu().numpy()) <= 1e-6
