@@ -204,8 +204,12 @@ inline ZTile zfwd_tile(const ZGeom& g, size_t optin, bool one) {
   const int xh = (xt + t.nxt - 1) / t.nxt, most = xh > zh ? xh : zh;
   t.nth = zround(most > gq ? most : gq, 32);
   if (t.nth > kZThreads) t.nth = kZThreads;
-  const int so = (int)((optin + 1024) / (t.smem + 1024)), ro = kZThreads / t.nth;
-  t.occ = so < ro ? so : ro;
+  const int so = (int)((optin + 1024) / (t.smem + 1024));
+  auto blocks = [&](int nth) { return so < kZThreads / nth ? so : kZThreads / nth; };
+  // twice the threads where shared memory leaves the SM short of warps (one
+  // slice of 128x128: 64 threads on ten blocks 49 us, 32 on fourteen 58 us)
+  if (2 * t.nth <= kZThreads && 2 * blocks(2 * t.nth) > blocks(t.nth) && so * t.nth < kZThreads) t.nth *= 2;
+  t.occ = blocks(t.nth);
   t.ystep = zdepth_step(g.ny);
   t.w = kZfwdX;
   return t;
@@ -256,8 +260,7 @@ inline ZsTiles zs_tiles(const ZGeom& g, size_t optin) {
 // one column of one slot).  16 columns a tile (8 of over 160 z): the blocks
 // are short enough to fill the last wave (128x128x80, 15 views: 46 us; 32
 // columns 48 us, 8 columns 46 us; 256x256x200, 8 views: 226 us, 8 columns 216
-// us), and images that leave the SMs short of threads split the slots
-// (64x64x64, 64 views: 32 columns 47 us, 16 columns in four groups 31 us).
+// us).
 constexpr int kZrotU = 2;          // units (column, four z) a thread
 constexpr int kZrotList = 9;       // list entries of a pair: its candidates at most
 constexpr int kZrotThreads = 512;  // nzp <= 256: 8 columns x 64 units / 2 = 256 a group at most
@@ -272,10 +275,19 @@ inline ZRotTile zrot_tile(const ZGeom& g, int nv, int sms) {
   r.ty = C / 4;
   r.grid = ((g.nx + r.tx - 1) / r.tx) * ((g.nx + r.ty - 1) / r.ty);
   const int gth = zround((C * n4 + kZrotU - 1) / kZrotU, 32);
-  r.S = (int)((long long)sms * 2 * kZrotThreads / ((long long)r.grid * gth));
-  if (r.S > nv) r.S = nv;
-  if (r.S > kZrotThreads / gth) r.S = kZrotThreads / gth;
-  if (r.S < 1) r.S = 1;
+  // slot groups: the fewest waves of blocks times their share of the slots,
+  // 15 % for each further group's lists and final sum (128x128x80, 15 views:
+  // two groups 42 us, one 46 us -- its last wave is nearly empty; 64x64x64, 64
+  // views: four groups 31 us)
+  double best = 0;
+  for (int S = 1; S <= nv && S * gth <= kZrotThreads; ++S) {
+    const int slots = sms * (2 * kZrotThreads / (S * gth));
+    const double cost = (double)((r.grid + slots - 1) / slots) / S * (1 + 0.15 * (S - 1));
+    if (S == 1 || cost < best) {
+      best = cost;
+      r.S = S;
+    }
+  }
   r.nth = r.S * gth;
   r.vb = r.nth / C;
   r.smem = (size_t)r.nth * 2 * kZrotList * 8;

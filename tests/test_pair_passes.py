@@ -199,7 +199,8 @@ def zrot_tile(g, nv, sms=148):
     tx, ty = 4, C // 4
     grid = -(-g["nx"] // tx) * -(-g["nx"] // ty)
     gth = zround((C * n4 + 1) // 2, 32)
-    S = max(1, min(sms * 1024 // (grid * gth), nv, 512 // gth))
+    S = min((s for s in range(1, min(nv, 512 // gth) + 1)),
+            key=lambda s: -(-grid // (sms * (1024 // (s * gth)))) / s * (1 + 0.15 * (s - 1)))
     return dict(C=C, tx=tx, ty=ty, grid=grid, gth=gth, S=S, nth=S * gth, vb=S * gth // C, n4=n4)
 
 
