@@ -207,6 +207,7 @@ struct ClassCols {
 __device__ __forceinline__ ClassCols class_cols(int nx, int c1) {
   ClassCols w;
   w.npt = (nx - c1 + 2) / 3;
+  if (w.npt <= 0) return ClassCols{0, 0, 0, 0x7fffffff, 0};  // no such column (nx 2, class 2): no row is walked
   w.dq = blockDim.x / w.npt;
   w.dm = blockDim.x - w.dq * w.npt;
   w.q0 = threadIdx.x / w.npt;
