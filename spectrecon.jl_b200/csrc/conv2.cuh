@@ -49,7 +49,7 @@ struct ConvGeom {
 struct Conv2Args {
   ConvGeom g;
   const float* P;       // forward input planes  [nv][ny][nz][nx]
-  float* T;             // adjoint output planes [nv][ny][nz][nx]
+  float* T;             // adjoint output planes [nv][ny][nz][nx], or [nv][ny][nx][nzp] when nzp > 0
   const float* Hs;      // [nset][ny][Q+1][Npx]
   const int* vidx;      // [nv] plan view of each slot
   const int* viewset;   // [nview] spectrum set of each view
@@ -66,6 +66,7 @@ struct Conv2Args {
   int att_mul;
   int* err;             // set to 1 when a bounded wait gives up
   int vsplit;           // k_vspec2: column blocks per view (work items nv * vsplit)
+  int nzp;              // adjoint output z fastest for k_zrot_adj, column pitch (a multiple of 4); 0: x fastest
 };
 
 struct Lanes {
@@ -249,6 +250,34 @@ __device__ __forceinline__ void store_plane(const ConvGeom& g, const PlaneWalk& 
   plane_walk(g, W, [&](int k, int x, int z) {
     dst[k] = att ? __fmul_rn(__ldg(att + k), Bf[x * rs + z]) : Bf[x * rs + z];
   });
+}
+
+// real rows of B -> z-fastest plane [nx][nzp] (zeros for z >= nz) in global
+// memory, times the attenuation plane [nz][nx] when given (shared or global
+// memory).  A warp's lanes are 32 columns, four z each: the attenuation rows
+// are read without bank conflicts, B's pairs with two-way ones, and a lane
+// writes 16 bytes.  The x-fastest store and a transpose kernel behind it moved
+// the planes three times: for 15 views of 128x128x80 (79 MB) 196 us + 58 us,
+// this store 211 us in all.
+__device__ __forceinline__ void store_plane_z(const ConvGeom& g, const float2* B, float* __restrict__ dst,
+                                              const float* att, int nzp, int warp, int lane) {
+  const int nxt = (g.nx + 31) / 32, tasks = nxt * (nzp / 4);
+  for (int t = warp; t < tasks; t += kConvWarps) {
+    const int z4 = t / nxt, x = (t - z4 * nxt) * 32 + lane, z = 4 * z4;
+    if (x >= g.nx) continue;
+    const float2* b = B + (size_t)x * g.QS + z / 2;
+    float2 u = make_float2(0.f, 0.f), w = u;  // a pair that starts inside the plane lies inside its B row
+    if (z < g.nz) u = b[0];
+    if (z + 2 < g.nz) w = b[1];
+    float r[4] = {u.x, u.y, w.x, w.y};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool in = z + k < g.nz;
+      if (att && in) r[k] = __fmul_rn(att[(size_t)(z + k) * g.nx + x], r[k]);
+      if (!in) r[k] = 0.f;
+    }
+    *reinterpret_cast<float4*>(dst + (size_t)x * nzp + z) = make_float4(r[0], r[1], r[2], r[3]);
+  }
 }
 
 // Per-lane index tables, computed once per kernel.
@@ -889,10 +918,17 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_adj2(Conv2Args a) {
           return;
         }
         phase ^= 1u;
-        store_plane_satt(g, W, B, a.T + ((size_t)slot * g.ny + y) * g.nz * g.nx, sA);
+        if (a.nzp > 0)
+          store_plane_z(g, B, a.T + ((size_t)slot * g.ny + y) * g.nx * a.nzp, sA, a.nzp, warp, lane);
+        else
+          store_plane_satt(g, W, B, a.T + ((size_t)slot * g.ny + y) * g.nz * g.nx, sA);
       } else {
         __syncthreads();
-        store_plane(g, W, B, a.T + ((size_t)slot * g.ny + y) * g.nz * g.nx, nullptr);
+        if (a.nzp > 0)  // the attenuation of planes too large to stage, from global memory
+          store_plane_z(g, B, a.T + ((size_t)slot * g.ny + y) * g.nx * a.nzp,
+                        a.att ? a.att + ((size_t)a.vidx[slot] * g.ny + y) * nplane : nullptr, a.nzp, warp, lane);
+        else
+          store_plane(g, W, B, a.T + ((size_t)slot * g.ny + y) * g.nz * g.nx, nullptr);
       }
     }
   }

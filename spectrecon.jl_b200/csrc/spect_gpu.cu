@@ -650,6 +650,10 @@ int forward_scratch(spect_plan_s* p, float* views, const float* image, const Vie
   }
   const int* const vidx = vsel.dev;
   const Geom& g = p->g;
+  // rotation by gathers from the z-fastest volume; calls on the static scratch
+  // keep off the plan's buffers, so they take the slice kernel
+  const bool gfwd = p->gadj && Pbuf == p->d_P;
+  if (gfwd && nidx > 0) LAUNCH(p, K_OTHER, st, "k_to_iz", zto_iz_launch(p->zg, st, image, p->d_imgIZ));
   for (int g0 = 0; g0 < nidx; g0 += gmax) {
     const int nv = std::min(gmax, nidx - g0);
     const int* vi = vidx + g0;
@@ -670,6 +674,9 @@ int forward_scratch(spect_plan_s* p, float* views, const float* image, const Vie
       LAUNCH(p, K_ROT_FWD, st, "k_att_combine",
              k_att_combine<false><<<(int)std::min<size_t>((n + 255) / 256, (size_t)p->sm_count * 16), 256, 0, st>>>(
                  att, p->d_R1, vi, nv, g.nx, g.ny, g.nz, Pbuf));
+    } else if (gfwd) {
+      LAUNCH(p, K_ROT_FWD, st, "k_zrot_fwd",
+             zrot_fwd_launch(p->zg, nv * g.ny, st, p->d_imgIZ, p->d_rot, vi, Pbuf));
     } else
     LAUNCH(p, K_ROT_FWD, st, "k_rot_fwd",
            if (p->rotf_smem_ok && att) k_rot_fwd<true, true><<<grid, thr, p->rotf_smem, st>>>(
@@ -763,7 +770,8 @@ int backward(spect_plan_s* p, float* image, const float* views, const ViewSel& v
       a.vsplit = std::max(1, std::min(8, cdiv(p->conv_grid, nv)));
       LAUNCH(p, K_VSPEC, st, "k_vspec", conv_launch(p, 2, std::min(p->conv_grid, nv * a.vsplit), st, a));
       a.Vs = p->d_Vs;
-      a.T = p->d_P;
+      a.T = p->gadj ? p->d_Tz : p->d_P;
+      a.nzp = p->gadj ? p->zg.nzp : 0;
       a.chunkY = cy;
       a.nchunks = nc;
       LAUNCH(p, K_CONV_ADJ, st, "k_conv_adj",
@@ -771,8 +779,9 @@ int backward(spect_plan_s* p, float* image, const float* views, const ViewSel& v
     }
     dim3 grid(g.nz, nsplit);
     const size_t rsm = p->rota_smem_ok ? p->rota_smem : 0;
-    if (p->gadj) {  // premultiplied planes -> z fastest -> gather into the IZ accumulator
-      LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
+    if (p->gadj) {  // premultiplied planes, z fastest (stored so by k_conv_adj2) -> gather into the IZ accumulator
+      if (p->sep_adj)
+        LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
              zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
              zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, view_list(ViewSel{vi, nullptr}, 0, nv), nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
@@ -1585,13 +1594,14 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       p->gadj = 1;
       p->zg = zg;
       p->izN = (size_t)zg.L * zg.L * zg.nzp;
-      if ((st = dalloc(p, &p->d_backIZ, p->izN)) ||
+      if ((st = dalloc(p, &p->d_imgIZ, p->izN)) || (st = dalloc(p, &p->d_backIZ, p->izN)) ||
           (st = dalloc(p, &p->d_Tz, (size_t)p->gmax * ny * nx * zg.nzp + zg.nzp)))
         return bail(st);
       p->tzero = (size_t)p->gmax * ny * nx * zg.nzp;
       const cudaError_t ze = zrot_adj_setup();
       if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("gather adjoint setup: ") + cudaGetErrorString(ze)));
-      if (cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
+      if (cudaMemsetAsync(p->d_imgIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
+          cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
           cudaMemsetAsync(p->d_Tz + p->tzero, 0, sizeof(float) * zg.nzp, p->home) != cudaSuccess)
         return bail(fail(SPECT_ERR_CUDA, "memset"));
     }

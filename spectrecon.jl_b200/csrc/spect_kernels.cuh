@@ -5,7 +5,8 @@
 //                src/rotatez.jl:331-362), depth-scan the rotated mu-map and
 //                write P[slot][y][z][x] = exp(-dy*(sum_{j<y} mu_j + mu_y/2)) * R(image)
 //                (src/project.jl:103-116).  One CTA per (z slice, view split);
-//                slices staged in shared memory.
+//                slices staged in shared memory.  (With the attenuation
+//                cache and nz <= 256 the planes come from k_zrot_fwd, zpath.cuh.)
 //   k_conv_fwd2  (conv2.cuh) depth-dependent PSF convolution and depth sum.
 //   k_reduce_views  sum of the chunk partials in chunk order (+ fused EM ratio).
 // Adjoint pass (backproject!, src/backproject.jl:69-124):

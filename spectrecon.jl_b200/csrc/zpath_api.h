@@ -310,6 +310,8 @@ cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const floa
                             const Rot1View* r1, const ViewList& vidx, int nv, const float* prev, float* out, const float* x,
                             const float* asum, int mode);  // T[zero ..]: a column of zeros; r1: null for :two
 cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, float* iz);
+cudaError_t zrot_fwd_launch(const ZGeom& g, int planes, cudaStream_t st, const float* iz, const float4* rot,
+                            const int* vidx, float* P);
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx);
 cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, float* dst, const float* asum, int mode);

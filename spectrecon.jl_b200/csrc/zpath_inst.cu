@@ -85,6 +85,12 @@ cudaError_t zto_iz_launch(const ZGeom& g, cudaStream_t st, const float* img, flo
   return launch_next(true, k_to_iz, dim3((g.nx + 31) / 32, g.ny, (g.nzp + 31) / 32), dim3(32, 8), 0, st, g, img, iz);
 }
 
+cudaError_t zrot_fwd_launch(const ZGeom& g, int planes, cudaStream_t st, const float* iz, const float4* rot,
+                            const int* vidx, float* P) {
+  return launch_next(zearly(g, planes / g.ny), k_zrot_fwd, dim3(planes, (g.nx + 31) / 32), 256,
+                     sizeof(float) * 33 * zround(g.nz, 4), st, g, iz, rot, vidx, P);
+}
+
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx) {
   k_t_to_z<<<dim3((g.nx + 31) / 32, planes, (g.nzp + 31) / 32), dim3(32, 8), 0, st>>>(g, src, dst, att, vidx);

@@ -186,3 +186,38 @@ def test_device_array_checks(S):
     S.project_(Interface(again), Interface(im), plan, index=np.arange(nview, dtype=np.int32))
     torch.cuda.synchronize()
     assert relerr(again.cpu().numpy(), out.cpu().numpy()) <= 1e-6
+
+
+@pytest.mark.parametrize("nx,nz,px,pz,nview,idx", [
+    (90, 53, 21, 17, 12, [11, 0, 4]),  # rows of 90: unstaged planes, an odd last row, z groups past the end
+    (128, 80, 37, 37, 8, None),        # staged planes, whole tiles of 32 columns
+    (36, 9, 5, 3, 9, [8, 2]),          # staged, one tile and four columns
+    (2, 1, 1, 1, 4, None),             # the smallest image
+    (66, 1, 9, 1, 6, [3, 5]),          # one slice
+    (32, 200, 7, 5, 5, None),          # many z groups of one column tile
+])
+@pytest.mark.parametrize("stage", ["1", "0"])
+def test_split_rotation_by_gathers(S, O, monkeypatch, nx, nz, px, pz, nview, idx, stage):
+    """PSFs that no two factors give: the rotation by gathers of z-fastest
+    columns and the convolution's z-fastest store against the slice kernels
+    (SPECT_GADJ=0), whose forward planes are the same bits, and the oracle."""
+    mumap, psfs, x, y = _plan_inputs(S, nx, nz, px, pz, nview, 11 * nx + nz)
+    i, j = np.meshgrid(np.arange(px) - px // 2, np.arange(pz) - pz // 2, indexing="ij")
+    psfs = psfs * (1 + 0.5 * np.cos(i * j)).astype(np.float32)[:, :, None, None]
+    psfs = np.asfortranarray(psfs / psfs.sum(axis=(0, 1), keepdims=True), np.float32)
+    ii = None if idx is None else np.array(idx, np.int32)
+    ys = y if ii is None else np.asfortranarray(y[:, :, ii])
+    monkeypatch.setenv("SPECT_ZPATH", "0")
+    monkeypatch.setenv("SPECT_NO_STAGE", "0" if stage == "1" else "1")
+    out = {}
+    for gather in ("1", "0"):
+        monkeypatch.setenv("SPECT_GADJ", gather)
+        plan = S.SPECTplan(mumap, psfs, 4.8)
+        assert plan.path == "split"
+        out[gather] = (S.project(x, plan, index=ii), S.backproject(ys, plan, index=ii))
+        plan.close()
+    np.testing.assert_array_equal(out["1"][0], out["0"][0])
+    assert relerr(out["1"][1], out["0"][1]) <= 1e-5
+    G = O.Geometry(mumap, psfs, 4.8)
+    assert relerr(out["1"][0], G.project(x, index=ii)) <= TOL
+    assert relerr(out["1"][1], G.backproject(ys, index=ii)) <= TOL
