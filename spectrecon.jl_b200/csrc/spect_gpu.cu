@@ -237,8 +237,9 @@ struct spect_plan_s {
   double ztaps[2] = {0, 0};    // mean kept taps per plane of the fused passes (z, x)
   ZsTiles zst{};               // tiling of the large-plane kernels (zpath == 2), their plane exchange buffer
   float* d_Q = nullptr;
-  // split kernels with the gather rotation adjoint: the premultiplied adjoint
-  // planes are transposed into d_Tz (z fastest) and gathered into d_backIZ
+  // split kernels with the gather rotation: forward planes from d_imgIZ; the
+  // premultiplied adjoint planes go z fastest into d_Tz (stored so by
+  // k_conv_adj2, transposed behind k_sconv_adj) and are gathered into d_backIZ
   int gadj = 0;
   float* d_Tz = nullptr;
   size_t tzero = 0;            // offset of the zero column behind the z-fastest adjoint planes (d_P or d_Tz)
@@ -548,7 +549,6 @@ ZArgs zargs(const spect_plan_s* p) {
   a.rot = p->d_rot;
   a.viewset = p->d_viewset;
   a.r1 = p->interp == SPECT_INTERP_ONE ? p->d_r1view : nullptr;
-  a.err = p->d_err;
   return a;
 }
 
@@ -1586,9 +1586,9 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       (st = dalloc(p, &p->d_Vs, (size_t)p->gmax * p->cg.Q * Npx)) ||
       (st = dalloc(p, &p->d_imgpart, (size_t)p->nsplit_adj_max * p->N)))
     return bail(st);
-  {  // split kernels with the attenuation cache (:two): rotation adjoint by the
-     // gather kernel, the attenuation applied by the convolution's store or by
-     // the transpose (SPECT_GADJ=0 keeps the scatter kernels)
+  {  // split kernels with the attenuation cache (:two): both rotations by the
+     // gather kernels, the adjoint's attenuation applied by the convolution's
+     // store or by the transpose (SPECT_GADJ=0 keeps the slice and scatter kernels)
     const char* genv = std::getenv("SPECT_GADJ");
     if (!p->zpath && p->d_att && interpmeth == SPECT_INTERP_TWO && zg.nzp <= 256 && !(genv && genv[0] == '0')) {
       p->gadj = 1;

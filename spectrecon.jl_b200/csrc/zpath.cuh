@@ -1,6 +1,5 @@
 // zpath.cuh -- the fused SPECT projector pair on z-fastest layouts (sm_100a),
-// for the common case: :two rotation, cached attenuation, separable (rank-1)
-// PSF planes.
+// for the common case: cached attenuation, separable (rank-1) PSF planes.
 //
 // Layouts (float32, z fastest; nzp = nz rounded up to 16; every entry with
 // z >= nz is zero):
@@ -14,33 +13,41 @@
 //   T     [slot][y][x][nzp]  adjoint planes att .* conv_adj(view) of a group
 //   views [slot][nz][nx]     the reference's views[nx, nz, nview], unchanged
 //
-// k_zfwd   project! (src/project.jl:77-135): work item (slot, depth chunk);
-//          per plane y the block gathers the rotated image (imrotate! :two,
-//          src/rotatez.jl:331-362) column by column from IZ, multiplies the
-//          attenuation plane (bulk-copied one plane ahead) and writes the
-//          z-pass buffer directly; then the z pass and the x pass of the
-//          replicate-boundary convolution that fft_conv! computes
-//          (src/fft_convolve.jl:33-55).  The x-pass outputs stay in
-//          registers across the chunk (the depth sum, src/project.jl:127-130).
-//          The rotated volume never leaves the SM.
-// k_zadj   backproject! (src/backproject.jl:69-124), convolution half: per
-//          plane the x pass and z pass of fft_conv_adj! (src/fft_convolve.jl:
-//          82-130) of the view, times the attenuation, stored as T.
-// The kernels for planes too large for these kernels' shared memory are in
-// zstrip.cuh (same layouts and passes, over plane tiles).
-// k_zrot_adj  imrotate_adj! :two (src/rotatez.jl:390-416) and the view sum
+// k_zfwd   project! (src/project.jl:77-135): the blocks share one flat walk
+//          over the planes (slot, y) of a group; per plane a block gathers the
+//          rotated image (imrotate!, src/rotatez.jl:331-362) column by column
+//          from IZ, times the attenuation, straight into the z pass's pair
+//          lines; then the z pass and the x pass of the replicate-boundary
+//          convolution that fft_conv! computes (src/fft_convolve.jl:33-55).
+//          A plane's x outputs are summed in registers and added to the
+//          block's partial view of the slot (the depth sum,
+//          src/project.jl:127-130); k_reduce_parts sums the partials in block
+//          order.  The rotated volume never leaves the SM.
+// k_zadj   backproject! (src/backproject.jl:69-124), convolution half, on row
+//          tiles of a view: per plane the z pass and the x pass of
+//          fft_conv_adj! (src/fft_convolve.jl:82-130), times the attenuation,
+//          stored as T.
+// The forward of planes too large for k_zfwd's shared memory is in zstrip.cuh
+// (same layouts and passes, over plane tiles).
+// k_zrot_adj  imrotate_adj! (src/rotatez.jl:390-416) and the view sum
 //          (src/backproject.jl:146-153): output-stationary gather.  Every image
-//          column sums, over the views in order, the bilinear weights of the
-//          rotated-grid points whose footprint covers it: the exact transpose
-//          of the forward sampling, without atomics.  The EM update
+//          column sums, over the views in order, the weights of the
+//          rotated-grid points whose footprint covers it, listed once per
+//          column and slot in shared memory: the exact transpose of the
+//          forward sampling, without atomics.  The EM update
 //          (src/ml-os-em.jl:111-126) is its epilogue.
+// ONE: the three shears of :one as eight taps of IZ (one_line).
 //
 // Convolution passes.  fft_conv! equals the replicate-boundary convolution
 // out[i] = sum_{m<p} w[m] in[clamp(i - h + m)] with the reversed factor w
-// (the plan factors each PSF plane as a[d] b[e]).  Here the input line sits
-// zero-padded in shared memory, data starting at an offset D0 = h rounded up
-// to 4, and the weights are shifted right by D0 - h, so a task of W = 8 or 16
-// consecutive outputs reads a window of 16-byte-aligned float4s; the clamped
+// (the plan factors each PSF plane as a[d] b[e]).  Here two input lines sit
+// interleaved and zero-padded in shared memory, one element f2 = (line a,
+// line b), and a task of W = 8 or 16 consecutive outputs of both runs packed
+// FMAs (fma.rn.f32x2): half the issue slots of a line at a time, which is what
+// bounds these loops next to their index and shared-memory work (63.4 against
+// 48.8 TFLOP/s beside one integer operation an FMA).  Data start at an offset
+// D0 = h rounded up to 4 and the weights are shifted right by D0 - h, so the
+// window is read in 16-byte-aligned pieces; the clamped
 // boundary is added as tail terms: the edge value times EL[i] =
 // sum_{m < h - i} w[m] (i < h) or ER[n-1-i] = sum_{m > h + n-1-i} w[m]
 // (i > n-1-h).  The adjoint passes are the zero-padded correlations with the
@@ -48,9 +55,10 @@
 // sums of the factor beyond k), as the reference's padding adjoint does.
 // The plan zeroes the outer taps of each factor whose summed magnitude per
 // side is within 2^-27 of the factor's (below Float32 resolution; a narrow
-// Gaussian plane keeps a few of its p taps) and every table, tails and folds
-// included, comes from those factors; per plane and pass a range table gives
-// the 8-tap blocks that hold the kept taps, and only those are run.
+// Gaussian plane keeps a few of its p taps) and cuts the rows to the widest
+// support that is left; every table, tails and folds included, comes from
+// those factors, and per plane and pass a range gives the 4-tap blocks that
+// hold the kept taps: only those are run.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -1033,7 +1041,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ Z
 // Bound: L1 (its tag stage is 55 % busy where an SM works: a column's 320
 // bytes straddle lines) and the latency of the misses.  Measured (the former
 // kernel tested the candidates in every 8-lane group): 128x128x80, 15 views 49
-// -> 46 us; 64x64x64, 64 views 57 -> 31 us; 64x64x40, 60 views 45 -> 24 us;
+// -> 42 us; 64x64x64, 64 views 57 -> 31 us; 64x64x40, 60 views 45 -> 24 us;
 // 256x256x200, 8 views 252 -> 216 us.
 // Epilogue (IZ layout): v = acc (+ prev); mode 1: zeros -> +Inf; mode 2:
 // v = x * (v / asum); out = v (z < nz only; out may be prev or x).

@@ -15,17 +15,9 @@ struct ZGeom {
   int R0, C0;       // first data row (z pass) / column (x pass) of the padded buffers
   int zpw, xpw;     // window taps of the z and x passes (shifted, multiples of 8)
   int hs, ts;       // weight-row and tail-row lengths of one direction
-  int rows, ast;    // z-pass buffer: rows per column, column stride (4 * odd)
-  int bs;           // x-pass buffer row stride (4 * odd)
 };
 
 __host__ __device__ constexpr int zround(int v, int m) { return (v + m - 1) / m * m; }
-// smallest 4 * odd >= v: 16-byte rows whose float4 chunk index is odd, so the
-// eight lanes of a 128-bit shared access phase hit distinct bank groups
-__host__ __device__ constexpr int zstride4(int v) {
-  return ((zround(v, 4) / 4) % 2 == 1) ? zround(v, 4) : zround(v, 4) + 4;
-}
-
 inline ZGeom zgeom_make(int nx, int ny, int nz, int px, int pz, int pad) {
   ZGeom g{};
   g.nx = nx;
@@ -45,9 +37,6 @@ inline ZGeom zgeom_make(int nx, int ny, int nz, int px, int pz, int pad) {
   g.xpw = zround(g.C0 - g.hx + px, 8);
   g.hs = g.zpw + g.xpw;
   g.ts = zround(2 * g.hx + 2 * g.hz, 4) < 4 ? 4 : zround(2 * g.hx + 2 * g.hz, 4);
-  g.rows = zround(nz, 16) + g.zpw;  // z tasks of 8 or 16 outputs
-  g.ast = zstride4(g.rows);
-  g.bs = zstride4(nx + g.xpw);
   return g;
 }
 
@@ -111,7 +100,6 @@ struct ZArgs {
   float* part;          // partial views [G + nv][nz][nx]
   const float* views;   // k_zadj input [nv][nz][nx]
   float* T;             // k_zadj output [nv][ny][nx][nzp]
-  int* err;
   float* Q;             // plane exchange of the large-plane kernels (zstrip.cuh), [nv][ny][row pair][nx][2]
   int tx, tz;           // their column and row tile sizes
   int zvst, xbst;       // their line strides (f2)
