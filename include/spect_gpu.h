@@ -261,6 +261,13 @@ unsigned long long spect_kernel_launches(void);
  * failed).  Synchronous; allocates 4 bytes. */
 int spect_plan_check_error(spect_plan_t plan, void* stream);
 int spect_selftest_wait_timeout(void);
+
+/* The launch shapes that a plan of the given sizes would take (test support,
+ * no device needed): in[] = nx (= ny), nz, px, pz, views, option, SMs, shared
+ * memory bytes a block may have.  what = "group": out[0] = views of a group
+ * for option 0 (slice kernels), 1 (split kernels with the gather rotation) or
+ * 2 (fused and large-plane kernels) of a plan of in[4] views. */
+int spect_selftest_tiling(const char* what, const int in[8], long long out[12]);
 int spect_plan_profile(spect_plan_t plan, int on);
 int spect_plan_kernel_times(spect_plan_t plan, double ms[8], long long counts[8]);
 

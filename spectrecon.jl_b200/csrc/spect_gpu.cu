@@ -91,6 +91,8 @@ inline int ilog2(int x) {
   while ((1 << l) < x) ++l;
   return l;
 }
+// zero ring of the rotation grid (src/plan-rotate.jl:56)
+inline int rotation_pad(int nx) { return (int)std::ceil(1.0 + nx * std::sqrt(2.0) / 2.0 - nx / 2.0); }
 inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 constexpr double kTwoPi = 6.283185307179586;
@@ -633,9 +635,11 @@ int zbackward(spect_plan_s* p, float* outIZ, const float* views, const ViewSel& 
     const int gs = (int)std::min<long long>((long long)p->sm_count * p->zat.occ, (long long)nv * p->zat.ntile * p->ny);
     LAUNCH(p, K_CONV_ADJ, st, "k_zadj", zadj_launch(gs, st, a));
     const bool last = g0 + nv >= nidx;
+    cudaError_t ze = cudaSuccess;
     LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-           zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, a.r1, a.vidx, nv, g0 > 0 ? p->d_backIZ : nullptr,
+           ze = zrot_adj_launch(p->zg, p->sm_count, st, p->d_P, p->tzero, p->d_rot, a.r1, a.vidx, nv, g0 > 0 ? p->d_backIZ : nullptr,
                            last ? outIZ : p->d_backIZ, xIZ, asumIZ, last ? mode : 0));
+    CUDA_TRY(ze);
   }
   return SPECT_OK;
 }
@@ -783,9 +787,11 @@ int backward(spect_plan_s* p, float* image, const float* views, const ViewSel& v
       if (p->sep_adj)
         LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
              zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
+      cudaError_t ze = cudaSuccess;
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
-             zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, view_list(ViewSel{vi, nullptr}, 0, nv), nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
+             ze = zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, view_list(ViewSel{vi, nullptr}, 0, nv), nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
                              nullptr, nullptr, 0));
+      CUDA_TRY(ze);
     } else if (p->interp == SPECT_INTERP_ONE) {
       const size_t n = (size_t)nv * p->N;
       LAUNCH(p, K_ROT_ADJ, st, "k_att_combine",
@@ -1466,7 +1472,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   const bool sep_host = factor_planes(psfs, uniq, ny, px, pz, opts, fa, fb);
   const char* conv_env = std::getenv("SPECT_CONV");
   const bool only_fft = conv_env && std::strcmp(conv_env, "fft") == 0;
-  const int pad_rot = (int)std::ceil(1.0 + nx * std::sqrt(2.0) / 2.0 - nx / 2.0);
+  const int pad_rot = rotation_pad(nx);
   // the fused path's factors: outer taps below Float32 resolution zeroed
   // (trim_taps), and the support cut to the widest kept half-widths over all
   // planes, which sizes the passes' line padding in shared memory
@@ -1564,12 +1570,15 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
   p->view_set = view_set;
   p->nset = (int)uniq.size();
 
-  // group size: rotated-plane scratch bounded by ~1 GiB
-  // (the fused path's adjoint planes T hold nzp >= nz values per column)
-  const size_t budget = (size_t)1 << 30;
+  // split kernels with the attenuation cache (:two): both rotations by the
+  // gather kernels, the adjoint's attenuation applied by the convolution's
+  // store or by the transpose (SPECT_GADJ=0 keeps the slice and scatter kernels)
+  const char* const genv = std::getenv("SPECT_GADJ");
+  p->gadj = !p->zpath && p->d_att && interpmeth == SPECT_INTERP_TWO && zg.nzp <= 256 && !(genv && genv[0] == '0');
+  // group size (the fused path's adjoint planes T hold nzp >= nz values per column)
   const size_t slot = p->zpath ? (size_t)ny * nx * zg.nzp : p->N;
   if (p->zpath) p->nsplit_adj = p->nsplit_adj_max = 1;  // no split partial images
-  p->gmax = (int)std::max<size_t>(1, std::min<size_t>((size_t)nview, budget / (sizeof(float) * slot)));
+  p->gmax = zgroup_views(nx, nview, slot, p->zpath || p->gadj);
   if (opts.gmax_cap > 0) p->gmax = std::min(p->gmax, opts.gmax_cap);
 
   if ((st = dalloc(p, &p->d_mumap, p->N)) || (st = dalloc(p, &p->d_rot, nview)) ||
@@ -1586,25 +1595,19 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
       (st = dalloc(p, &p->d_Vs, (size_t)p->gmax * p->cg.Q * Npx)) ||
       (st = dalloc(p, &p->d_imgpart, (size_t)p->nsplit_adj_max * p->N)))
     return bail(st);
-  {  // split kernels with the attenuation cache (:two): both rotations by the
-     // gather kernels, the adjoint's attenuation applied by the convolution's
-     // store or by the transpose (SPECT_GADJ=0 keeps the slice and scatter kernels)
-    const char* genv = std::getenv("SPECT_GADJ");
-    if (!p->zpath && p->d_att && interpmeth == SPECT_INTERP_TWO && zg.nzp <= 256 && !(genv && genv[0] == '0')) {
-      p->gadj = 1;
-      p->zg = zg;
-      p->izN = (size_t)zg.L * zg.L * zg.nzp;
-      if ((st = dalloc(p, &p->d_imgIZ, p->izN)) || (st = dalloc(p, &p->d_backIZ, p->izN)) ||
-          (st = dalloc(p, &p->d_Tz, (size_t)p->gmax * ny * nx * zg.nzp + zg.nzp)))
-        return bail(st);
-      p->tzero = (size_t)p->gmax * ny * nx * zg.nzp;
-      const cudaError_t ze = zrot_adj_setup();
-      if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("gather adjoint setup: ") + cudaGetErrorString(ze)));
-      if (cudaMemsetAsync(p->d_imgIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
-          cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
-          cudaMemsetAsync(p->d_Tz + p->tzero, 0, sizeof(float) * zg.nzp, p->home) != cudaSuccess)
-        return bail(fail(SPECT_ERR_CUDA, "memset"));
-    }
+  if (p->gadj) {
+    p->zg = zg;
+    p->izN = (size_t)zg.L * zg.L * zg.nzp;
+    p->tzero = (size_t)p->gmax * ny * nx * zg.nzp;
+    if ((st = dalloc(p, &p->d_imgIZ, p->izN)) || (st = dalloc(p, &p->d_backIZ, p->izN)) ||
+        (st = dalloc(p, &p->d_Tz, p->tzero + zg.nzp)))
+      return bail(st);
+    const cudaError_t ze = zrot_adj_setup();
+    if (ze != cudaSuccess) return bail(fail(SPECT_ERR_CUDA, std::string("gather adjoint setup: ") + cudaGetErrorString(ze)));
+    if (cudaMemsetAsync(p->d_imgIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
+        cudaMemsetAsync(p->d_backIZ, 0, sizeof(float) * p->izN, p->home) != cudaSuccess ||
+        cudaMemsetAsync(p->d_Tz + p->tzero, 0, sizeof(float) * zg.nzp, p->home) != cudaSuccess)
+      return bail(fail(SPECT_ERR_CUDA, "memset"));
   }
   if (p->zpath) {  // IZ volumes (zero ring and z padding) and zeroed adjoint planes
     if ((st = dalloc(p, &p->d_imgIZ, p->izN)) || (st = dalloc(p, &p->d_backIZ, p->izN)))
@@ -1635,7 +1638,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
 
   if (interpmeth == SPECT_INTERP_ONE) {
     // Rot1 geometry and per-view shear parameters (src/rotatez.jl:249-272)
-    const int pad1 = (int)std::ceil(1.0 + nx * std::sqrt(2.0) / 2.0 - nx / 2.0);
+    const int pad1 = rotation_pad(nx);
     p->r1 = Rot1Geom{nx, ny, nz, nx + 2 * pad1, pad1, nx + 2 * pad1 + 1};
     const int L = p->r1.L;
     p->r1f_smem = sizeof(float) * ((size_t)p->r1.LS * L + (size_t)kRot1Warps * L);
@@ -2236,6 +2239,19 @@ int spect_plan_check_error(spect_plan_t p, void* stream) {
     return fail(SPECT_ERR_TIMEOUT, "a bulk copy into shared memory did not complete");
   }
   return SPECT_OK;
+}
+
+int spect_selftest_tiling(const char* what, const int in[8], long long out[12]) {
+  if (!what || !in || !out) return fail(SPECT_ERR_ARG, "null pointer argument");
+  const int nx = in[0], nz = in[1], px = in[2], pz = in[3], nv = in[4], option = in[5];
+  if (nx <= 0 || nx % 2 || nz <= 0 || px <= 0 || pz <= 0 || nv <= 0) return fail(SPECT_ERR_ARG, "bad sizes");
+  std::memset(out, 0, 12 * sizeof(out[0]));
+  const ZGeom g = zgeom_make(nx, nx, nz, px, pz, rotation_pad(nx));
+  if (std::strcmp(what, "group") == 0) {
+    out[0] = zgroup_views(nx, nv, (size_t)nx * nx * (option == 2 ? g.nzp : nz), option != 0);
+    return SPECT_OK;
+  }
+  return fail(SPECT_ERR_ARG, std::string("unknown tiling ") + what);
 }
 
 int spect_selftest_wait_timeout(void) {

@@ -1057,8 +1057,8 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
   extern __shared__ float4 smem4[];
   const int nth = blockDim.x, tid = threadIdx.x, nx = g.nx, ny = g.ny, n4 = g.nzp / 4, C = r.tx * r.ty;
   const float c0 = g.c0;
-  // [2][nth][E]: the hits (T column, weight); the first entry's top five bits
-  // hold their count
+  // [2][nth][E]: the hits (T column, weight); the first entry's bits above the
+  // column hold their count
   int2* const list = reinterpret_cast<int2*>(smem4);
   const int ntx = (nx + r.tx - 1) / r.tx;
   const int X0 = (blockIdx.x % ntx) * r.tx, Y0 = (blockIdx.x / ntx) * r.ty;
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
     }
     const int m = (int)(L - L0);
     for (; L < L0 + 4; ++L) *L = make_int2(zcol, 0);
-    L0->x |= m << 27;
+    L0->x |= m << kZrotColumnBits;
   };
   // this thread's units: group, column of the tile, z group (a unit past the
   // last repeats it and is not stored)
@@ -1144,8 +1144,8 @@ __global__ void __launch_bounds__(kZrotThreads, 2) k_zrot_adj(ZGeom g, ZRotTile 
         for (int i = 0; i < 2; ++i) {
           const int2* const q = L + col[i0 + i] * E;
           const int2 e0 = q[0], e1 = q[1], e2 = q[2], e3 = q[3];
-          m[i] = (int)((unsigned)e0.x >> 27);
-          t[i][0] = load(i0 + i, e0.x & 0x07ffffff);
+          m[i] = (int)((unsigned)e0.x >> kZrotColumnBits);
+          t[i][0] = load(i0 + i, e0.x & kZrotColumnMask);
           t[i][1] = load(i0 + i, e1.x);
           t[i][2] = load(i0 + i, e2.x);
           t[i][3] = load(i0 + i, e3.x);

@@ -282,6 +282,23 @@ inline ZRotTile zrot_tile(const ZGeom& g, int nv, int sms) {
   return r;
 }
 
+// k_zrot_adj's lists keep a T column number below the count of hits in one
+// word: a group's columns and the zero column behind them are numbered in
+// kZrotColumnBits bits
+constexpr int kZrotColumnBits = 27;
+constexpr int kZrotColumnMask = (1 << kZrotColumnBits) - 1;
+// views of a group whose planes hold `slot` floats a view: about 1 GiB of
+// planes, and, where the gather adjoint runs, column numbers within their bits
+// (single slices on the split kernels: 512 views of 512x512x1 hold 2^27
+// columns in half that memory)
+inline int zgroup_views(int nx, int nview, size_t slot, bool gather) {
+  size_t n = ((size_t)1 << 30) / (sizeof(float) * slot);
+  if (n > (size_t)nview) n = nview;
+  const size_t most = (size_t)kZrotColumnMask / ((size_t)nx * nx);
+  if (gather && n > most) n = most;
+  return n < 1 ? 1 : (int)n;
+}
+
 // short work (about 100 us a kernel at most): nv planes stacks of nx x nx x nz
 inline bool zearly(const ZGeom& g, int nv) { return (long long)nv * g.nx * g.ny * g.nz <= (1LL << 25); }
 

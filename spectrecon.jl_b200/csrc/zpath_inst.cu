@@ -68,6 +68,7 @@ cudaError_t zadj_launch(int grid, cudaStream_t st, const ZArgs& a) {
 cudaError_t zrot_adj_launch(const ZGeom& g, int sms, cudaStream_t st, const float* T, size_t zero, const float4* rot,
                             const Rot1View* r1, const ViewList& vidx, int nv, const float* prev, float* out, const float* x,
                             const float* asum, int mode) {
+  if (zero / g.nzp > (size_t)kZrotColumnMask) return cudaErrorInvalidValue;  // zgroup_views rules it out
   const ZRotTile r = zrot_tile(g, nv, sms);
   const auto kernel = r1 ? k_zrot_adj<true> : k_zrot_adj<false>;
   return launch_next(zearly(g, nv), kernel, r.grid, r.nth, r.smem, st, g, r, T, (int)(zero / g.nzp), rot, r1, vidx, nv, prev, out, x,
