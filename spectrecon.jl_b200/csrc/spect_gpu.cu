@@ -784,10 +784,12 @@ int backward(spect_plan_s* p, float* image, const float* views, const ViewSel& v
     dim3 grid(g.nz, nsplit);
     const size_t rsm = p->rota_smem_ok ? p->rota_smem : 0;
     if (p->gadj) {  // premultiplied planes, z fastest (stored so by k_conv_adj2) -> gather into the IZ accumulator
-      if (p->sep_adj)
-        LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
-             zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
       cudaError_t ze = cudaSuccess;
+      if (p->sep_adj) {
+        LAUNCH(p, K_ROT_ADJ, st, "k_t_to_z",
+               ze = zt_to_z_launch(p->zg, nv * g.ny, st, p->d_P, p->d_Tz, p->adj_stage ? nullptr : p->d_att, vi));
+        CUDA_TRY(ze);
+      }
       LAUNCH(p, K_ROT_ADJ, st, "k_zrot_adj",
              ze = zrot_adj_launch(p->zg, p->sm_count, st, p->d_Tz, p->tzero, p->d_rot, nullptr, view_list(ViewSel{vi, nullptr}, 0, nv), nv, g0 > 0 ? p->d_backIZ : nullptr, p->d_backIZ,
                              nullptr, nullptr, 0));

@@ -7,6 +7,7 @@
 namespace spect {
 
 namespace {
+constexpr int kGridY = 65535;  // blocks of a grid's second dimension at most
 // [x tasks a thread - 1][rotation :two, :one]
 void (*const kZfwd[2][2])(const ZArgs) = {{k_zfwd<1, false>, k_zfwd<1, true>}, {k_zfwd<2, false>, k_zfwd<2, true>}};
 // launch with programmatic stream serialisation (grid_wait, zpath.cuh) where
@@ -94,8 +95,15 @@ cudaError_t zrot_fwd_launch(const ZGeom& g, int planes, cudaStream_t st, const f
 
 cudaError_t zt_to_z_launch(const ZGeom& g, int planes, cudaStream_t st, const float* src, float* dst,
                             const float* att, const int* vidx) {
-  k_t_to_z<<<dim3((g.nx + 31) / 32, planes, (g.nzp + 31) / 32), dim3(32, 8), 0, st>>>(g, src, dst, att, vidx);
-  return cudaGetLastError();
+  const int step = kGridY / g.ny * g.ny;  // whole slots a launch
+  for (int p0 = 0; p0 < planes; p0 += step) {
+    const int n = planes - p0 < step ? planes - p0 : step;
+    k_t_to_z<<<dim3((g.nx + 31) / 32, n, (g.nzp + 31) / 32), dim3(32, 8), 0, st>>>(
+        g, src + (size_t)p0 * g.nz * g.nx, dst + (size_t)p0 * g.nx * g.nzp, att, vidx + p0 / g.ny);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, float* dst, const float* asum, int mode) {

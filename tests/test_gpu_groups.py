@@ -37,3 +37,18 @@ def test_more_columns_than_a_list_word_holds(S, O):
     plan.close()
     assert relerr(whole, parts[0] + parts[1]) <= SAME
     assert relerr(whole, O.Geometry(mumap, psfs, 4.8).backproject(y)) <= TOL
+
+
+def test_more_planes_than_a_grid_holds(S, O, monkeypatch):
+    """520 views of 128x128x1 are 66 560 adjoint planes, above the 65 535
+    blocks of a grid's second dimension that the transpose of the direct
+    convolution's planes has."""
+    nx, nview = 128, 520
+    monkeypatch.setenv("SPECT_ZPATH", "0")
+    monkeypatch.setenv("SPECT_CONV", "direct")
+    mumap, psfs, y = _study(S, nx, nview, 2, separable=True)
+    plan = S.SPECTplan(mumap, psfs, 4.8)
+    assert plan.path == "split" and plan.conv_kernels()["adjoint"] == "direct"
+    out = S.backproject(y, plan)
+    plan.close()
+    assert relerr(out, O.Geometry(mumap, psfs, 4.8).backproject(y)) <= TOL
