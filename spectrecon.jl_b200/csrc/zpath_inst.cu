@@ -113,8 +113,12 @@ cudaError_t zfrom_iz_launch(const ZGeom& g, cudaStream_t st, const float* iz, fl
 
 cudaError_t zatten_launch(const ZGeom& g, int nview, cudaStream_t st, const float* muz, const float4* rot,
                           const Rot1View* r1, float dy, float* att) {
-  if (r1) k_zatten<true><<<dim3(g.nx, nview), g.nzp, 0, st>>>(g, muz, rot, r1, dy, att);
-  else k_zatten<false><<<dim3(g.nx, nview), g.nzp, 0, st>>>(g, muz, rot, r1, dy, att);
+  const size_t stack = (size_t)g.ny * g.nx * g.nzp;  // floats of a view
+  for (int v0 = 0; v0 < nview; v0 += kGridY) {
+    const dim3 grid(g.nx, nview - v0 < kGridY ? nview - v0 : kGridY);
+    if (r1) k_zatten<true><<<grid, g.nzp, 0, st>>>(g, muz, rot + v0, r1 + v0, dy, att + v0 * stack);
+    else k_zatten<false><<<grid, g.nzp, 0, st>>>(g, muz, rot + v0, r1, dy, att + v0 * stack);
+  }
   return cudaGetLastError();
 }
 

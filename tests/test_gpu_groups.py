@@ -52,3 +52,21 @@ def test_more_planes_than_a_grid_holds(S, O, monkeypatch):
     out = S.backproject(y, plan)
     plan.close()
     assert relerr(out, O.Geometry(mumap, psfs, 4.8).backproject(y)) <= TOL
+
+
+@pytest.mark.parametrize("interp", ["one", "two"])
+def test_more_views_than_a_grid_holds(S, O, interp):
+    """70 000 views of a 6x6x1 image on the fused pair: the attenuation of
+    views past the 65 535 blocks of a grid's second dimension."""
+    nx, nview = 6, 70000
+    mumap, _, _ = _study(S, nx, 1, 3)
+    psf = S.psf_gauss(ny=nx, px=3, pz=1, fwhm_start=1, fwhm_end=1.5)
+    psfs = np.asfortranarray(np.repeat(psf[:, :, :, None], nview, axis=3), np.float32)
+    plan = S.SPECTplan(mumap, psfs, 4.8, interpmeth=interp)
+    assert plan.path == "fused"
+    idx = np.array([69999, 0, 65535, 17501, 65534], np.int32)
+    x = np.asfortranarray(np.random.default_rng(4).random((nx, nx, 1)), np.float32)
+    out = S.project(x, plan, index=idx)
+    plan.close()
+    G = O.Geometry(mumap, psfs, 4.8, interp=interp)
+    assert relerr(out, G.project(x, index=idx)) <= TOL
