@@ -217,7 +217,10 @@ int spect_batch_destroy(spect_batch_t batch);
  * host arrays and returns at once; wait blocks until the job is done (or
  * timeout_ms, < 0 = forever), copies the reconstruction [nz][ny][nx] to `out`
  * and the submit-to-finish latency to latency_ms.  stats: submitted, done,
- * failed, active, pending, most active at once, bytes in use, budget. */
+ * failed, active, pending, most active at once, bytes in use, budget.  A
+ * request is active from its admission (its slot and memory are taken, then
+ * its plan is built and its OS-EM runs) until it has finished; never more than
+ * max_active are. */
 typedef struct {
   int nx, nz, px, pz, nview;     /* ny = nx */
   const float* mumap;            /* [nz][ny][nx] */

@@ -2454,9 +2454,12 @@ struct spect_server_s {
   std::unordered_map<long long, ServerJob*> jobs;
   long long next_ticket = 1;
   size_t used = 0;
-  int admitting = 0;  // jobs whose plan a scheduler thread is building (their memory is taken)
+  int admitting = 0;  // admitted jobs (slot and memory taken) whose plan a scheduler thread is building
   bool stop = false;
   long long n_submitted = 0, n_done = 0, n_failed = 0, max_active_seen = 0;
+  // slots taken: a job is active from its admission, while its plan is built
+  // and while it runs (a short job is over before the next one's plan stands)
+  long long slots() const { return (long long)active.size() + admitting; }
   // scheduler threads: each admits and retires jobs; while one prepares a
   // job's plan on the host (validation, uploads, PSF spectra) the others
   // keep admitting and retiring
@@ -2598,7 +2601,7 @@ void server_loop(spect_server_s* S) {
       S->cv_done.notify_all();
     }
     // admissions (FIFO) while slots and memory allow
-    while (!S->pending.empty() && (int)S->active.size() < S->max_active && !S->stop) {
+    while (!S->pending.empty() && S->slots() < S->max_active && !S->stop) {
       ServerJob* j = S->pending.front();
       if (j->est > S->budget) {
         S->pending.pop_front();
@@ -2614,10 +2617,8 @@ void server_loop(spect_server_s* S) {
       if (S->used + j->est > S->budget) break;  // wait for memory to free up
       S->pending.pop_front();
       S->used += j->est;
-      // jobs that hold device memory at once, those being prepared included (a
-      // short job may finish before the next one's plan stands)
       ++S->admitting;
-      S->max_active_seen = std::max<long long>(S->max_active_seen, (long long)S->active.size() + S->admitting);
+      S->max_active_seen = std::max(S->max_active_seen, S->slots());
       lk.unlock();
       j->t_admit = Clock::now();
       const int rc = job_admit(S, j, S->budget);
@@ -2754,7 +2755,7 @@ int spect_server_wait(spect_server_t S, long long ticket, float* out, double* la
 int spect_server_stats(spect_server_t S, long long out[8]) {
   if (!S || !out) return fail(SPECT_ERR_ARG, "null pointer argument");
   std::lock_guard<std::mutex> lk(S->mu);
-  long long v[8] = {S->n_submitted, S->n_done, S->n_failed, (long long)S->active.size(),
+  long long v[8] = {S->n_submitted, S->n_done, S->n_failed, S->slots(),
                     (long long)S->pending.size(), S->max_active_seen, (long long)S->used, (long long)S->budget};
   std::memcpy(out, v, sizeof(v));
   return SPECT_OK;
