@@ -265,11 +265,19 @@ unsigned long long spect_kernel_launches(void);
 int spect_plan_check_error(spect_plan_t plan, void* stream);
 int spect_selftest_wait_timeout(void);
 
-/* The launch shapes that a plan of the given sizes would take (test support,
- * no device needed): in[] = nx (= ny), nz, px, pz, views, option, SMs, shared
- * memory bytes a block may have.  what = "group": out[0] = views of a group
- * for option 0 (slice kernels), 1 (split kernels with the gather rotation) or
- * 2 (fused and large-plane kernels) of a plan of in[4] views. */
+/* The launch shapes that a plan of the given sizes takes (test support, no
+ * device needed): in[] = nx (= ny), nz, kept PSF support px, pz, views, option,
+ * SMs, shared memory bytes a block may have.  what and out[]:
+ *   "group"      views of a group; option 0 slice kernels, 1 split kernels with
+ *                the gather rotation, 2 fused and large-plane kernels
+ *   "geometry"   nzp, L, pad, hx, hz, R0, C0, zpw, xpw, hs, ts, table floats
+ *   "k_zadj"     w (0: none fits), tz, ntile, vst, bst, nxb, threads, blocks an
+ *                SM, depth step, x tasks a thread, shared memory bytes
+ *   "k_zfwd"     the same; option SPECT_INTERP_*
+ *   "k_zs"       tx, zvst, k_zs_fz threads (0: none fits), blocks an SM, tz,
+ *                xbst, k_zs_fx threads, blocks an SM, shared memory of both
+ *   "k_zrot_adj" tx, ty, slot groups, slots a batch, threads, blocks, shared
+ *                memory (in[4]: slots) */
 int spect_selftest_tiling(const char* what, const int in[8], long long out[12]);
 int spect_plan_profile(spect_plan_t plan, int on);
 int spect_plan_kernel_times(spect_plan_t plan, double ms[8], long long counts[8]);

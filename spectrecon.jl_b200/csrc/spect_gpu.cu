@@ -25,6 +25,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <deque>
+#include <initializer_list>
 #include <thread>
 #include <unordered_map>
 #include <cmath>
@@ -2252,6 +2253,27 @@ int spect_selftest_tiling(const char* what, const int in[8], long long out[12]) 
   if (std::strcmp(what, "group") == 0) {
     out[0] = zgroup_views(nx, nv, (size_t)nx * nx * (option == 2 ? g.nzp : nz), option != 0);
     return SPECT_OK;
+  }
+  const size_t optin = (size_t)std::max(0, in[7]);
+  auto put = [&](std::initializer_list<long long> v) {
+    std::copy(v.begin(), v.end(), out);
+    return SPECT_OK;
+  };
+  auto put_tile = [&](const ZTile& t) {
+    return put({t.w, t.tz, t.ntile, t.vst, t.bst, t.nxb, t.nth, t.occ, t.ystep, t.nxt, (long long)t.smem});
+  };
+  if (std::strcmp(what, "geometry") == 0) return put({g.nzp, g.L, g.pad, g.hx, g.hz, g.R0, g.C0, g.zpw, g.xpw, g.hs, g.ts,
+                                                      ztable_floats(g)});
+  if (std::strcmp(what, "k_zadj") == 0) return put_tile(zadj_tile(g, optin));
+  if (std::strcmp(what, "k_zfwd") == 0) return put_tile(zfwd_tile(g, optin, option == SPECT_INTERP_ONE));
+  if (std::strcmp(what, "k_zs") == 0) {
+    const ZsTiles t = zs_tiles(g, optin);
+    return put({t.tx, t.zvst, t.fz_nth, t.fz_occ, t.tz, t.xbst, t.fx_nth, t.fx_occ, (long long)t.fz_smem,
+                (long long)t.fx_smem});
+  }
+  if (std::strcmp(what, "k_zrot_adj") == 0) {
+    const ZRotTile t = zrot_tile(g, nv, std::max(1, in[6]));
+    return put({t.tx, t.ty, t.S, t.vb, t.nth, t.grid, (long long)t.smem});
   }
   return fail(SPECT_ERR_ARG, std::string("unknown tiling ") + what);
 }
