@@ -272,7 +272,8 @@ int spect_selftest_wait_timeout(void);
  *                the gather rotation, 2 fused and large-plane kernels
  *   "geometry"   nzp, L, pad, hx, hz, R0, C0, zpw, xpw, hs, ts, table floats
  *   "k_zadj"     w (0: none fits), tz, ntile, vst, bst, nxb, threads, blocks an
- *                SM, depth step, x tasks a thread, shared memory bytes
+ *                SM, depth step, x tasks a thread, shared memory bytes; option
+ *                w + 256 * row buffers + 65536 * row tiles, each 0 = free
  *   "k_zfwd"     the same; option SPECT_INTERP_*
  *   "k_zs"       tx, zvst, k_zs_fz threads (0: none fits), blocks an SM, tz,
  *                xbst, k_zs_fx threads, blocks an SM, shared memory of both

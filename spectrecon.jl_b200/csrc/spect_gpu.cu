@@ -1505,7 +1505,13 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
         sep_host && !only_fft && !(zenv && zenv[0] == '0') &&
         zg_full.zpw <= 72 && zg_full.xpw <= 72 &&  // pass rows of at most 9 blocks of 8 taps
         zg.nzp <= 256 && opts.atten_cache != 0) {
-      p->zat = zadj_tile(zg, (size_t)optin);
+      auto number = [](const char* name) {
+        const char* e = std::getenv(name);
+        return e ? std::atoi(e) : 0;
+      };
+      // comparisons and tests: outputs a z task, row tiles and row buffers of k_zadj
+      p->zat = zadj_tile(zg, (size_t)optin,
+                         ZadjForm{number("SPECT_ZW"), number("SPECT_ZADJ_TILES"), number("SPECT_ZADJ_BUFFERS")});
       const bool adj = p->zat.w != 0;
       const bool one = interpmeth == SPECT_INTERP_ONE;
       p->zft = zfwd_tile(zg, (size_t)optin, one);
@@ -2264,7 +2270,8 @@ int spect_selftest_tiling(const char* what, const int in[8], long long out[12]) 
   };
   if (std::strcmp(what, "geometry") == 0) return put({g.nzp, g.L, g.pad, g.hx, g.hz, g.R0, g.C0, g.zpw, g.xpw, g.hs, g.ts,
                                                       ztable_floats(g)});
-  if (std::strcmp(what, "k_zadj") == 0) return put_tile(zadj_tile(g, optin));
+  if (std::strcmp(what, "k_zadj") == 0) 
+    return put_tile(zadj_tile(g, optin, ZadjForm{option & 255, option >> 16, option >> 8 & 255}));
   if (std::strcmp(what, "k_zfwd") == 0) return put_tile(zfwd_tile(g, optin, option == SPECT_INTERP_ONE));
   if (std::strcmp(what, "k_zs") == 0) {
     const ZsTiles t = zs_tiles(g, optin);

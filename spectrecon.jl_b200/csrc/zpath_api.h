@@ -136,11 +136,17 @@ inline int zdepth_step(int ny) {
 // bytes per FMA, row tiles cut the shared memory of a block so that several
 // blocks (or a second row buffer) hide each other's barriers, and fewer than
 // 16 warps per SM no longer hide the latencies.
-inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
+// `want` fixes a field that is not 0, for comparisons; where nothing of that
+// form fits it is left out of account.
+struct ZadjForm {
+  int w, ntile, nxb;
+};
+inline ZTile zadj_tile(const ZGeom& g, size_t optin, const ZadjForm& want = {}) {
   ZTile best{};
   double bc = 0;
   for (int w : {16, 8})
     for (int nt = 1; nt <= (g.nz + 1) / 2; ++nt) {
+      if ((want.w && w != want.w) || (want.ntile && nt != want.ntile)) continue;
       ZTile t{};
       t.w = w;
       t.tz = zround((g.nz + nt - 1) / nt, nt > 1 ? 8 : 2);  // tiles of whole tasks
@@ -152,13 +158,14 @@ inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
       const int most = w == 16 || zt > xt ? zt : xt, rounds = (most + kZThreads - 1) / kZThreads;
       t.nth = zround((most + rounds - 1) / rounds, 32);
       for (int nxb : {1, 2}) {
+        if (want.nxb && nxb != want.nxb) continue;
         t.nxb = nxb;
         t.smem = zadj_smem(g, t);
         if (t.smem > optin) continue;
         const int so = (int)((optin + 1024) / (t.smem + 1024)), ro = kZThreads / t.nth;
         t.occ = so < ro ? so : ro;
         if (t.occ > 16) t.occ = 16;
-        if (nxb > 1 && t.occ > 1) continue;  // several blocks overlap already
+        if (nxb > 1 && t.occ > 1 && !want.nxb) continue;  // several blocks overlap already
         const double warps = t.occ * t.nth / 32.0;
         const double rz = (double)((zt + t.nth - 1) / t.nth), rx = (double)((xt + t.nth - 1) / t.nth);
         double c = t.ntile * t.nth * (rz * w * (w == 8 ? 1.15 : 1.0) + rx * kZadjX * 1.15);  // thread slots x outputs
@@ -170,6 +177,7 @@ inline ZTile zadj_tile(const ZGeom& g, size_t optin) {
         }
       }
     }
+  if (!best.w && (want.w || want.ntile || want.nxb)) return zadj_tile(g, optin);
   best.ystep = zdepth_step(g.ny);
   return best;
 }

@@ -43,7 +43,7 @@ SIZES = [(128, 80, 37, 37), (64, 64, 11, 11), (64, 40, 19, 19), (96, 48, 21, 21)
          (64, 1, 11, 1), (128, 1, 11, 1), (256, 200, 65, 65), (64, 90, 21, 21), (40, 37, 9, 9), (8, 5, 5, 5),
          (512, 96, 21, 21), (256, 17, 63, 3), (24, 230, 7, 65), (90, 53, 21, 17), (46, 80, 7, 7), (82, 73, 17, 17),
          (34, 9, 5, 3), (2, 1, 1, 1), (6, 3, 3, 3), (170, 1, 7, 1), (122, 100, 25, 25), (222, 150, 41, 41),
-         (512, 230, 65, 65), (32, 160, 5, 5), (512, 250, 5, 5), (4, 256, 1, 65)]
+         (512, 230, 65, 65), (32, 160, 5, 5), (512, 250, 5, 5), (4, 256, 1, 65), (46, 37, 9, 33)]
 X, NTH = 8, 640  # outputs of an x task; threads an SM's registers allow the pair-pass kernels
 GEO = ("nzp", "L", "pad", "hx", "hz", "R0", "C0", "zpw", "xpw", "hs", "ts", "trow")
 TILE = ("w", "tz", "ntile", "vst", "bst", "nxb", "nth", "occ", "ystep", "nxt", "smem")
@@ -106,6 +106,28 @@ def test_adjoint_tile(named, nx, nz, px, pz):
     g, t = named("geometry", nx, nz, px, pz), named("k_zadj", nx, nz, px, pz)
     assert g["trow"] % 4 == 0 and g["hs"] % 8 == 0 and g["nzp"] % 16 == 0
     check_adjoint_tile(nx, nz, g, t)
+
+
+@pytest.mark.parametrize("nx,nz,px,pz", SIZES)
+def test_adjoint_tile_forms(named, nx, nz, px, pz):
+    """Every form that the switches can ask for stays inside its buffers, and
+    one that fits nowhere falls back on the rule's own."""
+    g, own = named("geometry", nx, nz, px, pz), named("k_zadj", nx, nz, px, pz)
+    met = set()
+    for w in (0, 8, 16):
+        for nxb in (0, 1, 2):
+            for ntile in range(0, (nz + 1) // 2 + 1):
+                t = named("k_zadj", nx, nz, px, pz, option=w + 256 * nxb + 65536 * ntile)
+                check_adjoint_tile(nx, nz, g, t)
+                if (w or t["w"], nxb or t["nxb"], ntile or t["ntile"]) == (t["w"], t["nxb"], t["ntile"]):
+                    met.add((t["w"], t["nxb"], t["ntile"]))
+                else:
+                    assert t == own
+    assert (own["w"], own["nxb"], own["ntile"]) in met
+    if nx * nz <= 64 * 64:
+        ceil = lambda a, b: -(-a // b)  # noqa: E731
+        tiles = {nt for nt in range(1, (nz + 1) // 2 + 1) if nt == 1 or ceil(nz, 8 * ceil(ceil(nz, nt), 8)) == nt}
+        assert met == {(w, nxb, nt) for w in (8, 16) for nxb in (1, 2) for nt in tiles}
 
 
 @pytest.mark.parametrize("nx,nz,px,pz", SIZES)
