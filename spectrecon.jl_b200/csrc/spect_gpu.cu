@@ -995,12 +995,18 @@ struct TuneResult {
 std::mutex g_tune_mu;
 std::vector<std::pair<std::string, TuneResult>> g_tune_cache;
 
+// what decides the kernels of a call and their work: sizes, paths, and on the
+// fused paths the kept PSF support and the adjoint kernel's form
 std::string tune_key(const spect_plan_s* p, int nv) {
+  const std::string fused = !p->zpath ? std::string()
+                                      : "/t" + std::to_string(p->zg.hx) + "," + std::to_string(p->zg.hz) + "/f" +
+                                            std::to_string(p->zat.w) + "," + std::to_string(p->zat.nxb) + "," +
+                                            std::to_string(p->zat.ntile);
   return std::to_string(p->nx) + "x" + std::to_string(p->nz) + "/" + std::to_string(p->px) + "x" +
          std::to_string(p->pz) + "/v" + std::to_string(p->nview) + "/n" + std::to_string(nv) + "/i" +
          std::to_string(p->interp) + "/a" + std::to_string(p->d_att ? 1 : 0) + "/d" + std::to_string(p->device) +
          "/s" + std::to_string(p->sep_fwd_ok) + std::to_string(p->sep_adj_ok) + std::to_string(p->sep_forced) +
-         "/z" + std::to_string(p->zpath) + "/y" + std::to_string(p->ny);
+         "/z" + std::to_string(p->zpath) + "/y" + std::to_string(p->ny) + "/g" + std::to_string(p->gadj) + fused;
 }
 
 int time_pass(spect_plan_s* p, bool adj, int nv, int reps, double* ms) {
@@ -1081,9 +1087,11 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
     if (p->sep_adj_ok) aconv = {1, 0};
   }
   // forward: convolution kernel x depth tile x rotation split
-  std::vector<int> rsplits = {0};
+  // (the gather kernels have no split)
+  std::vector<int> rsplits = {0}, nsplits = {1, 2, 4, 8, 16};
   for (int f : {1, 2, 4, 8})
-    if (f * p->g.nz <= 8 * p->sm_count) rsplits.push_back(f);
+    if (!p->gadj && f * p->g.nz <= 8 * p->sm_count) rsplits.push_back(f);
+  if (p->gadj) nsplits = {p->nsplit_adj};
   double bf = 1e300;
   int bcy = cys[0], brs = 0, bsep = p->sep, rc = SPECT_OK;
   for (int sp : fconv)
@@ -1110,7 +1118,7 @@ int autotune(spect_plan_s* p, int nv, double* fwd_ms, double* adj_ms) {
   int bacy = cys[0], bns = p->nsplit_adj, basep = p->sep_adj;
   for (int sp : aconv)
     for (int cy : cys)
-      for (int ns : {1, 2, 4, 8, 16}) {
+      for (int ns : nsplits) {
         if (rc != SPECT_OK || ns > p->nsplit_adj_max) break;
         p->sep_adj = sp;
         p->tune_adj_cy = cy;
