@@ -213,12 +213,12 @@ def launch_work(plan, kind, nv):
         conv = plan.conv_kernels()
         ex = {"direct": direct_flops(nv, ny, nx, nz, px, pz), "fft": None}
         table = {
-            "k_rot_fwd": ("k_rot_fwd", "hbm", 8.0 * nv * N, 4.0 * (N + nv * N), None),
+            "k_rot_fwd": ("k_zrot_fwd|k_rot_fwd", "hbm", 8.0 * nv * N, 4.0 * (N + nv * N), None),
             "k_conv_fwd": ("k_sconv_fwd" if conv["forward"] == "direct" else "k_conv_fwd2", "fp32",
                            F, 4.0 * (2 * nv * N), ex[conv["forward"]]),
             "k_conv_adj": ("k_sconv_adj" if conv["adjoint"] == "direct" else "k_conv_adj2", "fp32",
                            F, 4.0 * (2 * nv * N), ex[conv["adjoint"]]),
-            "k_rot_adj": ("k_rot_adj", "hbm", 8.0 * nv * N, 4.0 * (nv * N + N), None),
+            "k_rot_adj": ("k_zrot_adj|k_rot_adj", "hbm", 8.0 * nv * N, 4.0 * (nv * N + N), None),
             "k_reduce_views": ("k_reduce_views", "hbm", 2.0 * nv * nxz, 4.0 * 4 * nv * nxz, None),
             "k_reduce_image": ("k_reduce_image", "hbm", 0.0, 4.0 * 3 * N, None),
         }

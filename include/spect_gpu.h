@@ -181,9 +181,11 @@ int spect_subset_sensitivity(spect_plan_t plan, float* asum, const int32_t* inde
 
 /* Autotuner (no counterpart in the reference).  Times candidate launch
  * shapes of the plan's forward and adjoint projector for nindex views on the
- * device (the depth-chunk tile of the FFT-convolution kernels, the view split
- * of the rotation kernels) and keeps the fastest for calls with nindex views;
- * results are cached per plan shape in the process.  ms[0], ms[1]: best
+ * device (the depth-chunk tile of the split convolution kernels, direct against
+ * FFT convolution, the view split of the slice and scatter rotations) and keeps
+ * the fastest for calls with nindex views; the launch shapes of the fused and
+ * large-plane kernels are fixed, so there it only measures.  Results are cached
+ * in the process for plans that run the same kernels.  ms[0], ms[1]: best
  * forward and adjoint times.  Synchronous; spect_batch_create runs it for
  * every job's subset size. */
 int spect_plan_autotune(spect_plan_t plan, int nindex, double ms[2]);

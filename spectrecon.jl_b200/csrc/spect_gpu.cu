@@ -228,8 +228,8 @@ struct spect_plan_s {
   // tuned launch shapes (0 = analytic default); tuned_nv = the view count they were tuned for
   int tune_fwd_cy = 0, tune_adj_cy = 0, tune_rotf_nsplit = 0, tuned_nv = 0;
   size_t rota_smem = 0;
-  // fused projector pair on z-fastest layouts (zpath.cuh): :two, attenuation
-  // cache, separable PSF planes, planes that fit in shared memory
+  // fused projector pair on z-fastest layouts (zpath.cuh):
+  // attenuation cache, separable PSF planes, planes that fit in shared memory
   int zpath = 0;
   ZGeom zg{};
   size_t izN = 0;              // floats of one IZ volume (L * L * nzp)
@@ -1478,7 +1478,7 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     return st;
   };
   // separable PSF planes (host factorisation) and the fused-path decision:
-  // :two, separable planes, attenuation cache, planes that fit in shared memory
+  // separable planes, attenuation cache, planes that fit in shared memory
   std::vector<double> fa, fb;
   const bool sep_host = factor_planes(psfs, uniq, ny, px, pz, opts, fa, fb);
   const char* conv_env = std::getenv("SPECT_CONV");

@@ -45,7 +45,7 @@
 // line b), and a task of W = 8 or 16 consecutive outputs of both runs packed
 // FMAs (fma.rn.f32x2): half the issue slots of a line at a time, which is what
 // bounds these loops next to their index and shared-memory work (63.4 against
-// 48.8 TFLOP/s beside one integer operation an FMA).  Data start at an offset
+// 48.9 TFLOP/s beside one integer operation per two FMAs).  Data start at an offset
 // D0 = h rounded up to 4 and the weights are shifted right by D0 - h, so the
 // window is read in 16-byte-aligned pieces; the clamped
 // boundary is added as tail terms: the edge value times EL[i] =
@@ -616,10 +616,9 @@ __global__ void __launch_bounds__(256) k_reduce_parts(const float* part, int nv,
 // thread at 96 registers, x outputs included (16 spilled them).
 // Bound: the shared-memory/L1 pipe (63 % busy at 128x128x80, 37 taps) and the
 // gather's L2 latency between the barriers; FFMA2 is 37 % of the
-// instructions.  Measured there: 15 views 107.7 -> 78.3 us, 120 views 695 ->
-// 573 us; 64x64x40, 19 taps, 60 views 107 -> 38 us; 128x128x1, 80 views 229 ->
-// 50 us (the former kernel staged the attenuation plane in shared memory, ran
-// one line a lane and one block per SM, and dealt chunks of 15 planes).
+// instructions.  Measured there: 15 views 78.3 us, 120 views 573 us; 64x64x40,
+// 19 taps, 60 views 38 us; 128x128x1, 80 views 45 us (one line a lane, chunks
+// of 15 planes on one block an SM: 107.7, 695, 107, 229 us).
 // ONE: the :one rotation (eight taps a column, one_geo).
 // Shared memory: [2 tables][geoW nx x (w00 w00 w10 w10 | w01 w01 w11 w11)]
 // [geoO nx int][ZB nxp * vst][XB (nz + 1) / 2 * bst] (lines: float2).
@@ -835,19 +834,18 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zfwd(const __grid_constant__ Z
 // Each pass is the zero-padded correlation with the factor plus the folded
 // padding at the two ends (z folds where the tile holds the image's first or
 // last row).  Lanes of the x pass are consecutive row pairs, so the
-// attenuation reads and the T stores are 256 contiguous bytes a warp (the
-// former x-then-z order read and wrote 16 bytes at a column stride, one line
-// a lane: the shared-memory/L1 pipe was its bound).  The plane's table
+// attenuation reads and the T stores are 256 contiguous bytes a warp (x then z
+// would read and write 16 bytes at a column stride).  The plane's table
 // (weights, folds, tap ranges) is copied one plane ahead and its attenuation
 // prefetched into L2; an x task loads its attenuation before its FMAs, which
 // hides the rest of that latency (8 outputs a task: 16 would need 32 more
 // registers).  Two barriers a plane with one XB (the host then runs several
 // blocks per SM, which fill each other's waits), one with two.
-// Bound: FFMA2 (13.1 M of 34.7 M warp instructions at 128x128x80, 37 taps, 15
-// views; the pipe is 44 % busy) and what the blocks wait for at their
-// barriers.  Measured there: 105 -> 66 us (51.9 M instructions before);
-// 64x64x64, 11 taps, 64 views 92 -> 38 us; 256x256x200, 65 taps, 8 views
-// (five row tiles, two XB) 735 -> 483 us.
+// Bound: FFMA2 (33.4 M warp instructions at 128x128x80, 37 taps, 15 views; the
+// pipe is 43 % busy) and what the blocks wait for at their barriers.  Measured
+// there: 66 us; 64x64x64, 11 taps, 64 views 38 us; 256x256x200, 65 taps, 8
+// views (five row tiles, two XB) 483 us (x then z, one line a lane: 105, 92,
+// 735 us).
 // Shared memory (float2): [VB nxp * vst][XB nxb * (tz / 2) * bst][3 tables].
 template <int W>
 __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ ZArgs a) {
@@ -1039,10 +1037,10 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zadj(const __grid_constant__ Z
 // zcol, so that a unit runs four unconditional loads a slot, the others under
 // a branch.  A group's sum runs over its slots and hits in order.
 // Bound: L1 (its tag stage is 55 % busy where an SM works: a column's 320
-// bytes straddle lines) and the latency of the misses.  Measured (the former
-// kernel tested the candidates in every 8-lane group): 128x128x80, 15 views 49
-// -> 42 us; 64x64x64, 64 views 57 -> 31 us; 64x64x40, 60 views 45 -> 24 us;
-// 256x256x200, 8 views 252 -> 216 us.
+// bytes straddle lines) and the latency of the misses.  Measured: 128x128x80,
+// 15 views 42 us; 64x64x64, 64 views 31 us; 64x64x40, 60 views 24 us;
+// 256x256x200, 8 views 216 us (candidates tested in every 8-lane group: 49, 57,
+// 45, 252 us).
 // Epilogue (IZ layout): v = acc (+ prev); mode 1: zeros -> +Inf; mode 2:
 // v = x * (v / asum); out = v (z < nz only; out may be prev or x).
 template <bool ONE>

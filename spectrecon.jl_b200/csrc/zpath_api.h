@@ -259,7 +259,7 @@ inline ZsTiles zs_tiles(const ZGeom& g, size_t optin) {
 // us).
 constexpr int kZrotU = 2;          // units (column, four z) a thread
 constexpr int kZrotList = 9;       // list entries of a pair: its candidates at most
-constexpr int kZrotThreads = 512;  // nzp <= 256: 8 columns x 64 units / 2 = 256 a group at most
+constexpr int kZrotThreads = 512;  // nzp <= 256: 16 columns x 40 z groups / 2 = 320 threads a group at most
 struct ZRotTile {
   int tx, ty, S, vb, nth, grid;
   size_t smem;
@@ -307,7 +307,13 @@ inline int zgroup_views(int nx, int nview, size_t slot, bool gather) {
   return n < 1 ? 1 : (int)n;
 }
 
-// short work (about 100 us a kernel at most): nv planes stacks of nx x nx x nz
+// short work: nv stacks of planes of nx x nz, below about 100 us a kernel.  The
+// kernels whose gathers live on L1 start early there.  Measured, two OS-EM
+// iterations, none of them early and all: 8 views of 64x64x64 (2.1 M samples)
+// 0.81 -> 0.69 ms; 15 and 25 views of 128x128x80 (20 M, 33 M) 2.09 -> 2.12 and
+// 3.23 -> 3.32 ms; 12 views of 192x192x120 (53 M) 6.57 -> 6.88; 8 views of
+// 256x256x128 (67 M) 8.13 -> 9.04; of 256x256x200 (105 M) 13.6 -> 14.4.  The line
+// keeps the large losses out; the crossing itself lies below 20 M.
 inline bool zearly(const ZGeom& g, int nv) { return (long long)nv * g.nx * g.ny * g.nz <= (1LL << 25); }
 
 // launchers (zpath_inst.cu)

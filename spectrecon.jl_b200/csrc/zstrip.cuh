@@ -30,8 +30,7 @@ namespace spect {
 // and image read, Q written: 1.1 GB for 8 views of 256x256x200, 65 taps) and
 // the latency of the gather's loads, not the FMAs.  Measured there: 392 us
 // (16-output tasks on two blocks 411 us, one plane an item 425 us, double ZB
-// with one barrier 511 us -- it takes the L1; the former single-line kernel,
-// which needed nx % 8 == 0, 394 us).
+// with one barrier 511 us -- it takes the L1; one line a lane 394 us).
 // Shared memory: [2 x 2 x (table | geoW tx x 2 float4 | geoO tx int)]
 // [ZB 2 x tx / 2 * vst f2].
 __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__ ZArgs a) {
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(kZsThreads, 3) k_zs_fz(const __grid_constant__
                            cols * nzp * (unsigned)sizeof(float));
       }
     }
-    // z pass: task (column pair, 16 rows) of plane y + pz -> Q
+    // z pass: task (column pair, W rows) of plane y + pz -> Q
     const float* const Wt = buf + pz * bufsz;
     const f2* const Wd = reinterpret_cast<const f2*>(Wt);
     const int2 rg = *reinterpret_cast<const int2*>(Wt + 2 * hs + ts);
