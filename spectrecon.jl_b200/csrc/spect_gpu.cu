@@ -2464,8 +2464,11 @@ size_t est_job_bytes(const ServerJob& j, bool att) {
              + nsub * N + nsub * 16 * nxz + 2 * nsub * Q * Npx  // P, part, Vs
              + 8 * N + 2 * (size_t)j.nview * nxz + (size_t)j.nblocks * N  // imgpart, EM buffers
              + 2 * N + 2 * (size_t)j.nview * nxz;     // job buffers
-  if (j.interp == SPECT_INTERP_ONE) f += nsub * N;
-  f += 2 * nsub * (size_t)j.nx * j.nx * ((j.nz + 15) / 16 * 16) + 2 * N;  // z-fastest planes and tiles, IZ volumes
+  // planes beside P, and the IZ volumes.  :one: the rotated slices of the split
+  // kernels, or the z padding of the fused pair's planes; :two: z-fastest
+  // planes and tiles
+  const size_t zcols = nsub * (size_t)j.nx * j.nx * ((j.nz + 15) / 16 * 16);
+  f += (j.interp == SPECT_INTERP_ONE ? std::max(nsub * N, zcols - nsub * N) : 2 * zcols) + 2 * N;
   size_t b = 4 * f + (size_t)j.nview * 32;
   // per-CTA global slabs of large planes (B, spectra accumulators)
   if ((size_t)j.nx * (Q + 1) * 8 + 8192 > 227 * 1024) b += (size_t)148 * j.nx * (Q + 1) * 8;
