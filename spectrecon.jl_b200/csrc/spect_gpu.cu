@@ -1533,26 +1533,28 @@ int plan_create_impl(spect_plan_t* out, int nx, int ny, int nz, int px, int pz, 
     }
     cudaGetLastError();
   }
-  const bool zcand = zkind != 0;
   // attenuation cache: on when it fits a quarter of the free device memory
   // (and 32 GiB); SPECT_ATTEN_CACHE=0 turns it off (and with it the fused
   // path).  The fused path keeps it z-fastest ([view][y][x][nzp]), the
-  // other kernels as [view][y][z][x].
+  // other kernels as [view][y][z][x]: where only the latter fits (single
+  // slices: a sixteenth), the split kernels take the plan.
   {
     const char* env = std::getenv("SPECT_ATTEN_CACHE");
-    const size_t cnt = zcand ? (size_t)nview * ny * nx * zg.nzp : p->N * (size_t)nview;
-    size_t need = sizeof(float) * cnt, fr = 0, tot = 0;
+    size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
       cudaGetLastError();
       fr = 0;
     }
-    bool want = !(env && env[0] == '0') && need <= std::min(fr / 4, (size_t)32 << 30);
-    if (opts.atten_cache >= 0) want = opts.atten_cache == 1;
-    if ((interpmeth == SPECT_INTERP_TWO || zcand) && want && dalloc(p, &p->d_att, cnt) != SPECT_OK) {
+    auto cache = [&](size_t cnt) {
+      bool want = !(env && env[0] == '0') && sizeof(float) * cnt <= std::min(fr / 4, (size_t)32 << 30);
+      if (opts.atten_cache >= 0) want = opts.atten_cache == 1;
+      if (!want || dalloc(p, &p->d_att, cnt) == SPECT_OK) return want;
       p->d_att = nullptr;
       g_err.clear();
-    }
-    p->zpath = (zcand && p->d_att) ? zkind : 0;
+      return false;
+    };
+    if (zkind != 0 && cache((size_t)nview * ny * nx * zg.nzp)) p->zpath = zkind;
+    else if (interpmeth == SPECT_INTERP_TWO) cache(p->N * (size_t)nview);
     if (interpmeth == SPECT_INTERP_ONE && !p->d_att) {
       // the split :one path reads its attenuation from the cache
       int st1 = dalloc(p, &p->d_att, p->N * (size_t)nview);

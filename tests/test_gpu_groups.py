@@ -70,3 +70,21 @@ def test_more_views_than_a_grid_holds(S, O, interp):
     plan.close()
     G = O.Geometry(mumap, psfs, 4.8, interp=interp)
     assert relerr(out, G.project(x, index=idx)) <= TOL
+
+
+def test_padded_cache_too_large_for_the_fused_pair(S, O):
+    """2200 views of 500x500x1: the fused pair's z-fastest attenuation (16 values
+    a column) would take 35 GB, above the cache's bound; the 2.2 GB of the split
+    kernels' cache still fit, and the plan keeps them."""
+    nx, nview = 500, 2200
+    mumap, _, _ = _study(S, nx, 1, 5)
+    psf = S.psf_gauss(ny=nx, px=3, pz=1, fwhm_start=1, fwhm_end=1.5)
+    psfs = np.asfortranarray(np.repeat(psf[:, :, :, None], nview, axis=3), np.float32)
+    plan = S.SPECTplan(mumap, psfs, 4.8)
+    assert plan.path == "split"
+    assert plan.info()["device_bytes"] > 4 * nx * nx * nview
+    idx = np.array([2199, 3, 1100], np.int32)
+    x = np.asfortranarray(np.random.default_rng(6).random((nx, nx, 1)), np.float32)
+    out = S.project(x, plan, index=idx)
+    plan.close()
+    assert relerr(out, O.Geometry(mumap, psfs, 4.8).project(x, index=idx)) <= TOL
